@@ -193,7 +193,6 @@ int launch_form_ab(const double *FI, const double *G, const double *RT, int K, i
 // ---------------------------------------------------------------------------
 // solvers
 // ---------------------------------------------------------------------------
-constexpr int SOLVE_THREADS = 512;
 constexpr int SMEM_SOLVE_MAX = 110;  // M1 up to which L lives in shared memory
 constexpr int TRI_MAXR = 32;  // registers per lane in the substitution: M1 <= 1024
 
@@ -534,31 +533,48 @@ TriKernel tri_solve_for(int nr)
     }
 }
 
-// Parallel cyclic Jacobi (round-robin pairing) on the symmetric A, then
-// W = V diag(1/lambda, 0 where lambda == 0) V^T B.
-__global__ void __launch_bounds__(SOLVE_THREADS) jacobi_solve_kernel(const double *__restrict__ A,
-                                                                    const double *__restrict__ B,
-                                                                    int M1, int D,
-                                                                    double *__restrict__ W,
-                                                                    double *__restrict__ work,
-                                                                    int *flag)
+// Parallel cyclic Jacobi (round-robin pairing) on the symmetric A; the
+// eigenvectors go to work[M1 M1 ..) and the inverted eigenvalues (0 where an
+// eigenvalue is exactly 0) to work[2 M1 M1 ..); then W = V diag(inv) V^T B.
+//
+// One CTA, because the M1 - 1 rounds of a sweep depend on each other; what
+// bounds it is the FP64 pipe (2 operations a clock) and, for small M1, the
+// chain of a round: angles, barrier, updates, barrier.  So S and V stay in
+// shared memory (in global memory beyond the 227 KB a block can hold:
+// M1 > SVD_SMEM_MAX); a round's rotations act on S as independent 2 x 2 blocks,
+// one per pair of pivot pairs (t <= u, mirrored), J_t^T S_tu J_u in one step
+// instead of a row pass, a barrier and a column pass; and the angle is taken
+// in FP32, with c = 1 / sqrt(1 + t^2) from it in FP64: c^2 + s^2 = 1 holds to
+// FP64, a pivot element is left at ~1e-7 of itself instead of at rounding, and
+// the next sweep removes it.  M1 = 26: 0.69 ms a solve, 5.73 ms with S and V in
+// global memory, FP64 angles and separate row and column passes.
+constexpr int SVD_THREADS = 512;
+constexpr int SVD_SMEM_MAX = 112;  // 2 M1^2 doubles within 200 KB
+
+__device__ __forceinline__ int jacobi_slot(int x, int n) { return x >= n - 1 ? x - (n - 1) : x; }
+
+template <bool SM>
+__global__ void __launch_bounds__(SVD_THREADS) jacobi_kernel(const double *__restrict__ A, int M1,
+                                                            double *__restrict__ work, int *flag)
 {
-    double *S = work;                        // M1 x M1 (becomes diagonal)
-    double *V = work + (size_t) M1 * M1;     // M1 x M1 eigenvectors (columns)
-    double *tmp = V + (size_t) M1 * M1;      // M1 x D
-    __shared__ double cs[SOLVE_THREADS], sn[SOLVE_THREADS];
-    __shared__ int pp[SOLVE_THREADS], qq[SOLVE_THREADS];
+    extern __shared__ double sh[];
+    double *S = SM ? sh : work;                       // M1 x M1 (becomes diagonal)
+    double *V = SM ? sh + (size_t) M1 * M1            // M1 x M1 eigenvectors (columns)
+                   : work + (size_t) M1 * M1;
+    __shared__ double cs[SVD_THREADS], sn[SVD_THREADS];
+    __shared__ short2 pq[SVD_THREADS];
     __shared__ double red[32];
-    __shared__ int done;
+    const int tid = threadIdx.x;
     const int n = M1 + (M1 & 1);  // even number of slots; slot M1 (if any) is a dummy
-    for (int i = threadIdx.x; i < M1 * M1; i += blockDim.x) {
+    const int h = n / 2;
+    for (int i = tid; i < M1 * M1; i += SVD_THREADS) {
         S[i] = A[i];
         V[i] = ((i / M1) == (i % M1)) ? 1.0 : 0.0;
     }
     __syncthreads();
     for (int sweep = 0; sweep < 60; sweep++) {
         double off = 0.0, tot = 0.0;
-        for (int i = threadIdx.x; i < M1 * M1; i += blockDim.x) {
+        for (int i = tid; i < M1 * M1; i += SVD_THREADS) {
             const double v = S[i] * S[i];
             tot += v;
             if ((i / M1) != (i % M1))
@@ -566,90 +582,141 @@ __global__ void __launch_bounds__(SOLVE_THREADS) jacobi_solve_kernel(const doubl
         }
         off = block_sum_fixed(off, red);
         tot = block_sum_fixed(tot, red);
-        if (threadIdx.x == 0)
-            done = (off <= 1e-32 * tot);
-        __syncthreads();
-        if (done)
+        if (off <= 1e-32 * tot)  // the same value in every thread
             break;
         for (int r = 0; r < n - 1; r++) {
             // round-robin: slot 0 fixed, the others rotate
-            for (int t = threadIdx.x; t < n / 2; t += blockDim.x) {
-                int a = (t == 0) ? 0 : 1 + ((t - 1 + r) % (n - 1));
-                int b = 1 + ((n - 2 - t + r) % (n - 1));
-                int p = min(a, b), q = max(a, b);
+            if (tid < h) {
+                const int a = (tid == 0) ? 0 : 1 + jacobi_slot(tid - 1 + r, n);
+                const int b = 1 + jacobi_slot(n - 2 - tid + r, n);
+                const int p = min(a, b), q = max(a, b);
                 double c = 1.0, s = 0.0;
                 if (q < M1) {
-                    const double apq = S[(size_t) p * M1 + q];
+                    const double apq = S[p * M1 + q];
                     if (apq != 0.0) {
-                        const double app = S[(size_t) p * M1 + p], aqq = S[(size_t) q * M1 + q];
-                        const double th = (aqq - app) / (2.0 * apq);
-                        const double tt = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-                        c = 1.0 / sqrt(tt * tt + 1.0);
-                        s = tt * c;
+                        const float th = (float) ((S[q * M1 + q] - S[p * M1 + p]) / (2.0 * apq));
+                        const float t = copysignf(1.0f / (fabsf(th) + sqrtf(fmaf(th, th, 1.0f))), th);
+                        const double d = fma((double) t, (double) t, 1.0);
+                        c = rsqrt_nr(d);
+                        c = fma(0.5 * c, fma(-d * c, c, 1.0), c);  // to half an ulp
+                        s = (double) t * c;
                     }
                 }
-                pp[t] = p;
-                qq[t] = q;
-                cs[t] = c;
-                sn[t] = s;
+                pq[tid] = make_short2((short) p, (short) q);
+                cs[tid] = c;
+                sn[tid] = s;
             }
             __syncthreads();
-            // rows: S <- J^T S
-            for (int idx = threadIdx.x; idx < (n / 2) * M1; idx += blockDim.x) {
-                const int t = idx / M1, k = idx % M1;
-                const int p = pp[t], q = qq[t];
-                if (q >= M1 || sn[t] == 0.0)
+            // S <- J^T S J: block (t, u) of the pairs t <= u; then V <- V J
+            const int nb = h * h;
+            for (int idx = tid; idx < nb; idx += SVD_THREADS) {
+                const int t = idx / h, u = idx - t * h;
+                if (t > u)
                     continue;
-                const double c = cs[t], s = sn[t];
-                const double sp = S[(size_t) p * M1 + k], sq = S[(size_t) q * M1 + k];
-                S[(size_t) p * M1 + k] = c * sp - s * sq;
-                S[(size_t) q * M1 + k] = s * sp + c * sq;
+                const int p = pq[t].x, q = pq[t].y;
+                const double c1 = cs[t], s1 = sn[t];
+                if (t == u) {
+                    if (q >= M1 || s1 == 0.0)
+                        continue;
+                    const double pp = S[p * M1 + p], qq = S[q * M1 + q], x = S[p * M1 + q];
+                    const double cx = c1 * pp - s1 * x, sx = s1 * pp + c1 * x;  // (J^T S) column p
+                    const double cy = c1 * x - s1 * qq, sy = s1 * x + c1 * qq;  // column q
+                    S[p * M1 + p] = c1 * cx - s1 * cy;
+                    S[q * M1 + q] = s1 * sx + c1 * sy;
+                    S[p * M1 + q] = S[q * M1 + p] = s1 * cx + c1 * cy;
+                    continue;
+                }
+                const int v = pq[u].x, w = pq[u].y;
+                const double c2 = cs[u], s2 = sn[u];
+                if (s1 == 0.0 && s2 == 0.0)
+                    continue;
+                const bool hq = q < M1, hw = w < M1;  // p and v are real slots
+                const double pv = S[p * M1 + v], pw = hw ? S[p * M1 + w] : 0.0;
+                const double qv = hq ? S[q * M1 + v] : 0.0, qw = hq && hw ? S[q * M1 + w] : 0.0;
+                const double rpv = c1 * pv - s1 * qv, rpw = c1 * pw - s1 * qw;
+                const double rqv = s1 * pv + c1 * qv, rqw = s1 * pw + c1 * qw;
+                S[p * M1 + v] = S[v * M1 + p] = c2 * rpv - s2 * rpw;
+                if (hw)
+                    S[p * M1 + w] = S[w * M1 + p] = s2 * rpv + c2 * rpw;
+                if (hq)
+                    S[q * M1 + v] = S[v * M1 + q] = c2 * rqv - s2 * rqw;
+                if (hq && hw)
+                    S[q * M1 + w] = S[w * M1 + q] = s2 * rqv + c2 * rqw;
             }
-            __syncthreads();
-            // columns: S <- S J, V <- V J
-            for (int idx = threadIdx.x; idx < (n / 2) * M1; idx += blockDim.x) {
-                const int t = idx / M1, k = idx % M1;
-                const int p = pp[t], q = qq[t];
-                if (q >= M1 || sn[t] == 0.0)
-                    continue;
+            for (int idx = tid; idx < h * M1; idx += SVD_THREADS) {
+                const int k = idx / h, t = idx - k * h;
+                const int p = pq[t].x, q = pq[t].y;
                 const double c = cs[t], s = sn[t];
-                const double sp = S[(size_t) k * M1 + p], sq = S[(size_t) k * M1 + q];
-                S[(size_t) k * M1 + p] = c * sp - s * sq;
-                S[(size_t) k * M1 + q] = s * sp + c * sq;
-                const double vp = V[(size_t) k * M1 + p], vq = V[(size_t) k * M1 + q];
-                V[(size_t) k * M1 + p] = c * vp - s * vq;
-                V[(size_t) k * M1 + q] = s * vp + c * vq;
+                if (s == 0.0)
+                    continue;
+                const double vp = V[k * M1 + p], vq = V[k * M1 + q];
+                V[k * M1 + p] = c * vp - s * vq;
+                V[k * M1 + q] = s * vp + c * vq;
             }
             __syncthreads();
         }
     }
-    // tmp = diag(1/lambda) V^T B
-    for (int idx = threadIdx.x; idx < M1 * D; idx += blockDim.x) {
-        const int i = idx / D, c = idx % D;
-        double acc = 0.0;
-        for (int r = 0; r < M1; r++)
-            acc += V[(size_t) r * M1 + i] * B[(size_t) r * D + c];
-        double lam = S[(size_t) i * M1 + i];
-        if (lam != 0.0)
-            lam = 1.0 / lam;
-        tmp[idx] = lam * acc;
+    // the inverted eigenvalues after V, which the global variant has in place
+    for (int i = tid; i < M1; i += SVD_THREADS) {
+        const double lam = S[i * M1 + i];
+        work[2 * M1 * M1 + i] = lam != 0.0 ? 1.0 / lam : 0.0;
+    }
+    if (SM)
+        for (int i = tid; i < M1 * M1; i += SVD_THREADS)
+            work[M1 * M1 + i] = V[i];
+    if (tid == 0)
+        flag[0] = 0;
+}
+
+// W = V diag(inv) V^T B, SVD_COLS columns of B per CTA (the columns are
+// independent, so they spread over the SMs)
+constexpr int SVD_COLS = 4;
+
+__global__ void __launch_bounds__(128) svd_apply_kernel(const double *__restrict__ V,
+                                                        const double *__restrict__ inv,
+                                                        const double *__restrict__ B, int M1, int D,
+                                                        double *__restrict__ W)
+{
+    extern __shared__ double sh[];
+    double *b = sh, *y = sh + SVD_COLS * M1;  // [M1][SVD_COLS] each
+    const int c0 = blockIdx.x * SVD_COLS;
+    for (int e = threadIdx.x; e < M1 * SVD_COLS; e += blockDim.x) {
+        const int r = e / SVD_COLS, c = c0 + e % SVD_COLS;
+        b[e] = c < D ? B[(size_t) r * D + c] : 0.0;
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < M1 * D; idx += blockDim.x) {
-        const int r = idx / D, c = idx % D;
-        double acc = 0.0;
-        for (int i = 0; i < M1; i++)
-            acc += V[(size_t) r * M1 + i] * tmp[(size_t) i * D + c];
-        W[idx] = acc;
+    for (int i = threadIdx.x; i < M1; i += blockDim.x) {
+        double acc[SVD_COLS] = {};
+        for (int r = 0; r < M1; r++) {
+            const double v = V[(size_t) r * M1 + i];
+#pragma unroll
+            for (int c = 0; c < SVD_COLS; c++)
+                acc[c] = fma(v, b[r * SVD_COLS + c], acc[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < SVD_COLS; c++)
+            y[i * SVD_COLS + c] = inv[i] * acc[c];
     }
-    if (threadIdx.x == 0)
-        flag[0] = 0;
+    __syncthreads();
+    for (int r = threadIdx.x; r < M1; r += blockDim.x) {
+        double acc[SVD_COLS] = {};
+        for (int i = 0; i < M1; i++) {
+            const double v = V[(size_t) r * M1 + i];
+#pragma unroll
+            for (int c = 0; c < SVD_COLS; c++)
+                acc[c] = fma(v, y[i * SVD_COLS + c], acc[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < SVD_COLS; c++)
+            if (c0 + c < D)
+                W[(size_t) r * D + c0 + c] = acc[c];
+    }
 }
 
 int solve_launches(int M1, int solver)
 {
     if (solver == DGTM_SOLVE_SVD)
-        return 1;
+        return 2;
     if (M1 <= SMEM_SOLVE_MAX)
         return 2;
     // np panels, np - 1 trailing updates (none after the last), the substitution
@@ -665,12 +732,26 @@ int launch_solve(const double *A, const double *B, int M1, int D, int solver, do
         set_error(DGTM_ENOTSUP, "the Cholesky solver supports M1 <= %d", 32 * TRI_MAXR);
         return DGTM_ENOTSUP;
     }
-    if (solver == DGTM_SOLVE_SVD && M1 > 2 * SOLVE_THREADS - 2) {
-        set_error(DGTM_ENOTSUP, "the eigen-SVD solver supports M1 <= %d", 2 * SOLVE_THREADS - 2);
+    if (solver == DGTM_SOLVE_SVD && M1 > 2 * SVD_THREADS - 2) {
+        set_error(DGTM_ENOTSUP, "the eigen-SVD solver supports M1 <= %d", 2 * SVD_THREADS - 2);
         return DGTM_ENOTSUP;
     }
     if (solver == DGTM_SOLVE_SVD) {
-        jacobi_solve_kernel<<<1, SOLVE_THREADS, 0, s>>>(A, B, M1, D, W, work, flag);
+        if (M1 <= SVD_SMEM_MAX) {
+            const size_t smem = sizeof(double) * 2 * (size_t) M1 * M1;
+            DGTM_CUDA_TRY(cudaFuncSetAttribute(jacobi_kernel<true>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int) smem));
+            jacobi_kernel<true><<<1, SVD_THREADS, smem, s>>>(A, M1, work, flag);
+        } else {
+            jacobi_kernel<false><<<1, SVD_THREADS, 0, s>>>(A, M1, work, flag);
+        }
+        DGTM_CUDA_TRY(cudaGetLastError());
+        const size_t asmem = sizeof(double) * 2 * SVD_COLS * (size_t) M1;
+        DGTM_CUDA_TRY(cudaFuncSetAttribute(svd_apply_kernel,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int) asmem));
+        svd_apply_kernel<<<ceil_div(D, SVD_COLS), 128, asmem, s>>>(
+            work + (size_t) M1 * M1, work + 2 * (size_t) M1 * M1, B, M1, D, W);
     } else {
         if (M1 <= SMEM_SOLVE_MAX) {
             const size_t smem = sizeof(double) * (3 * (size_t) M1 + (size_t) M1 * M1) +
