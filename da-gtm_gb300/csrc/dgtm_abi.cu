@@ -5,6 +5,7 @@
 // fixed-order on-device reduction and only scalars cross to the host.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "oz.cuh"
 #include "tc.cuh"
 #include "x64.cuh"
 
@@ -73,13 +74,16 @@ struct dgtm_ctx {
     double *Gpart, *RTpart;
     double *G, *RT, *A, *B, *work, *bterm, *abpart;
     double *scal;      // device scalars
-    int *flag;         // device status: [0..1] the solver's, [2] update_y's pair counter
+    int *flag;         // device status: [0..1] the solver's, [2] update_y's pair counter,
+                       // [3] the digit-slice products' bounded waits
     double *hscal;     // pinned host scalars
     int *hflag;
     // split-BF16 form
     TcState *tc;
     // exact-slice FP64 form (0/1 data on sm_10x; otherwise the CUDA-core form)
     XState *x64;
+    // normal equations by digit slices on the tensor cores (large K M1 (M1 + D))
+    OzAB *ozab;
     // phase timers (dgtm_set_timing)
     int timing;
     cudaEvent_t ev[DGTM_NPHASES][2];
@@ -161,6 +165,18 @@ int sync_and_check(dgtm_ctx *c)
     return DGTM_OK;
 }
 
+// the digit-slice products' status word, fetched into hflag[3]
+int check_oz_status(dgtm_ctx *c)
+{
+    if (c->hflag[3] == 0)
+        return DGTM_OK;
+    const int site = c->hflag[3];
+    c->hflag[3] = 0;
+    cudaMemsetAsync(c->flag + 3, 0, sizeof(int), c->stream);
+    set_error(DGTM_ETIMEOUT, "a wait in the digit-slice product gave up (site %d)", site);
+    return DGTM_ETIMEOUT;
+}
+
 int phase_begin(dgtm_ctx *c, int p)
 {
     if (c->timing)
@@ -213,6 +229,7 @@ void free_ctx(dgtm_ctx *c)
         tc_destroy(c->tc);
     if (c->x64)
         x64_destroy(c->x64);
+    ozab_destroy(c->ozab);
     for (int p = 0; p < DGTM_NPHASES; p++)
         for (int q = 0; q < 2; q++)
             if (c->ev[p][q])
@@ -305,16 +322,27 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
     CK(dev_alloc(&c->B, (size_t) M1 * D));
     CK(dev_alloc(&c->work, 2 * (size_t) M1 * M1 + (size_t) M1 * D));
     CK(dev_alloc(&c->bterm, K));
-    CK(dev_alloc(&c->abpart, form_ab_scratch_doubles(M1, D)));
+    // The FP32 and split forms keep form_ab's multiply-add chain: their E-step
+    // rounds the centres to FP32 / BF16 pieces, so a W that differs in its last
+    // bits flips some of those roundings, and a run would no longer repeat what
+    // it gave before to better than the form's own 1e-5.
+    if (precision == DGTM_FP64 && ozab_wanted(K, M1, D))
+        CK(ozab_create(&c->ozab, K, M1, D, c->sms));
+    else
+        CK(dev_alloc(&c->abpart, form_ab_scratch_doubles(M1, D)));
     CK(dev_alloc(&c->scal, 8));
     CK(dev_alloc(&c->flag, 4));
     CKC(cudaMallocHost((void **) &c->hscal, 8 * sizeof(double)));
     CKC(cudaMallocHost((void **) &c->hflag, 4 * sizeof(int)));
+    CKC(cudaMemsetAsync(c->flag, 0, 4 * sizeof(int), c->stream));
+    memset(c->hflag, 0, 4 * sizeof(int));
 
     CKC(copy_rows(c->T64, sizeof(double) * D, T, sizeof(double) * (size_t) ldT,
                           sizeof(double) * D, N, cudaMemcpyHostToDevice, c->stream));
     CKC(copy_rows(c->FI, sizeof(double) * M1, FI, sizeof(double) * (size_t) ldFI,
                           sizeof(double) * M1, K, cudaMemcpyHostToDevice, c->stream));
+    if (c->ozab)
+        CK(ozab_basis(c->ozab, c->FI, c->stream));
     if (precision != DGTM_FP64) {
         CK(dev_alloc(&c->FIp, (size_t) K * M1));
         CK(launch_to_pairs(c->FI, (size_t) K * M1, c->FIp, c->stream));
@@ -534,8 +562,15 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
                                       ctx->RT, ctx->stream));
         nsmall += 1;
     }
-    DGTM_TRY(launch_form_ab(ctx->FI, ctx->G, ctx->RT, K, M1, D, ctx->A, ctx->B, ctx->abpart,
-                            ctx->stream));
+    if (ctx->ozab) {
+        int nab = 0;
+        DGTM_TRY(ozab_form(ctx->ozab, ctx->FI, ctx->G, ctx->RT, ctx->A, ctx->B, ctx->flag + 3, &nab,
+                           ctx->stream));
+        nsmall += nab - 2;
+    } else {
+        DGTM_TRY(launch_form_ab(ctx->FI, ctx->G, ctx->RT, K, M1, D, ctx->A, ctx->B, ctx->abpart,
+                                ctx->stream));
+    }
     DGTM_TRY(launch_solve(ctx->A, ctx->B, M1, D, ctx->solver, ctx->W, ctx->work, ctx->flag,
                           ctx->stream));
     // the E-step's copies of the new centres come out of the same kernel
@@ -560,7 +595,7 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
     DGTM_TRY(phase_end(ctx, DGTM_PHASE_MSTEP_SOLVE, nsmall));
     DGTM_CUDA_TRY(cudaMemcpyAsync(ctx->hscal, ctx->scal, 2 * sizeof(double),
                                   cudaMemcpyDeviceToHost, ctx->stream));
-    DGTM_CUDA_TRY(cudaMemcpyAsync(ctx->hflag, ctx->flag, 2 * sizeof(int), cudaMemcpyDeviceToHost,
+    DGTM_CUDA_TRY(cudaMemcpyAsync(ctx->hflag, ctx->flag, 4 * sizeof(int), cudaMemcpyDeviceToHost,
                                   ctx->stream));
     if (W)
         DGTM_CUDA_TRY(copy_rows(W, sizeof(double) * (size_t) ldW, ctx->W,
@@ -575,6 +610,7 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
     DGTM_TRY(sync_and_check(ctx));
     if (ctx->tc)
         DGTM_TRY(tc_check_status(ctx->tc));
+    DGTM_TRY(check_oz_status(ctx));
     ctx->stats_valid = 0;
     ctx->prev_valid = 1;
     ctx->rt_valid = 1;

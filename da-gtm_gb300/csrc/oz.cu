@@ -1,0 +1,613 @@
+// oz.cu -- FP64-accurate matrix products on the tensor cores (tcgen05 + TMA +
+// TMEM, sm_103a) by exact digit slices.
+//
+// GB300's FP64 pipe does 2 FMA per clock per SM (0.63 TFMA/s measured on the
+// whole GPU), its BF16 tensor pipe 4096.  Each FP64 operand value is therefore
+// written as a 56-bit integer on its row's (or the matrix's) power-of-two grid
+// and cut into eight balanced base-128 digits, |d| <= 64, exact in BF16 (the
+// error-free splitting of Ozaki, Ogita, Oishi and Rump, "Error-free
+// transformations of matrix multiplication by using fast routines of matrix
+// multiplication and its applications", Numer. Algorithms 59, 2012).  Products
+// of digits i and j carry the weight of level l = i + j, so one FP32
+// accumulator per level holds them all:
+//     C = sum_l 128^(14 - l) S_l,  S_l = sum_{i + j = l} sum_k a_i[k] b_j[k],
+// |S_l| <= (l + 1) 512 4096 <= 2^24 over 512 elements of k: an exact FP32
+// integer whatever the order.  Levels 0 .. 7 are kept (36 of the 64 digit
+// products); what is dropped is below 2^-58 of the operands' largest products
+// per term, under the rounding of an FP64 multiply-add chain.  The levels are
+// combined in 64-bit integers every 512 elements; FP64 comes back only once per
+// result.
+//
+// oz_gemm_kernel: persistent, one CTA per SM (TMEM: 8 levels x 64 columns = all
+// 512).  Tile 128 (A rows, TMEM lanes) x 64 (B rows).  Per 64-deep panel the
+// eight B planes (64 KB, double-buffered) stay while the A planes stream
+// through a ring of 16 KB slots; A plane i multiplies B planes 0 .. 7 - i in one
+// or two instructions, because consecutive planes of B are consecutive rows in
+// shared memory and their levels i .. 7 consecutive column blocks in TMEM
+// (N up to 256: the tensor pipe's full rate, where an N = 64 instruction per
+// digit pair is bound by shared-memory reads).  Per panel 36 x 128 clocks of
+// MMA against 192 KB of loads.
+#include "common.cuh"
+#include "kernels.cuh"
+#include "oz.cuh"
+#include "sm100.cuh"
+
+#include <vector>
+
+namespace dgtm {
+
+int make_tmap_bf16(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t cols, uint64_t ld,
+                   uint32_t box_rows, uint32_t box_cols);
+
+using namespace sm100;
+
+namespace {
+
+constexpr int OZ_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 drain
+constexpr int TM = 128, TN = 64; // tile
+constexpr int PANEL = 64;
+constexpr int SB = oz::DIGITS;   // planes of B, levels
+constexpr int A_SLOT = TM * 128;           // one A plane of one panel: 16 KB
+constexpr int B_PLANE = TN * 128;          // 8 KB
+constexpr int B_BUF = SB * B_PLANE;        // 64 KB
+constexpr int A_SLOTS = 5;
+constexpr int SEG = 8;                     // panels per exact segment (512 elements)
+constexpr size_t OZ_SMEM = 1024 + 2 * (size_t) B_BUF + A_SLOTS * (size_t) A_SLOT + 256;
+
+struct OzParams {
+    int panels, a_rows, b_rows, a_tile0, mtiles, ntiles, nitems, splits, item_panels;
+    const int *tiles;
+    int64_t *out64;
+    int ext;
+    int64_t *out;
+    size_t ldm;
+    int mrows, ncols;
+    const int *shift;
+    int *status;
+};
+
+__device__ __forceinline__ void oz_item(const OzParams &p, int it, int &mt, int &nt, int &p0, int &p1)
+{
+    const int t = it / p.splits, sp = it - t * p.splits;
+    if (p.tiles) {
+        const int v = p.tiles[t];
+        mt = v >> 16;
+        nt = v & 0xFFFF;
+    } else {
+        mt = t / p.ntiles;
+        nt = t - mt * p.ntiles;
+    }
+    p0 = sp * p.item_panels;
+    p1 = min(p.panels, p0 + p.item_panels);
+}
+
+// the levels of one element as hi 2^28 + lo: the four pairs are exact in 32 bits
+__device__ __forceinline__ void level_pairs(const uint32_t *v, int c, int64_t &hi, int64_t &lo)
+{
+    int q[4];
+#pragma unroll
+    for (int h = 0; h < 4; h++)
+        q[h] = __float2int_rz(__uint_as_float(v[16 * h + c])) * 128 +
+               __float2int_rz(__uint_as_float(v[16 * h + 8 + c]));
+    hi = (int64_t) q[0] * 16384 + q[1];
+    lo = (int64_t) q[2] * 16384 + q[3];
+}
+
+template <int SA, bool SUM>
+__global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
+                                                               const __grid_constant__ CUtensorMap tmB,
+                                                               const OzParams p)
+{
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char *sm = (unsigned char *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
+    unsigned char *Bst = sm, *Ast = sm + 2 * B_BUF;
+    uint64_t *bars = (uint64_t *) (Ast + A_SLOTS * A_SLOT);
+    uint64_t *a_full = bars, *a_empty = bars + A_SLOTS;
+    uint64_t *b_full = bars + 2 * A_SLOTS, *b_empty = b_full + 2;
+    uint64_t *acc_full = b_full + 4, *acc_empty = acc_full + 1, *drain = acc_full + 2;
+    uint32_t *tmem_sh = (uint32_t *) (drain + 1);
+    __shared__ int failed;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        failed = 0;
+        for (int i = 0; i < A_SLOTS; i++) {
+            mbar_init(&a_full[i], 1);
+            mbar_init(&a_empty[i], 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&b_full[i], 1);
+            mbar_init(&b_empty[i], 1);
+        }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, 256);
+        mbar_init(drain, 1);
+        fence_barrier_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(tmem_sh, 512);
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_sh, 0);
+
+    if (warp == 0 && lane == 0) {
+        // ---------------- producer ----------------
+        prefetch_tmap(&tmA);
+        prefetch_tmap(&tmB);
+        int as = 0, na = 0, nb = 0;
+        uint32_t aph = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; ok && it < p.nitems; it += gridDim.x) {
+            int mt, nt, p0, p1;
+            oz_item(p, it, mt, nt, p0, p1);
+            for (int pn = p0; ok && pn < p1; pn++, nb++) {
+                const int b = nb & 1;
+                if (nb >= 2 && !mbar_wait(&b_empty[b], (uint32_t) (((nb >> 1) & 1) ^ 1), p.status, 71)) {
+                    ok = false;
+                    break;
+                }
+                mbar_expect_tx(&b_full[b], (uint32_t) B_BUF);
+#pragma unroll
+                for (int j = 0; j < SB; j++)
+                    tma_load_2d(Bst + b * B_BUF + j * B_PLANE, &tmB, &b_full[b], PANEL * pn,
+                                j * p.b_rows + nt * TN);
+                for (int i = 0; i < SA; i++, na++) {
+                    if (na >= A_SLOTS && !mbar_wait(&a_empty[as], aph ^ 1u, p.status, 72)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&a_full[as], (uint32_t) A_SLOT);
+                    tma_load_2d(Ast + as * A_SLOT, &tmA, &a_full[as], PANEL * pn,
+                                i * p.a_rows + (p.a_tile0 + mt) * TM);
+                    if (++as == A_SLOTS) {
+                        as = 0;
+                        aph ^= 1u;
+                    }
+                }
+            }
+        }
+        if (!ok)
+            failed = 1;
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        const uint64_t adesc0 = sdesc_sw128(smem_u32(Ast), 16, 1024);
+        const uint64_t bdesc0 = sdesc_sw128(smem_u32(Bst), 16, 1024);
+        int as = 0, nb = 0, nseg = 0;
+        uint32_t aph = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; ok && it < p.nitems; it += gridDim.x) {
+            int mt, nt, p0, p1;
+            oz_item(p, it, mt, nt, p0, p1);
+            for (int pn = p0; ok && pn < p1; pn++, nb++) {
+                const int in_seg = (pn - p0) % SEG;
+                if (in_seg == 0 && nseg > 0 &&
+                    !mbar_wait_w(acc_empty, (uint32_t) ((nseg - 1) & 1), p.status, 73)) {
+                    ok = false;
+                    break;
+                }
+                const int b = nb & 1;
+                if (!mbar_wait_w(&b_full[b], (uint32_t) ((nb >> 1) & 1), p.status, 74)) {
+                    ok = false;
+                    break;
+                }
+                const uint64_t bd = bdesc0 + (uint64_t) ((b * B_BUF) >> 4);
+#pragma unroll
+                for (int i = 0; i < SA; i++) {
+                    if (!mbar_wait_w(&a_full[as], aph, p.status, 75)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t ad = adesc0 + (uint64_t) ((as * A_SLOT) >> 4);
+#pragma unroll
+                    for (int ks = 0; ks < 4; ks++) {
+                        const int first = SB - i < 4 ? SB - i : 4;  // B planes of the first instruction
+                        mma_ss_w(tmem + (uint32_t) (i * TN), ad + 2 * ks, bd + 2 * ks,
+                                 idesc_bf16(TM, TN * first, 0, 0),
+                                 (in_seg || i || ks) ? 1u : 0u);
+                        if (SB - i > 4)
+                            mma_ss_w(tmem + (uint32_t) ((i + 4) * TN), ad + 2 * ks,
+                                     bd + (uint64_t) ((4 * B_PLANE) >> 4) + 2 * ks,
+                                     idesc_bf16(TM, TN * (SB - i - 4), 0, 0),
+                                     (in_seg || i || ks) ? 1u : 0u);
+                    }
+                    mma_commit_w(&a_empty[as]);
+                    if (++as == A_SLOTS) {
+                        as = 0;
+                        aph ^= 1u;
+                    }
+                }
+                if (!ok)
+                    break;
+                mma_commit_w(&b_empty[b]);
+                if (in_seg == SEG - 1 || pn == p1 - 1) {
+                    mma_commit_w(acc_full);
+                    nseg++;
+                }
+            }
+        }
+        if (!ok)
+            failed = 1;
+    } else if (warp >= 2) {
+        // ---------------- drain: levels to 64-bit integers ----------------
+        const int q = warp & 3, h = (warp - 2) >> 2;  // lane quarter, half of the columns
+        const uint32_t lane_base = tmem + ((uint32_t) (q * 32) << 16) + (uint32_t) (32 * h);
+        const int row = q * 32 + lane;
+        const int shift = SUM ? 8 + p.ext : (p.shift ? *p.shift : 0);
+        const int64_t half = SUM ? (1ll << (shift - 1)) : 0;
+        int nseg = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; ok && it < p.nitems; it += gridDim.x) {
+            int mt, nt, p0, p1;
+            oz_item(p, it, mt, nt, p0, p1);
+            int64_t acc[SUM ? 32 : 1];
+            if constexpr (SUM) {
+#pragma unroll
+                for (int c = 0; c < 32; c++)
+                    acc[c] = 0;
+            }
+            for (int pn = p0; pn < p1; pn += SEG, nseg++) {
+                if (!mbar_wait(acc_full, (uint32_t) (nseg & 1), p.status, 76)) {
+                    ok = false;
+                    break;
+                }
+                __syncwarp();
+                tc_fence_after();
+#pragma unroll
+                for (int cb = 0; cb < 4; cb++) {
+                    uint32_t v[64];
+#pragma unroll
+                    for (int l = 0; l < SB; l++)
+                        tmem_ld8p(lane_base + (uint32_t) (l * TN + 8 * cb), v + 8 * l);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        int64_t hi, lo;
+                        level_pairs(v, c, hi, lo);
+                        if constexpr (SUM) {
+                            // hi 2^28 + lo may need 72 bits: both are shifted down by >= 8
+                            acc[8 * cb + c] += hi * (1 << (28 - shift)) + ((lo + half) >> shift);
+                        } else {
+                            // units 2^-61 (sa = 8): 8 bits down; sa = 1: exact in 2^-55
+                            int64_t I = SA == 1 ? hi * 268435456 + lo : hi * 1048576 + ((lo + 128) >> 8);
+                            I >>= shift;
+                            const int n = nt * TN + 32 * h + 8 * cb + c, m = mt * TM + row;
+                            if (m < p.mrows && n < p.ncols)
+                                p.out[(size_t) n * p.ldm + m] = I;
+                        }
+                    }
+                }
+                tc_fence_before();
+                mbar_arrive(acc_empty);
+            }
+            if constexpr (SUM) {
+                if (ok) {
+                    int64_t *dst = p.out64 + (size_t) it * (TM * TN) + (size_t) (32 * h) * TM + row;
+#pragma unroll
+                    for (int c = 0; c < 32; c++)
+                        dst[(size_t) c * TM] = acc[c];
+                }
+            }
+        }
+        if (!ok)
+            failed = 1;
+    }
+    __syncthreads();
+    if (failed && warp == 1) {
+        mma_commit_w(drain);
+        mbar_wait_w(drain, 0, p.status, 77, 100000000ull);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        tmem_dealloc(tmem, 512);
+}
+
+// ---------------------------------------------------------------------------
+// slicing
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t bf16_pair(int a, int b) { return pack_bf16((float) a, (float) b); }
+
+// Column c of the source: c < c1: G[k] X1[k][c] (G may be null), else X2[k][c - c1].
+struct OzSource {
+    const double *G, *X1, *X2;
+    int c1, ld1, ld2;
+    __device__ __forceinline__ double at(int k, int c) const
+    {
+        if (c < c1) {
+            const double v = X1[(size_t) k * ld1 + c];
+            return G ? G[k] * v : v;
+        }
+        return X2[(size_t) k * ld2 + (c - c1)];
+    }
+};
+
+// bits[c] = max(bits[c], the largest |value| of column c over the block's rows)
+__global__ void __launch_bounds__(256) oz_colmax_kernel(OzSource src, int rows, int cols, int rows_per,
+                                                        unsigned long long *__restrict__ bits)
+{
+    __shared__ unsigned long long red[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c = blockIdx.y * 32 + lane;
+    const int k0 = blockIdx.x * rows_per, k1 = min(rows, k0 + rows_per);
+    unsigned long long m = 0ull;
+    if (c < cols)
+        for (int k = k0 + w; k < k1; k += 8) {
+            const unsigned long long b = oz::double_bits(src.at(k, c)) & oz::ABS_MASK;
+            m = b > m ? b : m;
+        }
+    red[w][lane] = m;
+    __syncthreads();
+    if (w == 0 && c < cols) {
+        for (int i = 1; i < 8; i++)
+            m = red[i][lane] > m ? red[i][lane] : m;
+        atomicMax(&bits[c], m);
+    }
+}
+
+// planes[i][c][k] = digit i of column c of the source on the column's grid:
+// the transposed operand (contraction over the source's rows), zero past rows
+// and cols.  Block: 64 rows x 32 columns.
+__global__ void __launch_bounds__(256) oz_slice_t_kernel(OzSource src, int rows, int cols, int prows,
+                                                         int ld, const unsigned long long *__restrict__ bits,
+                                                         __nv_bfloat16 *__restrict__ planes)
+{
+    __shared__ int64_t qs[32][65];
+    const int k0 = blockIdx.x * 64, c0 = blockIdx.y * 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c = c0 + lane;
+    const int e = c < cols ? oz::exponent_of(bits[c]) : 0;
+#pragma unroll
+    for (int r = w; r < 64; r += 8) {
+        const int k = k0 + r;
+        qs[lane][r] = (k < rows && c < cols) ? oz::to_fixed(src.at(k, c), e) : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int cc = w; cc < 32; cc += 8) {
+        int64_t a = qs[cc][2 * lane], b = qs[cc][2 * lane + 1];
+        uint32_t *dst = (uint32_t *) (planes + (size_t) (c0 + cc) * ld + k0) + lane;
+        const size_t plane = (size_t) prows * ld / 2;
+#pragma unroll
+        for (int i = oz::DIGITS - 1; i > 0; i--) {
+            const int da = oz::next_digit(a), db = oz::next_digit(b);
+            dst[(size_t) i * plane] = bf16_pair(da, db);
+        }
+        dst[0] = bf16_pair((int) a, (int) b);
+    }
+}
+
+__host__ __device__ constexpr int rup(int a, int b) { return (a + b - 1) / b * b; }
+
+}  // namespace
+
+// One term is below 2^53 units of 2^-53: 512 terms fit 62 bits, longer
+// contractions drop one bit per doubling (of the sum's magnitude, which grows
+// alike: the unit stays below the FP64 rounding of a sum of that many terms).
+int oz_sum_ext(int panels)
+{
+    int ext = 0;
+    while ((512ll << ext) < (long long) panels * PANEL)
+        ext++;
+    return ext;
+}
+
+int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
+{
+    CUtensorMap tmA, tmB;
+    const uint64_t ld = (uint64_t) g.panels * PANEL;
+    int rc = make_tmap_bf16(&tmA, g.A, (uint64_t) g.sa * g.a_rows, ld, ld, TM, PANEL);
+    if (rc == DGTM_OK)
+        rc = make_tmap_bf16(&tmB, g.B, (uint64_t) SB * g.b_rows, ld, ld, TN, PANEL);
+    if (rc != DGTM_OK)
+        return rc;
+    OzParams p{};
+    p.panels = g.panels;
+    p.a_rows = g.a_rows;
+    p.b_rows = g.b_rows;
+    p.a_tile0 = g.a_tile0;
+    p.mtiles = g.mtiles;
+    p.ntiles = g.ntiles;
+    p.item_panels = g.out64 ? g.item_panels : g.panels;
+    p.splits = ceil_div(g.panels, p.item_panels);
+    p.nitems = (g.tiles ? g.ntile : g.mtiles * g.ntiles) * p.splits;
+    p.tiles = g.tiles;
+    p.out64 = g.out64;
+    p.ext = oz_sum_ext(g.panels);
+    p.out = g.out;
+    p.ldm = g.ldm;
+    p.mrows = g.mrows;
+    p.ncols = g.ncols;
+    p.shift = g.shift;
+    p.status = status;
+    using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const OzParams);
+    const Kernel k = g.out64 ? (Kernel) oz_gemm_kernel<8, true>
+                             : (g.sa == 1 ? (Kernel) oz_gemm_kernel<1, false> : (Kernel) oz_gemm_kernel<8, false>);
+    DGTM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) OZ_SMEM));
+    k<<<p.nitems < sms ? p.nitems : sms, OZ_THREADS, OZ_SMEM, s>>>(tmA, tmB, p);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    return DGTM_OK;
+}
+
+// ---------------------------------------------------------------------------
+// the M-step's normal equations
+// ---------------------------------------------------------------------------
+struct OzAB {
+    int K = 0, M1 = 0, D = 0, sms = 0;
+    int Kp = 0, panels = 0, Mp = 0, Ap = 0, Wp = 0;  // Ap: columns of diag(G) FI, padded to 64
+    int ntile = 0, splits = 0, item_panels = 0;
+    __nv_bfloat16 *Fp = nullptr, *Wpl = nullptr;
+    unsigned long long *fbits = nullptr, *wbits = nullptr;
+    int64_t *part = nullptr;
+    int *tiles = nullptr;
+};
+
+namespace {
+
+// A and B from the tiles' split sums (exact integers); a column with a
+// non-finite value gives NaN.
+__global__ void __launch_bounds__(256) ozab_reduce_kernel(const int64_t *__restrict__ part,
+                                                          const int *__restrict__ tiles, int splits,
+                                                          int ext, int M1, int D, int Ap,
+                                                          const unsigned long long *__restrict__ fbits,
+                                                          const unsigned long long *__restrict__ wbits,
+                                                          double *__restrict__ A, double *__restrict__ B)
+{
+    const int t = blockIdx.x, v = tiles[t], mt = v >> 16, nt = v & 0xFFFF;
+    for (int e = blockIdx.y * 256 + threadIdx.x; e < TM * TN; e += 256 * gridDim.y) {
+        const int m = mt * TM + (e & (TM - 1)), c = nt * TN + (e >> 7);
+        const bool isA = c < Ap;
+        const int j = isA ? c : c - Ap;
+        if (m >= M1 || (isA ? (j >= M1 || j < m) : j >= D))
+            continue;
+        int64_t sum = 0;
+        for (int sp = 0; sp < splits; sp++)
+            sum += part[((size_t) t * splits + sp) * (TM * TN) + e];
+        const unsigned long long fb = fbits[m], wb = wbits[isA ? j : M1 + j];
+        double r = scalbn((double) sum, oz::exponent_of(fb) + oz::exponent_of(wb) - 53 + ext);
+        if (fb >= oz::INF_BITS || wb >= oz::INF_BITS)
+            r = NAN;
+        if (isA) {
+            A[(size_t) m * M1 + j] = r;
+            A[(size_t) j * M1 + m] = r;
+        } else {
+            B[(size_t) m * D + j] = r;
+        }
+    }
+}
+
+}  // namespace
+
+bool ozab_wanted(int K, int M1, int D)
+{
+    return K <= (1 << 26) && (double) K * M1 * (0.5 * M1 + D) >= 2e7;
+}
+
+void ozab_destroy(OzAB *st)
+{
+    if (!st)
+        return;
+    void *ptrs[] = {st->Fp, st->Wpl, st->fbits, st->wbits, st->part, st->tiles};
+    for (void *p : ptrs)
+        if (p)
+            cudaFree(p);
+    delete st;
+}
+
+int ozab_create(OzAB **out, int K, int M1, int D, int sms)
+{
+    *out = nullptr;
+    OzAB *st = new OzAB();
+    st->K = K;
+    st->M1 = M1;
+    st->D = D;
+    st->sms = sms;
+    st->Kp = rup(K, PANEL);
+    st->panels = st->Kp / PANEL;
+    st->Mp = rup(M1, TM);
+    st->Ap = rup(M1, TN);
+    st->Wp = st->Ap + rup(D, TN);
+    // the tiles that reach the upper triangle of A, and all of B's
+    std::vector<int> tiles;
+    for (int mt = 0; mt < st->Mp / TM; mt++)
+        for (int nt = 0; nt < st->Wp / TN; nt++)
+            if (nt * TN >= st->Ap || nt * TN + TN - 1 >= mt * TM)
+                tiles.push_back(mt << 16 | nt);
+    st->ntile = (int) tiles.size();
+    // splits of the contraction: whole panels, the count that gives the shortest
+    // schedule of equal items on `sms` CTAs (36 x 128 clocks of MMA a panel, about
+    // 5000 clocks to fill the pipeline and drain the accumulator, 60 an item to
+    // write its sums and read them back)
+    int per = 1;
+    double best = 1e300;
+    for (int c = 1; c <= st->panels; c++) {
+        const double items = (double) st->ntile * ceil_div(st->panels, c);
+        const double cost = ceil(items / sms) * (c * 4608.0 + 5000.0) + 60.0 * items;
+        if (cost < best) {
+            best = cost;
+            per = c;
+        }
+    }
+    st->item_panels = per;
+    st->splits = ceil_div(st->panels, per);
+    cudaError_t e = cudaMalloc((void **) &st->Fp, sizeof(__nv_bfloat16) * oz::DIGITS * (size_t) st->Mp * st->Kp);
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **) &st->Wpl, sizeof(__nv_bfloat16) * oz::DIGITS * (size_t) st->Wp * st->Kp);
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **) &st->fbits, sizeof(unsigned long long) * M1);
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **) &st->wbits, sizeof(unsigned long long) * (M1 + D));
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **) &st->part, sizeof(int64_t) * TM * TN * (size_t) st->ntile * st->splits);
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **) &st->tiles, sizeof(int) * tiles.size());
+    if (e == cudaSuccess)
+        e = cudaMemcpy(st->tiles, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        const int code = e == cudaErrorMemoryAllocation ? DGTM_ENOMEM : DGTM_ECUDA;
+        set_error(code, "ozab_create: %s", cudaGetErrorString(e));
+        ozab_destroy(st);
+        return code;
+    }
+    *out = st;
+    return DGTM_OK;
+}
+
+// FI's digit planes, once per basis; the padding rows of both operands are zero
+int ozab_basis(OzAB *st, const double *FI, cudaStream_t s)
+{
+    const int K = st->K, M1 = st->M1;
+    DGTM_CUDA_TRY(cudaMemsetAsync(st->Fp, 0, sizeof(__nv_bfloat16) * oz::DIGITS * (size_t) st->Mp * st->Kp, s));
+    DGTM_CUDA_TRY(cudaMemsetAsync(st->Wpl, 0, sizeof(__nv_bfloat16) * oz::DIGITS * (size_t) st->Wp * st->Kp, s));
+    DGTM_CUDA_TRY(cudaMemsetAsync(st->fbits, 0, sizeof(unsigned long long) * M1, s));
+    const OzSource src{nullptr, FI, nullptr, M1, M1, 0};
+    oz_colmax_kernel<<<dim3(ceil_div(K, 128), ceil_div(M1, 32)), 256, 0, s>>>(src, K, M1, 128, st->fbits);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    oz_slice_t_kernel<<<dim3(st->panels, ceil_div(M1, 32)), 256, 0, s>>>(src, K, M1, st->Mp, st->Kp,
+                                                                        st->fbits, st->Fp);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    return DGTM_OK;
+}
+
+int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, double *A, double *B,
+              int *status, int *nlaunch, cudaStream_t s)
+{
+    const int K = st->K, M1 = st->M1, D = st->D, W = M1 + D;
+    DGTM_CUDA_TRY(cudaMemsetAsync(st->wbits, 0, sizeof(unsigned long long) * W, s));
+    // diag(G) FI at rows 0 .. M1 of the planes, RT at rows Ap ..
+    const OzSource both{G, FI, RT, M1, M1, D};
+    oz_colmax_kernel<<<dim3(ceil_div(K, 128), ceil_div(W, 32)), 256, 0, s>>>(both, K, W, 128, st->wbits);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    const OzSource left{G, FI, nullptr, M1, M1, 0}, right{nullptr, RT, nullptr, D, D, 0};
+    oz_slice_t_kernel<<<dim3(st->panels, ceil_div(M1, 32)), 256, 0, s>>>(left, K, M1, st->Wp, st->Kp,
+                                                                        st->wbits, st->Wpl);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    oz_slice_t_kernel<<<dim3(st->panels, ceil_div(D, 32)), 256, 0, s>>>(
+        right, K, D, st->Wp, st->Kp, st->wbits + M1, st->Wpl + (size_t) st->Ap * st->Kp);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    OzGemm g;
+    g.A = st->Fp;
+    g.B = st->Wpl;
+    g.a_rows = st->Mp;
+    g.b_rows = st->Wp;
+    g.panels = st->panels;
+    g.mtiles = st->Mp / TM;
+    g.ntiles = st->Wp / TN;
+    g.tiles = st->tiles;
+    g.ntile = st->ntile;
+    g.out64 = st->part;
+    g.item_panels = st->item_panels;
+    const int rc = launch_oz_gemm(g, st->sms, status, s);
+    if (rc != DGTM_OK)
+        return rc;
+    ozab_reduce_kernel<<<dim3(st->ntile, 32), 256, 0, s>>>(st->part, st->tiles, st->splits, oz_sum_ext(st->panels), M1, D, st->Ap,
+                                                          st->fbits, st->wbits, A, B);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    if (nlaunch)
+        *nlaunch = 5;
+    return DGTM_OK;
+}
+
+}  // namespace dgtm

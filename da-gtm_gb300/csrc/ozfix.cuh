@@ -1,0 +1,196 @@
+// ozfix.cuh -- fixed-point pieces of the digit-slice products (oz.cu): FP64
+// values as 56-bit integers in eight balanced base-128 digits, and powers of
+// two of a fixed-point exponent in 64-bit integer arithmetic.
+//
+// GB300 issues FP64 at 2 operations per clock per SM, 1/64 of its FP32 rate and
+// 1/32 of its integer rate.  A library exp(double) is about 20 such operations;
+// exp2_neg below is about 50 integer ones, and more exact: its argument is a
+// fixed-point number with an absolute error of 2^-53, where an FP64 argument of
+// 10 already carries 2^-50.
+//
+// Everything here is host/device code so that it can be checked on the CPU.
+#pragma once
+
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#if defined(__CUDACC__)
+#define OZ_HD __host__ __device__ __forceinline__
+#else
+#define OZ_HD static inline
+#endif
+
+namespace dgtm {
+namespace oz {
+
+constexpr int DIGITS = 8;        // balanced base-128 digits, each |d| <= 64
+constexpr int FIX = 55;          // |v| < 2^e is held as rint(v 2^(FIX - e)), |q| <= 2^55
+constexpr int TAB_BITS = 12;     // exp2_neg: 2^-(i / 4096), i = 0 .. 4095
+constexpr int TAB = 1 << TAB_BITS;
+constexpr int WFRAC = 53;        // exponents in units of 2^-53
+constexpr int WBIAS = 4;         // exponents carry + 4, so a slightly negative one fits
+
+OZ_HD uint64_t mulhi(uint64_t a, uint64_t b)
+{
+#if defined(__CUDA_ARCH__)
+    return __umul64hi(a, b);
+#else
+    return (uint64_t) (((unsigned __int128) a * b) >> 64);
+#endif
+}
+
+OZ_HD uint32_t mulhi32(uint32_t a, uint32_t b) { return (uint32_t) (((uint64_t) a * b) >> 32); }
+
+OZ_HD uint64_t double_bits(double v)
+{
+#if defined(__CUDA_ARCH__)
+    return (uint64_t) __double_as_longlong(v);
+#else
+    uint64_t b;
+    memcpy(&b, &v, sizeof b);
+    return b;
+#endif
+}
+
+OZ_HD double bits_double(uint64_t b)
+{
+#if defined(__CUDA_ARCH__)
+    return __longlong_as_double((long long) b);
+#else
+    double v;
+    memcpy(&v, &b, sizeof v);
+    return v;
+#endif
+}
+
+// the bits of |v| order like |v| (with infinities and NaN on top)
+constexpr uint64_t ABS_MASK = 0x7FFFFFFFFFFFFFFFull;
+constexpr uint64_t INF_BITS = 0x7FF0000000000000ull;
+
+// e with |v| < 2^e for every |v| up to the one with these bits
+OZ_HD int exponent_of(uint64_t absbits)
+{
+    const int E = (int) (absbits >> 52);
+    return (E ? E : 1) - 1022;
+}
+
+// rint(v 2^(FIX - e)) (ties away from zero), for |v| < 2^e; integer operations only
+OZ_HD int64_t to_fixed(double v, int e)
+{
+    const uint64_t b = double_bits(v);
+    const int E = (int) ((b >> 52) & 0x7FF);
+    const uint64_t m = (b & 0xFFFFFFFFFFFFFull) | (E ? (1ull << 52) : 0ull);
+    const int sh = (E ? E : 1) - 1020 - e;  // at most 2
+    uint64_t q;
+    if (sh >= 0)
+        q = m << (sh & 3);
+    else if (sh > -60)
+        q = (m + (1ull << (-sh - 1))) >> (-sh);
+    else
+        q = 0;
+    return (b >> 63) ? -(int64_t) q : (int64_t) q;
+}
+
+// q 2^k as an int64 from a double q, rounded to nearest, saturated
+OZ_HD int64_t scaled_int(double v, int k)
+{
+    const uint64_t b = double_bits(v);
+    const int E = (int) ((b >> 52) & 0x7FF);
+    const uint64_t m = (b & 0xFFFFFFFFFFFFFull) | (E ? (1ull << 52) : 0ull);
+    const int sh = (E ? E : 1) - 1075 + k;
+    uint64_t q;
+    if (sh >= 10)
+        q = m ? 0x7FFFFFFFFFFFFFFFull : 0ull;
+    else if (sh >= 0)
+        q = m << sh;
+    else if (sh > -63)
+        q = (m + (1ull << (-sh - 1))) >> (-sh);
+    else
+        q = 0;
+    return (b >> 63) ? -(int64_t) q : (int64_t) q;
+}
+
+// the least digit of the running value r, taken out of it; after DIGITS - 1
+// calls on r = q what is left in r is the top digit (-64 .. 64)
+OZ_HD int next_digit(int64_t &r)
+{
+    const int d = (int) ((r + 64) & 127) - 64;
+    r = (r - d) >> 7;
+    return d;
+}
+
+// w = x kappa in units of 2^-53, for 0 <= x <= lim: (mulhi(x << a, m)) >> b
+struct Mul {
+    uint64_t m;
+    uint64_t lim;  // beyond it w leaves the exponents' range: the power is 0
+    int a, b;
+};
+
+// kappa: the exponent (base 2) of one unit of x; the product is kept below 2000
+inline Mul make_mul(double kappa)
+{
+    Mul r;
+    int ex = 0;
+    const double f = frexp(kappa, &ex);  // kappa = f 2^ex, f in [0.5, 1)
+    r.m = (uint64_t) ldexp(f, 64);
+    if (f >= 1.0)
+        r.m = ~0ull;
+    // x kappa 2^53 = x m 2^(ex + 53 - 64) = mulhi(x << a, m) >> b
+    const int sh = ex + WFRAC;  // a - b
+    r.a = sh > 0 ? (sh < 63 ? sh : 63) : 0;
+    r.b = sh < 0 ? (-sh < 63 ? -sh : 63) : 0;
+    const double l = 2000.0 / kappa;
+    const double cap = ldexp(1.0, 63 - r.a);  // x << a below 2^63
+    const double t = l < cap ? l : cap;
+    r.lim = t < 9.0e18 ? (uint64_t) t : 9000000000000000000ull;
+    if (sh > 63)
+        r.lim = 0;
+    return r;
+}
+
+OZ_HD uint64_t mul_w(const Mul &k, uint64_t x) { return mulhi(x << k.a, k.m) >> k.b; }
+
+// 2^-(W 2^-53) = E 2^-63 2^-n with n = W >> 53: returns E in (2^62, 2^63].
+// 2^-f = T[f's top 12 bits] (1 - x), x = y - y^2/2 + y^3/6 - y^4/24 for
+// y = rho ln 2 below 2^-12.5; x within 2^-57, T within 2^-63.
+OZ_HD uint64_t exp2_neg(uint64_t W, const uint64_t *tab)
+{
+    const uint32_t i = (uint32_t) (W >> (WFRAC - TAB_BITS)) & (TAB - 1);
+    const uint64_t T = tab[i];
+    const uint64_t rho = W << (64 - (WFRAC - TAB_BITS));      // the low 41 bits on top
+    const uint64_t y = mulhi(rho, 0xB17217F7D1CF79ACull) >> TAB_BITS;  // ln 2; y in 2^-64
+    const uint32_t yh = (uint32_t) ((y + (1ull << 19)) >> 20);         // y in 2^-44
+    const uint64_t yy = (uint64_t) yh * yh;                            // y^2 in 2^-88
+    const uint32_t s = (uint32_t) (yy >> 32);                          // y^2 in 2^-56
+    const uint32_t s6 = mulhi32(s, 715827883u);                        // y^2 / 6
+    const uint64_t y3 = ((uint64_t) s6 * yh) >> 36;                    // y^3 / 6 in 2^-64
+    const uint32_t y4 = mulhi32(mulhi32(s, s), 178956971u) >> 16;      // y^4 / 24 in 2^-64
+    const uint64_t x = y - (yy >> 25) + y3 - y4;
+    return T - mulhi(T, x);
+}
+
+// E 2^-63 2^(-n) as a double, E in (2^62, 2^63]
+OZ_HD double to_double(uint64_t E, int n)
+{
+    // round to 53 bits: E + half an ulp, carried into the exponent by the add
+    const bool one = (E >> 63) != 0;
+    const uint64_t m = one ? 0ull : ((E << 2) + (1ull << 11)) >> 12;  // 52 fraction bits (may carry)
+    const int e = (one ? 0 : -1) - n;
+    if (e < -1021)
+        return e < -1100 ? 0.0 : scalbn((double) (int64_t) (E >> 1), -62 - n);
+    return bits_double(((uint64_t) (e + 1023) << 52) + m);
+}
+
+// an unsigned fixed-point value in units of 2^-53 from a double (v >= 0)
+OZ_HD uint64_t to_wfix(double v) { return (uint64_t) scaled_int(v, WFRAC); }
+
+// table entry: 2^-(i / 4096) in units of 2^-63
+inline void fill_table(uint64_t *tab)
+{
+    for (int i = 0; i < TAB; i++)
+        tab[i] = (uint64_t) (exp2l(-(long double) i / TAB) * 9223372036854775808.0L + 0.5L);
+}
+
+}  // namespace oz
+}  // namespace dgtm

@@ -27,3 +27,11 @@ def solve_case(pkg, M1, D, K, solver, precision="fp64"):
 @pytest.mark.parametrize("M1,D", [(1, 3), (2, 5), (3, 1), (26, 9), (65, 33), (112, 6), (113, 6)])
 def test_svd_sizes(pkg, M1, D):
     solve_case(pkg, M1, D, 3 * M1 + 20, "svd")
+
+
+# the normal equations by digit slices: one tile and several, ragged K, M1 and D,
+# contractions of one segment (512 centres) and of many
+@pytest.mark.parametrize("K,M1,D", [(8000, 65, 166), (5003, 129, 33), (1500, 513, 7), (2111, 200, 190),
+                                    (33000, 30, 64), (700, 250, 20)])
+def test_normal_equations_by_slices(pkg, K, M1, D):
+    solve_case(pkg, M1, D, K, "cholesky")

@@ -1,0 +1,22 @@
+"""The fixed-point pieces of the digit-slice products
+(da-gtm_gb300/csrc/ozfix.cuh), compiled for the host from the same header and
+checked against long-double references (tests/oz_check.cc): digits rebuild the
+56-bit integer and the integer the value to half a unit; exp2_neg within 2^-57
+and its double within one FP64 rounding (2^-53); the fixed-point product of an
+exponent within one unit plus the 64-bit constant's own 2^-63."""
+import os
+import subprocess
+
+from conftest import ROOT
+
+
+def test_fixed_point_pieces(tmp_path):
+    exe = str(tmp_path / "oz_check")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-o", exe,
+                           os.path.join(ROOT, "tests", "oz_check.cc"), "-lm"])
+    bad, exp2, dbl, prod = subprocess.run([exe], capture_output=True, text=True, timeout=300,
+                                          check=True).stdout.split()
+    assert float(bad) == 0
+    assert float(exp2) <= 2.0 ** -57
+    assert float(dbl) <= 2.0 ** -53 + 2.0 ** -57
+    assert float(prod) <= 2.0
