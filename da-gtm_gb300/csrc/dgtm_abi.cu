@@ -84,6 +84,10 @@ struct dgtm_ctx {
     XState *x64;
     // normal equations by digit slices on the tensor cores (large K M1 (M1 + D))
     OzAB *ozab;
+    // digit-slice E-step, responsibility pass and map (FP64 form, other data), and
+    // for the map of the other contexts, made by the first large dgtm_map
+    OzE *oze, *ozmap;
+    int ozmap_tried;
     // phase timers (dgtm_set_timing)
     int timing;
     cudaEvent_t ev[DGTM_NPHASES][2];
@@ -165,6 +169,13 @@ int sync_and_check(dgtm_ctx *c)
     return DGTM_OK;
 }
 
+int fetch_oz_status(dgtm_ctx *c)
+{
+    DGTM_CUDA_TRY(cudaMemcpyAsync(c->hflag + 3, c->flag + 3, sizeof(int), cudaMemcpyDeviceToHost,
+                                  c->stream));
+    return DGTM_OK;
+}
+
 // the digit-slice products' status word, fetched into hflag[3]
 int check_oz_status(dgtm_ctx *c)
 {
@@ -210,6 +221,49 @@ int refresh_y_copies(dgtm_ctx *c, int *n)
     return DGTM_OK;
 }
 
+// Digit-slice state is larger than what the CUDA-core kernels need: without
+// memory for it a context falls back to them.
+int unless_enomem(int code)
+{
+    if (code != DGTM_ENOMEM)
+        return code;
+    g_err[0] = 0;
+    return DGTM_OK;
+}
+
+// DGTM_X64=0 keeps FP64 work on the CUDA cores
+bool slices_on()
+{
+    const char *env = getenv("DGTM_X64");
+    return !(env && strcmp(env, "0") == 0);
+}
+
+OzEArgs oze_args(const dgtm_ctx *c, bool mstep)
+{
+    OzEArgs a{};
+    a.T64 = c->T64;
+    a.tt = c->tt;
+    a.N = c->N;
+    a.D = c->D;
+    a.K = c->K;
+    a.sms = c->sms;
+    a.mstep = mstep;
+    a.status = c->flag + 3;
+    // 0/1 data that a context already holds in BF16
+    if (c->x64) {
+        a.Tb = (const __nv_bfloat16 *) x64_data(c->x64, &a.Tb_rows, &a.Tb_ld);
+    } else if (c->tc) {
+        TcView v;
+        tc_view(c->tc, &v);
+        if (v.binary && v.nT == 1) {
+            a.Tb = (const __nv_bfloat16 *) v.Tb;
+            a.Tb_rows = v.Npad;
+            a.Tb_ld = v.Dp;
+        }
+    }
+    return a;
+}
+
 void free_ctx(dgtm_ctx *c)
 {
     if (!c)
@@ -230,6 +284,8 @@ void free_ctx(dgtm_ctx *c)
     if (c->x64)
         x64_destroy(c->x64);
     ozab_destroy(c->ozab);
+    oze_destroy(c->oze);
+    oze_destroy(c->ozmap);
     for (int p = 0; p < DGTM_NPHASES; p++)
         for (int q = 0; q < 2; q++)
             if (c->ev[p][q])
@@ -327,8 +383,8 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
     // bits flips some of those roundings, and a run would no longer repeat what
     // it gave before to better than the form's own 1e-5.
     if (precision == DGTM_FP64 && ozab_wanted(K, M1, D))
-        CK(ozab_create(&c->ozab, K, M1, D, c->sms));
-    else
+        CK(unless_enomem(ozab_create(&c->ozab, K, M1, D, c->sms)));
+    if (!c->ozab)
         CK(dev_alloc(&c->abpart, form_ab_scratch_doubles(M1, D)));
     CK(dev_alloc(&c->scal, 8));
     CK(dev_alloc(&c->flag, 4));
@@ -369,10 +425,16 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
                 CK(xr);
             if (c->x64)
                 c->nblk1 = x64_pass1_blocks(c->x64);
+            else if (slices_on() && oze_wanted(N, D, K))
+                CK(unless_enomem(oze_create(&c->oze, oze_args(c, true), c->stream)));
+            if (c->oze)
+                c->nblk1 = oze_estep_blocks(c->oze);
         }
         CK(dev_alloc(&c->part, 2 * (size_t) c->nblk1));
-        CK(dev_alloc(&c->Gpart, (size_t) c->nsplit * K));
-        CK(dev_alloc(&c->RTpart, (size_t) c->nsplit * KD));
+        if (!c->oze) {
+            CK(dev_alloc(&c->Gpart, (size_t) c->nsplit * K));
+            CK(dev_alloc(&c->RTpart, (size_t) c->nsplit * KD));
+        }
         if (precision == DGTM_FP32) {
             CK(dev_alloc(&c->T32, ND));
             CK(dev_alloc(&c->Y32, KD));
@@ -475,6 +537,9 @@ int dgtm_estep(dgtm_ctx *ctx, double beta, int isDA, double temp, double *llh, d
     if (ctx->x64) {
         r = x64_estep(ctx->x64, ctx->Y64, ctx->yy, ctx->tt, c1, c2, isDA, ctx->colstat, ctx->part,
                       ctx->stream, &nl);
+    } else if (ctx->oze) {
+        r = oze_estep(ctx->oze, ctx->Y64, ctx->yy, c1, c2, isDA, ctx->colstat, ctx->part,
+                      ref_dcut(beta), &nl, ctx->stream);
     } else if (ctx->precision == DGTM_FP64) {
         Pass1Args<double> a{ctx->T64, ctx->Y64, ctx->tt, ctx->yy, ctx->N, ctx->D, ctx->K,
                             c1, c2, isDA, ctx->colstat, ctx->part};
@@ -497,7 +562,11 @@ int dgtm_estep(dgtm_ctx *ctx, double beta, int isDA, double temp, double *llh, d
         DGTM_TRY(tc_fetch_status(ctx->tc, ctx->stream));
     if (ctx->x64)
         DGTM_TRY(x64_fetch_status(ctx->x64, ctx->stream));
+    if (ctx->oze)
+        DGTM_TRY(fetch_oz_status(ctx));
     DGTM_TRY(sync_and_check(ctx));
+    if (ctx->oze)
+        DGTM_TRY(check_oz_status(ctx));
     if (ctx->tc)
         DGTM_TRY(tc_check_status(ctx->tc));
     if (ctx->x64)
@@ -540,6 +609,8 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
     DGTM_TRY(phase_begin(ctx, DGTM_PHASE_MSTEP_PASS));
     if (ctx->x64) {
         DGTM_TRY(x64_mstep_pass(ctx->x64, c, ctx->G, ctx->RT, ctx->stream, &npass));  // cut: pass 1
+    } else if (ctx->oze) {
+        DGTM_TRY(oze_mstep_pass(ctx->oze, c, ctx->G, ctx->RT, &npass, ctx->stream));
     } else if (ctx->precision == DGTM_FP64) {
         Pass2Args<double> a{ctx->T64, ctx->Y64, ctx->tt, ctx->yy, ctx->colstat, N, D, K, c,
                             ctx->n_per_split, ctx->Gpart, ctx->RTpart, ref_dcut(ctx->beta)};
@@ -557,7 +628,7 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
         int nr = 0;
         DGTM_TRY(tc_mstep_reduce(ctx->tc, ctx->G, ctx->RT, ctx->stream, &nr));
         nsmall += nr;
-    } else if (!ctx->x64) {
+    } else if (!ctx->x64 && !ctx->oze) {
         DGTM_TRY(launch_reduce_slices(ctx->Gpart, ctx->RTpart, ctx->nsplit, K, D, ctx->G,
                                       ctx->RT, ctx->stream));
         nsmall += 1;
@@ -709,13 +780,28 @@ int dgtm_get_path(dgtm_ctx *ctx, int *path)
         set_error(DGTM_EINVAL, "path is null");
         return DGTM_EINVAL;
     }
-    *path = ctx->x64 ? DGTM_PATH_EXACT_SLICES : ctx->tc ? DGTM_PATH_SPLIT_BF16 : DGTM_PATH_CUDA_CORES;
+    *path = ctx->x64 || ctx->oze ? DGTM_PATH_EXACT_SLICES : ctx->tc ? DGTM_PATH_SPLIT_BF16 : DGTM_PATH_CUDA_CORES;
     return DGTM_OK;
 }
 
 }  // extern "C"
 
 namespace {
+
+// The context's digit-slice state for the map, made on first use and kept; null
+// where the problem is small, the data are not finite or memory is short (the
+// CUDA-core kernel then does it).
+OzE *map_slices(dgtm_ctx *c)
+{
+    if (c->oze)
+        return c->oze;
+    if (!c->ozmap_tried && slices_on() && oze_wanted(c->N, c->D, c->K)) {
+        c->ozmap_tried = 1;
+        if (oze_create(&c->ozmap, oze_args(c, false), c->stream) != DGTM_OK)
+            g_err[0] = 0;
+    }
+    return c->ozmap;
+}
 
 // M = R^T X, or with rd (R o D)^T X: R of the last E-step, which an M-step has
 // followed, times the squared distances to the new centres.
@@ -743,10 +829,15 @@ int map_impl(dgtm_ctx *ctx, const double *X, int L, double *M, int ldM, bool rd)
         return r;
     }
     r = DGTM_OK;
+    OzE *oz = rd ? nullptr : map_slices(ctx);
     cudaError_t e = cudaMemcpyAsync(dX, X, sizeof(double) * ctx->K * L, cudaMemcpyHostToDevice,
                                     ctx->stream);
     if (e == cudaSuccess) {
-        if (rd)
+        if (oz) {
+            r = oze_map(oz, ctx->Y64, ctx->yy, ctx->colstat, c, dX, L, dM, ctx->stream);
+            if (r == DGTM_OK)
+                r = fetch_oz_status(ctx);
+        } else if (rd)
             r = launch_map(ctx->T64, ctx->Yprev, ctx->tt, ctx->yyprev, ctx->colstat, ctx->N, ctx->D,
                            ctx->K, c, dX, L, dM, ctx->stream, ctx->Y64, ctx->yy);
         else
@@ -759,6 +850,8 @@ int map_impl(dgtm_ctx *ctx, const double *X, int L, double *M, int ldM, bool rd)
     }
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(ctx->stream);
+    if (oz && e == cudaSuccess && r == DGTM_OK)
+        r = check_oz_status(ctx);
     cudaFree(dX);
     cudaFree(dM);
     if (e != cudaSuccess) {

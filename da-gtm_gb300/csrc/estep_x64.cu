@@ -1075,6 +1075,13 @@ void x64_destroy(XState *st)
     delete st;
 }
 
+const void *x64_data(const XState *st, int *Npad, int *Dp)
+{
+    *Npad = st->Npad;
+    *Dp = st->Dp;
+    return st->Tx;
+}
+
 int x64_create(XState **out, int N, int D, int K, int sms, const double *T64, cudaStream_t s)
 {
     *out = nullptr;

@@ -30,8 +30,10 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "oz.cuh"
+#include "oz_slice.cuh"
 #include "sm100.cuh"
 
+#include <math.h>
 #include <vector>
 
 namespace dgtm {
@@ -55,7 +57,7 @@ constexpr int SEG = 8;                     // panels per exact segment (512 elem
 constexpr size_t OZ_SMEM = 1024 + 2 * (size_t) B_BUF + A_SLOTS * (size_t) A_SLOT + 256;
 
 struct OzParams {
-    int panels, a_rows, b_rows, a_tile0, mtiles, ntiles, nitems, splits, item_panels;
+    int panels, b_panel0, a_rows, b_rows, a_tile0, mtiles, ntiles, nitems, splits, item_panels;
     const int *tiles;
     int64_t *out64;
     int ext;
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
                 mbar_expect_tx(&b_full[b], (uint32_t) B_BUF);
 #pragma unroll
                 for (int j = 0; j < SB; j++)
-                    tma_load_2d(Bst + b * B_BUF + j * B_PLANE, &tmB, &b_full[b], PANEL * pn,
+                    tma_load_2d(Bst + b * B_BUF + j * B_PLANE, &tmB, &b_full[b], PANEL * (pn + p.b_panel0),
                                 j * p.b_rows + nt * TN);
                 for (int i = 0; i < SA; i++, na++) {
                     if (na >= A_SLOTS && !mbar_wait(&a_empty[as], aph ^ 1u, p.status, 72)) {
@@ -305,80 +307,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
         tmem_dealloc(tmem, 512);
 }
 
-// ---------------------------------------------------------------------------
-// slicing
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t bf16_pair(int a, int b) { return pack_bf16((float) a, (float) b); }
-
-// Column c of the source: c < c1: G[k] X1[k][c] (G may be null), else X2[k][c - c1].
-struct OzSource {
-    const double *G, *X1, *X2;
-    int c1, ld1, ld2;
-    __device__ __forceinline__ double at(int k, int c) const
-    {
-        if (c < c1) {
-            const double v = X1[(size_t) k * ld1 + c];
-            return G ? G[k] * v : v;
-        }
-        return X2[(size_t) k * ld2 + (c - c1)];
-    }
-};
-
-// bits[c] = max(bits[c], the largest |value| of column c over the block's rows)
-__global__ void __launch_bounds__(256) oz_colmax_kernel(OzSource src, int rows, int cols, int rows_per,
-                                                        unsigned long long *__restrict__ bits)
-{
-    __shared__ unsigned long long red[8][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int c = blockIdx.y * 32 + lane;
-    const int k0 = blockIdx.x * rows_per, k1 = min(rows, k0 + rows_per);
-    unsigned long long m = 0ull;
-    if (c < cols)
-        for (int k = k0 + w; k < k1; k += 8) {
-            const unsigned long long b = oz::double_bits(src.at(k, c)) & oz::ABS_MASK;
-            m = b > m ? b : m;
-        }
-    red[w][lane] = m;
-    __syncthreads();
-    if (w == 0 && c < cols) {
-        for (int i = 1; i < 8; i++)
-            m = red[i][lane] > m ? red[i][lane] : m;
-        atomicMax(&bits[c], m);
-    }
-}
-
-// planes[i][c][k] = digit i of column c of the source on the column's grid:
-// the transposed operand (contraction over the source's rows), zero past rows
-// and cols.  Block: 64 rows x 32 columns.
-__global__ void __launch_bounds__(256) oz_slice_t_kernel(OzSource src, int rows, int cols, int prows,
-                                                         int ld, const unsigned long long *__restrict__ bits,
-                                                         __nv_bfloat16 *__restrict__ planes)
-{
-    __shared__ int64_t qs[32][65];
-    const int k0 = blockIdx.x * 64, c0 = blockIdx.y * 32;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int c = c0 + lane;
-    const int e = c < cols ? oz::exponent_of(bits[c]) : 0;
-#pragma unroll
-    for (int r = w; r < 64; r += 8) {
-        const int k = k0 + r;
-        qs[lane][r] = (k < rows && c < cols) ? oz::to_fixed(src.at(k, c), e) : 0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int cc = w; cc < 32; cc += 8) {
-        int64_t a = qs[cc][2 * lane], b = qs[cc][2 * lane + 1];
-        uint32_t *dst = (uint32_t *) (planes + (size_t) (c0 + cc) * ld + k0) + lane;
-        const size_t plane = (size_t) prows * ld / 2;
-#pragma unroll
-        for (int i = oz::DIGITS - 1; i > 0; i--) {
-            const int da = oz::next_digit(a), db = oz::next_digit(b);
-            dst[(size_t) i * plane] = bf16_pair(da, db);
-        }
-        dst[0] = bf16_pair((int) a, (int) b);
-    }
-}
-
 __host__ __device__ constexpr int rup(int a, int b) { return (a + b - 1) / b * b; }
 
 }  // namespace
@@ -394,17 +322,37 @@ int oz_sum_ext(int panels)
     return ext;
 }
 
+// Splits of the contraction: whole panels an item, the count that gives the
+// shortest schedule of equal items on `sms` CTAs (36 x 128 clocks of MMA a panel,
+// about 5000 clocks to fill the pipeline and drain the accumulator, 60 an item to
+// write its sums and read them back).
+int oz_item_panels(int ntile, int panels, int sms)
+{
+    int per = 1;
+    double best = 1e300;
+    for (int c = 1; c <= panels; c++) {
+        const double items = (double) ntile * ceil_div(panels, c);
+        const double cost = ceil(items / sms) * (c * 4608.0 + 5000.0) + 60.0 * items;
+        if (cost < best) {
+            best = cost;
+            per = c;
+        }
+    }
+    return per;
+}
+
 int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
 {
     CUtensorMap tmA, tmB;
-    const uint64_t ld = (uint64_t) g.panels * PANEL;
-    int rc = make_tmap_bf16(&tmA, g.A, (uint64_t) g.sa * g.a_rows, ld, ld, TM, PANEL);
+    const uint64_t lda = (uint64_t) g.a_panels * PANEL, ldb = (uint64_t) g.b_panels * PANEL;
+    int rc = make_tmap_bf16(&tmA, g.A, (uint64_t) g.sa * g.a_rows, lda, lda, TM, PANEL);
     if (rc == DGTM_OK)
-        rc = make_tmap_bf16(&tmB, g.B, (uint64_t) SB * g.b_rows, ld, ld, TN, PANEL);
+        rc = make_tmap_bf16(&tmB, g.B, (uint64_t) SB * g.b_rows, ldb, ldb, TN, PANEL);
     if (rc != DGTM_OK)
         return rc;
     OzParams p{};
     p.panels = g.panels;
+    p.b_panel0 = g.b_panel0;
     p.a_rows = g.a_rows;
     p.b_rows = g.b_rows;
     p.a_tile0 = g.a_tile0;
@@ -516,20 +464,7 @@ int ozab_create(OzAB **out, int K, int M1, int D, int sms)
             if (nt * TN >= st->Ap || nt * TN + TN - 1 >= mt * TM)
                 tiles.push_back(mt << 16 | nt);
     st->ntile = (int) tiles.size();
-    // splits of the contraction: whole panels, the count that gives the shortest
-    // schedule of equal items on `sms` CTAs (36 x 128 clocks of MMA a panel, about
-    // 5000 clocks to fill the pipeline and drain the accumulator, 60 an item to
-    // write its sums and read them back)
-    int per = 1;
-    double best = 1e300;
-    for (int c = 1; c <= st->panels; c++) {
-        const double items = (double) st->ntile * ceil_div(st->panels, c);
-        const double cost = ceil(items / sms) * (c * 4608.0 + 5000.0) + 60.0 * items;
-        if (cost < best) {
-            best = cost;
-            per = c;
-        }
-    }
+    const int per = oz_item_panels(st->ntile, st->panels, sms);
     st->item_panels = per;
     st->splits = ceil_div(st->panels, per);
     cudaError_t e = cudaMalloc((void **) &st->Fp, sizeof(__nv_bfloat16) * oz::DIGITS * (size_t) st->Mp * st->Kp);
@@ -547,6 +482,7 @@ int ozab_create(OzAB **out, int K, int M1, int D, int sms)
         e = cudaMemcpy(st->tiles, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         const int code = e == cudaErrorMemoryAllocation ? DGTM_ENOMEM : DGTM_ECUDA;
+        cudaGetLastError();
         set_error(code, "ozab_create: %s", cudaGetErrorString(e));
         ozab_destroy(st);
         return code;
@@ -592,7 +528,7 @@ int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, dou
     g.B = st->Wpl;
     g.a_rows = st->Mp;
     g.b_rows = st->Wp;
-    g.panels = st->panels;
+    g.panels = g.a_panels = g.b_panels = st->panels;
     g.mtiles = st->Mp / TM;
     g.ntiles = st->Wp / TN;
     g.tiles = st->tiles;

@@ -11,14 +11,16 @@
 namespace dgtm {
 
 // One product C[m][n] = sum_k A[m][k] B[n][k] over digit planes: A has sa planes
-// (8, or 1 for values that are small integers themselves) of a_rows x ld BF16,
-// B has 8 planes of b_rows x ld; ld = 64 panels; a_rows a multiple of 128,
-// b_rows of 64.
+// (8, or 1 for values that are small integers themselves) of a_rows x 64
+// a_panels BF16, B has 8 planes of b_rows x 64 b_panels; a_rows a multiple of
+// 128, b_rows of 64.  The contraction runs over `panels` panels of 64, from
+// panel 0 of A and panel b_panel0 of B.
 struct OzGemm {
     const __nv_bfloat16 *A = nullptr, *B = nullptr;
     int sa = 8;
     int a_rows = 0, b_rows = 0;
     int panels = 0;        // 64-deep panels of the contraction
+    int a_panels = 0, b_panels = 0, b_panel0 = 0;
     int a_tile0 = 0;       // first 128-row tile of A
     int mtiles = 0, ntiles = 0;
     const int *tiles = nullptr;  // (mt << 16 | nt) of each tile, or null: all mtiles x ntiles
@@ -38,6 +40,7 @@ struct OzGemm {
 };
 
 int oz_sum_ext(int panels);
+int oz_item_panels(int ntile, int panels, int sms);
 int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s);
 
 // A = FI^T diag(G) FI and B = FI^T RT by digit slices; FI's planes are kept.
@@ -49,5 +52,30 @@ int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, dou
               int *status, int *nlaunch, cudaStream_t s);
 // whether the digit-slice product is the faster one at this size
 bool ozab_wanted(int K, int M1, int D);
+
+// The E-step, responsibility pass and map from digit-slice distances
+// (oz_estep.cu).
+struct OzE;
+struct OzEArgs {
+    const double *T64, *tt;  // N x D, N
+    int N, D, K, sms;
+    // 0/1 data already in BF16 (rows_pad a multiple of 128, ld = 64 panels; columns
+    // past D meet zeros), or null: eight digit planes of T64 are made
+    const __nv_bfloat16 *Tb;
+    int Tb_rows, Tb_ld;
+    bool mstep;              // with what the responsibility pass needs
+    int *status;             // device: the bounded waits' status word
+};
+bool oze_wanted(int N, int D, int K);
+// *out stays null (and the call succeeds) where the data have a non-finite value
+int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s);
+void oze_destroy(OzE *st);
+int oze_estep_blocks(const OzE *st);
+int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, int isDA,
+              double2 *colstat, double *part, double dcut, int *nlaunch, cudaStream_t s);
+int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaStream_t s);
+// M = R^T X from a context's column statistics
+int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c,
+            const double *X, int L, double *M, cudaStream_t s);
 
 }  // namespace dgtm

@@ -1,0 +1,779 @@
+// oz_estep.cu -- the E-step, the responsibility pass and the MAP projection in
+// FP64 accuracy from digit-slice distances (oz.cu): real-valued data of the FP64
+// form, and the map of every form.
+//
+// The CUDA-core kernels (estep_simt.cu) spend D FP64 multiply-adds and about 20
+// FP64 operations of exp a centre-point pair, on a pipe of two per clock and SM.
+// Here the contraction runs on the tensor cores and what is left per pair on the
+// integer pipe:
+//
+//   distances.  acc_kn = y_k.t_n - |y_k|^2 / 2 = (|t_n|^2 - d_kn) / 2 as a 64-bit
+//     integer on one power-of-two grid (unit 2^u, at most 2^-53 of the largest
+//     product), so the best centre is an integer comparison and
+//     d_kn - d_min = 2 (acc_max - acc_kn) 2^u an exact integer difference.
+//   exponentials.  2^-W for the fixed-point W = c log2(e) (d_kn - d_min) (+ log2 of
+//     the column sum), units of 2^-53 (ozfix.cuh): no FP64 operation.
+//   column sums.  2^-63 integers with a carry word: exact, order-free.
+//   G and R T.  R_kn on its centre's power-of-two grid (the chunk's largest
+//     R of the centre within [2^-56, 1] of it: small responsibilities keep their
+//     relative precision), in eight digit planes, times the digit planes of
+//     T^T and a row of ones: 64-bit integer sums per chunk, FP64 across chunks.
+//
+// Points go in chunks whose K x nn integers stay in L2 (8 M of them, 64 MB).
+// Everything per chunk is a launch of its own: the distances cross L2 once more
+// than in a fused kernel (16 bytes a pair, against ~150 integer operations), and
+// one layout serves the statistics, the responsibilities and the map.
+#include "common.cuh"
+#include "kernels.cuh"
+#include "oz.cuh"
+#include "oz_slice.cuh"
+
+#include <math.h>
+#include <new>
+
+namespace dgtm {
+
+namespace {
+
+constexpr int PANEL = 64;
+constexpr long long CHUNK = 8LL << 20;  // centre-point pairs a chunk
+constexpr int ST_PTS = 8;               // points of a statistics block
+constexpr int ST_THREADS = 512;
+constexpr int ST_WARPS = ST_THREADS / 32;
+constexpr int ST_KG = ST_THREADS / ST_PTS;  // centre groups of a block
+constexpr int64_t ZERO_COLUMN = INT64_MIN;  // aref of a point whose R is 1/K
+constexpr size_t TAB_BYTES = sizeof(uint64_t) * oz::TAB;
+
+__host__ __device__ constexpr int rup(int a, int b) { return (a + b - 1) / b * b; }
+
+// the centres' grid, set by oz_slice_rows_kernel
+struct OzScale {
+    int shift;  // right shift of the product's integers (oz.cuh)
+    int u;      // one unit of acc is 2^u
+    int bad;    // a centre is not finite
+};
+
+// a point's reference and the exponent its responsibilities start from
+struct OzPoint {
+    int64_t aref;   // (t^2 - d_ref) / 2 in units, or ZERO_COLUMN
+    uint64_t lam;   // log2 s + WBIAS (2^-53)
+};
+
+// max |y| and max |y|^2 of the centres, as bits
+__global__ void __launch_bounds__(256) oz_absmax_kernel(const double *__restrict__ X, size_t n,
+                                                        const double *__restrict__ xx, int rows,
+                                                        unsigned long long *__restrict__ bits)
+{
+    unsigned long long m = 0ull, q = 0ull;
+    for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < n; i += (size_t) gridDim.x * 256) {
+        const unsigned long long b = oz::double_bits(X[i]) & oz::ABS_MASK;
+        m = b > m ? b : m;
+        if (i < (size_t) rows) {
+            const unsigned long long c = oz::double_bits(xx[i]) & oz::ABS_MASK;
+            q = c > q ? c : q;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long a = __shfl_xor_sync(0xffffffffu, m, o), b = __shfl_xor_sync(0xffffffffu, q, o);
+        m = a > m ? a : m;
+        q = b > q ? b : q;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&bits[0], m);
+        atomicMax(&bits[1], q);
+    }
+}
+
+// planes[i][r][d] = digit i of X[r][d] on the common grid of bits[0]; zero past rows
+// and D.  With sc: the grid of the products with T (tbits: its max |t| and |t|^2;
+// sa its planes) and h_k = |y_k|^2 / 2 on it.
+__global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__restrict__ X, int rows, int D,
+                                                            int prows, int ld,
+                                                            const unsigned long long *__restrict__ bits,
+                                                            __nv_bfloat16 *__restrict__ planes,
+                                                            const unsigned long long *__restrict__ tbits,
+                                                            int sa, const double *__restrict__ xx,
+                                                            OzScale *sc, int64_t *__restrict__ h)
+{
+    const int e = oz::exponent_of(bits[0]);
+    const size_t n2 = (size_t) prows * ld / 2;
+    if (sc) {
+        // |t.y| + |y|^2 / 2, and differences of two such, within 2^62 units
+        const int base = sa == 1 ? e - 55 : oz::exponent_of(tbits[0]) + e - 53;
+        const double tt = oz::bits_double(tbits[1]), yy = oz::bits_double(bits[1]);
+        const double bound = 2.0 * (sqrt(tt) * sqrt(yy) + 0.5 * yy);
+        const int need = oz::exponent_of(oz::double_bits(bound)) - 62;
+        const int u = need > base ? need : base;
+        const int bad = bits[0] >= oz::INF_BITS || bits[1] >= oz::INF_BITS;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            sc->shift = u - base < 60 ? u - base : 60;
+            sc->u = u;
+            sc->bad = bad;
+        }
+        for (int k = blockIdx.x * 256 + threadIdx.x; k < rows; k += gridDim.x * 256)
+            h[k] = bad ? 0 : oz::scaled_int(xx[k], -1 - u);
+    }
+    for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < n2; i += (size_t) gridDim.x * 256) {
+        const int r = (int) (2 * i / ld), d = (int) (2 * i % ld);
+        int64_t a = 0, b = 0;
+        if (r < rows) {
+            const double *x = X + (size_t) r * D;
+            a = d < D ? oz::to_fixed(x[d], e) : 0;
+            b = d + 1 < D ? oz::to_fixed(x[d + 1], e) : 0;
+        }
+        uint32_t *dst = (uint32_t *) planes + i;
+#pragma unroll
+        for (int p = oz::DIGITS - 1; p > 0; p--) {
+            const int da = oz::next_digit(a), db = oz::next_digit(b);
+            dst[(size_t) p * n2] = bf16_pair(da, db);
+        }
+        dst[0] = bf16_pair((int) a, (int) b);
+    }
+}
+
+__device__ __forceinline__ void load_table(uint64_t *tab, const uint64_t *__restrict__ gtab)
+{
+    for (int i = threadIdx.x; i < oz::TAB; i += blockDim.x)
+        tab[i] = gtab[i];
+}
+
+// the base-2 exponent of a double's natural logarithm term, as a fixed-point value
+__device__ __forceinline__ uint64_t lam_of(double ln_s)
+{
+    return oz::to_wfix(ln_s * 1.4426950408889634 + (double) oz::WBIAS);
+}
+
+struct OzStatsArgs {
+    const int64_t *acc;    // K x ldm
+    size_t ldm;
+    const int64_t *h;      // K
+    const OzScale *sc;
+    const uint64_t *tab;
+    const double *tt;      // this chunk's points
+    int nn, K, isDA;
+    double c1, c2, dcut;
+    oz::MulBase k1, k2;    // 2 c log2(e) for the two exponents
+    double2 *colstat;
+    OzPoint *pt;
+    int64_t *thr;
+    double *part;          // 2 per block
+};
+
+// Column statistics of a chunk.  Block: 8 points x 64 centre groups (a warp
+// reads four 64-byte rows at once); the maximum first, then the sums against it.
+// Bound by the integer pipe: about 75 instructions an exponential.
+template <bool TWO>
+__global__ void __launch_bounds__(ST_THREADS) oz_stats_kernel(const OzStatsArgs a)
+{
+    extern __shared__ uint64_t tab[];
+    __shared__ int64_t smax[ST_WARPS][ST_PTS];
+    __shared__ uint64_t slo[2][ST_WARPS][ST_PTS];
+    __shared__ uint32_t shi[2][ST_WARPS][ST_PTS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int pl = lane & (ST_PTS - 1), kg = w * (32 / ST_PTS) + lane / ST_PTS;
+    const int p = blockIdx.x * ST_PTS + pl;
+    const bool live = p < a.nn;
+    const int64_t *acc = a.acc + (live ? p : 0);
+    load_table(tab, a.tab);
+    int64_t m = INT64_MIN;
+#pragma unroll 4
+    for (int k = kg; k < a.K; k += ST_KG) {
+        const int64_t v = acc[(size_t) k * a.ldm] - a.h[k];
+        m = v > m ? v : m;
+    }
+#pragma unroll
+    for (int o = ST_PTS; o < 32; o <<= 1) {
+        const int64_t v = __shfl_xor_sync(0xffffffffu, m, o);
+        m = v > m ? v : m;
+    }
+    if (lane < ST_PTS)
+        smax[w][lane] = m;
+    __syncthreads();
+    m = smax[0][pl];
+#pragma unroll
+    for (int i = 1; i < ST_WARPS; i++)
+        m = smax[i][pl] > m ? smax[i][pl] : m;
+    const int u = a.sc->u;
+    const oz::Mul k1 = oz::mul_at(a.k1, u), k2 = oz::mul_at(a.k2, u);
+    uint64_t lo1 = 0, lo2 = 0;
+    uint32_t hi1 = 0, hi2 = 0;
+#pragma unroll 2
+    for (int k = kg; k < a.K; k += ST_KG) {
+        const uint64_t x = (uint64_t) (m - (acc[(size_t) k * a.ldm] - a.h[k]));
+        if (x <= k1.lim) {
+            const uint64_t W = oz::mul_w(k1, x);
+            const int n = (int) (W >> oz::WFRAC);
+            const uint64_t t = n < 64 ? oz::exp2_neg(W, tab) >> n : 0ull;
+            lo1 += t;
+            hi1 += lo1 < t;
+        }
+        if (TWO && x <= k2.lim) {
+            const uint64_t W = oz::mul_w(k2, x);
+            const int n = (int) (W >> oz::WFRAC);
+            const uint64_t t = n < 64 ? oz::exp2_neg(W, tab) >> n : 0ull;
+            lo2 += t;
+            hi2 += lo2 < t;
+        }
+    }
+#pragma unroll
+    for (int o = ST_PTS; o < 32; o <<= 1) {
+        uint64_t v = __shfl_xor_sync(0xffffffffu, lo1, o);
+        hi1 += __shfl_xor_sync(0xffffffffu, hi1, o);
+        lo1 += v;
+        hi1 += lo1 < v;
+        if (TWO) {
+            v = __shfl_xor_sync(0xffffffffu, lo2, o);
+            hi2 += __shfl_xor_sync(0xffffffffu, hi2, o);
+            lo2 += v;
+            hi2 += lo2 < v;
+        }
+    }
+    if (lane < ST_PTS) {
+        slo[0][w][lane] = lo1;
+        shi[0][w][lane] = hi1;
+        slo[1][w][lane] = lo2;
+        shi[1][w][lane] = hi2;
+    }
+    __syncthreads();
+    if (w != 0)
+        return;
+    double t1 = 0.0, t2 = 0.0;
+    if (lane < ST_PTS && live) {
+#pragma unroll
+        for (int i = 1; i < ST_WARPS; i++) {
+            const uint64_t v1 = slo[0][i][lane], v2 = slo[1][i][lane];
+            lo1 += v1;
+            hi1 += shi[0][i][lane] + (lo1 < v1);
+            lo2 += v2;
+            hi2 += shi[1][i][lane] + (lo2 < v2);
+        }
+        const double s1 = (double) hi1 * 2.0 + (double) lo1 * 0x1p-63;
+        const double s2 = TWO ? (double) hi2 * 2.0 + (double) lo2 * 0x1p-63 : s1;
+        const double dmin = a.tt[p] - 2.0 * scalbn((double) m, u);
+        const double ln1 = log(s1), ln2 = TWO ? log(s2) : ln1;
+        t1 = -a.c1 * dmin + ln1;
+        t2 = a.isDA ? -a.c2 * dmin + ln2 : 0.0;
+        double lsn = a.isDA ? ln2 : ln1;
+        int64_t aref = m;
+        uint64_t lam = lam_of(lsn);
+        // comm/mpicomm.c:382-389: a column whose every exp(-beta d/2) underflows
+        // is replaced by R = 1/K with v = K
+        if (exp(-a.c1 * dmin) == 0.0 || a.sc->bad) {
+            lsn = NAN;
+            aref = ZERO_COLUMN;
+            lam = lam_of(log((double) a.K));
+            if (a.isDA) {
+                t1 = -INFINITY;
+                t2 = log((double) a.K);
+            } else {
+                t1 = log((double) a.K);
+            }
+            if (a.sc->bad)
+                t1 = t2 = NAN;
+        }
+        a.colstat[p] = make_double2(dmin, lsn);
+        a.pt[p] = OzPoint{aref, lam};
+        // R = 0 beyond the distance where the reference's exp(-beta d / 2) underflows
+        a.thr[p] = aref == ZERO_COLUMN ? INT64_MIN : oz::scaled_int(a.tt[p] - a.dcut, -1 - u);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        t1 += __shfl_down_sync(0xffffffffu, t1, o);
+        t2 += __shfl_down_sync(0xffffffffu, t2, o);
+    }
+    if (lane == 0) {
+        a.part[2 * blockIdx.x] = t1;
+        a.part[2 * blockIdx.x + 1] = t2;
+    }
+}
+
+// references and exponents from a context's column statistics (d_ref, ln s)
+__global__ void oz_points_kernel(const double2 *__restrict__ colstat, const double *__restrict__ tt, int N,
+                                 int K, const OzScale *__restrict__ sc, OzPoint *__restrict__ pt)
+{
+    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
+        const double2 cs = colstat[n];
+        OzPoint o;
+        if (isnan(cs.y) || sc->bad) {
+            o.aref = ZERO_COLUMN;
+            o.lam = lam_of(log((double) K));
+        } else {
+            o.aref = oz::scaled_int(tt[n] - cs.x, -1 - sc->u);
+            o.lam = lam_of(cs.y);
+        }
+        pt[n] = o;
+    }
+}
+
+// W of R = 2^(WBIAS - W): w(aref - acc) + lam; ~0 where R is 0
+__device__ __forceinline__ uint64_t r_exponent(const OzPoint &o, int64_t v, const oz::Mul &k)
+{
+    if (o.aref == ZERO_COLUMN)
+        return o.lam;
+    const int64_t x = o.aref - v;
+    const uint64_t ax = (uint64_t) (x < 0 ? -x : x);
+    if (ax > k.lim)
+        return x < 0 ? 0ull : ~0ull;
+    const uint64_t wv = oz::mul_w(k, ax);
+    if (x >= 0)
+        return o.lam + wv;
+    return o.lam > wv ? o.lam - wv : 0ull;
+}
+
+// Responsibilities of a chunk as digit planes, planes[i][k][n] (n fastest), each
+// centre on the grid of its largest R in the chunk; nmin[k] is that R's integer
+// exponent.  Zero past nn up to ldn.  One block per centre; the exponents are
+// formed twice, which is cheaper than keeping them.
+__global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn,
+                                                        const int64_t *__restrict__ h,
+                                                        const OzScale *__restrict__ sc,
+                                                        const uint64_t *__restrict__ gtab,
+                                                        const OzPoint *__restrict__ pt,
+                                                        const int64_t *__restrict__ thr, oz::MulBase kb, int prows, int ldn,
+                                                        __nv_bfloat16 *__restrict__ planes,
+                                                        int *__restrict__ nmin_out)
+{
+    extern __shared__ uint64_t tab[];
+    __shared__ int red[8];
+    const int k = blockIdx.x;
+    const oz::Mul km = oz::mul_at(kb, sc->u);
+    const int64_t hk = h[k];
+    const int64_t *row = acc + (size_t) k * ldm;
+    load_table(tab, gtab);
+    int nmin = 1 << 20;
+    for (int n = threadIdx.x; n < nn; n += 256) {
+        const int64_t v = row[n] - hk;
+        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, km);
+        const int e = (int) (W >> oz::WFRAC);
+        if (e < 2047)
+            nmin = e < nmin ? e : nmin;
+    }
+    nmin = __reduce_min_sync(0xffffffffu, nmin);
+    if ((threadIdx.x & 31) == 0)
+        red[threadIdx.x >> 5] = nmin;
+    __syncthreads();
+    nmin = red[0];
+#pragma unroll
+    for (int i = 1; i < 8; i++)
+        nmin = red[i] < nmin ? red[i] : nmin;
+    if (threadIdx.x == 0)
+        nmin_out[k] = nmin;
+    const size_t plane = (size_t) prows * ldn / 2;
+    uint32_t *dst = (uint32_t *) planes + (size_t) k * ldn / 2;
+    for (int j = threadIdx.x; j < ldn / 2; j += 256) {
+        int64_t q[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int n = 2 * j + e;
+            q[e] = 0;
+            if (n < nn) {
+                const int64_t v = row[n] - hk;
+                const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, km);
+                const int ex = (int) (W >> oz::WFRAC);
+                // R 2^(55 - (5 - nmin)) = E >> (9 + ex - nmin), rounded
+                const int sh = 9 + ex - nmin;
+                if (ex < 2047 && sh < 64)
+                    q[e] = (int64_t) ((oz::exp2_neg(W, tab) + (1ull << (sh - 1))) >> sh);
+            }
+        }
+#pragma unroll
+        for (int i = oz::DIGITS - 1; i > 0; i--) {
+            const int da = oz::next_digit(q[0]), db = oz::next_digit(q[1]);
+            dst[(size_t) i * plane + j] = bf16_pair(da, db);
+        }
+        dst[j] = bf16_pair((int) q[0], (int) q[1]);
+    }
+}
+
+// G and R T of a chunk from the products' split sums; the first chunk sets, the
+// others add.  Column D of the product is the row of ones: G.
+__global__ void __launch_bounds__(256) oz_rt_kernel(const int64_t *__restrict__ part, int ntiles, int splits,
+                                                    int ext, const int *__restrict__ nmin,
+                                                    const unsigned long long *__restrict__ cbits, int K, int D,
+                                                    int first, double *__restrict__ G, double *__restrict__ RT)
+{
+    const int t = blockIdx.x, mt = t / ntiles, nt = t - mt * ntiles;
+    for (int e = blockIdx.y * 256 + threadIdx.x; e < 128 * 64; e += 256 * gridDim.y) {
+        const int k = mt * 128 + (e & 127), d = nt * 64 + (e >> 7);
+        if (k >= K || d > D)
+            continue;
+        int64_t sum = 0;
+        for (int sp = 0; sp < splits; sp++)
+            sum += part[((size_t) t * splits + sp) * (128 * 64) + e];
+        const int nm = nmin[k];
+        const double v = nm < 2047 ? scalbn((double) sum, 5 - nm + oz::exponent_of(cbits[d]) - 53 + ext) : 0.0;
+        double *dst = d < D ? RT + (size_t) k * D + d : G + k;
+        *dst = first ? v : *dst + v;
+    }
+}
+
+// M = R^T X of a chunk, blocks as in oz_stats_kernel.
+template <int LMAX>
+__global__ void __launch_bounds__(ST_THREADS) oz_map_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn,
+                                                            const int64_t *__restrict__ h,
+                                                            const OzScale *__restrict__ sc,
+                                                            const uint64_t *__restrict__ gtab,
+                                                            const OzPoint *__restrict__ pt, oz::MulBase kb,
+                                                            int K, const double *__restrict__ X, int L,
+                                                            double *__restrict__ M)
+{
+    extern __shared__ uint64_t tab[];
+    __shared__ double sm[ST_WARPS][LMAX][ST_PTS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int pl = lane & (ST_PTS - 1), kg = w * (32 / ST_PTS) + lane / ST_PTS;
+    const int p = blockIdx.x * ST_PTS + pl;
+    const bool live = p < nn;
+    const int64_t *a = acc + (live ? p : 0);
+    const OzPoint o = pt[live ? p : 0];
+    const oz::Mul km = oz::mul_at(kb, sc->u);
+    load_table(tab, gtab);
+    __syncthreads();
+    double m[LMAX] = {};
+#pragma unroll 2
+    for (int k = kg; k < K; k += ST_KG) {
+        const uint64_t W = r_exponent(o, a[(size_t) k * ldm] - h[k], km);
+        const double r = W == ~0ull ? 0.0
+                                    : oz::to_double(oz::exp2_neg(W, tab), (int) (W >> oz::WFRAC) - oz::WBIAS);
+#pragma unroll
+        for (int l = 0; l < LMAX; l++)
+            if (l < L)
+                m[l] = fma(r, X[(size_t) k * L + l], m[l]);
+    }
+#pragma unroll
+    for (int l = 0; l < LMAX; l++) {
+#pragma unroll
+        for (int s = ST_PTS; s < 32; s <<= 1)
+            m[l] += __shfl_xor_sync(0xffffffffu, m[l], s);
+        if (lane < ST_PTS)
+            sm[w][l][lane] = m[l];
+    }
+    __syncthreads();
+    if (threadIdx.x < LMAX * ST_PTS) {
+        const int l = threadIdx.x / ST_PTS, q = blockIdx.x * ST_PTS + threadIdx.x % ST_PTS;
+        if (l < L && q < nn) {
+            double s = 0.0;
+            for (int i = 0; i < ST_WARPS; i++)
+                s += sm[i][l][threadIdx.x % ST_PTS];
+            M[(size_t) q * L + l] = s;
+        }
+    }
+}
+
+int grid_of(size_t n, int cap)
+{
+    const size_t b = (n + 255) / 256;
+    return (int) (b < 1 ? 1 : b > (size_t) cap ? (size_t) cap : b);
+}
+
+}  // namespace
+
+struct OzE {
+    OzEArgs a;
+    int sa = 8, panels = 0, Dp = 0, Np = 0, Kp = 0, chunk = 0, nchunks = 0;
+    const __nv_bfloat16 *Tp = nullptr;  // data planes (own or the caller's)
+    __nv_bfloat16 *Town = nullptr, *Yp = nullptr;
+    unsigned long long *bits = nullptr;  // 0, 1: T; 2, 3: Y; 4 ..: columns of T, then ones
+    OzScale *sc = nullptr;
+    uint64_t *tab = nullptr;
+    int64_t *h = nullptr, *acc = nullptr;
+    size_t ldm = 0;
+    OzPoint *pt = nullptr;
+    int64_t *thr = nullptr;  // acc below it: the reference's R is 0
+    int acc_whole = 0;  // acc holds all points of the centres in Yp
+    int own_stats = 0;  // Yp, h and pt are those of the last oze_estep
+    // responsibility pass
+    int Wp = 0, Kp128 = 0, Npk = 0, rt_tiles = 0, rt_per = 0;
+    __nv_bfloat16 *Tt = nullptr, *Rp = nullptr;
+    int64_t *part = nullptr;
+    int *nmin = nullptr;
+};
+
+// The digit-slice path has fixed costs (planes of the centres, four launches a
+// chunk, tiles of 128 x 64): below this the CUDA-core kernels are as fast.
+bool oze_wanted(int N, int D, int K)
+{
+    return D <= 4 * PANEL && K <= (1 << 20) && (double) N * K >= 2e6 && N >= 256;
+}
+
+void oze_destroy(OzE *st)
+{
+    if (!st)
+        return;
+    void *ptrs[] = {st->Town, st->Yp, st->bits, st->sc, st->tab, st->h, st->acc, st->pt, st->thr,
+                    st->Tt, st->Rp, st->part, st->nmin};
+    for (void *p : ptrs)
+        if (p)
+            cudaFree(p);
+    delete st;
+}
+
+// the table of exp2_neg, filled once in the process (4096 long-double powers)
+static const uint64_t *host_table()
+{
+    struct Table {
+        uint64_t v[oz::TAB];
+        Table() { oz::fill_table(v); }
+    };
+    static const Table t;
+    return t.v;
+}
+
+int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
+{
+    *out = nullptr;
+    OzE *st = new (std::nothrow) OzE();
+    if (!st) {
+        set_error(DGTM_ENOMEM, "host allocation failed");
+        return DGTM_ENOMEM;
+    }
+    st->a = a;
+    const int N = a.N, D = a.D, K = a.K;
+    st->sa = a.Tb ? 1 : 8;
+    st->Dp = a.Tb ? a.Tb_ld : rup(D, PANEL);
+    st->panels = st->Dp / PANEL;
+    st->Np = a.Tb ? a.Tb_rows : rup(N, 128);
+    st->Kp = rup(K, 64);
+    long long c = CHUNK / K / 128 * 128;
+    c = c < 128 ? 128 : c > st->Np ? st->Np : c;
+    st->chunk = (int) c;
+    st->nchunks = ceil_div(N, st->chunk);
+    st->ldm = (size_t) st->chunk;
+    st->Wp = rup(D + 1, 64);
+    st->Kp128 = rup(K, 128);
+    st->Npk = rup(N, PANEL);
+    const size_t planes = sizeof(__nv_bfloat16) * oz::DIGITS;
+    cudaError_t e = cudaSuccess;
+    auto get = [&](void *pp, size_t bytes) {
+        if (e == cudaSuccess)
+            e = cudaMalloc((void **) pp, bytes);
+    };
+    if (!a.Tb)
+        get(&st->Town, planes * st->Np * st->Dp);
+    get(&st->Yp, planes * st->Kp * st->Dp);
+    get(&st->bits, sizeof(unsigned long long) * (4 + D + 1));
+    get(&st->sc, sizeof(OzScale));
+    get(&st->tab, TAB_BYTES);
+    get(&st->h, sizeof(int64_t) * K);
+    get(&st->acc, sizeof(int64_t) * st->ldm * K);
+    get(&st->pt, sizeof(OzPoint) * N);
+    if (a.mstep)
+        get(&st->thr, sizeof(int64_t) * N);
+    if (a.mstep) {
+        const int cp = rup(st->chunk, PANEL) / PANEL;
+        st->rt_tiles = (st->Kp128 / 128) * (st->Wp / 64);
+        st->rt_per = oz_item_panels(st->rt_tiles, cp, a.sms);
+        get(&st->Tt, planes * st->Wp * st->Npk);
+        get(&st->Rp, planes * st->Kp128 * st->chunk);
+        get(&st->part, sizeof(int64_t) * 8192 * (size_t) st->rt_tiles * ceil_div(cp, st->rt_per));
+        get(&st->nmin, sizeof(int) * K);
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpy(st->tab, host_table(), TAB_BYTES, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(st->bits, 0, sizeof(unsigned long long) * (4 + D + 1), s);
+    if (e == cudaSuccess) {
+        oz_absmax_kernel<<<grid_of((size_t) N * D, 4864), 256, 0, s>>>(a.T64, (size_t) N * D, a.tt, N, st->bits);
+        if (!a.Tb)
+            oz_slice_rows_kernel<<<grid_of((size_t) st->Np * st->Dp / 2, 16384), 256, 0, s>>>(
+                a.T64, N, D, st->Np, st->Dp, st->bits, st->Town, nullptr, 8, nullptr, nullptr, nullptr);
+        e = cudaGetLastError();
+        st->Tp = a.Tb ? a.Tb : st->Town;
+    }
+    if (e == cudaSuccess && a.mstep) {
+        const OzSource src{nullptr, a.T64, nullptr, D, D, 0};
+        e = cudaMemsetAsync(st->Tt, 0, planes * st->Wp * st->Npk, s);
+        oz_colmax_kernel<<<dim3(ceil_div(N, 512), ceil_div(D + 1, 32)), 256, 0, s>>>(src, N, D + 1, 512,
+                                                                                    st->bits + 4);
+        oz_slice_t_kernel<<<dim3(st->Npk / PANEL, ceil_div(D + 1, 32)), 256, 0, s>>>(
+            src, N, D + 1, st->Wp, st->Npk, st->bits + 4, st->Tt);
+        if (e == cudaSuccess)
+            e = cudaGetLastError();
+    }
+    unsigned long long tb[2] = {0, 0};
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(tb, st->bits, sizeof(tb), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        const int code = e == cudaErrorMemoryAllocation ? DGTM_ENOMEM : DGTM_ECUDA;
+        cudaGetLastError();
+        set_error(code, "oze_create: %s", cudaGetErrorString(e));
+        oze_destroy(st);
+        return code;
+    }
+    if (tb[0] >= oz::INF_BITS || tb[1] >= oz::INF_BITS) {
+        oze_destroy(st);  // non-finite data: the CUDA-core kernels carry them
+        return DGTM_OK;
+    }
+    *out = st;
+    return DGTM_OK;
+}
+
+int oze_estep_blocks(const OzE *st)
+{
+    return (st->nchunks - 1) * (st->chunk / ST_PTS) +
+           ceil_div(st->a.N - (st->nchunks - 1) * st->chunk, ST_PTS);
+}
+
+namespace {
+
+// the centres' planes, grid and h
+int slice_centres(OzE *st, const double *Y, const double *yy, cudaStream_t s)
+{
+    const int K = st->a.K, D = st->a.D;
+    DGTM_CUDA_TRY(cudaMemsetAsync(st->bits + 2, 0, 2 * sizeof(unsigned long long), s));
+    oz_absmax_kernel<<<grid_of((size_t) K * D, 608), 256, 0, s>>>(Y, (size_t) K * D, yy, K, st->bits + 2);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    oz_slice_rows_kernel<<<grid_of((size_t) st->Kp * st->Dp / 2, 4864), 256, 0, s>>>(
+        Y, K, D, st->Kp, st->Dp, st->bits + 2, st->Yp, st->bits, st->sa, yy, st->sc, st->h);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    st->acc_whole = st->own_stats = 0;
+    return DGTM_OK;
+}
+
+// the integer products of chunk c
+int chunk_products(OzE *st, int c, cudaStream_t s)
+{
+    OzGemm g;
+    g.A = st->Tp;
+    g.B = st->Yp;
+    g.sa = st->sa;
+    g.a_rows = st->Np;
+    g.b_rows = st->Kp;
+    g.panels = g.a_panels = g.b_panels = st->panels;
+    const int n0 = c * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
+    g.a_tile0 = n0 / 128;
+    g.mtiles = ceil_div(nn, 128);
+    g.ntiles = st->Kp / 64;
+    g.out = st->acc;
+    g.ldm = st->ldm;
+    g.mrows = nn;
+    g.ncols = st->a.K;
+    g.shift = &st->sc->shift;
+    return launch_oz_gemm(g, st->a.sms, st->a.status, s);
+}
+
+template <typename Kernel>
+int table_smem(Kernel k)
+{
+    DGTM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) TAB_BYTES));
+    return DGTM_OK;
+}
+
+constexpr double LOG2E_2 = 2.0 * 1.4426950408889634;
+
+}  // namespace
+
+#define OZ_TRY(expr)           \
+    do {                       \
+        const int _r = (expr); \
+        if (_r != DGTM_OK)     \
+            return _r;         \
+    } while (0)
+
+int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, int isDA, double2 *colstat,
+              double *part, double dcut, int *nlaunch, cudaStream_t s)
+{
+    OZ_TRY(slice_centres(st, Y, yy, s));
+    const bool two = isDA && c1 != c2;
+    OZ_TRY(two ? table_smem(oz_stats_kernel<true>) : table_smem(oz_stats_kernel<false>));
+    for (int c = 0; c < st->nchunks; c++) {
+        OZ_TRY(chunk_products(st, c, s));
+        const int n0 = c * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
+        OzStatsArgs a{};
+        a.acc = st->acc;
+        a.ldm = st->ldm;
+        a.h = st->h;
+        a.sc = st->sc;
+        a.tab = st->tab;
+        a.tt = st->a.tt + n0;
+        a.nn = nn;
+        a.K = st->a.K;
+        a.isDA = isDA;
+        a.c1 = c1;
+        a.c2 = c2;
+        a.k1 = oz::make_mul(c1 * LOG2E_2);
+        a.k2 = oz::make_mul(c2 * LOG2E_2);
+        a.colstat = colstat + n0;
+        a.pt = st->pt + n0;
+        a.thr = st->thr + n0;
+        a.dcut = dcut;
+        a.part = part + 2 * (size_t) (n0 / ST_PTS);
+        if (two)
+            oz_stats_kernel<true><<<ceil_div(nn, ST_PTS), ST_THREADS, TAB_BYTES, s>>>(a);
+        else
+            oz_stats_kernel<false><<<ceil_div(nn, ST_PTS), ST_THREADS, TAB_BYTES, s>>>(a);
+        DGTM_CUDA_TRY(cudaGetLastError());
+    }
+    st->acc_whole = st->nchunks == 1;
+    st->own_stats = 1;
+    if (nlaunch)
+        *nlaunch = 2 + 2 * st->nchunks;
+    return DGTM_OK;
+}
+
+int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaStream_t s)
+{
+    const int K = st->a.K, D = st->a.D;
+    OZ_TRY(table_smem(oz_digits_kernel));
+    int nl = 0;
+    for (int ch = 0; ch < st->nchunks; ch++) {
+        if (!st->acc_whole) {
+            OZ_TRY(chunk_products(st, ch, s));
+            nl++;
+        }
+        const int n0 = ch * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
+        const int ldn = rup(nn, PANEL);
+        oz_digits_kernel<<<K, 256, TAB_BYTES, s>>>(st->acc, st->ldm, nn, st->h, st->sc, st->tab, st->pt + n0,
+                                                   st->thr + n0, oz::make_mul(c * LOG2E_2), st->Kp128, ldn,
+                                                   st->Rp, st->nmin);
+        DGTM_CUDA_TRY(cudaGetLastError());
+        OzGemm g;
+        g.A = st->Rp;
+        g.B = st->Tt;
+        g.a_rows = st->Kp128;
+        g.b_rows = st->Wp;
+        g.panels = g.a_panels = ldn / PANEL;
+        g.b_panels = st->Npk / PANEL;
+        g.b_panel0 = n0 / PANEL;
+        g.mtiles = st->Kp128 / 128;
+        g.ntiles = st->Wp / 64;
+        g.out64 = st->part;
+        g.item_panels = st->rt_per;
+        OZ_TRY(launch_oz_gemm(g, st->a.sms, st->a.status, s));
+        oz_rt_kernel<<<dim3(st->rt_tiles, 32), 256, 0, s>>>(st->part, g.ntiles, ceil_div(g.panels, st->rt_per),
+                                                            oz_sum_ext(g.panels), st->nmin, st->bits + 4, K, D,
+                                                            ch == 0 ? 1 : 0, G, RT);
+        DGTM_CUDA_TRY(cudaGetLastError());
+        nl += 3;
+    }
+    if (nlaunch)
+        *nlaunch = nl;
+    return DGTM_OK;
+}
+
+int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c, const double *X,
+            int L, double *M, cudaStream_t s)
+{
+    const int N = st->a.N, K = st->a.K;
+    if (!st->own_stats) {
+        OZ_TRY(slice_centres(st, Y, yy, s));
+        oz_points_kernel<<<grid_of((size_t) N, 1216), 256, 0, s>>>(colstat, st->a.tt, N, K, st->sc, st->pt);
+        DGTM_CUDA_TRY(cudaGetLastError());
+    }
+    const auto kernel = L <= 2 ? oz_map_kernel<2> : L == 3 ? oz_map_kernel<3> : oz_map_kernel<8>;
+    OZ_TRY(table_smem(kernel));
+    for (int ch = 0; ch < st->nchunks; ch++) {
+        if (!st->acc_whole)
+            OZ_TRY(chunk_products(st, ch, s));
+        const int n0 = ch * st->chunk, nn = N - n0 < st->chunk ? N - n0 : st->chunk;
+        kernel<<<ceil_div(nn, ST_PTS), ST_THREADS, TAB_BYTES, s>>>(st->acc, st->ldm, nn, st->h, st->sc, st->tab,
+                                                                   st->pt + n0, oz::make_mul(c * LOG2E_2), K,
+                                                                   X, L, M + (size_t) n0 * L);
+        DGTM_CUDA_TRY(cudaGetLastError());
+    }
+    return DGTM_OK;
+}
+
+}  // namespace dgtm

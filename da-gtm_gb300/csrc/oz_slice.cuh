@@ -1,0 +1,88 @@
+// oz_slice.cuh -- kernels that cut FP64 matrices into the digit planes of the
+// digit-slice products (oz.cu).  Bound by memory: 8 bytes in, 16 out a value.
+#pragma once
+
+#include "ozfix.cuh"
+#include "sm100.cuh"
+
+#include <cuda_bf16.h>
+
+namespace dgtm {
+namespace {
+
+using sm100::pack_bf16;
+
+__device__ __forceinline__ uint32_t bf16_pair(int a, int b) { return pack_bf16((float) a, (float) b); }
+
+// Column c of the source: c < c1: G[k] X1[k][c] (G may be null), else X2[k][c - c1]
+// (X2 null: 1).
+struct OzSource {
+    const double *G, *X1, *X2;
+    int c1, ld1, ld2;
+    __device__ __forceinline__ double at(int k, int c) const
+    {
+        if (c < c1) {
+            const double v = X1[(size_t) k * ld1 + c];
+            return G ? G[k] * v : v;
+        }
+        return X2 ? X2[(size_t) k * ld2 + (c - c1)] : 1.0;
+    }
+};
+
+// bits[c] = max(bits[c], the largest |value| of column c over the block's rows)
+static __global__ void __launch_bounds__(256) oz_colmax_kernel(OzSource src, int rows, int cols, int rows_per,
+                                                        unsigned long long *__restrict__ bits)
+{
+    __shared__ unsigned long long red[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c = blockIdx.y * 32 + lane;
+    const int k0 = blockIdx.x * rows_per, k1 = min(rows, k0 + rows_per);
+    unsigned long long m = 0ull;
+    if (c < cols)
+        for (int k = k0 + w; k < k1; k += 8) {
+            const unsigned long long b = oz::double_bits(src.at(k, c)) & oz::ABS_MASK;
+            m = b > m ? b : m;
+        }
+    red[w][lane] = m;
+    __syncthreads();
+    if (w == 0 && c < cols) {
+        for (int i = 1; i < 8; i++)
+            m = red[i][lane] > m ? red[i][lane] : m;
+        atomicMax(&bits[c], m);
+    }
+}
+
+// planes[i][c][k] = digit i of column c of the source on the column's grid:
+// the transposed operand (contraction over the source's rows), zero past rows
+// and cols.  Block: 64 rows x 32 columns.
+static __global__ void __launch_bounds__(256) oz_slice_t_kernel(OzSource src, int rows, int cols, int prows,
+                                                         int ld, const unsigned long long *__restrict__ bits,
+                                                         __nv_bfloat16 *__restrict__ planes)
+{
+    __shared__ int64_t qs[32][65];
+    const int k0 = blockIdx.x * 64, c0 = blockIdx.y * 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c = c0 + lane;
+    const int e = c < cols ? oz::exponent_of(bits[c]) : 0;
+#pragma unroll
+    for (int r = w; r < 64; r += 8) {
+        const int k = k0 + r;
+        qs[lane][r] = (k < rows && c < cols) ? oz::to_fixed(src.at(k, c), e) : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int cc = w; cc < 32; cc += 8) {
+        int64_t a = qs[cc][2 * lane], b = qs[cc][2 * lane + 1];
+        uint32_t *dst = (uint32_t *) (planes + (size_t) (c0 + cc) * ld + k0) + lane;
+        const size_t plane = (size_t) prows * ld / 2;
+#pragma unroll
+        for (int i = oz::DIGITS - 1; i > 0; i--) {
+            const int da = oz::next_digit(a), db = oz::next_digit(b);
+            dst[(size_t) i * plane] = bf16_pair(da, db);
+        }
+        dst[0] = bf16_pair((int) a, (int) b);
+    }
+}
+
+}  // namespace
+}  // namespace dgtm

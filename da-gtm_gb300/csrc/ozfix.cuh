@@ -127,25 +127,36 @@ struct Mul {
     int a, b;
 };
 
-// kappa: the exponent (base 2) of one unit of x; the product is kept below 2000
-inline Mul make_mul(double kappa)
+// kappa = k0 2^u with k0 known on the host and u (the unit of x) on the device
+struct MulBase {
+    uint64_t m;   // k0 = m 2^(ex - 64), m's top bit set
+    uint64_t l0;  // 2000 / (m 2^-64) in units of 2^-20
+    int ex;
+};
+
+static inline MulBase make_mul(double k0)
+{
+    MulBase r;
+    int ex = 0;
+    const double f = frexp(k0, &ex);  // k0 = f 2^ex, f in [0.5, 1)
+    r.m = (uint64_t) ldexp(f, 64);
+    r.l0 = (uint64_t) (2000.0 / f * 1048576.0);
+    r.ex = ex;
+    return r;
+}
+
+OZ_HD Mul mul_at(const MulBase &k, int u)
 {
     Mul r;
-    int ex = 0;
-    const double f = frexp(kappa, &ex);  // kappa = f 2^ex, f in [0.5, 1)
-    r.m = (uint64_t) ldexp(f, 64);
-    if (f >= 1.0)
-        r.m = ~0ull;
-    // x kappa 2^53 = x m 2^(ex + 53 - 64) = mulhi(x << a, m) >> b
-    const int sh = ex + WFRAC;  // a - b
+    r.m = k.m;
+    // x kappa 2^53 = x m 2^(ex + u + 53 - 64) = mulhi(x << a, m) >> b
+    const int sh = k.ex + u + WFRAC;  // a - b
     r.a = sh > 0 ? (sh < 63 ? sh : 63) : 0;
-    r.b = sh < 0 ? (-sh < 63 ? -sh : 63) : 0;
-    const double l = 2000.0 / kappa;
-    const double cap = ldexp(1.0, 63 - r.a);  // x << a below 2^63
-    const double t = l < cap ? l : cap;
-    r.lim = t < 9.0e18 ? (uint64_t) t : 9000000000000000000ull;
-    if (sh > 63)
-        r.lim = 0;
+    r.b = sh < 0 ? (sh > -63 ? -sh : 63) : 0;
+    const uint64_t cap = (1ull << (63 - r.a)) - 1;  // x << a below 2^63
+    const int ls = -(k.ex + u) - 20;                // lim = l0 2^ls, l0 < 2^32
+    uint64_t l = ls >= 31 ? ~0ull >> 1 : ls >= 0 ? k.l0 << ls : ls > -64 ? k.l0 >> -ls : 0ull;
+    r.lim = sh > 63 ? 0ull : (l < cap ? l : cap);
     return r;
 }
 
@@ -186,7 +197,7 @@ OZ_HD double to_double(uint64_t E, int n)
 OZ_HD uint64_t to_wfix(double v) { return (uint64_t) scaled_int(v, WFRAC); }
 
 // table entry: 2^-(i / 4096) in units of 2^-63
-inline void fill_table(uint64_t *tab)
+static inline void fill_table(uint64_t *tab)
 {
     for (int i = 0; i < TAB; i++)
         tab[i] = (uint64_t) (exp2l(-(long double) i / TAB) * 9223372036854775808.0L + 0.5L);

@@ -21,6 +21,8 @@ struct XState;
 // CUDA-core FP64 form.
 int x64_create(XState **out, int N, int D, int K, int sms, const double *T64, cudaStream_t s);
 void x64_destroy(XState *st);
+// the 0/1 data in BF16 (Npad x Dp, ones in the padding columns)
+const void *x64_data(const XState *st, int *Npad, int *Dp);
 // E-step: the digit slices of Y64, then pass 1: column statistics (d_ref,
 // log s_n) as the CUDA-core FP64 pass writes them, and two partial sums per
 // CTA of the quality terms into part (x64_pass1_blocks pairs).

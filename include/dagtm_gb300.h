@@ -206,8 +206,9 @@ int dgtm_get_stream(dgtm_ctx *ctx, void **stream);
  * (D <= 189, K <= 60000) on an sm_10x GPU use the exact-slice path: distance
  * products from fixed-point digit slices of the centres on the tensor cores
  * (exact integers), exponentials and sums in double-float and 2^-48 fixed
- * point.  Setting DGTM_X64=0 before dgtm_ctx_create keeps them on the
- * CUDA-core FP64 kernels. */
+ * point.  On other data they use digit slices of both operands and fixed-point
+ * exponentials when N K is at least 2e6 (N >= 256, D <= 256).  Setting
+ * DGTM_X64=0 before dgtm_ctx_create keeps them on the CUDA-core FP64 kernels. */
 #define DGTM_PATH_CUDA_CORES 0
 #define DGTM_PATH_SPLIT_BF16 1
 #define DGTM_PATH_EXACT_SLICES 2

@@ -66,16 +66,21 @@ int main()
     }
     // products
     long double worstm = 0;
-    const double ks[] = {0x1.8p-53, 0x1.234p-40, 3e-20, 0x1.fp-58};
-    for (double k : ks) {
-        const Mul m = make_mul(k);
-        for (int it = 0; it < 100000; it++) {
-            uint64_t x = (uint64_t) (fabs(u(g)) * (double) m.lim);
-            const long double ref = (long double) x * (long double) k * 0x1p53L;
-            const long double err = fabsl((long double) mul_w(m, x) - ref);
-            worstm = fmaxl(worstm, err / fmaxl(1.0L, ref * 0x1p-52L));
+    const double ks[] = {1.5, 0x1.234p3, 3e-4, 0x1.fp-8, 900.0};
+    for (double k : ks)
+        for (int e = -60; e <= 0; e += 3) {
+            const Mul m = mul_at(make_mul(k), e);
+            for (int it = 0; it < 20000; it++) {
+                uint64_t x = (uint64_t) (fabs(u(g)) * (double) m.lim);
+                if (x > m.lim)
+                    x = m.lim;
+                const long double ref = (long double) x * (long double) k * ldexpl(1.0L, e + 53);
+                const long double err = fabsl((long double) mul_w(m, x) - ref);
+                if (ref > 2001.0L * 0x1p53L)
+                    bad += 1;
+                worstm = fmaxl(worstm, err);
+            }
         }
-    }
     printf("%.0f %.3Le %.3Le %.3Le\n", bad, worst, worstd, worstm);
     return 0;
 }

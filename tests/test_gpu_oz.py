@@ -1,0 +1,109 @@
+"""The digit-slice E-step, responsibility pass and map (real-valued data of the
+FP64 form, and the map of every form) against the oracle, at the sizes where
+tiles, panels and chunks are only partly filled.  The FP64 form's stated bounds
+apply: 1e-12 relative on the qualities, G, RT and the map, 1e-13 on R."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    a, b = np.asarray(a, float), np.asarray(b, float)
+    return float(np.max(np.abs(a - b)) / max(np.max(np.abs(b)), 1e-300))
+
+
+def problem(N, D, K, seed, scale=None, binary=False):
+    rng = np.random.default_rng(seed)
+    T = (rng.random((N, D)) < 0.4).astype(float) if binary else rng.normal(size=(N, D))
+    Y = rng.normal(size=(K, D)) * 0.7
+    if scale is not None:
+        s = np.logspace(-scale, scale, D)
+        T, Y = T * s, Y * s
+    FI = np.concatenate([rng.random((K, 3)), np.ones((K, 1))], axis=1)
+    return T, Y, FI, rng.normal(size=(K, 3))
+
+
+def oracle(orc, T, Y, beta, isDA, temp):
+    R, vgc, vgc2 = orc.resp(orc.dist(Y, T), beta, isDA, temp)
+    N, D = T.shape
+    K = Y.shape[0]
+    llh = orc.qual(N, K, D, beta, vgc, 0, temp)
+    return R, llh, orc.qual(N, K, D, beta, vgc2, 1, temp) if isDA else -llh
+
+
+# one panel and four, one dimension, ragged N and K, one chunk and several
+# (chunks hold 8 M pairs, 128 points at least), both temperatures, plain EM
+@pytest.mark.parametrize("N,D,K,isDA,temp,scale", [
+    (256, 1, 8000, 1, 1.5, None), (4001, 3, 517, 1, 1.0, None), (2050, 64, 1001, 1, 2.0, None),
+    (2177, 65, 8000, 1, 1.3, None), (1000, 130, 2049, 0, 1.0, None), (700, 200, 3000, 1, 3.0, None),
+    (513, 256, 4097, 1, 2.0, None), (3000, 12, 700, 1, 1.2, 2.0), (90001, 7, 130, 1, 2.0, None)])
+def test_em_step_and_map(pkg, orc, N, D, K, isDA, temp, scale):
+    T, Y, FI, X = problem(N, D, K, N + D, scale)
+    beta = 2.0 / max(1.0, np.mean(np.sum(T * T, axis=1)) / 8)
+    with pkg.Context(T, FI, "fp64") as c:
+        assert c.path == "exact_slices"
+        c.set_Y(Y)
+        llh, nfree = c.estep(beta, isDA, temp)
+        M = c.map(X)
+        Rb = c.R_block(0, 17, 0, N)
+        c.mstep()
+        G, RT = c.get_stats()
+    R, ollh, onfree = oracle(orc, T, Y, beta, isDA, temp)
+    assert llh == pytest.approx(ollh, rel=1e-12)
+    assert nfree == pytest.approx(onfree, rel=1e-12)
+    assert np.max(np.abs(Rb - R[:17])) <= 1e-13
+    assert rel(G, R.sum(1)) <= 1e-12
+    assert rel(RT, R @ T) <= 1e-12
+    assert rel(M, R.T @ X) <= 1e-12
+
+
+def test_far_centre_keeps_its_statistics(pkg, orc):
+    """A centre whose largest responsibility is far below 2^-56 keeps G and RT to
+    the form's relative accuracy (its own power-of-two grid)."""
+    T, Y, FI, X = problem(3000, 5, 700, 1)
+    Y[3] = 8.0
+    beta, temp = 1.0, 1.1
+    R, _, _ = oracle(orc, T, Y, beta, 1, temp)
+    assert 0 < R[3].max() < 1e-20
+    with pkg.Context(T, FI, "fp64") as c:
+        c.set_Y(Y)
+        c.estep(beta, 1, temp)
+        c.mstep()
+        G, RT = c.get_stats()
+    assert G[3] == pytest.approx(R[3].sum(), rel=1e-10)
+    assert rel(RT[3], R[3] @ T) <= 1e-10
+
+
+def test_zero_column_and_nonfinite_centre(pkg, orc):
+    T, Y, FI, X = problem(3000, 4, 700, 2)
+    T[5] = 500.0  # exp(-beta d / 2) underflows for every centre
+    with pkg.Context(T, FI, "fp64") as c:
+        c.set_Y(Y)
+        llh, nfree = c.estep(4.0, 1, 1.5)
+        assert llh == -np.inf and np.isfinite(nfree)
+        assert np.max(np.abs(c.R_block(0, 20, 5, 1) - 1 / 700)) <= 1e-15
+        M = c.map(X)
+        assert np.max(np.abs(M[5] - X.mean(0))) <= 1e-12
+        Y[7, 2] = np.nan
+        c.set_Y(Y)
+        llh, nfree = c.estep(4.0, 1, 1.5)
+        assert np.isnan(llh) and np.isnan(nfree)
+
+
+@pytest.mark.parametrize("form,binary,D", [("bf16x3", True, 166), ("bf16x3", False, 64), ("fp32", False, 31),
+                                           ("fp64", True, 100), ("fp32", True, 200)])
+def test_map_matches_cuda_cores(pkg, monkeypatch, form, binary, D):
+    """The map of every form against the CUDA-core map kernel on the same column
+    statistics."""
+    T, Y, FI, X = problem(2100, D, 1050, D, binary=binary)
+    Y = 0.4 + 0.2 * Y if binary else Y
+    out = []
+    for on in ("1", "0"):
+        monkeypatch.setenv("DGTM_X64", on if form != "fp64" else "1")
+        with pkg.Context(T, FI, form) as c:
+            c.set_Y(Y)
+            c.estep(1.5, 1, 1.2)
+            monkeypatch.setenv("DGTM_X64", on)
+            out.append(c.map(X))
+    assert rel(out[0], out[1]) <= 1e-12
