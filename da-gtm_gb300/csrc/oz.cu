@@ -45,7 +45,8 @@ using namespace sm100;
 
 namespace {
 
-constexpr int OZ_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 drain
+constexpr int DRAIN_WARPS = 16;
+constexpr int OZ_THREADS = 64 + 32 * DRAIN_WARPS;  // warp 0 TMA, warp 1 MMA, then the drain
 constexpr int TM = 128, TN = 64; // tile
 constexpr int PANEL = 64;
 constexpr int SB = oz::DIGITS;   // planes of B, levels
@@ -83,19 +84,30 @@ __device__ __forceinline__ void oz_item(const OzParams &p, int it, int &mt, int 
     p1 = min(p.panels, p0 + p.item_panels);
 }
 
-// the levels of one element as hi 2^28 + lo: the four pairs are exact in 32 bits
-__device__ __forceinline__ void level_pairs(const uint32_t *v, int c, int64_t &hi, int64_t &lo)
+// One element's levels v[0], v[4], .., v[28] as hi 2^28 + lo; the four pairs of
+// levels are exact in 32 bits.  NARROW: every |S_l| is at most 2^22, so
+// 1.5 2^23 + S_l has the integer in its low bits; a conversion instruction runs
+// at an eighth of the adder's rate.
+template <bool NARROW>
+__device__ __forceinline__ void level_pairs(const uint32_t *v, int64_t &hi, int64_t &lo)
 {
     int q[4];
 #pragma unroll
-    for (int h = 0; h < 4; h++)
-        q[h] = __float2int_rz(__uint_as_float(v[16 * h + c])) * 128 +
-               __float2int_rz(__uint_as_float(v[16 * h + 8 + c]));
+    for (int h = 0; h < 4; h++) {
+        const float a = __uint_as_float(v[8 * h]), b = __uint_as_float(v[8 * h + 4]);
+        if (NARROW) {
+            const uint32_t x = __float_as_uint(__fadd_rn(a, 12582912.f));
+            const uint32_t y = __float_as_uint(__fadd_rn(b, 12582912.f));
+            q[h] = (int) (x * 128u + (y - 0x4B400000u * 129u));
+        } else {
+            q[h] = __float2int_rz(a) * 128 + __float2int_rz(b);
+        }
+    }
     hi = (int64_t) q[0] * 16384 + q[1];
     lo = (int64_t) q[2] * 16384 + q[3];
 }
 
-template <int SA, bool SUM>
+template <int SA, bool SUM, bool NARROW>
 __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                const __grid_constant__ CUtensorMap tmB,
                                                                const OzParams p)
@@ -121,7 +133,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
             mbar_init(&b_empty[i], 1);
         }
         mbar_init(acc_full, 1);
-        mbar_init(acc_empty, 256);
+        mbar_init(acc_empty, 32 * DRAIN_WARPS);
         mbar_init(drain, 1);
         fence_barrier_init();
     }
@@ -233,8 +245,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
             failed = 1;
     } else if (warp >= 2) {
         // ---------------- drain: levels to 64-bit integers ----------------
-        const int q = warp & 3, h = (warp - 2) >> 2;  // lane quarter, half of the columns
-        const uint32_t lane_base = tmem + ((uint32_t) (q * 32) << 16) + (uint32_t) (32 * h);
+        const int q = warp & 3, h = (warp - 2) >> 2;  // lane quarter, 16 of the columns
+        const uint32_t lane_base = tmem + ((uint32_t) (q * 32) << 16) + (uint32_t) (16 * h);
         const int row = q * 32 + lane;
         const int shift = SUM ? 8 + p.ext : (p.shift ? *p.shift : 0);
         const int64_t half = SUM ? (1ll << (shift - 1)) : 0;
@@ -243,10 +255,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
         for (int it = blockIdx.x; ok && it < p.nitems; it += gridDim.x) {
             int mt, nt, p0, p1;
             oz_item(p, it, mt, nt, p0, p1);
-            int64_t acc[SUM ? 32 : 1];
+            int64_t acc[SUM ? 16 : 1];
             if constexpr (SUM) {
 #pragma unroll
-                for (int c = 0; c < 32; c++)
+                for (int c = 0; c < 16; c++)
                     acc[c] = 0;
             }
             for (int pn = p0; pn < p1; pn += SEG, nseg++) {
@@ -258,23 +270,23 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
                 tc_fence_after();
 #pragma unroll
                 for (int cb = 0; cb < 4; cb++) {
-                    uint32_t v[64];
+                    uint32_t v[4 * SB];
 #pragma unroll
                     for (int l = 0; l < SB; l++)
-                        tmem_ld8p(lane_base + (uint32_t) (l * TN + 8 * cb), v + 8 * l);
+                        tmem_ld4p(lane_base + (uint32_t) (l * TN + 4 * cb), v + 4 * l);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int c = 0; c < 8; c++) {
+                    for (int c = 0; c < 4; c++) {
                         int64_t hi, lo;
-                        level_pairs(v, c, hi, lo);
+                        level_pairs<NARROW>(v + c, hi, lo);
                         if constexpr (SUM) {
                             // hi 2^28 + lo may need 72 bits: both are shifted down by >= 8
-                            acc[8 * cb + c] += hi * (1 << (28 - shift)) + ((lo + half) >> shift);
+                            acc[4 * cb + c] += hi * (1 << (28 - shift)) + ((lo + half) >> shift);
                         } else {
                             // units 2^-61 (sa = 8): 8 bits down; sa = 1: exact in 2^-55
                             int64_t I = SA == 1 ? hi * 268435456 + lo : hi * 1048576 + ((lo + 128) >> 8);
                             I >>= shift;
-                            const int n = nt * TN + 32 * h + 8 * cb + c, m = mt * TM + row;
+                            const int n = nt * TN + 16 * h + 4 * cb + c, m = mt * TM + row;
                             if (m < p.mrows && n < p.ncols)
                                 p.out[(size_t) n * p.ldm + m] = I;
                         }
@@ -285,9 +297,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
             }
             if constexpr (SUM) {
                 if (ok) {
-                    int64_t *dst = p.out64 + (size_t) it * (TM * TN) + (size_t) (32 * h) * TM + row;
+                    int64_t *dst = p.out64 + (size_t) it * (TM * TN) + (size_t) (16 * h) * TM + row;
 #pragma unroll
-                    for (int c = 0; c < 32; c++)
+                    for (int c = 0; c < 16; c++)
                         dst[(size_t) c * TM] = acc[c];
                 }
             }
@@ -371,8 +383,11 @@ int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
     p.shift = g.shift;
     p.status = status;
     using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const OzParams);
-    const Kernel k = g.out64 ? (Kernel) oz_gemm_kernel<8, true>
-                             : (g.sa == 1 ? (Kernel) oz_gemm_kernel<1, false> : (Kernel) oz_gemm_kernel<8, false>);
+    // |S_l| <= (l + 1) 64 panels 4096: at most 2^22 for two panels, and for 0/1 data
+    const Kernel k = g.out64      ? (Kernel) oz_gemm_kernel<8, true, false>
+                     : g.sa == 1  ? (Kernel) oz_gemm_kernel<1, false, true>
+                     : g.panels <= 2 ? (Kernel) oz_gemm_kernel<8, false, true>
+                                     : (Kernel) oz_gemm_kernel<8, false, false>;
     DGTM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) OZ_SMEM));
     k<<<p.nitems < sms ? p.nitems : sms, OZ_THREADS, OZ_SMEM, s>>>(tmA, tmB, p);
     DGTM_CUDA_TRY(cudaGetLastError());

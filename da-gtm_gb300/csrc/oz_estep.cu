@@ -36,11 +36,9 @@ namespace dgtm {
 namespace {
 
 constexpr int PANEL = 64;
-constexpr long long CHUNK = 8LL << 20;  // centre-point pairs a chunk
-constexpr int ST_PTS = 8;               // points of a statistics block
-constexpr int ST_THREADS = 512;
-constexpr int ST_WARPS = ST_THREADS / 32;
-constexpr int ST_KG = ST_THREADS / ST_PTS;  // centre groups of a block
+constexpr long long CHUNK = 10000000;   // centre-point pairs a chunk
+constexpr int ST_PTS = 8;               // points of a statistics or map block
+constexpr int DG_K = 4;                 // centres of a digits block
 constexpr int64_t ZERO_COLUMN = INT64_MIN;  // aref of a point whose R is 1/K
 constexpr size_t TAB_BYTES = sizeof(uint64_t) * oz::TAB;
 
@@ -122,13 +120,11 @@ __global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__rest
             a = d < D ? oz::to_fixed(x[d], e) : 0;
             b = d + 1 < D ? oz::to_fixed(x[d + 1], e) : 0;
         }
-        uint32_t *dst = (uint32_t *) planes + i;
+        uint32_t *dst = (uint32_t *) planes + i, w[oz::DIGITS];
+        digit_pairs(a, b, w);
 #pragma unroll
-        for (int p = oz::DIGITS - 1; p > 0; p--) {
-            const int da = oz::next_digit(a), db = oz::next_digit(b);
-            dst[(size_t) p * n2] = bf16_pair(da, db);
-        }
-        dst[0] = bf16_pair((int) a, (int) b);
+        for (int p = 0; p < oz::DIGITS; p++)
+            dst[(size_t) p * n2] = w[p];
     }
 }
 
@@ -160,12 +156,26 @@ struct OzStatsArgs {
     double *part;          // 2 per block
 };
 
-// Column statistics of a chunk.  Block: 8 points x 64 centre groups (a warp
-// reads four 64-byte rows at once); the maximum first, then the sums against it.
-// Bound by the integer pipe: about 75 instructions an exponential.
-template <bool TWO>
-__global__ void __launch_bounds__(ST_THREADS) oz_stats_kernel(const OzStatsArgs a)
+// (hi, lo) += 2^-(x kappa) in units of 2^-63
+__device__ __forceinline__ void add_power(uint64_t x, const oz::Mul &k, const uint64_t *tab, uint64_t &lo,
+                                          uint32_t &hi)
 {
+    const uint64_t W = oz::mul_w(k, x <= k.lim ? x : k.lim);  // lim is 2000 bits down (or 0)
+    const int n = (int) (W >> oz::WFRAC);
+    if (n < 64 && x <= k.lim) {
+        const uint64_t t = oz::exp2_neg(W, tab) >> n;
+        lo += t;
+        hi += lo < t;
+    }
+}
+
+// Column statistics of a chunk.  Block: 8 points x 64 or 128 centre groups (a
+// warp reads four 64-byte rows at once); the maximum first, then the sums against it.
+// Bound by the integer pipe: about 75 instructions an exponential.
+template <int NT, bool TWO>
+__global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
+{
+    constexpr int ST_WARPS = NT / 32, ST_KG = NT / ST_PTS;  // warps, centre groups
     extern __shared__ uint64_t tab[];
     __shared__ int64_t smax[ST_WARPS][ST_PTS];
     __shared__ uint64_t slo[2][ST_WARPS][ST_PTS];
@@ -177,10 +187,16 @@ __global__ void __launch_bounds__(ST_THREADS) oz_stats_kernel(const OzStatsArgs 
     const int64_t *acc = a.acc + (live ? p : 0);
     load_table(tab, a.tab);
     int64_t m = INT64_MIN;
-#pragma unroll 4
-    for (int k = kg; k < a.K; k += ST_KG) {
-        const int64_t v = acc[(size_t) k * a.ldm] - a.h[k];
-        m = v > m ? v : m;
+    for (int k0 = kg; k0 < a.K; k0 += 8 * ST_KG) {
+        int64_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int k = min(k0 + j * ST_KG, a.K - 1);  // a repeated centre changes no maximum
+            v[j] = acc[(size_t) k * a.ldm] - a.h[k];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            m = v[j] > m ? v[j] : m;
     }
 #pragma unroll
     for (int o = ST_PTS; o < 32; o <<= 1) {
@@ -198,22 +214,20 @@ __global__ void __launch_bounds__(ST_THREADS) oz_stats_kernel(const OzStatsArgs 
     const oz::Mul k1 = oz::mul_at(a.k1, u), k2 = oz::mul_at(a.k2, u);
     uint64_t lo1 = 0, lo2 = 0;
     uint32_t hi1 = 0, hi2 = 0;
-#pragma unroll 2
-    for (int k = kg; k < a.K; k += ST_KG) {
-        const uint64_t x = (uint64_t) (m - (acc[(size_t) k * a.ldm] - a.h[k]));
-        if (x <= k1.lim) {
-            const uint64_t W = oz::mul_w(k1, x);
-            const int n = (int) (W >> oz::WFRAC);
-            const uint64_t t = n < 64 ? oz::exp2_neg(W, tab) >> n : 0ull;
-            lo1 += t;
-            hi1 += lo1 < t;
+    for (int k0 = kg; k0 < a.K; k0 += 4 * ST_KG) {
+        uint64_t x[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int k = min(k0 + j * ST_KG, a.K - 1);
+            x[j] = (uint64_t) (m - (acc[(size_t) k * a.ldm] - a.h[k]));
+            if (k0 + j * ST_KG >= a.K)
+                x[j] = ~0ull;
         }
-        if (TWO && x <= k2.lim) {
-            const uint64_t W = oz::mul_w(k2, x);
-            const int n = (int) (W >> oz::WFRAC);
-            const uint64_t t = n < 64 ? oz::exp2_neg(W, tab) >> n : 0ull;
-            lo2 += t;
-            hi2 += lo2 < t;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            add_power(x[j], k1, tab, lo1, hi1);
+            if (TWO)
+                add_power(x[j], k2, tab, lo2, hi2);
         }
     }
 #pragma unroll
@@ -322,67 +336,105 @@ __device__ __forceinline__ uint64_t r_exponent(const OzPoint &o, int64_t v, cons
 }
 
 // Responsibilities of a chunk as digit planes, planes[i][k][n] (n fastest), each
-// centre on the grid of its largest R in the chunk; nmin[k] is that R's integer
-// exponent.  Zero past nn up to ldn.  One block per centre; the exponents are
-// formed twice, which is cheaper than keeping them.
+// centre on the grid of its largest R in the chunk; nmin[k] is an integer bound of
+// that R's exponent.  Zero past nn up to ldn.  A block takes DG_K centres, so that
+// a point's constants are read once for all of them.  The first loop finds the
+// grids from the exponents in FP32 (a margin of 2^-6 and 2^-10 of the exponent
+// taken): one conversion and one FMA a pair instead of a 64-bit product.
 __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn,
-                                                        const int64_t *__restrict__ h,
+                                                        int K, const int64_t *__restrict__ h,
                                                         const OzScale *__restrict__ sc,
                                                         const uint64_t *__restrict__ gtab,
                                                         const OzPoint *__restrict__ pt,
-                                                        const int64_t *__restrict__ thr, oz::MulBase kb, int prows, int ldn,
-                                                        __nv_bfloat16 *__restrict__ planes,
+                                                        const int64_t *__restrict__ thr, oz::MulBase kb,
+                                                        int prows, int ldn, __nv_bfloat16 *__restrict__ planes,
                                                         int *__restrict__ nmin_out)
 {
     extern __shared__ uint64_t tab[];
-    __shared__ int red[8];
-    const int k = blockIdx.x;
-    const oz::Mul km = oz::mul_at(kb, sc->u);
-    const int64_t hk = h[k];
-    const int64_t *row = acc + (size_t) k * ldm;
-    load_table(tab, gtab);
-    int nmin = 1 << 20;
-    for (int n = threadIdx.x; n < nn; n += 256) {
-        const int64_t v = row[n] - hk;
-        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, km);
-        const int e = (int) (W >> oz::WFRAC);
-        if (e < 2047)
-            nmin = e < nmin ? e : nmin;
-    }
-    nmin = __reduce_min_sync(0xffffffffu, nmin);
-    if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = nmin;
-    __syncthreads();
-    nmin = red[0];
+    __shared__ float red[8][DG_K];
+    const int k0 = blockIdx.x * DG_K;
+    const int u = sc->u;
+    const oz::Mul km = oz::mul_at(kb, u);
+    const float kf = scalbnf((float) (kb.m >> 40), kb.ex - 24 + u);  // exponent of one unit
+    int64_t hk[DG_K];
+    const int64_t *row[DG_K];
 #pragma unroll
-    for (int i = 1; i < 8; i++)
-        nmin = red[i] < nmin ? red[i] : nmin;
-    if (threadIdx.x == 0)
-        nmin_out[k] = nmin;
+    for (int i = 0; i < DG_K; i++) {
+        const int k = min(k0 + i, K - 1);
+        hk[i] = h[k];
+        row[i] = acc + (size_t) k * ldm;
+    }
+    load_table(tab, gtab);
+    float wmin[DG_K];
+#pragma unroll
+    for (int i = 0; i < DG_K; i++)
+        wmin[i] = 4096.f;
+    for (int n = threadIdx.x; n < nn; n += 256) {
+        const OzPoint o = pt[n];
+        const int64_t t = thr[n];
+        const float lf = (float) (uint32_t) (o.lam >> 32) * 0x1p-21f;  // 53 - 32 bits of fraction
+#pragma unroll
+        for (int i = 0; i < DG_K; i++) {
+            const int64_t v = row[i][n] - hk[i];
+            const float w = o.aref == ZERO_COLUMN ? lf : fmaf(__ll2float_rn(o.aref - v), kf, lf);
+            wmin[i] = fminf(wmin[i], v < t ? 4096.f : w);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < DG_K; i++) {
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+            wmin[i] = fminf(wmin[i], __shfl_xor_sync(0xffffffffu, wmin[i], s));
+        if ((threadIdx.x & 31) == 0)
+            red[threadIdx.x >> 5][i] = wmin[i];
+    }
+    __syncthreads();
+    int nmin[DG_K];
+#pragma unroll
+    for (int i = 0; i < DG_K; i++) {
+        float w = red[0][i];
+#pragma unroll
+        for (int j = 1; j < 8; j++)
+            w = fminf(w, red[j][i]);
+        // the integer part of a W at most 2^-6 + 2^-10 w below w
+        w = floorf(w - 0.015625f - w * 0.0009765625f);
+        nmin[i] = w < 0.f ? 0 : (int) w;
+        if (threadIdx.x == 0 && k0 + i < K)
+            nmin_out[k0 + i] = nmin[i];
+    }
     const size_t plane = (size_t) prows * ldn / 2;
-    uint32_t *dst = (uint32_t *) planes + (size_t) k * ldn / 2;
     for (int j = threadIdx.x; j < ldn / 2; j += 256) {
-        int64_t q[2];
+        OzPoint o[2];
+        int64_t t[2];
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-            const int n = 2 * j + e;
-            q[e] = 0;
-            if (n < nn) {
-                const int64_t v = row[n] - hk;
-                const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, km);
+            const int n = min(2 * j + e, nn - 1);
+            o[e] = pt[n];
+            t[e] = 2 * j + e < nn ? thr[n] : INT64_MAX;  // padding: R = 0
+        }
+#pragma unroll
+        for (int i = 0; i < DG_K; i++) {
+            if (k0 + i >= K)
+                break;
+            int64_t q[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int64_t v = row[i][min(2 * j + e, nn - 1)] - hk[i];
+                const uint64_t W = v < t[e] ? ~0ull : r_exponent(o[e], v, km);
                 const int ex = (int) (W >> oz::WFRAC);
                 // R 2^(55 - (5 - nmin)) = E >> (9 + ex - nmin), rounded
-                const int sh = 9 + ex - nmin;
+                const int sh = 9 + ex - nmin[i];
+                q[e] = 0;
                 if (ex < 2047 && sh < 64)
                     q[e] = (int64_t) ((oz::exp2_neg(W, tab) + (1ull << (sh - 1))) >> sh);
             }
-        }
+            uint32_t *dst = (uint32_t *) planes + (size_t) (k0 + i) * ldn / 2 + j;
+            uint32_t w[oz::DIGITS];
+            digit_pairs(q[0], q[1], w);
 #pragma unroll
-        for (int i = oz::DIGITS - 1; i > 0; i--) {
-            const int da = oz::next_digit(q[0]), db = oz::next_digit(q[1]);
-            dst[(size_t) i * plane + j] = bf16_pair(da, db);
+            for (int d = 0; d < oz::DIGITS; d++)
+                dst[(size_t) d * plane] = w[d];
         }
-        dst[j] = bf16_pair((int) q[0], (int) q[1]);
     }
 }
 
@@ -409,8 +461,8 @@ __global__ void __launch_bounds__(256) oz_rt_kernel(const int64_t *__restrict__ 
 }
 
 // M = R^T X of a chunk, blocks as in oz_stats_kernel.
-template <int LMAX>
-__global__ void __launch_bounds__(ST_THREADS) oz_map_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn,
+template <int NT, int LMAX>
+__global__ void __launch_bounds__(NT) oz_map_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn,
                                                             const int64_t *__restrict__ h,
                                                             const OzScale *__restrict__ sc,
                                                             const uint64_t *__restrict__ gtab,
@@ -418,6 +470,7 @@ __global__ void __launch_bounds__(ST_THREADS) oz_map_kernel(const int64_t *__res
                                                             int K, const double *__restrict__ X, int L,
                                                             double *__restrict__ M)
 {
+    constexpr int ST_WARPS = NT / 32, ST_KG = NT / ST_PTS;
     extern __shared__ uint64_t tab[];
     __shared__ double sm[ST_WARPS][LMAX][ST_PTS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -430,15 +483,26 @@ __global__ void __launch_bounds__(ST_THREADS) oz_map_kernel(const int64_t *__res
     load_table(tab, gtab);
     __syncthreads();
     double m[LMAX] = {};
-#pragma unroll 2
-    for (int k = kg; k < K; k += ST_KG) {
-        const uint64_t W = r_exponent(o, a[(size_t) k * ldm] - h[k], km);
-        const double r = W == ~0ull ? 0.0
-                                    : oz::to_double(oz::exp2_neg(W, tab), (int) (W >> oz::WFRAC) - oz::WBIAS);
+    for (int k0 = kg; k0 < K; k0 += 4 * ST_KG) {
+        int64_t v[4];
 #pragma unroll
-        for (int l = 0; l < LMAX; l++)
-            if (l < L)
-                m[l] = fma(r, X[(size_t) k * L + l], m[l]);
+        for (int j = 0; j < 4; j++) {
+            const int k = min(k0 + j * ST_KG, K - 1);
+            v[j] = a[(size_t) k * ldm] - h[k];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int k = k0 + j * ST_KG;
+            const uint64_t W = k < K ? r_exponent(o, v[j], km) : ~0ull;
+            const int n = (int) (W >> oz::WFRAC) - oz::WBIAS;
+            if (n > 1080)  // R is 0 in FP64
+                continue;
+            const double r = oz::to_double(oz::exp2_neg(W, tab), n);
+#pragma unroll
+            for (int l = 0; l < LMAX; l++)
+                if (l < L)
+                    m[l] = fma(r, X[(size_t) k * L + l], m[l]);
+        }
     }
 #pragma unroll
     for (int l = 0; l < LMAX; l++) {
@@ -534,7 +598,17 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     st->panels = st->Dp / PANEL;
     st->Np = a.Tb ? a.Tb_rows : rup(N, 128);
     st->Kp = rup(K, 64);
-    long long c = CHUNK / K / 128 * 128;
+    // points a chunk: equal chunks near CHUNK pairs, in whole tiles of 128; with
+    // room for few of them, whole waves of statistics blocks (8 points on each SM)
+    const long long wave = (long long) ST_PTS * a.sms;
+    long long c = CHUNK / K;
+    if (c >= 2 * wave) {
+        const long long parts = (N + c / 2) / c;
+        c = parts > 1 ? rup(ceil_div(N, parts), 128) : st->Np;
+    } else if (c >= wave) {
+        c = wave;
+    }
+    c = c / 128 * 128;
     c = c < 128 ? 128 : c > st->Np ? st->Np : c;
     st->chunk = (int) c;
     st->nchunks = ceil_div(N, st->chunk);
@@ -661,6 +735,10 @@ int table_smem(Kernel k)
     return DGTM_OK;
 }
 
+// Few points a chunk (many centres): fewer than two blocks an SM, so that a block
+// of 1024 threads keeps the SM's schedulers busier than one of 512
+bool wide_blocks(int K) { return K > 4096; }
+
 constexpr double LOG2E_2 = 2.0 * 1.4426950408889634;
 
 }  // namespace
@@ -677,7 +755,10 @@ int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, 
 {
     OZ_TRY(slice_centres(st, Y, yy, s));
     const bool two = isDA && c1 != c2;
-    OZ_TRY(two ? table_smem(oz_stats_kernel<true>) : table_smem(oz_stats_kernel<false>));
+    const int nt = wide_blocks(st->a.K) ? 1024 : 512;
+    const auto kernel = nt == 512 ? (two ? oz_stats_kernel<512, true> : oz_stats_kernel<512, false>)
+                                  : (two ? oz_stats_kernel<1024, true> : oz_stats_kernel<1024, false>);
+    OZ_TRY(table_smem(kernel));
     for (int c = 0; c < st->nchunks; c++) {
         OZ_TRY(chunk_products(st, c, s));
         const int n0 = c * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
@@ -700,10 +781,7 @@ int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, 
         a.thr = st->thr + n0;
         a.dcut = dcut;
         a.part = part + 2 * (size_t) (n0 / ST_PTS);
-        if (two)
-            oz_stats_kernel<true><<<ceil_div(nn, ST_PTS), ST_THREADS, TAB_BYTES, s>>>(a);
-        else
-            oz_stats_kernel<false><<<ceil_div(nn, ST_PTS), ST_THREADS, TAB_BYTES, s>>>(a);
+        kernel<<<ceil_div(nn, ST_PTS), nt, TAB_BYTES, s>>>(a);
         DGTM_CUDA_TRY(cudaGetLastError());
     }
     st->acc_whole = st->nchunks == 1;
@@ -725,7 +803,7 @@ int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaS
         }
         const int n0 = ch * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
         const int ldn = rup(nn, PANEL);
-        oz_digits_kernel<<<K, 256, TAB_BYTES, s>>>(st->acc, st->ldm, nn, st->h, st->sc, st->tab, st->pt + n0,
+        oz_digits_kernel<<<ceil_div(K, DG_K), 256, TAB_BYTES, s>>>(st->acc, st->ldm, nn, K, st->h, st->sc, st->tab, st->pt + n0,
                                                    st->thr + n0, oz::make_mul(c * LOG2E_2), st->Kp128, ldn,
                                                    st->Rp, st->nmin);
         DGTM_CUDA_TRY(cudaGetLastError());
@@ -762,13 +840,15 @@ int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, 
         oz_points_kernel<<<grid_of((size_t) N, 1216), 256, 0, s>>>(colstat, st->a.tt, N, K, st->sc, st->pt);
         DGTM_CUDA_TRY(cudaGetLastError());
     }
-    const auto kernel = L <= 2 ? oz_map_kernel<2> : L == 3 ? oz_map_kernel<3> : oz_map_kernel<8>;
+    const int nt = wide_blocks(K) ? 1024 : 512;
+    const auto kernel = nt == 512 ? (L <= 2 ? oz_map_kernel<512, 2> : L == 3 ? oz_map_kernel<512, 3> : oz_map_kernel<512, 8>)
+                                  : (L <= 2 ? oz_map_kernel<1024, 2> : L == 3 ? oz_map_kernel<1024, 3> : oz_map_kernel<1024, 8>);
     OZ_TRY(table_smem(kernel));
     for (int ch = 0; ch < st->nchunks; ch++) {
         if (!st->acc_whole)
             OZ_TRY(chunk_products(st, ch, s));
         const int n0 = ch * st->chunk, nn = N - n0 < st->chunk ? N - n0 : st->chunk;
-        kernel<<<ceil_div(nn, ST_PTS), ST_THREADS, TAB_BYTES, s>>>(st->acc, st->ldm, nn, st->h, st->sc, st->tab,
+        kernel<<<ceil_div(nn, ST_PTS), nt, TAB_BYTES, s>>>(st->acc, st->ldm, nn, st->h, st->sc, st->tab,
                                                                    st->pt + n0, oz::make_mul(c * LOG2E_2), K,
                                                                    X, L, M + (size_t) n0 * L);
         DGTM_CUDA_TRY(cudaGetLastError());

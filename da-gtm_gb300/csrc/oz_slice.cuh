@@ -10,9 +10,19 @@
 namespace dgtm {
 namespace {
 
-using sm100::pack_bf16;
-
-__device__ __forceinline__ uint32_t bf16_pair(int a, int b) { return pack_bf16((float) a, (float) b); }
+// The digits of two values as BF16 pairs, w[i] = (digit i of a, digit i of b):
+// a field f becomes the float 2^23 + f by its bits, f - 64 by one subtraction, and
+// its upper half is the BF16, since eight bits hold it.
+__device__ __forceinline__ void digit_pairs(int64_t a, int64_t b, uint32_t (&w)[oz::DIGITS])
+{
+    const uint64_t ua = (uint64_t) a + oz::digit_bias(), ub = (uint64_t) b + oz::digit_bias();
+#pragma unroll
+    for (int i = 0; i < oz::DIGITS; i++) {
+        const float x = __fsub_rn(__uint_as_float(oz::digit_field(ua, i) | 0x4B000000u), 8388672.f);
+        const float y = __fsub_rn(__uint_as_float(oz::digit_field(ub, i) | 0x4B000000u), 8388672.f);
+        w[i] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+    }
+}
 
 // Column c of the source: c < c1: G[k] X1[k][c] (G may be null), else X2[k][c - c1]
 // (X2 null: 1).
@@ -72,15 +82,13 @@ static __global__ void __launch_bounds__(256) oz_slice_t_kernel(OzSource src, in
     __syncthreads();
 #pragma unroll
     for (int cc = w; cc < 32; cc += 8) {
-        int64_t a = qs[cc][2 * lane], b = qs[cc][2 * lane + 1];
+        uint32_t v[oz::DIGITS];
+        digit_pairs(qs[cc][2 * lane], qs[cc][2 * lane + 1], v);
         uint32_t *dst = (uint32_t *) (planes + (size_t) (c0 + cc) * ld + k0) + lane;
         const size_t plane = (size_t) prows * ld / 2;
 #pragma unroll
-        for (int i = oz::DIGITS - 1; i > 0; i--) {
-            const int da = oz::next_digit(a), db = oz::next_digit(b);
-            dst[(size_t) i * plane] = bf16_pair(da, db);
-        }
-        dst[0] = bf16_pair((int) a, (int) b);
+        for (int i = 0; i < oz::DIGITS; i++)
+            dst[(size_t) i * plane] = v[i];
     }
 }
 

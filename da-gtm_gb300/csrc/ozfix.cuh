@@ -111,13 +111,18 @@ OZ_HD int64_t scaled_int(double v, int k)
     return (b >> 63) ? -(int64_t) q : (int64_t) q;
 }
 
-// the least digit of the running value r, taken out of it; after DIGITS - 1
-// calls on r = q what is left in r is the top digit (-64 .. 64)
-OZ_HD int next_digit(int64_t &r)
+// digit i (0 the top one) of q: with 64 added to every digit the digits are the
+// 7-bit fields of an unsigned number (the top one 8 bits), so none waits for another
+OZ_HD uint64_t digit_bias()
 {
-    const int d = (int) ((r + 64) & 127) - 64;
-    r = (r - d) >> 7;
-    return d;
+    // 64 (1 + 2^7 + ... + 2^49)
+    return (64ull << 0) + (64ull << 7) + (64ull << 14) + (64ull << 21) + (64ull << 28) + (64ull << 35) +
+           (64ull << 42) + (64ull << 49);
+}
+
+OZ_HD uint32_t digit_field(uint64_t biased, int i)
+{
+    return (uint32_t) (biased >> (7 * (DIGITS - 1 - i))) & (i == 0 ? 255u : 127u);
 }
 
 // w = x kappa in units of 2^-53, for 0 <= x <= lim: (mulhi(x << a, m)) >> b

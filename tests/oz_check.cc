@@ -21,9 +21,8 @@ int main()
             bad += 1;
         int64_t r = q, back = 0;
         int d[DIGITS];
-        for (int i = DIGITS - 1; i > 0; i--)
-            d[i] = next_digit(r);
-        d[0] = (int) r;
+        for (int i = 0; i < DIGITS; i++)
+            d[i] = (int) digit_field((uint64_t) r + digit_bias(), i) - 64;
         for (int i = 0; i < DIGITS; i++) {
             if (d[i] < -64 || d[i] > 64)
                 bad += 1;
@@ -37,9 +36,8 @@ int main()
     for (double v : ext) {
         int64_t r = to_fixed(v, 0), q = r, back = 0;
         int d[DIGITS];
-        for (int i = DIGITS - 1; i > 0; i--)
-            d[i] = next_digit(r);
-        d[0] = (int) r;
+        for (int i = 0; i < DIGITS; i++)
+            d[i] = (int) digit_field((uint64_t) r + digit_bias(), i) - 64;
         for (int i = 0; i < DIGITS; i++) {
             back = back * 128 + d[i];
             if (d[i] < -64 || d[i] > 64)
