@@ -38,7 +38,7 @@ namespace {
 constexpr int PANEL = 64;
 constexpr long long CHUNK = 10000000;   // centre-point pairs a chunk
 constexpr int ST_PTS = 8;               // points of a statistics or map block
-constexpr int DG_K = 4;                 // centres of a digits block
+constexpr int DG_K = 2;                 // centres of a digits block
 constexpr int64_t ZERO_COLUMN = INT64_MIN;  // aref of a point whose R is 1/K
 constexpr size_t TAB_BYTES = sizeof(uint64_t) * oz::TAB;
 
@@ -355,7 +355,9 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
     const int k0 = blockIdx.x * DG_K;
     const int u = sc->u;
     const oz::Mul km = oz::mul_at(kb, u);
-    const float kf = scalbnf((float) (kb.m >> 40), kb.ex - 24 + u);  // exponent of one unit
+    // exponents in FP32 from x >> xs, xs such that one of its units is at most 2^-8
+    const int xs = min(max(-8 - kb.ex - u, 0), 40);
+    const float kf = scalbnf((float) (kb.m >> 40), kb.ex - 24 + u + xs);
     int64_t hk[DG_K];
     const int64_t *row[DG_K];
 #pragma unroll
@@ -376,7 +378,9 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
 #pragma unroll
         for (int i = 0; i < DG_K; i++) {
             const int64_t v = row[i][n] - hk[i];
-            const float w = o.aref == ZERO_COLUMN ? lf : fmaf(__ll2float_rn(o.aref - v), kf, lf);
+            const int64_t x = (o.aref - v) >> xs;
+            const int xi = x > 0x7FFFFFFF ? 0x7FFFFFFF : (int) x;  // x >= -(a few): d_ref is the least
+            const float w = o.aref == ZERO_COLUMN ? lf : fmaf((float) xi, kf, lf);
             wmin[i] = fminf(wmin[i], v < t ? 4096.f : w);
         }
     }
@@ -598,16 +602,11 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     st->panels = st->Dp / PANEL;
     st->Np = a.Tb ? a.Tb_rows : rup(N, 128);
     st->Kp = rup(K, 64);
-    // points a chunk: equal chunks near CHUNK pairs, in whole tiles of 128; with
-    // room for few of them, whole waves of statistics blocks (8 points on each SM)
+    // points a chunk: whole waves of statistics blocks (8 points on each SM) where
+    // that many fit, in whole tiles of 128
     const long long wave = (long long) ST_PTS * a.sms;
     long long c = CHUNK / K;
-    if (c >= 2 * wave) {
-        const long long parts = (N + c / 2) / c;
-        c = parts > 1 ? rup(ceil_div(N, parts), 128) : st->Np;
-    } else if (c >= wave) {
-        c = wave;
-    }
+    c = c >= wave ? c / wave * wave : c;
     c = c / 128 * 128;
     c = c < 128 ? 128 : c > st->Np ? st->Np : c;
     st->chunk = (int) c;

@@ -40,6 +40,14 @@ OZ_HD uint64_t mulhi(uint64_t a, uint64_t b)
 #endif
 }
 
+// mulhi(a, b) or up to two less (without the low halves' product): three 32-bit
+// multiplies instead of four and their carries
+OZ_HD uint64_t mulhi_low(uint64_t a, uint64_t b)
+{
+    const uint32_t ah = (uint32_t) (a >> 32), al = (uint32_t) a, bh = (uint32_t) (b >> 32), bl = (uint32_t) b;
+    return (uint64_t) ah * bh + (((uint64_t) ah * bl) >> 32) + (((uint64_t) al * bh) >> 32);
+}
+
 OZ_HD uint32_t mulhi32(uint32_t a, uint32_t b) { return (uint32_t) (((uint64_t) a * b) >> 32); }
 
 OZ_HD uint64_t double_bits(double v)
@@ -175,7 +183,7 @@ OZ_HD uint64_t exp2_neg(uint64_t W, const uint64_t *tab)
     const uint32_t i = (uint32_t) (W >> (WFRAC - TAB_BITS)) & (TAB - 1);
     const uint64_t T = tab[i];
     const uint64_t rho = W << (64 - (WFRAC - TAB_BITS));      // the low 41 bits on top
-    const uint64_t y = mulhi(rho, 0xB17217F7D1CF79ACull) >> TAB_BITS;  // ln 2; y in 2^-64
+    const uint64_t y = mulhi_low(rho, 0xB17217F7D1CF79ACull) >> TAB_BITS;  // ln 2; y in 2^-64
     const uint32_t yh = (uint32_t) ((y + (1ull << 19)) >> 20);         // y in 2^-44
     const uint64_t yy = (uint64_t) yh * yh;                            // y^2 in 2^-88
     const uint32_t s = (uint32_t) (yy >> 32);                          // y^2 in 2^-56
@@ -183,7 +191,7 @@ OZ_HD uint64_t exp2_neg(uint64_t W, const uint64_t *tab)
     const uint64_t y3 = ((uint64_t) s6 * yh) >> 36;                    // y^3 / 6 in 2^-64
     const uint32_t y4 = mulhi32(mulhi32(s, s), 178956971u) >> 16;      // y^4 / 24 in 2^-64
     const uint64_t x = y - (yy >> 25) + y3 - y4;
-    return T - mulhi(T, x);
+    return T - mulhi_low(T, x);
 }
 
 // E 2^-63 2^(-n) as a double, E in (2^62, 2^63]
