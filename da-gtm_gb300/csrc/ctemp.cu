@@ -221,6 +221,16 @@ size_t eig_smem_bytes(int D)
     return sizeof(F) * ((size_t) D * D + 4 * (size_t) D + 34);
 }
 
+// eig64_kernel: the matrix with an odd row stride, four vectors and the column
+// groups' partial products
+constexpr size_t EIG64_SMEM_MAX = 232448 - 128;
+
+size_t eig64_smem_bytes(int D, bool in_smem)
+{
+    const int nt = D <= EIG_SMALL_D ? 256 : 512, rw = (D + 31) & ~31;
+    return sizeof(double) * ((in_smem ? (size_t) D * (D | 1) : 0) + 4 * (size_t) D + (size_t) (nt / rw) * rw);
+}
+
 template <typename F>
 __device__ __forceinline__ F warp_sum(F a)
 {
@@ -432,19 +442,240 @@ __global__ void __launch_bounds__(EIG_THREADS) eig_kernel(const double *__restri
         out[(size_t) kl * 2 + which] = mx;
 }
 
+// The FP64 eigenvalue step: the same reduction and bisection, laid out for a pipe
+// of two FP64 operations a clock and SM, where a warp's FP64 instruction takes 16
+// clocks of the SM whatever the other warps do.  So no scalar is formed by more
+// than one warp (sums, square root and division of a column by warp 0 only), the
+// matrix-vector product gives a thread one row and a share of the columns (no
+// shuffle sums), the rank-2 update computes the lower triangle and mirrors it, and
+// the Sturm count divides by a reciprocal from an FP32 seed and two Newton steps
+// (on the matrix scaled to norm 1, where every pivot above 1e-30 is in FP32's
+// range; the pivot floor is that 1e-30).  250 blocks of D = 64: 0.61 ms, 1.38 ms
+// with every warp forming the scalars.
+constexpr double EIG_PIVMIN = 1e-30;
+
+// 1/q for 1e-30 <= |q| <= 1e30
+__device__ __forceinline__ double rcp_nr(double q)
+{
+    double r = (double) (1.0f / (float) q);
+    r = fma(r, fma(-q, r, 1.0), r);
+    return fma(r, fma(-q, r, 1.0), r);
+}
+
+// eigenvalues below x of the tridiagonal matrix (norm about 1)
+__device__ int count_below_nr(const double *dg, const double *od2, int D, double x)
+{
+    double q = dg[0] - x;
+    if (fabs(q) < EIG_PIVMIN)
+        q = -EIG_PIVMIN;
+    int c = q < 0.0;
+    for (int i = 1; i < D; i++) {
+        // far out of the spectrum q stays of the order of the norm; a huge q comes
+        // from a tiny pivot and is bounded by od2 / 1e-30
+        q = fma(-od2[i - 1], rcp_nr(q), dg[i] - x);
+        if (fabs(q) < EIG_PIVMIN)
+            q = -EIG_PIVMIN;
+        c += q < 0.0;
+    }
+    return c;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT) eig64_kernel(const double *__restrict__ S, int D, int in_smem,
+                                                   double *__restrict__ Mg, const double *__restrict__ gg,
+                                                   double lim_scale, double *__restrict__ out)
+{
+    constexpr int NW = NT / 32;
+    extern __shared__ __align__(16) unsigned char sh_raw[];
+    double *sh = reinterpret_cast<double *>(sh_raw);
+    const int LD = in_smem ? (D | 1) : D;
+    const int kl = blockIdx.x, which = blockIdx.y;
+    double *M = in_smem ? sh : Mg + ((size_t) kl * 2 + which) * D * D;
+    double *v = in_smem ? sh + (size_t) D * LD : sh;  // Householder vector
+    double *p = v + D;                                 // tau M v, then w
+    double *dg = p + D, *od = dg + D;                  // diagonal, off-diagonal (then squares)
+    double *pp = od + D;                               // partial products
+    __shared__ double s_tau;
+    __shared__ int s_skip;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double *S1 = S + (size_t) kl * 2 * D * D, *S2 = S1 + (size_t) D * D;
+    const double gk = gg[kl];
+    if (gk == 0.0) {
+        // the reference returns HUGE_VAL before any eigen work (comm/mpicomm.c:582-585)
+        if (tid == 0)
+            out[(size_t) kl * 2 + which] = 0.0;
+        return;
+    }
+    // gg < GG_MIN: the reference scales H by 1 / GG_MIN and the eigenvalues back
+    const double sc = gk < GG_MIN ? 1.0 / GG_MIN : 1.0, back = gk < GG_MIN ? GG_MIN : 1.0;
+    for (int e = tid; e < D * D; e += NT) {
+        const int i = e / D, j = e - i * D;
+        const size_t at = i <= j ? (size_t) i * D + j : (size_t) j * D + i;
+        M[i * LD + j] = (which == 0 ? 2.0 * S1[at] : 2.0 * (S1[at] - S2[at])) * sc;
+    }
+    const int rw = (D + 31) & ~31;       // row threads
+    const int ng = NT / rw;              // column groups
+    const int ri = tid % rw, rg = tid / rw;
+    __syncthreads();
+    for (int k = 0; k + 2 < D; k++) {
+        const int m = D - k - 1;
+        double *A = M + (size_t) (k + 1) * LD + (k + 1);
+        if (warp == 0) {
+            const double *x = M + (size_t) k * LD + k + 1;
+            double part = 0.0;
+            for (int i = 1 + lane; i < m; i += 32)
+                part = fma(x[i], x[i], part);
+            const double sigma = warp_sum(part), x0 = x[0];
+            double tau = 0.0, v0 = 0.0, alpha = x0;
+            if (sigma != 0.0) {
+                const double mu = sqrt(fma(x0, x0, sigma));
+                alpha = x0 <= 0.0 ? mu : -mu;
+                v0 = x0 - alpha;  // |v0| = |x0| + mu: no cancellation
+                tau = 2.0 / fma(v0, v0, sigma);
+            }
+            // already reduced, or |x| underflows: the column counts as reduced
+            const bool skip = sigma == 0.0 || !isfinite(tau);
+            for (int i = lane; i < m; i += 32)
+                v[i] = i == 0 ? v0 : x[i];
+            if (lane == 0) {
+                dg[k] = M[(size_t) k * LD + k];
+                od[k] = skip ? x0 : alpha;
+                s_tau = tau;
+                s_skip = skip;
+            }
+        }
+        __syncthreads();
+        const bool skip = s_skip;
+        if (!skip) {
+            if (rg < ng && ri < m) {
+                double a0 = 0.0, a1 = 0.0;
+                int j = rg;
+                for (; j + ng < m; j += 2 * ng) {
+                    a0 = fma(A[(size_t) j * LD + ri], v[j], a0);
+                    a1 = fma(A[(size_t) (j + ng) * LD + ri], v[j + ng], a1);
+                }
+                if (j < m)
+                    a0 = fma(A[(size_t) j * LD + ri], v[j], a0);
+                pp[rg * rw + ri] = a0 + a1;
+            }
+            __syncthreads();
+            if (warp == 0) {
+                const double tau = s_tau;
+                double part = 0.0;
+                for (int i = lane; i < m; i += 32) {
+                    double s = pp[i];
+                    for (int g = 1; g < ng; g++)
+                        s += pp[g * rw + i];
+                    s *= tau;
+                    p[i] = s;
+                    part = fma(s, v[i], part);
+                }
+                const double half_k = 0.5 * tau * warp_sum(part);
+                for (int i = lane; i < m; i += 32)
+                    p[i] = fma(-half_k, v[i], p[i]);
+            }
+            __syncthreads();
+            for (int i = warp; i < m; i += NW) {
+                double *row = A + (size_t) i * LD;
+                const double vi = v[i], wi = p[i];
+                for (int j = lane; j <= i; j += 32) {
+                    const double a = fma(-wi, v[j], fma(-vi, p[j], row[j]));
+                    row[j] = a;
+                    A[(size_t) j * LD + i] = a;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        if (D >= 2) {
+            dg[D - 2] = M[(size_t) (D - 2) * LD + (D - 2)];
+            od[D - 2] = M[(size_t) (D - 2) * LD + (D - 1)];
+        }
+        dg[D - 1] = M[(size_t) (D - 1) * LD + (D - 1)];
+    }
+    __syncthreads();
+    if (warp != 0)
+        return;
+    // Gershgorin bounds; then everything in units of a power of two near the norm
+    double lo = INFINITY, hi = -INFINITY;
+    for (int i = lane; i < D; i += 32) {
+        const double el = i > 0 ? fabs(od[i - 1]) : 0.0, er = i + 1 < D ? fabs(od[i]) : 0.0;
+        lo = fmin(lo, dg[i] - el - er);
+        hi = fmax(hi, dg[i] + el + er);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    const double norm = fmax(fabs(lo), fabs(hi));
+    const double limit = lim_scale * gk / back;
+    double mx = 0.0;
+    if (norm > 0.0 && isfinite(norm)) {
+        const int ex = ilogb(norm);
+        // 2^-ex in two factors, so that neither leaves the range
+        const double u1 = ldexp(1.0, -(ex / 2)), u2 = ldexp(1.0, -(ex - ex / 2));
+        __syncwarp();
+        for (int i = lane; i < D; i += 32) {
+            dg[i] = dg[i] * u1 * u2;
+            if (i + 1 < D) {
+                const double o = od[i] * u1 * u2;
+                od[i] = o * o;
+            }
+        }
+        __syncwarp();
+        lo = lo * u1 * u2;
+        hi = hi * u1 * u2;
+        // a limit outside the spectrum counts none or all of it
+        double lim_s = limit > norm * 4.0 ? 8.0 : limit < -norm * 4.0 ? -8.0 : limit * u1 * u2;
+        // eigenvalues at or above the limit count as 0, then the largest
+        const int c = count_below_nr(dg, od, D, lim_s);
+        if (c > 0) {
+            // the c-th smallest eigenvalue lies in [lo, min(hi, lim_s)]
+            const double pad = DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + EIG_PIVMIN;
+            lo -= pad;
+            hi = fmin(hi + pad, lim_s);
+            for (int it = 0; it < 64 && hi - lo > 0.5 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + EIG_PIVMIN; it++) {
+                const double xl = fma((hi - lo) * (1.0 / 33.0), (double) (lane + 1), lo);
+                const unsigned up = __ballot_sync(0xffffffffu, count_below_nr(dg, od, D, xl) >= c);
+                // the first point with at least c eigenvalues below it
+                const int f = up ? __ffs(up) - 1 : 32;
+                const double nlo = f == 0 ? lo : __shfl_sync(0xffffffffu, xl, f - 1 < 0 ? 0 : f - 1);
+                const double nhi = f == 32 ? hi : __shfl_sync(0xffffffffu, xl, f == 32 ? 0 : f);
+                lo = nlo;
+                hi = nhi;
+            }
+            const double lam = ldexp(0.5 * (lo + hi), ex) * back;
+            mx = (c < D) ? fmax(lam, 0.0) : lam;
+        }
+    }  // else the zero matrix, or non-finite entries: 0
+    if (lane == 0)
+        out[(size_t) kl * 2 + which] = mx;
+}
+
 template <int NT, typename F>
 int launch_eig(int kb, int D, bool in_smem, const double *S, F *Mg, const double *gg,
                double lim_scale, double *out, cudaStream_t s,
                const unsigned long long *rmax = nullptr)
 {
-    const size_t smem = in_smem ? eig_smem_bytes<F>(D)
-                                : eig_smem_bytes<F>(D) - sizeof(F) * (size_t) D * D;
-    DGTM_CUDA_TRY(cudaFuncSetAttribute(eig_kernel<NT, F>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    eig_kernel<NT, F><<<dim3(kb, 2), NT, smem, s>>>(S, D, in_smem ? 1 : 0, Mg, gg, lim_scale, out,
-                                                    rmax);
-    DGTM_CUDA_TRY(cudaGetLastError());
-    return DGTM_OK;
+    if constexpr (std::is_same<F, double>::value) {
+        const size_t smem = eig64_smem_bytes(D, in_smem);
+        DGTM_CUDA_TRY(cudaFuncSetAttribute(eig64_kernel<NT>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        eig64_kernel<NT><<<dim3(kb, 2), NT, smem, s>>>(S, D, in_smem ? 1 : 0, Mg, gg, lim_scale, out);
+        DGTM_CUDA_TRY(cudaGetLastError());
+        return DGTM_OK;
+    } else {
+        const size_t smem = in_smem ? eig_smem_bytes<F>(D)
+                                    : eig_smem_bytes<F>(D) - sizeof(F) * (size_t) D * D;
+        DGTM_CUDA_TRY(cudaFuncSetAttribute(eig_kernel<NT, F>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        eig_kernel<NT, F><<<dim3(kb, 2), NT, smem, s>>>(S, D, in_smem ? 1 : 0, Mg, gg, lim_scale, out,
+                                                        rmax);
+        DGTM_CUDA_TRY(cudaGetLastError());
+        return DGTM_OK;
+    }
 }
 
 template <typename F>
@@ -521,7 +752,7 @@ CtempPlan ctemp_plan(int N, int D, int K, bool f32, bool have_t32, size_t budget
     if (pl.nn < 1)
         pl.nn = 1;
     const size_t fsz = f32 ? sizeof(float) : sizeof(double);
-    pl.eig_in_smem = (f32 ? eig_smem_bytes<float>(D) : eig_smem_bytes<double>(D)) <= EIG_SMEM_MAX;
+    pl.eig_in_smem = f32 ? eig_smem_bytes<float>(D) <= EIG_SMEM_MAX : eig64_smem_bytes(D, true) <= EIG64_SMEM_MAX;
     const size_t dd = (size_t) D * D;
     const size_t per = sizeof(double) * 2 * dd + (pl.eig_in_smem ? 0 : fsz * 2 * dd) +
                        sizeof(double) * (size_t) pl.nn;

@@ -957,8 +957,14 @@ int dgtm_next_ctemp_k(dgtm_ctx *ctx, double temp, double beta, double eps, const
     const int kb = pl.kb;
     double *scratch = nullptr, *dgg = nullptr, *dgsum = nullptr, *dout = nullptr;
     std::vector<double> out((size_t) 2 * K), gsum(K);
-    int rc = pairs ? DGTM_OK
-                   : dev_alloc(&scratch, (pl.scratch_bytes + sizeof(double) - 1) / sizeof(double));
+    // FP64 form: the scatter as digit-slice products, where the problem is large
+    // enough for its fixed costs (an explicit DGTM_CTEMP_SCRATCH_MB bounds it too)
+    OzE *slices = nullptr;
+    if (ctx->precision == DGTM_FP64 && env_int("DGTM_CTEMP_PAIRS", 1, 0, 1) &&
+        (double) N * K * D * D >= 1e8 && D >= 2)
+        slices = map_slices(ctx);
+    const bool bounded = env_int("DGTM_CTEMP_SCRATCH_MB", -1, 1, 1 << 20) > 0;
+    int rc = DGTM_OK;
     if (rc == DGTM_OK)
         rc = dev_alloc(&dgsum, K);
     if (rc == DGTM_OK)
@@ -972,6 +978,34 @@ int dgtm_next_ctemp_k(dgtm_ctx *ctx, double temp, double beta, double eps, const
     std::vector<int> redo;
     std::vector<double> out_sel, gsum_sel;
     const double dcut = ref_dcut(ctx->beta);
+    if (slices && rc == DGTM_OK && e == cudaSuccess) {
+        const size_t gbudget = (size_t) env_int("DGTM_CTEMP_GEMM_MB", 8192, 64, 1 << 22) << 20;
+        double *dspread = nullptr;
+        std::vector<double> spread(K);
+        rc = dev_alloc(&dspread, (size_t) K);
+        if (rc == DGTM_OK)
+            rc = oz_ctemp(slices, ctx->T64, ctx->Y64, ctx->yy, ctx->colstat, N, D, K, ctx->sms, c, dcut,
+                          gg ? dgg : nullptr, lim_scale, bounded ? budget : gbudget, dgsum, dout, dspread,
+                          ctx->flag + 3, ctx->stream);
+        if (rc == DGTM_OK)
+            rc = fetch_oz_status(ctx);
+        if (rc == DGTM_OK)
+            e = cudaMemcpyAsync(spread.data(), dspread, sizeof(double) * K, cudaMemcpyDeviceToHost,
+                                ctx->stream);
+        if (rc == DGTM_OK && e == cudaSuccess && (e = cudaStreamSynchronize(ctx->stream)) == cudaSuccess)
+            rc = check_oz_status(ctx);
+        cudaFree(dspread);
+        // centres whose expansion about the data's mean cancels more than 8 bits
+        for (int k = 0; rc == DGTM_OK && e == cudaSuccess && k < K; k++)
+            if (!(spread[k] <= 256.0))
+                redo.push_back(k);
+        if (rc == DGTM_ENOMEM) {  // no room: the CUDA-core scatter
+            rc = unless_enomem(rc);
+            slices = nullptr;
+        }
+    }
+    if (!pairs && !slices && rc == DGTM_OK)
+        rc = dev_alloc(&scratch, (pl.scratch_bytes + sizeof(double) - 1) / sizeof(double));
     if (pairs && rc == DGTM_OK && e == cudaSuccess) {
         TcView v;
         tc_view(ctx->tc, &v);
@@ -1051,7 +1085,7 @@ int dgtm_next_ctemp_k(dgtm_ctx *ctx, double temp, double beta, double eps, const
         cudaFree(gs);
         cudaFree(os);
     }
-    for (int k0 = 0; !pairs && rc == DGTM_OK && e == cudaSuccess && k0 < K; k0 += kb) {
+    for (int k0 = 0; !pairs && !slices && rc == DGTM_OK && e == cudaSuccess && k0 < K; k0 += kb) {
         const int nb = (K - k0 < kb) ? K - k0 : kb;
         rc = launch_ctemp_batch(pl, ctx->T64, ctx->T32, ctx->Y64, ctx->tt, ctx->yy, ctx->colstat,
                                 N, D, K, c, k0, nb, gg ? dgg + k0 : nullptr, lim_scale, scratch,

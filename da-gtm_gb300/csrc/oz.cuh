@@ -74,8 +74,28 @@ int oze_estep_blocks(const OzE *st);
 int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, int isDA,
               double2 *colstat, double *part, double dcut, int *nlaunch, cudaStream_t s);
 int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaStream_t s);
+// The parts other products with R are made of.  oze_refer: the centres' planes and
+// the points' references (kept when they are those of the last oze_estep);
+// oze_chunks: how many chunks, and their points; oze_r_digits: R (or R^2) of the
+// centres k0 .. k0 + kb over a chunk as eight planes of prows x (points rounded
+// up to 64), and the integer exponents of their grids: an integer sum of the
+// product with B counts 2^(5 - nmin[k]) of B's grid (oz_sum_ext).  products: form
+// the chunk's distances first (they stay until the next chunk's).
+int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat, double dcut, cudaStream_t s);
+int oze_chunks(const OzE *st, int *points);
+int oze_r_digits(OzE *st, int ch, int k0, int kb, double c, bool squares, bool products, int prows,
+                 __nv_bfloat16 *planes, int *nmin, cudaStream_t s);
 // M = R^T X from a context's column statistics
 int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c,
             const double *X, int L, double *M, cudaStream_t s);
+
+// The AUTO schedule's scatter in FP64 accuracy as digit-slice products of R and
+// R^2 with pair features (oz_ctemp.cu): out and gsum as launch_ctemp_batch;
+// spread[k] = tr(sum R x x^T) / tr(S1) about the data's mean: what the expansion
+// cancels.  DGTM_ENOMEM (nothing done) if not even 128 centres fit the budget.
+int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, const double2 *colstat, int N,
+             int D, int K, int sms, double c, double dcut, const double *gg_dev, double lim_scale,
+             size_t budget, double *gsum_dev, double *out_dev, double *spread_dev, int *status,
+             cudaStream_t s);
 
 }  // namespace dgtm

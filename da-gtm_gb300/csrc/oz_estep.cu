@@ -30,6 +30,7 @@
 
 #include <math.h>
 #include <new>
+#include <type_traits>
 
 namespace dgtm {
 
@@ -77,9 +78,17 @@ __global__ void __launch_bounds__(256) oz_absmax_kernel(const double *__restrict
         m = a > m ? a : m;
         q = b > q ? b : q;
     }
+    __shared__ unsigned long long red[2][8];
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(&bits[0], m);
-        atomicMax(&bits[1], q);
+        red[0][threadIdx.x >> 5] = m;
+        red[1][threadIdx.x >> 5] = q;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        m = 0ull;
+        for (int i = 0; i < 8; i++)
+            m = red[threadIdx.x][i] > m ? red[threadIdx.x][i] : m;
+        atomicMax(&bits[threadIdx.x], m);
     }
 }
 
@@ -304,7 +313,8 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
 
 // references and exponents from a context's column statistics (d_ref, ln s)
 __global__ void oz_points_kernel(const double2 *__restrict__ colstat, const double *__restrict__ tt, int N,
-                                 int K, const OzScale *__restrict__ sc, OzPoint *__restrict__ pt)
+                                 int K, const OzScale *__restrict__ sc, double dcut,
+                                 OzPoint *__restrict__ pt, int64_t *__restrict__ thr)
 {
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
         const double2 cs = colstat[n];
@@ -317,6 +327,7 @@ __global__ void oz_points_kernel(const double2 *__restrict__ colstat, const doub
             o.lam = lam_of(cs.y);
         }
         pt[n] = o;
+        thr[n] = o.aref == ZERO_COLUMN ? INT64_MIN : oz::scaled_int(tt[n] - dcut, -1 - sc->u);
     }
 }
 
@@ -335,43 +346,51 @@ __device__ __forceinline__ uint64_t r_exponent(const OzPoint &o, int64_t v, cons
     return o.lam > wv ? o.lam - wv : 0ull;
 }
 
-// Responsibilities of a chunk as digit planes, planes[i][k][n] (n fastest), each
-// centre on the grid of its largest R in the chunk; nmin[k] is an integer bound of
-// that R's exponent.  Zero past nn up to ldn.  A block takes DG_K centres, so that
-// a point's constants are read once for all of them.  The first loop finds the
-// grids from the exponents in FP32 (a margin of 2^-6 and 2^-10 of the exponent
-// taken): one conversion and one FMA a pair instead of a 64-bit product.
-__global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn,
-                                                        int K, const int64_t *__restrict__ h,
-                                                        const OzScale *__restrict__ sc,
-                                                        const uint64_t *__restrict__ gtab,
-                                                        const OzPoint *__restrict__ pt,
-                                                        const int64_t *__restrict__ thr, oz::MulBase kb,
-                                                        int prows, int ldn, __nv_bfloat16 *__restrict__ planes,
-                                                        int *__restrict__ nmin_out)
+// the exponent of R^2
+__device__ __forceinline__ uint64_t r_square(uint64_t W)
 {
-    extern __shared__ uint64_t tab[];
-    __shared__ float red[8][DG_K];
-    const int k0 = blockIdx.x * DG_K;
+    constexpr uint64_t bias = (uint64_t) oz::WBIAS << oz::WFRAC;
+    return W >> 63 ? ~0ull : 2 * W > bias ? 2 * W - bias : 0ull;
+}
+
+// W of a centre's values from W of its R: the grid bound and the digits agree on it
+template <bool SQ>
+__device__ __forceinline__ int grid_of_w(float w)
+{
+    if (SQ)
+        w = 2.f * w - (float) oz::WBIAS;
+    // the integer part of a W at most 2^-5 + 2^-9 w below w
+    w = floorf(w - 0.03125f - w * 0.001953125f);
+    return w < 0.f ? 0 : (int) w;
+}
+
+// wmin[k] = the least exponent W of the chunk's R_kn (FP32 bits, 4096 where all R
+// are 0): the grid of a centre's responsibilities.  FP32 is enough (grid_of_w takes
+// a margin): one conversion and one FMA a pair.  Block: DG_K centres (a point's
+// constants are read once for all of them), a range of points.
+__global__ void __launch_bounds__(256) oz_rmax_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn, int K,
+                                                      const int64_t *__restrict__ h,
+                                                      const OzScale *__restrict__ sc,
+                                                      const OzPoint *__restrict__ pt,
+                                                      const int64_t *__restrict__ thr, oz::MulBase kb, int range,
+                                                      unsigned *__restrict__ wmin)
+{
+    const int k0 = blockIdx.x * DG_K, na = blockIdx.y * range, nb = min(nn, na + range);
     const int u = sc->u;
-    const oz::Mul km = oz::mul_at(kb, u);
-    // exponents in FP32 from x >> xs, xs such that one of its units is at most 2^-8
+    // exponents from x >> xs, xs such that one of its units is at most 2^-8
     const int xs = min(max(-8 - kb.ex - u, 0), 40);
     const float kf = scalbnf((float) (kb.m >> 40), kb.ex - 24 + u + xs);
     int64_t hk[DG_K];
     const int64_t *row[DG_K];
+    float w[DG_K];
 #pragma unroll
     for (int i = 0; i < DG_K; i++) {
         const int k = min(k0 + i, K - 1);
         hk[i] = h[k];
         row[i] = acc + (size_t) k * ldm;
+        w[i] = 4096.f;
     }
-    load_table(tab, gtab);
-    float wmin[DG_K];
-#pragma unroll
-    for (int i = 0; i < DG_K; i++)
-        wmin[i] = 4096.f;
-    for (int n = threadIdx.x; n < nn; n += 256) {
+    for (int n = na + threadIdx.x; n < nb; n += 256) {
         const OzPoint o = pt[n];
         const int64_t t = thr[n];
         const float lf = (float) (uint32_t) (o.lam >> 32) * 0x1p-21f;  // 53 - 32 bits of fraction
@@ -380,34 +399,55 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
             const int64_t v = row[i][n] - hk[i];
             const int64_t x = (o.aref - v) >> xs;
             const int xi = x > 0x7FFFFFFF ? 0x7FFFFFFF : (int) x;  // x >= -(a few): d_ref is the least
-            const float w = o.aref == ZERO_COLUMN ? lf : fmaf((float) xi, kf, lf);
-            wmin[i] = fminf(wmin[i], v < t ? 4096.f : w);
+            const float f = o.aref == ZERO_COLUMN ? lf : fmaf((float) xi, kf, lf);
+            w[i] = fminf(w[i], v < t ? 4096.f : f);
         }
     }
 #pragma unroll
     for (int i = 0; i < DG_K; i++) {
 #pragma unroll
         for (int s = 16; s > 0; s >>= 1)
-            wmin[i] = fminf(wmin[i], __shfl_xor_sync(0xffffffffu, wmin[i], s));
-        if ((threadIdx.x & 31) == 0)
-            red[threadIdx.x >> 5][i] = wmin[i];
+            w[i] = fminf(w[i], __shfl_xor_sync(0xffffffffu, w[i], s));
+        if ((threadIdx.x & 31) == 0 && k0 + i < K)
+            atomicMin(&wmin[k0 + i], __float_as_uint(fmaxf(w[i], 0.f)));
     }
-    __syncthreads();
+}
+
+// Responsibilities (SQ: their squares) of a chunk as digit planes, planes[i][k][n]
+// (n fastest), each centre on the grid of its largest value in the chunk; nmin[k] is
+// an integer bound of that value's exponent.  Zero past nn up to ldn.  Blocks as in
+// oz_rmax_kernel, two points a thread.  Bound by the integer pipe: about 120
+// instructions a pair, half of them the exponential.
+template <bool SQ>
+__global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn, int K,
+                                                        const int64_t *__restrict__ h,
+                                                        const OzScale *__restrict__ sc,
+                                                        const uint64_t *__restrict__ gtab,
+                                                        const OzPoint *__restrict__ pt,
+                                                        const int64_t *__restrict__ thr, oz::MulBase kb, int range,
+                                                        const unsigned *__restrict__ wmin, int prows, int ldn,
+                                                        __nv_bfloat16 *__restrict__ planes,
+                                                        int *__restrict__ nmin_out)
+{
+    extern __shared__ uint64_t tab[];
+    const int k0 = blockIdx.x * DG_K, ja = blockIdx.y * (range / 2), jb = min(ldn / 2, ja + range / 2);
+    const oz::Mul km = oz::mul_at(kb, sc->u);
+    int64_t hk[DG_K];
+    const int64_t *row[DG_K];
     int nmin[DG_K];
+    load_table(tab, gtab);
 #pragma unroll
     for (int i = 0; i < DG_K; i++) {
-        float w = red[0][i];
-#pragma unroll
-        for (int j = 1; j < 8; j++)
-            w = fminf(w, red[j][i]);
-        // the integer part of a W at most 2^-6 + 2^-10 w below w
-        w = floorf(w - 0.015625f - w * 0.0009765625f);
-        nmin[i] = w < 0.f ? 0 : (int) w;
-        if (threadIdx.x == 0 && k0 + i < K)
+        const int k = min(k0 + i, K - 1);
+        hk[i] = h[k];
+        row[i] = acc + (size_t) k * ldm;
+        nmin[i] = grid_of_w<SQ>(__uint_as_float(wmin[k]));
+        if (threadIdx.x == 0 && blockIdx.y == 0 && k0 + i < K)
             nmin_out[k0 + i] = nmin[i];
     }
+    __syncthreads();
     const size_t plane = (size_t) prows * ldn / 2;
-    for (int j = threadIdx.x; j < ldn / 2; j += 256) {
+    for (int j = ja + threadIdx.x; j < jb; j += 256) {
         OzPoint o[2];
         int64_t t[2];
 #pragma unroll
@@ -424,7 +464,9 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 const int64_t v = row[i][min(2 * j + e, nn - 1)] - hk[i];
-                const uint64_t W = v < t[e] ? ~0ull : r_exponent(o[e], v, km);
+                uint64_t W = v < t[e] ? ~0ull : r_exponent(o[e], v, km);
+                if (SQ)
+                    W = r_square(W);
                 const int ex = (int) (W >> oz::WFRAC);
                 // R 2^(55 - (5 - nmin)) = E >> (9 + ex - nmin), rounded
                 const int sh = 9 + ex - nmin[i];
@@ -538,6 +580,7 @@ int grid_of(size_t n, int cap)
 
 struct OzE {
     OzEArgs a;
+    unsigned char *arena = nullptr;  // every buffer below, one allocation
     int sa = 8, panels = 0, Dp = 0, Np = 0, Kp = 0, chunk = 0, nchunks = 0;
     const __nv_bfloat16 *Tp = nullptr;  // data planes (own or the caller's)
     __nv_bfloat16 *Town = nullptr, *Yp = nullptr;
@@ -555,6 +598,7 @@ struct OzE {
     __nv_bfloat16 *Tt = nullptr, *Rp = nullptr;
     int64_t *part = nullptr;
     int *nmin = nullptr;
+    unsigned *wmin = nullptr;
 };
 
 // The digit-slice path has fixed costs (planes of the centres, four launches a
@@ -568,11 +612,8 @@ void oze_destroy(OzE *st)
 {
     if (!st)
         return;
-    void *ptrs[] = {st->Town, st->Yp, st->bits, st->sc, st->tab, st->h, st->acc, st->pt, st->thr,
-                    st->Tt, st->Rp, st->part, st->nmin};
-    for (void *p : ptrs)
-        if (p)
-            cudaFree(p);
+    if (st->arena)
+        cudaFree(st->arena);
     delete st;
 }
 
@@ -616,37 +657,45 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     st->Kp128 = rup(K, 128);
     st->Npk = rup(N, PANEL);
     const size_t planes = sizeof(__nv_bfloat16) * oz::DIGITS;
-    cudaError_t e = cudaSuccess;
-    auto get = [&](void *pp, size_t bytes) {
-        if (e == cudaSuccess)
-            e = cudaMalloc((void **) pp, bytes);
+    const int cp = rup(st->chunk, PANEL) / PANEL;
+    st->rt_tiles = (st->Kp128 / 128) * (st->Wp / 64);
+    st->rt_per = oz_item_panels(st->rt_tiles, cp, a.sms);
+    size_t bytes = 0;
+    auto lay = [&](auto **pp, size_t n, unsigned char *base) {
+        if (base)
+            *pp = reinterpret_cast<std::remove_reference_t<decltype(*pp)>>(base + bytes);
+        bytes += (n + 255) / 256 * 256;
     };
-    if (!a.Tb)
-        get(&st->Town, planes * st->Np * st->Dp);
-    get(&st->Yp, planes * st->Kp * st->Dp);
-    get(&st->bits, sizeof(unsigned long long) * (4 + D + 1));
-    get(&st->sc, sizeof(OzScale));
-    get(&st->tab, TAB_BYTES);
-    get(&st->h, sizeof(int64_t) * K);
-    get(&st->acc, sizeof(int64_t) * st->ldm * K);
-    get(&st->pt, sizeof(OzPoint) * N);
-    if (a.mstep)
-        get(&st->thr, sizeof(int64_t) * N);
-    if (a.mstep) {
-        const int cp = rup(st->chunk, PANEL) / PANEL;
-        st->rt_tiles = (st->Kp128 / 128) * (st->Wp / 64);
-        st->rt_per = oz_item_panels(st->rt_tiles, cp, a.sms);
-        get(&st->Tt, planes * st->Wp * st->Npk);
-        get(&st->Rp, planes * st->Kp128 * st->chunk);
-        get(&st->part, sizeof(int64_t) * 8192 * (size_t) st->rt_tiles * ceil_div(cp, st->rt_per));
-        get(&st->nmin, sizeof(int) * K);
-    }
+    auto lay_out = [&](unsigned char *base) {
+        bytes = 0;
+        if (!a.Tb)
+            lay(&st->Town, planes * st->Np * st->Dp, base);
+        lay(&st->Yp, planes * st->Kp * st->Dp, base);
+        lay(&st->bits, sizeof(unsigned long long) * (4 + D + 1), base);
+        lay(&st->sc, sizeof(OzScale), base);
+        lay(&st->tab, TAB_BYTES, base);
+        lay(&st->h, sizeof(int64_t) * K, base);
+        lay(&st->acc, sizeof(int64_t) * st->ldm * K, base);
+        lay(&st->pt, sizeof(OzPoint) * N, base);
+        lay(&st->thr, sizeof(int64_t) * N, base);
+        lay(&st->wmin, sizeof(unsigned) * K, base);
+        if (a.mstep) {
+            lay(&st->Tt, planes * st->Wp * st->Npk, base);
+            lay(&st->Rp, planes * st->Kp128 * st->chunk, base);
+            lay(&st->part, sizeof(int64_t) * 8192 * (size_t) st->rt_tiles * ceil_div(cp, st->rt_per), base);
+            lay(&st->nmin, sizeof(int) * K, base);
+        }
+    };
+    lay_out(nullptr);
+    cudaError_t e = cudaMalloc((void **) &st->arena, bytes);
+    if (e == cudaSuccess)
+        lay_out(st->arena);
     if (e == cudaSuccess)
         e = cudaMemcpy(st->tab, host_table(), TAB_BYTES, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(st->bits, 0, sizeof(unsigned long long) * (4 + D + 1), s);
     if (e == cudaSuccess) {
-        oz_absmax_kernel<<<grid_of((size_t) N * D, 4864), 256, 0, s>>>(a.T64, (size_t) N * D, a.tt, N, st->bits);
+        oz_absmax_kernel<<<grid_of((size_t) N * D, 1216), 256, 0, s>>>(a.T64, (size_t) N * D, a.tt, N, st->bits);
         if (!a.Tb)
             oz_slice_rows_kernel<<<grid_of((size_t) st->Np * st->Dp / 2, 16384), 256, 0, s>>>(
                 a.T64, N, D, st->Np, st->Dp, st->bits, st->Town, nullptr, 8, nullptr, nullptr, nullptr);
@@ -793,7 +842,6 @@ int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, 
 int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaStream_t s)
 {
     const int K = st->a.K, D = st->a.D;
-    OZ_TRY(table_smem(oz_digits_kernel));
     int nl = 0;
     for (int ch = 0; ch < st->nchunks; ch++) {
         if (!st->acc_whole) {
@@ -802,10 +850,7 @@ int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaS
         }
         const int n0 = ch * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
         const int ldn = rup(nn, PANEL);
-        oz_digits_kernel<<<ceil_div(K, DG_K), 256, TAB_BYTES, s>>>(st->acc, st->ldm, nn, K, st->h, st->sc, st->tab, st->pt + n0,
-                                                   st->thr + n0, oz::make_mul(c * LOG2E_2), st->Kp128, ldn,
-                                                   st->Rp, st->nmin);
-        DGTM_CUDA_TRY(cudaGetLastError());
+        OZ_TRY(oze_r_digits(st, ch, 0, K, c, false, false, st->Kp128, st->Rp, st->nmin, s));
         OzGemm g;
         g.A = st->Rp;
         g.B = st->Tt;
@@ -823,10 +868,56 @@ int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaS
                                                             oz_sum_ext(g.panels), st->nmin, st->bits + 4, K, D,
                                                             ch == 0 ? 1 : 0, G, RT);
         DGTM_CUDA_TRY(cudaGetLastError());
-        nl += 3;
+        nl += 4;
     }
     if (nlaunch)
         *nlaunch = nl;
+    return DGTM_OK;
+}
+
+// the centres' planes and the points' references for a context's column statistics
+int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat, double dcut, cudaStream_t s)
+{
+    if (st->own_stats)
+        return DGTM_OK;
+    OZ_TRY(slice_centres(st, Y, yy, s));
+    oz_points_kernel<<<grid_of((size_t) st->a.N, 1216), 256, 0, s>>>(colstat, st->a.tt, st->a.N, st->a.K,
+                                                                    st->sc, dcut, st->pt, st->thr);
+    DGTM_CUDA_TRY(cudaGetLastError());
+    return DGTM_OK;
+}
+
+int oze_chunks(const OzE *st, int *points)
+{
+    *points = st->chunk;
+    return st->nchunks;
+}
+
+int oze_r_digits(OzE *st, int ch, int k0, int kb, double c, bool squares, bool products, int prows,
+                 __nv_bfloat16 *planes, int *nmin, cudaStream_t s)
+{
+    if (products && !st->acc_whole)
+        OZ_TRY(chunk_products(st, ch, s));
+    const auto kernel = squares ? oz_digits_kernel<true> : oz_digits_kernel<false>;
+    OZ_TRY(table_smem(kernel));
+    const int n0 = ch * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
+    const int ldn = rup(nn, PANEL), kblocks = ceil_div(kb, DG_K);
+    // ranges of points: about four blocks an SM, at least 1024 points each
+    int parts = ceil_div(4LL * st->a.sms, kblocks);
+    const int range = rup(ceil_div(ldn, parts) < 1024 ? 1024 : ceil_div(ldn, parts), PANEL);
+    parts = ceil_div(ldn, range);
+    const int64_t *acc = st->acc + (size_t) k0 * st->ldm;
+    const oz::MulBase base = oz::make_mul(c * LOG2E_2);
+    if (!squares) {  // the squares' grids follow from the same exponents
+        DGTM_CUDA_TRY(cudaMemsetAsync(st->wmin, 0x7F, sizeof(unsigned) * kb, s));
+        oz_rmax_kernel<<<dim3(kblocks, parts), 256, 0, s>>>(acc, st->ldm, nn, kb, st->h + k0, st->sc, st->pt + n0,
+                                                            st->thr + n0, base, range, st->wmin);
+        DGTM_CUDA_TRY(cudaGetLastError());
+    }
+    kernel<<<dim3(kblocks, parts), 256, TAB_BYTES, s>>>(acc, st->ldm, nn, kb, st->h + k0, st->sc, st->tab,
+                                                        st->pt + n0, st->thr + n0, base, range, st->wmin, prows,
+                                                        ldn, planes, nmin);
+    DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
 
@@ -834,11 +925,7 @@ int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, 
             int L, double *M, cudaStream_t s)
 {
     const int N = st->a.N, K = st->a.K;
-    if (!st->own_stats) {
-        OZ_TRY(slice_centres(st, Y, yy, s));
-        oz_points_kernel<<<grid_of((size_t) N, 1216), 256, 0, s>>>(colstat, st->a.tt, N, K, st->sc, st->pt);
-        DGTM_CUDA_TRY(cudaGetLastError());
-    }
+    OZ_TRY(oze_refer(st, Y, yy, colstat, 1e300, s));
     const int nt = wide_blocks(K) ? 1024 : 512;
     const auto kernel = nt == 512 ? (L <= 2 ? oz_map_kernel<512, 2> : L == 3 ? oz_map_kernel<512, 3> : oz_map_kernel<512, 8>)
                                   : (L <= 2 ? oz_map_kernel<1024, 2> : L == 3 ? oz_map_kernel<1024, 3> : oz_map_kernel<1024, 8>);

@@ -166,6 +166,10 @@ int dgtm_get_RD_block(dgtm_ctx *ctx, int k0, int nk, int n0, int nn, double *R, 
  * R and R^2 (split BF16) against the pair features (t_i t_j, t_i, 1), which
  * are exact in BF16, with DGTM_CTEMP_GEMM_MB (default 8192) of scratch;
  * DGTM_CTEMP_PAIRS=0 selects the CUDA-core scatter for those contexts too.
+ * The FP64 form does the same at large sizes (N K D^2 at least 1e8, N K at
+ * least 2e6) with FP64-accurate digit-slice products, in DGTM_CTEMP_GEMM_MB of
+ * scratch, or in DGTM_CTEMP_SCRATCH_MB where that is set (the CUDA-core
+ * scatter where not even 128 centres fit).
  * Replaces dagtm_mpi_next_ctemp and its helper (comm/mpicomm.c:562-674) with
  * dagtm_vector_max (comm/comm.c:2149-2161), called at dagtm/dagtm.cxx:1919-1934.
  */

@@ -107,3 +107,43 @@ def test_map_matches_cuda_cores(pkg, monkeypatch, form, binary, D):
             monkeypatch.setenv("DGTM_X64", on)
             out.append(c.map(X))
     assert rel(out[0], out[1]) <= 1e-12
+
+
+# the FP64 critical temperatures by digit slices against the CUDA-core scatter,
+# centre by centre: two dimensions, one and several tiles of features and of
+# centres, several batches of centres (a small budget), several chunks of points
+@pytest.mark.parametrize("N,D,K,binary,mb", [
+    (7000, 2, 4001, False, 8192), (2000, 65, 1001, False, 8192), (2100, 20, 1500, False, 64),
+    (9000, 33, 1301, False, 8192), (2500, 40, 900, True, 8192), (20000, 64, 125, False, 8192)])
+def test_ctemp_matches_cuda_cores(pkg, monkeypatch, N, D, K, binary, mb):
+    T, Y, FI, _ = problem(N, D, K, N + D, binary=binary)
+    beta = 8.0 / D
+    out = []
+    for pairs in ("1", "0"):
+        monkeypatch.setenv("DGTM_CTEMP_PAIRS", pairs)
+        monkeypatch.setenv("DGTM_CTEMP_GEMM_MB", str(mb))
+        with pkg.Context(T, FI, "fp64") as c:
+            c.set_Y(Y if not binary else 0.4 + 0.2 * Y)
+            c.estep(beta, 1, 2.0)
+            out.append(c.next_ctemp(50.0, beta, 1e-6, per_centre=True))
+    (a, ak), (b, bk) = out
+    assert a == pytest.approx(b, rel=1e-12)
+    # the expansion may cancel 8 bits of 2^-53: 2.8e-14 of the largest eigenvalue
+    assert np.max(np.abs(ak - bk) / bk) <= 1e-13
+
+
+def test_ctemp_tight_clusters_are_redone(pkg, monkeypatch):
+    """Clusters of width 1e-4 far from the mean: the expansion would cancel 24
+    bits, so those centres go through the CUDA-core scatter."""
+    rng = np.random.default_rng(3)
+    mu = rng.normal(size=(700, 8))
+    T = mu[rng.integers(0, 700, 4000)] + 1e-4 * rng.normal(size=(4000, 8))
+    FI = np.ones((700, 1))
+    out = []
+    for pairs in ("1", "0"):
+        monkeypatch.setenv("DGTM_CTEMP_PAIRS", pairs)
+        with pkg.Context(T, FI, "fp64") as c:
+            c.set_Y(mu)
+            c.estep(1e5, 1, 1.5)
+            out.append(c.next_ctemp(1e6, 1e5, 1e-6, per_centre=True)[1])
+    np.testing.assert_allclose(out[0], out[1], rtol=1e-13)  # zeros and HUGE_VAL alike
