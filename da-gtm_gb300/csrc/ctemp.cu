@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(NT) eig64_kernel(const double *__restrict__ S,
             const double pad = DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + EIG_PIVMIN;
             lo -= pad;
             hi = fmin(hi + pad, lim_s);
-            for (int it = 0; it < 64 && hi - lo > 0.5 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + EIG_PIVMIN; it++) {
+            for (int it = 0; it < 64 && hi - lo > DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + EIG_PIVMIN; it++) {
                 const double xl = fma((hi - lo) * (1.0 / 33.0), (double) (lane + 1), lo);
                 const unsigned up = __ballot_sync(0xffffffffu, count_below_nr(dg, od, D, xl) >= c);
                 // the first point with at least c eigenvalues below it

@@ -364,32 +364,20 @@ __device__ __forceinline__ int grid_of_w(float w)
     return w < 0.f ? 0 : (int) w;
 }
 
-// wmin[k] = the least exponent W of the chunk's R_kn (FP32 bits, 4096 where all R
-// are 0): the grid of a centre's responsibilities.  FP32 is enough (grid_of_w takes
-// a margin): one conversion and one FMA a pair.  Block: DG_K centres (a point's
-// constants are read once for all of them), a range of points.
-__global__ void __launch_bounds__(256) oz_rmax_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn, int K,
-                                                      const int64_t *__restrict__ h,
-                                                      const OzScale *__restrict__ sc,
-                                                      const OzPoint *__restrict__ pt,
-                                                      const int64_t *__restrict__ thr, oz::MulBase kb, int range,
-                                                      unsigned *__restrict__ wmin)
+// The least exponents W of R_kn of DG_K centres over the points na .. nb (each
+// warp's own share), in FP32: enough for the grid of a centre's responsibilities
+// (grid_of_w takes a margin), and one conversion and one FMA a pair.
+__device__ __forceinline__ void least_exponents(const int64_t *const (&row)[DG_K], const int64_t (&hk)[DG_K],
+                                                int na, int nb, int u, const oz::MulBase &kb,
+                                                const OzPoint *__restrict__ pt, const int64_t *__restrict__ thr,
+                                                float (&w)[DG_K])
 {
-    const int k0 = blockIdx.x * DG_K, na = blockIdx.y * range, nb = min(nn, na + range);
-    const int u = sc->u;
     // exponents from x >> xs, xs such that one of its units is at most 2^-8
     const int xs = min(max(-8 - kb.ex - u, 0), 40);
     const float kf = scalbnf((float) (kb.m >> 40), kb.ex - 24 + u + xs);
-    int64_t hk[DG_K];
-    const int64_t *row[DG_K];
-    float w[DG_K];
 #pragma unroll
-    for (int i = 0; i < DG_K; i++) {
-        const int k = min(k0 + i, K - 1);
-        hk[i] = h[k];
-        row[i] = acc + (size_t) k * ldm;
+    for (int i = 0; i < DG_K; i++)
         w[i] = 4096.f;
-    }
     for (int n = na + threadIdx.x; n < nb; n += 256) {
         const OzPoint o = pt[n];
         const int64_t t = thr[n];
@@ -408,24 +396,51 @@ __global__ void __launch_bounds__(256) oz_rmax_kernel(const int64_t *__restrict_
 #pragma unroll
         for (int s = 16; s > 0; s >>= 1)
             w[i] = fminf(w[i], __shfl_xor_sync(0xffffffffu, w[i], s));
-        if ((threadIdx.x & 31) == 0 && k0 + i < K)
-            atomicMin(&wmin[k0 + i], __float_as_uint(fmaxf(w[i], 0.f)));
+        w[i] = fmaxf(w[i], 0.f);
     }
+}
+
+// wmin[k] = that of the whole chunk as FP32 bits (4096 where all R are 0).  Block:
+// DG_K centres (a point's constants are read once for all of them), a range of points.
+__global__ void __launch_bounds__(256) oz_rmax_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn, int K,
+                                                      const int64_t *__restrict__ h,
+                                                      const OzScale *__restrict__ sc,
+                                                      const OzPoint *__restrict__ pt,
+                                                      const int64_t *__restrict__ thr, oz::MulBase kb, int range,
+                                                      unsigned *__restrict__ wmin)
+{
+    const int k0 = blockIdx.x * DG_K, na = blockIdx.y * range, nb = min(nn, na + range);
+    int64_t hk[DG_K];
+    const int64_t *row[DG_K];
+    float w[DG_K];
+#pragma unroll
+    for (int i = 0; i < DG_K; i++) {
+        const int k = min(k0 + i, K - 1);
+        hk[i] = h[k];
+        row[i] = acc + (size_t) k * ldm;
+    }
+    least_exponents(row, hk, na, nb, sc->u, kb, pt, thr, w);
+#pragma unroll
+    for (int i = 0; i < DG_K; i++)
+        if ((threadIdx.x & 31) == 0 && k0 + i < K)
+            atomicMin(&wmin[k0 + i], __float_as_uint(w[i]));
 }
 
 // Responsibilities (SQ: their squares) of a chunk as digit planes, planes[i][k][n]
 // (n fastest), each centre on the grid of its largest value in the chunk; nmin[k] is
 // an integer bound of that value's exponent.  Zero past nn up to ldn.  Blocks as in
-// oz_rmax_kernel, two points a thread.  Bound by the integer pipe: about 120
+// oz_rmax_kernel, two points a thread.  FIND: the block covers the whole chunk and
+// finds the grids itself (a second launch reads the distances from L2 again: 100 us
+// a chunk of 1e7 pairs against 87).  Bound by the integer pipe: about 120
 // instructions a pair, half of them the exponential.
-template <bool SQ>
+template <bool SQ, bool FIND>
 __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn, int K,
                                                         const int64_t *__restrict__ h,
                                                         const OzScale *__restrict__ sc,
                                                         const uint64_t *__restrict__ gtab,
                                                         const OzPoint *__restrict__ pt,
                                                         const int64_t *__restrict__ thr, oz::MulBase kb, int range,
-                                                        const unsigned *__restrict__ wmin, int prows, int ldn,
+                                                        unsigned *__restrict__ wmin, int prows, int ldn,
                                                         __nv_bfloat16 *__restrict__ planes,
                                                         int *__restrict__ nmin_out)
 {
@@ -441,11 +456,31 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
         const int k = min(k0 + i, K - 1);
         hk[i] = h[k];
         row[i] = acc + (size_t) k * ldm;
-        nmin[i] = grid_of_w<SQ>(__uint_as_float(wmin[k]));
+    }
+    if constexpr (FIND) {
+        __shared__ float red[8][DG_K];
+        float w[DG_K];
+        least_exponents(row, hk, 0, nn, sc->u, kb, pt, thr, w);
+        if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+            for (int i = 0; i < DG_K; i++)
+                red[threadIdx.x >> 5][i] = w[i];
+        }
+        __syncthreads();
+        if (threadIdx.x < DG_K && k0 + (int) threadIdx.x < K) {
+            float m = red[0][threadIdx.x];
+            for (int i = 1; i < 8; i++)
+                m = fminf(m, red[i][threadIdx.x]);
+            wmin[k0 + threadIdx.x] = __float_as_uint(m);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < DG_K; i++) {
+        nmin[i] = grid_of_w<SQ>(__uint_as_float(wmin[min(k0 + i, K - 1)]));
         if (threadIdx.x == 0 && blockIdx.y == 0 && k0 + i < K)
             nmin_out[k0 + i] = nmin[i];
     }
-    __syncthreads();
     const size_t plane = (size_t) prows * ldn / 2;
     for (int j = ja + threadIdx.x; j < jb; j += 256) {
         OzPoint o[2];
@@ -898,8 +933,6 @@ int oze_r_digits(OzE *st, int ch, int k0, int kb, double c, bool squares, bool p
 {
     if (products && !st->acc_whole)
         OZ_TRY(chunk_products(st, ch, s));
-    const auto kernel = squares ? oz_digits_kernel<true> : oz_digits_kernel<false>;
-    OZ_TRY(table_smem(kernel));
     const int n0 = ch * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
     const int ldn = rup(nn, PANEL), kblocks = ceil_div(kb, DG_K);
     // ranges of points: about four blocks an SM, at least 1024 points each
@@ -908,7 +941,11 @@ int oze_r_digits(OzE *st, int ch, int k0, int kb, double c, bool squares, bool p
     parts = ceil_div(ldn, range);
     const int64_t *acc = st->acc + (size_t) k0 * st->ldm;
     const oz::MulBase base = oz::make_mul(c * LOG2E_2);
-    if (!squares) {  // the squares' grids follow from the same exponents
+    // the squares' grids follow from the same exponents
+    const auto kernel = squares ? oz_digits_kernel<true, false>
+                                : parts == 1 ? oz_digits_kernel<false, true> : oz_digits_kernel<false, false>;
+    OZ_TRY(table_smem(kernel));
+    if (!squares && parts > 1) {
         DGTM_CUDA_TRY(cudaMemsetAsync(st->wmin, 0x7F, sizeof(unsigned) * kb, s));
         oz_rmax_kernel<<<dim3(kblocks, parts), 256, 0, s>>>(acc, st->ldm, nn, kb, st->h + k0, st->sc, st->pt + n0,
                                                             st->thr + n0, base, range, st->wmin);
