@@ -49,6 +49,12 @@ void set_error(int code, const char *fmt, ...)
 
 using namespace dgtm;
 
+// One small device-to-host copy brings back a call's scalars and status words.
+constexpr size_t CTL_DOUBLES = 10;
+// W up to this size comes back through pinned memory with them: a copy into the
+// caller's pageable memory waits for the stream by itself.
+constexpr size_t W_STAGE_MAX = 1 << 18;
+
 struct dgtm_ctx {
     int N, D, K, M1, precision, solver, device, sms;
     cudaStream_t stream;
@@ -73,11 +79,13 @@ struct dgtm_ctx {
     int nsplit, n_per_split;
     double *Gpart, *RTpart;
     double *G, *RT, *A, *B, *work, *bterm, *abpart;
-    double *scal;      // device scalars
-    int *flag;         // device status: [0..1] the solver's, [2] update_y's pair counter,
+    double *scal;      // device scalars (CTL_DOUBLES with the status words)
+    int *flag;         // device status, behind the scalars: [0..1] the solver's, [2] update_y's pair counter,
                        // [3] the digit-slice products' bounded waits
-    double *hscal;     // pinned host scalars
+    double *hscal;     // pinned host copies of scal and flag
     int *hflag;
+    double *hW;        // pinned staging of W (w_staged)
+    int w_staged;
     // split-BF16 form
     TcState *tc;
     // exact-slice FP64 form (0/1 data on sm_10x; otherwise the CUDA-core form)
@@ -169,9 +177,10 @@ int sync_and_check(dgtm_ctx *c)
     return DGTM_OK;
 }
 
-int fetch_oz_status(dgtm_ctx *c)
+// scalars and status words
+int fetch_ctl(dgtm_ctx *c)
 {
-    DGTM_CUDA_TRY(cudaMemcpyAsync(c->hflag + 3, c->flag + 3, sizeof(int), cudaMemcpyDeviceToHost,
+    DGTM_CUDA_TRY(cudaMemcpyAsync(c->hscal, c->scal, sizeof(double) * CTL_DOUBLES, cudaMemcpyDeviceToHost,
                                   c->stream));
     return DGTM_OK;
 }
@@ -271,14 +280,12 @@ void free_ctx(dgtm_ctx *c)
     void *ptrs[] = {c->T64, c->T32, c->tt, c->FI, c->FIp, c->Y64, c->Yprev, c->yyprev, c->Y32, c->yy,
                     c->W, c->colstat,
                     c->part, c->Gpart, c->RTpart, c->G, c->RT, c->A, c->B, c->work, c->bterm, c->abpart,
-                    c->scal, c->flag};
+                    c->scal};
     for (void *p : ptrs)
         if (p)
             cudaFree(p);
     if (c->hscal)
         cudaFreeHost(c->hscal);
-    if (c->hflag)
-        cudaFreeHost(c->hflag);
     if (c->tc)
         tc_destroy(c->tc);
     if (c->x64)
@@ -386,10 +393,14 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
         CK(unless_enomem(ozab_create(&c->ozab, K, M1, D, c->sms)));
     if (!c->ozab)
         CK(dev_alloc(&c->abpart, form_ab_scratch_doubles(M1, D)));
-    CK(dev_alloc(&c->scal, 8));
-    CK(dev_alloc(&c->flag, 4));
-    CKC(cudaMallocHost((void **) &c->hscal, 8 * sizeof(double)));
-    CKC(cudaMallocHost((void **) &c->hflag, 4 * sizeof(int)));
+    // scalars, then the status words; on the host W follows where it is small
+    CK(dev_alloc(&c->scal, CTL_DOUBLES));
+    c->flag = (int *) (c->scal + 8);
+    c->w_staged = (size_t) M1 * D <= W_STAGE_MAX;
+    CKC(cudaMallocHost((void **) &c->hscal,
+                       sizeof(double) * (CTL_DOUBLES + (c->w_staged ? (size_t) M1 * D : 0))));
+    c->hflag = (int *) (c->hscal + 8);
+    c->hW = c->hscal + CTL_DOUBLES;
     CKC(cudaMemsetAsync(c->flag, 0, 4 * sizeof(int), c->stream));
     memset(c->hflag, 0, 4 * sizeof(int));
 
@@ -539,7 +550,7 @@ int dgtm_estep(dgtm_ctx *ctx, double beta, int isDA, double temp, double *llh, d
                       ctx->stream, &nl);
     } else if (ctx->oze) {
         r = oze_estep(ctx->oze, ctx->Y64, ctx->yy, c1, c2, isDA, ctx->colstat, ctx->part,
-                      ref_dcut(beta), &nl, ctx->stream);
+                      ref_dcut(beta), ctx->scal, &nl, ctx->stream);
     } else if (ctx->precision == DGTM_FP64) {
         Pass1Args<double> a{ctx->T64, ctx->Y64, ctx->tt, ctx->yy, ctx->N, ctx->D, ctx->K,
                             c1, c2, isDA, ctx->colstat, ctx->part};
@@ -554,16 +565,14 @@ int dgtm_estep(dgtm_ctx *ctx, double beta, int isDA, double temp, double *llh, d
     DGTM_TRY(r);
     DGTM_TRY(phase_end(ctx, DGTM_PHASE_ESTEP, nl));
     DGTM_TRY(phase_begin(ctx, DGTM_PHASE_ESTEP_REDUCE));
-    DGTM_TRY(launch_sum_pairs(ctx->part, ctx->nblk1, ctx->scal, ctx->stream));
-    DGTM_TRY(phase_end(ctx, DGTM_PHASE_ESTEP_REDUCE, 1));
-    DGTM_CUDA_TRY(cudaMemcpyAsync(ctx->hscal, ctx->scal, 2 * sizeof(double),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
+    if (!ctx->oze)  // its last statistics block sums the terms
+        DGTM_TRY(launch_sum_pairs(ctx->part, ctx->nblk1, ctx->scal, ctx->stream));
+    DGTM_TRY(phase_end(ctx, DGTM_PHASE_ESTEP_REDUCE, ctx->oze ? 0 : 1));
+    DGTM_TRY(fetch_ctl(ctx));
     if (ctx->tc)
         DGTM_TRY(tc_fetch_status(ctx->tc, ctx->stream));
     if (ctx->x64)
         DGTM_TRY(x64_fetch_status(ctx->x64, ctx->stream));
-    if (ctx->oze)
-        DGTM_TRY(fetch_oz_status(ctx));
     DGTM_TRY(sync_and_check(ctx));
     if (ctx->oze)
         DGTM_TRY(check_oz_status(ctx));
@@ -635,12 +644,12 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
     }
     if (ctx->ozab) {
         int nab = 0;
-        DGTM_TRY(ozab_form(ctx->ozab, ctx->FI, ctx->G, ctx->RT, ctx->A, ctx->B, ctx->flag + 3, &nab,
+        DGTM_TRY(ozab_form(ctx->ozab, ctx->FI, ctx->G, ctx->RT, ctx->A, ctx->B, ctx->flag, &nab,
                            ctx->stream));
         nsmall += nab - 2;
     } else {
         DGTM_TRY(launch_form_ab(ctx->FI, ctx->G, ctx->RT, K, M1, D, ctx->A, ctx->B, ctx->abpart,
-                                ctx->stream));
+                                ctx->flag, ctx->stream));
     }
     DGTM_TRY(launch_solve(ctx->A, ctx->B, M1, D, ctx->solver, ctx->W, ctx->work, ctx->flag,
                           ctx->stream));
@@ -664,11 +673,11 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
     DGTM_TRY(launch_sum_ratio(ctx->bterm, K, ctx->sum_tt, (double) ((long long) N * D),
                               ctx->scal, ctx->stream));
     DGTM_TRY(phase_end(ctx, DGTM_PHASE_MSTEP_SOLVE, nsmall));
-    DGTM_CUDA_TRY(cudaMemcpyAsync(ctx->hscal, ctx->scal, 2 * sizeof(double),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-    DGTM_CUDA_TRY(cudaMemcpyAsync(ctx->hflag, ctx->flag, 4 * sizeof(int), cudaMemcpyDeviceToHost,
-                                  ctx->stream));
-    if (W)
+    DGTM_TRY(fetch_ctl(ctx));
+    if (W && ctx->w_staged)
+        DGTM_CUDA_TRY(cudaMemcpyAsync(ctx->hW, ctx->W, sizeof(double) * (size_t) M1 * D,
+                                      cudaMemcpyDeviceToHost, ctx->stream));
+    else if (W)
         DGTM_CUDA_TRY(copy_rows(W, sizeof(double) * (size_t) ldW, ctx->W,
                                         sizeof(double) * D, sizeof(double) * D, M1,
                                         cudaMemcpyDeviceToHost, ctx->stream));
@@ -682,6 +691,9 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
     if (ctx->tc)
         DGTM_TRY(tc_check_status(ctx->tc));
     DGTM_TRY(check_oz_status(ctx));
+    if (W && ctx->w_staged)
+        for (int m = 0; m < M1; m++)
+            memcpy(W + (size_t) m * ldW, ctx->hW + (size_t) m * D, sizeof(double) * D);
     ctx->stats_valid = 0;
     ctx->prev_valid = 1;
     ctx->rt_valid = 1;
@@ -795,7 +807,9 @@ OzE *map_slices(dgtm_ctx *c)
 {
     if (c->oze)
         return c->oze;
-    if (!c->ozmap_tried && slices_on() && oze_wanted(c->N, c->D, c->K)) {
+    // making it takes about a millisecond, which the CUDA-core map of a small problem
+    // does not
+    if (!c->ozmap_tried && slices_on() && oze_wanted(c->N, c->D, c->K) && (double) c->N * c->K >= 2e6) {
         c->ozmap_tried = 1;
         if (oze_create(&c->ozmap, oze_args(c, false), c->stream) != DGTM_OK)
             g_err[0] = 0;
@@ -836,7 +850,7 @@ int map_impl(dgtm_ctx *ctx, const double *X, int L, double *M, int ldM, bool rd)
         if (oz) {
             r = oze_map(oz, ctx->Y64, ctx->yy, ctx->colstat, c, dX, L, dM, ctx->stream);
             if (r == DGTM_OK)
-                r = fetch_oz_status(ctx);
+                r = fetch_ctl(ctx);
         } else if (rd)
             r = launch_map(ctx->T64, ctx->Yprev, ctx->tt, ctx->yyprev, ctx->colstat, ctx->N, ctx->D,
                            ctx->K, c, dX, L, dM, ctx->stream, ctx->Y64, ctx->yy);
@@ -882,7 +896,11 @@ int r_block_impl(dgtm_ctx *ctx, int k0, int nk, int n0, int nn, double *R, int l
     DGTM_TRY(dev_alloc(&dR, (size_t) nk * nn));
     // R_kn = 0 where the reference's exp(-beta d / 2) underflows
     const double dcut = ref_dcut(ctx->beta);
-    int r = rd ? launch_r_block(ctx->T64, ctx->Yprev, ctx->tt, ctx->yyprev, ctx->colstat, ctx->D,
+    // from the E-step's own distances where those are digit slices; the other forms
+    // have the slices after a large map, and use them for blocks worth their launches
+    OzE *oz = rd ? nullptr : ctx->oze ? ctx->oze : (size_t) nk * nn >= 65536 ? ctx->ozmap : nullptr;
+    int r = oz ? oze_r_block(oz, ctx->Y64, ctx->yy, ctx->colstat, c, dcut, k0, nk, n0, nn, dR, ctx->stream)
+            : rd ? launch_r_block(ctx->T64, ctx->Yprev, ctx->tt, ctx->yyprev, ctx->colstat, ctx->D,
                                 ctx->K, c, k0, nk, n0, nn, dR, ctx->stream, ctx->Y64, ctx->yy, dcut)
                : launch_r_block(ctx->T64, ctx->Y64, ctx->tt, ctx->yy, ctx->colstat, ctx->D, ctx->K,
                                 c, k0, nk, n0, nn, dR, ctx->stream, nullptr, nullptr, dcut);
@@ -890,8 +908,12 @@ int r_block_impl(dgtm_ctx *ctx, int k0, int nk, int n0, int nn, double *R, int l
     if (r == DGTM_OK)
         e = copy_rows(R, sizeof(double) * (size_t) ldR, dR, sizeof(double) * nn,
                               sizeof(double) * nn, nk, cudaMemcpyDeviceToHost, ctx->stream);
+    if (oz && r == DGTM_OK)
+        r = fetch_ctl(ctx);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(ctx->stream);
+    if (oz && e == cudaSuccess && r == DGTM_OK)
+        r = check_oz_status(ctx);
     cudaFree(dR);
     if (e != cudaSuccess) {
         set_error(DGTM_ECUDA, "dgtm_get_R_block: %s", cudaGetErrorString(e));
@@ -988,7 +1010,7 @@ int dgtm_next_ctemp_k(dgtm_ctx *ctx, double temp, double beta, double eps, const
                           gg ? dgg : nullptr, lim_scale, bounded ? budget : gbudget, dgsum, dout, dspread,
                           ctx->flag + 3, ctx->stream);
         if (rc == DGTM_OK)
-            rc = fetch_oz_status(ctx);
+            rc = fetch_ctl(ctx);
         if (rc == DGTM_OK)
             e = cudaMemcpyAsync(spread.data(), dspread, sizeof(double) * K, cudaMemcpyDeviceToHost,
                                 ctx->stream);

@@ -65,12 +65,14 @@ int launch_r_block(const double *T, const double *Y, const double *tt, const dou
 int launch_reduce_slices(const double *Gpart, const double *RTpart, int nsplit, int K,
                          int D, double *G, double *RT, cudaStream_t s);
 // A = FI^T diag(G) FI (M1 x M1), B = FI^T RT (M1 x D); scratch holds
-// form_ab_scratch_doubles(M1, D) doubles of slice partials.
+// form_ab_scratch_doubles(M1, D) doubles of slice partials.  flag[0..2], the
+// solver's status words and update_y's ticket, are set to 0.
 size_t form_ab_scratch_doubles(int M1, int D);
 int launch_form_ab(const double *FI, const double *G, const double *RT, int K, int M1,
-                   int D, double *A, double *B, double *scratch, cudaStream_t s);
+                   int D, double *A, double *B, double *scratch, int *flag, cudaStream_t s);
 // W = A^{-1} B by Cholesky (solver 0) or symmetric-eigen pseudo-inverse (solver 1).
-// work: M1*M1 + M1 doubles (+ M1*M1 for solver 1).  flag[0] != 0 on failure.
+// work: M1*M1 + M1 doubles (+ M1*M1 for solver 1).  flag[0] != 0 on failure
+// (flag[0..1] zero before).
 // kernel launches of one launch_solve
 int solve_launches(int M1, int solver);
 int launch_solve(const double *A, const double *B, int M1, int D, int solver, double *W,
@@ -87,7 +89,7 @@ struct YCopies {
 // Y = FI W, yy = |y|^2, bterm_k = G_k yy_k - 2 y_k.RT_k (G/RT may be null: no
 // bterm), and the copies in cp.  FIp: FI as (hi, lo) FP32 pairs for the
 // compensated FP32 product (FP32 and split forms), or null for FP64 FMAs.
-// ticket: one device int of scratch.  scratch (scratch_doubles doubles, may be
+// ticket: one device int, zero before.  scratch (scratch_doubles doubles, may be
 // null): room for W as FP32 pairs when W is too large for shared memory, so
 // that the compensated product does not convert it per centre; *nlaunch
 // receives the kernels launched.

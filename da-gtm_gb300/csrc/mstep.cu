@@ -140,8 +140,11 @@ __global__ void __launch_bounds__(AB_THREADS) form_ab_partial_kernel(
 // sum over slices in slice order; A is written from its upper triangle and
 // mirrored, so it is exactly symmetric
 __global__ void form_ab_reduce_kernel(const double *__restrict__ Cpart, int nslice, int M1, int D,
-                                      double *__restrict__ A, double *__restrict__ B)
+                                      double *__restrict__ A, double *__restrict__ B,
+                                      int *__restrict__ flag)
 {
+    if (blockIdx.x == 0 && threadIdx.x < 3)
+        flag[threadIdx.x] = 0;
     const int W = D + M1;
     const size_t total = (size_t) M1 * W;
     for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < total;
@@ -149,8 +152,20 @@ __global__ void form_ab_reduce_kernel(const double *__restrict__ Cpart, int nsli
         const int m = (int) (i / W), c = (int) (i % W);
         if (c >= D && c - D < m)
             continue;
+        // in slice order; sixteen loads in flight (one at a time the 67 to 76 slices
+        // of a small basis cost their memory latency each)
         double sum = 0.0;
-        for (int sl = 0; sl < nslice; sl++)
+        int sl = 0;
+        for (; sl + 16 <= nslice; sl += 16) {
+            double v[16];
+#pragma unroll
+            for (int q = 0; q < 16; q++)
+                v[q] = Cpart[(size_t) (sl + q) * total + i];
+#pragma unroll
+            for (int q = 0; q < 16; q++)
+                sum += v[q];
+        }
+        for (; sl < nslice; sl++)
             sum += Cpart[(size_t) sl * total + i];
         if (c < D) {
             B[(size_t) m * D + c] = sum;
@@ -165,7 +180,7 @@ __global__ void form_ab_reduce_kernel(const double *__restrict__ Cpart, int nsli
 size_t form_ab_scratch_doubles(int M1, int D) { return (size_t) AB_SLICES * M1 * (D + M1); }
 
 int launch_form_ab(const double *FI, const double *G, const double *RT, int K, int M1, int D,
-                   double *A, double *B, double *scratch, cudaStream_t s)
+                   double *A, double *B, double *scratch, int *flag, cudaStream_t s)
 {
     const int M1p = (M1 + 3) / 4 * 4, Wp = (D + M1 + 3) / 4 * 4;
     int kc = (int) ((48 * 1024) / (sizeof(double) * (size_t) (M1p + Wp)));
@@ -184,8 +199,9 @@ int launch_form_ab(const double *FI, const double *G, const double *RT, int K, i
                                                           slice_len, scratch);
     DGTM_CUDA_TRY(cudaGetLastError());
     const size_t total = (size_t) M1 * (D + M1);
-    int blocks = (int) ((total + 255) / 256);
-    form_ab_reduce_kernel<<<blocks, 256, 0, s>>>(scratch, nslice, M1, D, A, B);
+    // small blocks: a small basis has few elements, and their loads spread over the SMs
+    const int blocks = (int) ((total + 63) / 64);
+    form_ab_reduce_kernel<<<blocks, 64, 0, s>>>(scratch, nslice, M1, D, A, B, flag);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
@@ -727,7 +743,6 @@ int solve_launches(int M1, int solver)
 int launch_solve(const double *A, const double *B, int M1, int D, int solver, double *W,
                  double *work, int *flag, cudaStream_t s)
 {
-    DGTM_CUDA_TRY(cudaMemsetAsync(flag, 0, 2 * sizeof(int), s));
     if (solver != DGTM_SOLVE_SVD && M1 > 32 * TRI_MAXR) {
         set_error(DGTM_ENOTSUP, "the Cholesky solver supports M1 <= %d", 32 * TRI_MAXR);
         return DGTM_ENOTSUP;
@@ -1031,7 +1046,6 @@ int launch_update_y(const double *FI, const float2 *FIp, const double *W, const 
                     const YCopies &cp, int *ticket, double *scratch, size_t scratch_doubles,
                     int *nlaunch, cudaStream_t s)
 {
-    DGTM_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(int), s));
     int dev = 0, sms = 0;
     DGTM_CUDA_TRY(cudaGetDevice(&dev));
     DGTM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

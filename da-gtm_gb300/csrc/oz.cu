@@ -58,7 +58,7 @@ constexpr int SEG = 8;                     // panels per exact segment (512 elem
 constexpr size_t OZ_SMEM = 1024 + 2 * (size_t) B_BUF + A_SLOTS * (size_t) A_SLOT + 256;
 
 struct OzParams {
-    int panels, b_panel0, a_rows, b_rows, a_tile0, mtiles, ntiles, nitems, splits, item_panels;
+    int panels, b_panel0, a_rows, b_rows, a_tile0, b_row0, mtiles, ntiles, nitems, splits, item_panels;
     const int *tiles;
     int64_t *out64;
     int ext;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
 #pragma unroll
                 for (int j = 0; j < SB; j++)
                     tma_load_2d(Bst + b * B_BUF + j * B_PLANE, &tmB, &b_full[b], PANEL * (pn + p.b_panel0),
-                                j * p.b_rows + nt * TN);
+                                j * p.b_rows + p.b_row0 + nt * TN);
                 for (int i = 0; i < SA; i++, na++) {
                     if (na >= A_SLOTS && !mbar_wait(&a_empty[as], aph ^ 1u, p.status, 72)) {
                         ok = false;
@@ -368,6 +368,7 @@ int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
     p.a_rows = g.a_rows;
     p.b_rows = g.b_rows;
     p.a_tile0 = g.a_tile0;
+    p.b_row0 = g.b_row0;
     p.mtiles = g.mtiles;
     p.ntiles = g.ntiles;
     p.item_panels = g.out64 ? g.item_panels : g.panels;
@@ -416,8 +417,11 @@ __global__ void __launch_bounds__(256) ozab_reduce_kernel(const int64_t *__restr
                                                           int ext, int M1, int D, int Ap,
                                                           const unsigned long long *__restrict__ fbits,
                                                           const unsigned long long *__restrict__ wbits,
-                                                          double *__restrict__ A, double *__restrict__ B)
+                                                          double *__restrict__ A, double *__restrict__ B,
+                                                          int *__restrict__ flag)
 {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 3)
+        flag[threadIdx.x] = 0;
     const int t = blockIdx.x, v = tiles[t], mt = v >> 16, nt = v & 0xFFFF;
     for (int e = blockIdx.y * 256 + threadIdx.x; e < TM * TN; e += 256 * gridDim.y) {
         const int m = mt * TM + (e & (TM - 1)), c = nt * TN + (e >> 7);
@@ -523,7 +527,7 @@ int ozab_basis(OzAB *st, const double *FI, cudaStream_t s)
 }
 
 int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, double *A, double *B,
-              int *status, int *nlaunch, cudaStream_t s)
+              int *flag, int *nlaunch, cudaStream_t s)
 {
     const int K = st->K, M1 = st->M1, D = st->D, W = M1 + D;
     DGTM_CUDA_TRY(cudaMemsetAsync(st->wbits, 0, sizeof(unsigned long long) * W, s));
@@ -550,11 +554,11 @@ int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, dou
     g.ntile = st->ntile;
     g.out64 = st->part;
     g.item_panels = st->item_panels;
-    const int rc = launch_oz_gemm(g, st->sms, status, s);
+    const int rc = launch_oz_gemm(g, st->sms, flag + 3, s);
     if (rc != DGTM_OK)
         return rc;
     ozab_reduce_kernel<<<dim3(st->ntile, 32), 256, 0, s>>>(st->part, st->tiles, st->splits, oz_sum_ext(st->panels), M1, D, st->Ap,
-                                                          st->fbits, st->wbits, A, B);
+                                                          st->fbits, st->wbits, A, B, flag);
     DGTM_CUDA_TRY(cudaGetLastError());
     if (nlaunch)
         *nlaunch = 5;

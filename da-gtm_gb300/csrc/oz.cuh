@@ -22,6 +22,7 @@ struct OzGemm {
     int panels = 0;        // 64-deep panels of the contraction
     int a_panels = 0, b_panels = 0, b_panel0 = 0;
     int a_tile0 = 0;       // first 128-row tile of A
+    int b_row0 = 0;        // first row of B (tiles of 64 from there)
     int mtiles = 0, ntiles = 0;
     const int *tiles = nullptr;  // (mt << 16 | nt) of each tile, or null: all mtiles x ntiles
     int ntile = 0;               // entries of tiles
@@ -48,8 +49,9 @@ struct OzAB;
 int ozab_create(OzAB **out, int K, int M1, int D, int sms);
 int ozab_basis(OzAB *st, const double *FI, cudaStream_t s);
 void ozab_destroy(OzAB *st);
+// flag: [0..2] set to 0 (as launch_form_ab does), [3] the bounded waits' status word
 int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, double *A, double *B,
-              int *status, int *nlaunch, cudaStream_t s);
+              int *flag, int *nlaunch, cudaStream_t s);
 // whether the digit-slice product is the faster one at this size
 bool ozab_wanted(int K, int M1, int D);
 
@@ -71,8 +73,9 @@ bool oze_wanted(int N, int D, int K);
 int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s);
 void oze_destroy(OzE *st);
 int oze_estep_blocks(const OzE *st);
+// sums: the two totals of part
 int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, int isDA,
-              double2 *colstat, double *part, double dcut, int *nlaunch, cudaStream_t s);
+              double2 *colstat, double *part, double dcut, double *sums, int *nlaunch, cudaStream_t s);
 int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaStream_t s);
 // The parts other products with R are made of.  oze_refer: the centres' planes and
 // the points' references (kept when they are those of the last oze_estep);
@@ -85,6 +88,9 @@ int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat
 int oze_chunks(const OzE *st, int *points);
 int oze_r_digits(OzE *st, int ch, int k0, int kb, double c, bool squares, bool products, int prows,
                  __nv_bfloat16 *planes, int *nmin, cudaStream_t s);
+// R of the centres k0 .. k0 + nk and the points n0 .. n0 + nn (nk x nn)
+int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c, double dcut,
+                int k0, int nk, int n0, int nn, double *R, cudaStream_t s);
 // M = R^T X from a context's column statistics
 int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c,
             const double *X, int L, double *M, cudaStream_t s);

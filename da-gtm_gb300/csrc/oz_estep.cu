@@ -162,7 +162,12 @@ struct OzStatsArgs {
     double2 *colstat;
     OzPoint *pt;
     int64_t *thr;
-    double *part;          // 2 per block
+    unsigned long long *ybits;  // the centres' maxima, zeroed for the next call
+    double *part;          // 2 per block of the call
+    double *block_part;    // of this launch
+    double *sums;          // totals, from the last block of the call
+    int nblocks;           // of the call
+    unsigned *done;        // blocks finished (zero between calls)
 };
 
 // (hi, lo) += 2^-(x kappa) in units of 2^-63
@@ -189,11 +194,15 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
     __shared__ int64_t smax[ST_WARPS][ST_PTS];
     __shared__ uint64_t slo[2][ST_WARPS][ST_PTS];
     __shared__ uint32_t shi[2][ST_WARPS][ST_PTS];
+    __shared__ double red[32];
+    __shared__ int last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int pl = lane & (ST_PTS - 1), kg = w * (32 / ST_PTS) + lane / ST_PTS;
     const int p = blockIdx.x * ST_PTS + pl;
     const bool live = p < a.nn;
     const int64_t *acc = a.acc + (live ? p : 0);
+    if (blockIdx.x == 0 && threadIdx.x < 2)
+        a.ybits[threadIdx.x] = 0ull;
     load_table(tab, a.tab);
     int64_t m = INT64_MIN;
     for (int k0 = kg; k0 < a.K; k0 += 8 * ST_KG) {
@@ -259,10 +268,8 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
         shi[1][w][lane] = hi2;
     }
     __syncthreads();
-    if (w != 0)
-        return;
     double t1 = 0.0, t2 = 0.0;
-    if (lane < ST_PTS && live) {
+    if (w == 0 && lane < ST_PTS && live) {
 #pragma unroll
         for (int i = 1; i < ST_WARPS; i++) {
             const uint64_t v1 = slo[0][i][lane], v2 = slo[1][i][lane];
@@ -300,22 +307,46 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
         // R = 0 beyond the distance where the reference's exp(-beta d / 2) underflows
         a.thr[p] = aref == ZERO_COLUMN ? INT64_MIN : oz::scaled_int(a.tt[p] - a.dcut, -1 - u);
     }
+    if (w == 0) {
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-        t1 += __shfl_down_sync(0xffffffffu, t1, o);
-        t2 += __shfl_down_sync(0xffffffffu, t2, o);
+        for (int o = 4; o > 0; o >>= 1) {
+            t1 += __shfl_down_sync(0xffffffffu, t1, o);
+            t2 += __shfl_down_sync(0xffffffffu, t2, o);
+        }
+        if (lane == 0) {
+            a.block_part[2 * blockIdx.x] = t1;
+            a.block_part[2 * blockIdx.x + 1] = t2;
+            __threadfence();
+            last = atomicAdd(a.done, 1u) == (unsigned) a.nblocks - 1;
+        }
     }
-    if (lane == 0) {
-        a.part[2 * blockIdx.x] = t1;
-        a.part[2 * blockIdx.x + 1] = t2;
+    __syncthreads();
+    if (!last)
+        return;
+    // the call's last block: all terms, in a fixed order
+    __threadfence();
+    double u1 = 0.0, u2 = 0.0;
+    for (int i = threadIdx.x; i < a.nblocks; i += NT) {
+        u1 += __ldcg(a.part + 2 * (size_t) i);
+        u2 += __ldcg(a.part + 2 * (size_t) i + 1);
+    }
+    u1 = block_sum_fixed(u1, red);
+    u2 = block_sum_fixed(u2, red);
+    if (threadIdx.x == 0) {
+        a.sums[0] = u1;
+        a.sums[1] = u2;
+        *a.done = 0u;
     }
 }
 
 // references and exponents from a context's column statistics (d_ref, ln s)
 __global__ void oz_points_kernel(const double2 *__restrict__ colstat, const double *__restrict__ tt, int N,
                                  int K, const OzScale *__restrict__ sc, double dcut,
-                                 OzPoint *__restrict__ pt, int64_t *__restrict__ thr)
+                                 OzPoint *__restrict__ pt, int64_t *__restrict__ thr,
+                                 unsigned long long *__restrict__ ybits)
 {
+    if (blockIdx.x == 0 && threadIdx.x < 2)
+        ybits[threadIdx.x] = 0ull;
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
         const double2 cs = colstat[n];
         OzPoint o;
@@ -605,6 +636,29 @@ __global__ void __launch_bounds__(NT) oz_map_kernel(const int64_t *__restrict__ 
     }
 }
 
+// R of a block of centres and points from its distances (acc: nk rows of ldm)
+__global__ void __launch_bounds__(256) oz_rblock_kernel(const int64_t *__restrict__ acc, size_t ldm, int nk, int nn,
+                                                        const int64_t *__restrict__ h,
+                                                        const OzScale *__restrict__ sc,
+                                                        const uint64_t *__restrict__ gtab,
+                                                        const OzPoint *__restrict__ pt,
+                                                        const int64_t *__restrict__ thr, oz::MulBase kb, size_t ldR,
+                                                        double *__restrict__ R)
+{
+    extern __shared__ uint64_t tab[];
+    load_table(tab, gtab);
+    __syncthreads();
+    const oz::Mul km = oz::mul_at(kb, sc->u);
+    const size_t total = (size_t) nk * nn;
+    for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < total; i += (size_t) gridDim.x * 256) {
+        const int k = (int) (i / nn), n = (int) (i - (size_t) k * nn);
+        const int64_t v = acc[(size_t) k * ldm + n] - h[k];
+        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, km);
+        R[(size_t) k * ldR + n] =
+            W == ~0ull ? 0.0 : oz::to_double(oz::exp2_neg(W, tab), (int) (W >> oz::WFRAC) - oz::WBIAS);
+    }
+}
+
 int grid_of(size_t n, int cap)
 {
     const size_t b = (n + 255) / 256;
@@ -634,13 +688,16 @@ struct OzE {
     int64_t *part = nullptr;
     int *nmin = nullptr;
     unsigned *wmin = nullptr;
+    unsigned *done = nullptr;  // statistics blocks finished in a call
 };
 
 // The digit-slice path has fixed costs (planes of the centres, four launches a
-// chunk, tiles of 128 x 64): below this the CUDA-core kernels are as fast.
+// chunk, tiles of 128 x 64), about 60 us an EM iteration.  The CUDA-core kernels
+// take that for about 3e4 pairs: few blocks, each walking all centres (N = 1000,
+// K = 400, D = 12: 600 us).
 bool oze_wanted(int N, int D, int K)
 {
-    return D <= 4 * PANEL && K <= (1 << 20) && (double) N * K >= 2e6 && N >= 256;
+    return D <= 4 * PANEL && K <= (1 << 20) && (double) N * K >= 32768;
 }
 
 void oze_destroy(OzE *st)
@@ -714,6 +771,7 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         lay(&st->pt, sizeof(OzPoint) * N, base);
         lay(&st->thr, sizeof(int64_t) * N, base);
         lay(&st->wmin, sizeof(unsigned) * K, base);
+        lay(&st->done, sizeof(unsigned), base);
         if (a.mstep) {
             lay(&st->Tt, planes * st->Wp * st->Npk, base);
             lay(&st->Rp, planes * st->Kp128 * st->chunk, base);
@@ -729,6 +787,8 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         e = cudaMemcpy(st->tab, host_table(), TAB_BYTES, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(st->bits, 0, sizeof(unsigned long long) * (4 + D + 1), s);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(st->done, 0, sizeof(unsigned), s);
     if (e == cudaSuccess) {
         oz_absmax_kernel<<<grid_of((size_t) N * D, 1216), 256, 0, s>>>(a.T64, (size_t) N * D, a.tt, N, st->bits);
         if (!a.Tb)
@@ -775,11 +835,11 @@ int oze_estep_blocks(const OzE *st)
 
 namespace {
 
-// the centres' planes, grid and h
+// the centres' planes, grid and h (what follows zeroes bits[2..3] for the next call)
 int slice_centres(OzE *st, const double *Y, const double *yy, cudaStream_t s)
 {
     const int K = st->a.K, D = st->a.D;
-    DGTM_CUDA_TRY(cudaMemsetAsync(st->bits + 2, 0, 2 * sizeof(unsigned long long), s));
+    // bits[2..3] are 0: set so at the start and by the kernel that reads them last
     oz_absmax_kernel<<<grid_of((size_t) K * D, 608), 256, 0, s>>>(Y, (size_t) K * D, yy, K, st->bits + 2);
     DGTM_CUDA_TRY(cudaGetLastError());
     oz_slice_rows_kernel<<<grid_of((size_t) st->Kp * st->Dp / 2, 4864), 256, 0, s>>>(
@@ -834,7 +894,7 @@ constexpr double LOG2E_2 = 2.0 * 1.4426950408889634;
     } while (0)
 
 int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, int isDA, double2 *colstat,
-              double *part, double dcut, int *nlaunch, cudaStream_t s)
+              double *part, double dcut, double *sums, int *nlaunch, cudaStream_t s)
 {
     OZ_TRY(slice_centres(st, Y, yy, s));
     const bool two = isDA && c1 != c2;
@@ -863,7 +923,12 @@ int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, 
         a.pt = st->pt + n0;
         a.thr = st->thr + n0;
         a.dcut = dcut;
-        a.part = part + 2 * (size_t) (n0 / ST_PTS);
+        a.ybits = st->bits + 2;
+        a.part = part;
+        a.block_part = part + 2 * (size_t) (n0 / ST_PTS);
+        a.sums = sums;
+        a.nblocks = oze_estep_blocks(st);
+        a.done = st->done;
         kernel<<<ceil_div(nn, ST_PTS), nt, TAB_BYTES, s>>>(a);
         DGTM_CUDA_TRY(cudaGetLastError());
     }
@@ -917,7 +982,7 @@ int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat
         return DGTM_OK;
     OZ_TRY(slice_centres(st, Y, yy, s));
     oz_points_kernel<<<grid_of((size_t) st->a.N, 1216), 256, 0, s>>>(colstat, st->a.tt, st->a.N, st->a.K,
-                                                                    st->sc, dcut, st->pt, st->thr);
+                                                                    st->sc, dcut, st->pt, st->thr, st->bits + 2);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
@@ -955,6 +1020,48 @@ int oze_r_digits(OzE *st, int ch, int k0, int kb, double c, bool squares, bool p
                                                         st->pt + n0, st->thr + n0, base, range, st->wmin, prows,
                                                         ldn, planes, nmin);
     DGTM_CUDA_TRY(cudaGetLastError());
+    return DGTM_OK;
+}
+
+int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c, double dcut,
+                int k0, int nk, int n0, int nn, double *R, cudaStream_t s)
+{
+    OZ_TRY(oze_refer(st, Y, yy, colstat, dcut, s));
+    OZ_TRY(table_smem(oz_rblock_kernel));
+    const oz::MulBase base = oz::make_mul(c * LOG2E_2);
+    auto launch = [&](const int64_t *acc, size_t ldm, int n, int np) -> int {
+        oz_rblock_kernel<<<grid_of((size_t) nk * np, 1216), 256, TAB_BYTES, s>>>(
+            acc, ldm, nk, np, st->h + k0, st->sc, st->tab, st->pt + n, st->thr + n, base, (size_t) nn, R + (n - n0));
+        DGTM_CUDA_TRY(cudaGetLastError());
+        return DGTM_OK;
+    };
+    if (st->acc_whole)
+        return launch(st->acc + (size_t) k0 * st->ldm + n0, st->ldm, n0, nn);
+    // as many points at a time as the chunk buffer has room for with nk rows
+    OzGemm g;
+    g.A = st->Tp;
+    g.B = st->Yp;
+    g.sa = st->sa;
+    g.a_rows = st->Np;
+    g.b_rows = st->Kp;
+    g.b_row0 = k0;
+    g.panels = g.a_panels = g.b_panels = st->panels;
+    g.ntiles = ceil_div(nk, 64);
+    g.out = st->acc;
+    g.ncols = nk;
+    g.shift = &st->sc->shift;
+    const int first = n0 / 128 * 128;
+    const long long room = (long long) st->ldm * st->a.K / nk / 128 * 128;
+    for (long long m0 = first; m0 < n0 + nn; m0 += room) {
+        const int m1 = (int) (m0 + room < n0 + nn ? m0 + room : n0 + nn);
+        g.a_tile0 = (int) (m0 / 128);
+        g.mtiles = ceil_div(m1 - m0, 128);
+        g.mrows = (int) (m1 - m0);
+        g.ldm = (size_t) g.mrows;
+        OZ_TRY(launch_oz_gemm(g, st->a.sms, st->a.status, s));
+        const int na = m0 < n0 ? n0 : (int) m0;
+        OZ_TRY(launch(st->acc + (na - m0), g.ldm, na, m1 - na));
+    }
     return DGTM_OK;
 }
 

@@ -147,3 +147,22 @@ def test_ctemp_tight_clusters_are_redone(pkg, monkeypatch):
             c.estep(1e5, 1, 1.5)
             out.append(c.next_ctemp(1e6, 1e5, 1e-6, per_centre=True)[1])
     np.testing.assert_allclose(out[0], out[1], rtol=1e-13)  # zeros and HUGE_VAL alike
+
+
+@pytest.mark.parametrize("N,D,K,k0,nk,n0,nn", [(5000, 20, 3000, 2900, 100, 4871, 129),
+                                               (5000, 20, 3000, 1, 3, 127, 4000), (70000, 3, 500, 63, 130, 1, 69999),
+                                               (300, 5, 200, 199, 1, 299, 1)])
+def test_r_blocks(pkg, orc, N, D, K, k0, nk, n0, nn):
+    """Blocks that start and end off the tiles, from kept distances and from
+    recomputed ones, and the M-step after them."""
+    T, Y, FI, X = problem(N, D, K, K + nk)
+    beta, temp = 2.0, 1.4
+    with pkg.Context(T, FI, "fp64") as c:
+        c.set_Y(Y)
+        c.estep(beta, 1, temp)
+        Rb = c.R_block(k0, nk, n0, nn)
+        c.mstep()
+        G, _ = c.get_stats()
+    R, _, _ = oracle(orc, T, Y, beta, 1, temp)
+    assert np.max(np.abs(Rb - R[k0:k0 + nk, n0:n0 + nn])) <= 1e-13
+    assert rel(G, R.sum(1)) <= 1e-12
