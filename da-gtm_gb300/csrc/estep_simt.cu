@@ -1,5 +1,6 @@
-// estep_simt.cu -- FP64 / FP32 CUDA-core kernels of the E-step and of the
-// responsibility pass of the M-step (the "plain" precision forms).
+// estep_simt.cu -- FP64 CUDA-core kernels of the E-step and of the
+// responsibility pass of the M-step, and their FP32 form with the roles
+// exchanged (the FP32 form's own two passes are in estep_f32.cu).
 //
 // Pass 1 (n-owner): one block per 64 data points; the block streams all K
 // centres in chunks of 64 and keeps, per point, the running minimum distance
@@ -593,12 +594,16 @@ size_t pass2_simt_smem(int D)
 template <typename F>
 int launch_pass1_simt(const Pass1Args<F> &a, cudaStream_t s)
 {
-    const size_t smem = pass1_simt_smem<F>(a.D);
-    DGTM_CUDA_TRY(cudaFuncSetAttribute(pass1_simt_kernel<F>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    pass1_simt_kernel<F><<<ceil_div(a.N, BN), NT, smem, s>>>(a);
-    DGTM_CUDA_TRY(cudaGetLastError());
-    return DGTM_OK;
+    if constexpr (sizeof(F) == 4) {
+        return launch_pass1_f32(a, s);
+    } else {
+        const size_t smem = pass1_simt_smem<F>(a.D);
+        DGTM_CUDA_TRY(cudaFuncSetAttribute(pass1_simt_kernel<F>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        pass1_simt_kernel<F><<<ceil_div(a.N, BN), NT, smem, s>>>(a);
+        DGTM_CUDA_TRY(cudaGetLastError());
+        return DGTM_OK;
+    }
 }
 
 int pass1_simt_blocks(int N) { return ceil_div(N, BN); }
@@ -623,14 +628,14 @@ int launch_pass2_simt(const Pass2Args<F> &a, int nsplit, cudaStream_t s, bool ow
         set_error(DGTM_ENOTSUP, "the exchanged-role pass exists in FP32 only");
         return DGTM_ENOTSUP;
     }
+    if constexpr (sizeof(F) == 4) {
+        if (!own)
+            return launch_pass2_f32(a, nsplit, s);
+    }
     switch (ndj) {
 #define DGTM_CASE(n)                                                    \
     case n:                                                             \
-        if constexpr (sizeof(F) == 4) {                                 \
-            if (own)                                                    \
-                return launch_pass2_ndj<F, n, true>(a, nsplit, s);      \
-        }                                                               \
-        return launch_pass2_ndj<F, n, false>(a, nsplit, s);
+        return launch_pass2_ndj<F, n, sizeof(F) == 4>(a, nsplit, s);
         DGTM_CASE(1) DGTM_CASE(2) DGTM_CASE(3) DGTM_CASE(4) DGTM_CASE(5) DGTM_CASE(6)
         DGTM_CASE(7) DGTM_CASE(8) DGTM_CASE(9) DGTM_CASE(10) DGTM_CASE(11) DGTM_CASE(12)
         DGTM_CASE(13) DGTM_CASE(14) DGTM_CASE(15) DGTM_CASE(16)

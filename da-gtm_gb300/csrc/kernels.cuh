@@ -46,6 +46,9 @@ template <typename F> int launch_pass1_simt(const Pass1Args<F> &a, cudaStream_t 
 // own = true: statistics indexed by the owner rows (see estep_simt.cu).
 template <typename F>
 int launch_pass2_simt(const Pass2Args<F> &a, int nsplit, cudaStream_t s, bool own = false);
+// the FP32 form's passes (estep_f32.cu)
+int launch_pass1_f32(const Pass1Args<float> &a, cudaStream_t s);
+int launch_pass2_f32(const Pass2Args<float> &a, int nsplit, cudaStream_t s);
 int pass1_simt_blocks(int N);
 int pass2_simt_ktiles(int K);
 // M = R^T X (N x L, L <= 8) and explicit R blocks, FP64, from the column

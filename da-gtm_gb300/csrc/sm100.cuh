@@ -395,6 +395,14 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
     return r;
 }
 
+// a b + c per lane, one rounding
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
 // Fire-and-forget FP32 add of four consecutive floats in global memory
 // (performed at L2, round-to-nearest); addr must be 16-byte aligned.
 __device__ __forceinline__ void red_add_f32x4(float *addr, float a, float b, float c, float d)
