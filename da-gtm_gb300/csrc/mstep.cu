@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 
 #include <math.h>
+#include <type_traits>
 
 namespace dgtm {
 
@@ -61,14 +62,28 @@ int launch_reduce_slices(const double *Gpart, const double *RTpart, int nsplit, 
 
 // C = FI^T [RT | diag(G) FI] (M1 x (D + M1)): B = C[:, :D], A = C[:, D:]
 // (the upper triangle of A and its diagonal tiles only).
-// The K rows are cut into slices; each thread keeps a 4 x 4 FP64 tile of C
-// over its slice, fed from shared-memory copies of KC rows of FI and of the
-// right operand; the slices' partial tiles are then summed in slice order.
-// The FP64 pipe (about 2 FMA per clock per SM on this part) bounds this.
+// The K rows are cut into slices; each thread keeps a 4 x 4 FP64 tile of C over its
+// slice, fed from shared memory; the slices' partial tiles are then summed in slice
+// order.  Every element is one multiply-add chain over its slice, whichever kernel
+// forms it.  The FP64 pipe (about 2 FMA per clock per SM on this part) bounds both.
+//
+// form_ab_rows_kernel (M1 <= AB_ROWS_MAX): a block stages whole rows of both
+// operands for 256 consecutive 4 x 4 tiles, so no tile of a small basis is padding.
+// form_ab_partial_kernel (above): a block forms a 64 x 64 tile of C over its
+// slice, a thread 4 x 4 of it, from shared-memory copies of AB_KC rows of its
+// FI and right-operand columns (the next rows' loads in flight meanwhile).  A warp
+// covers 8 rows x 64 columns; warps past M1 or below A's diagonal do nothing.
+// K = 32768, M1 = 513, D = 166: 14.3 ms (11.3 ms at the pipe's 0.63 TFMA/s), by
+// whole rows, staged and scaled by 86 blocks, 19.4 ms.  K = 8000, M1 = 65: 0.37 ms,
+// its second tile row holding one row, against 0.25 ms by whole rows.
+constexpr int AB_ROWS_MAX = 128;
 constexpr int AB_THREADS = 256;
 constexpr int AB_SLICES = 76;
+constexpr int AB_TILE = 64;
+constexpr int AB_KC = 16;
+constexpr int AB_LD = AB_TILE + 2;
 
-__global__ void __launch_bounds__(AB_THREADS) form_ab_partial_kernel(
+__global__ void __launch_bounds__(AB_THREADS) form_ab_rows_kernel(
     const double *__restrict__ FI, const double *__restrict__ G, const double *__restrict__ RT,
     int K, int M1, int D, int M1p, int Wp, int kc, int slice_len, double *__restrict__ Cpart)
 {
@@ -137,6 +152,87 @@ __global__ void __launch_bounds__(AB_THREADS) form_ab_partial_kernel(
                 dst[(size_t) (m0 + i) * W + c0 + j] = acc[i][j];
 }
 
+__global__ void __launch_bounds__(AB_THREADS) form_ab_partial_kernel(
+    const double *__restrict__ FI, const double *__restrict__ G, const double *__restrict__ RT,
+    int K, int M1, int D, int nct, int slice_len, double *__restrict__ Cpart)
+{
+    __shared__ __align__(16) double FIs[AB_KC * AB_LD], Rs[AB_KC * AB_LD];
+    const int W = D + M1;
+    const int mt = (blockIdx.y / nct) * AB_TILE, ct = (blockIdx.y % nct) * AB_TILE;
+    // a tile of A strictly below the diagonal is not formed: the reduction
+    // takes A from its upper triangle and mirrors it
+    if (ct >= D && ct + AB_TILE - 1 - D < mt)
+        return;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    const int m0 = mt + 4 * ty, c0 = ct + 4 * tx;
+    const int wm = mt + 8 * (threadIdx.x >> 5);  // the warp's first row
+    const bool active = wm < M1 && !(ct >= D && ct + AB_TILE - 1 - D < wm);
+    const int kb = blockIdx.x * slice_len, ke = min(K, kb + slice_len);
+    // staging: row sr + 4 q, column sc of both operands
+    const int sr = threadIdx.x >> 6, sc = threadIdx.x & 63;
+    const int gm = mt + sc, gc = ct + sc;
+    double fv[AB_KC / 4], rv[AB_KC / 4];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < AB_KC / 4; q++) {
+            const int k = k0 + sr + 4 * q;
+            fv[q] = (k < ke && gm < M1) ? FI[(size_t) k * M1 + gm] : 0.0;
+            double v = 0.0;
+            if (k < ke) {
+                if (gc < D)
+                    v = RT[(size_t) k * D + gc];
+                else if (gc < W)
+                    v = G[k] * FI[(size_t) k * M1 + (gc - D)];
+            }
+            rv[q] = v;
+        }
+    };
+    double acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            acc[i][j] = 0.0;
+    fetch(kb);
+    for (int k0 = kb; k0 < ke; k0 += AB_KC) {
+        const int nk = min(AB_KC, ke - k0);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < AB_KC / 4; q++) {
+            FIs[(sr + 4 * q) * AB_LD + sc] = fv[q];
+            Rs[(sr + 4 * q) * AB_LD + sc] = rv[q];
+        }
+        __syncthreads();
+        if (k0 + AB_KC < ke)
+            fetch(k0 + AB_KC);
+        if (active) {
+#pragma unroll 4
+            for (int r = 0; r < nk; r++) {
+                const double2 a01 = *(const double2 *) &FIs[r * AB_LD + 4 * ty];
+                const double2 a23 = *(const double2 *) &FIs[r * AB_LD + 4 * ty + 2];
+                const double2 b01 = *(const double2 *) &Rs[r * AB_LD + 4 * tx];
+                const double2 b23 = *(const double2 *) &Rs[r * AB_LD + 4 * tx + 2];
+                const double av[4] = {a01.x, a01.y, a23.x, a23.y};
+                const double bv[4] = {b01.x, b01.y, b23.x, b23.y};
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+            }
+        }
+    }
+    if (!active)
+        return;
+    double *dst = Cpart + (size_t) blockIdx.x * M1 * W;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (m0 + i < M1 && c0 + j < W)
+                dst[(size_t) (m0 + i) * W + c0 + j] = acc[i][j];
+}
+
 // sum over slices in slice order; A is written from its upper triangle and
 // mirrored, so it is exactly symmetric
 __global__ void form_ab_reduce_kernel(const double *__restrict__ Cpart, int nslice, int M1, int D,
@@ -182,21 +278,20 @@ size_t form_ab_scratch_doubles(int M1, int D) { return (size_t) AB_SLICES * M1 *
 int launch_form_ab(const double *FI, const double *G, const double *RT, int K, int M1, int D,
                    double *A, double *B, double *scratch, int *flag, cudaStream_t s)
 {
-    const int M1p = (M1 + 3) / 4 * 4, Wp = (D + M1 + 3) / 4 * 4;
-    int kc = (int) ((48 * 1024) / (sizeof(double) * (size_t) (M1p + Wp)));
-    if (kc > 16)
-        kc = 16;
-    if (kc < 1) {
-        set_error(DGTM_ENOTSUP, "form_ab: M1 + D too large (%d)", M1 + D);
-        return DGTM_ENOTSUP;
-    }
     const int slice_len = ceil_div(K, AB_SLICES);
     const int nslice = ceil_div(K, slice_len);
-    const int ntiles = (M1p / 4) * (Wp / 4);
-    const dim3 grid(nslice, ceil_div(ntiles, AB_THREADS));
-    const size_t smem = sizeof(double) * (size_t) kc * (M1p + Wp);
-    form_ab_partial_kernel<<<grid, AB_THREADS, smem, s>>>(FI, G, RT, K, M1, D, M1p, Wp, kc,
-                                                          slice_len, scratch);
+    if (M1 <= AB_ROWS_MAX) {
+        const int M1p = (M1 + 3) / 4 * 4, Wp = (D + M1 + 3) / 4 * 4;
+        int kc = (int) ((48 * 1024) / (sizeof(double) * (size_t) (M1p + Wp)));
+        kc = kc > 16 ? 16 : kc;  // at least 11: M1 + D <= 384
+        form_ab_rows_kernel<<<dim3(nslice, ceil_div((M1p / 4) * (Wp / 4), AB_THREADS)), AB_THREADS,
+                              sizeof(double) * (size_t) kc * (M1p + Wp), s>>>(FI, G, RT, K, M1, D, M1p, Wp, kc,
+                                                                              slice_len, scratch);
+    } else {
+        const int nct = ceil_div(D + M1, AB_TILE);
+        form_ab_partial_kernel<<<dim3(nslice, ceil_div(M1, AB_TILE) * nct), AB_THREADS, 0, s>>>(
+            FI, G, RT, K, M1, D, nct, slice_len, scratch);
+    }
     DGTM_CUDA_TRY(cudaGetLastError());
     const size_t total = (size_t) M1 * (D + M1);
     // small blocks: a small basis has few elements, and their loads spread over the SMs
@@ -210,7 +305,7 @@ int launch_form_ab(const double *FI, const double *G, const double *RT, int K, i
 // solvers
 // ---------------------------------------------------------------------------
 constexpr int SMEM_SOLVE_MAX = 110;  // M1 up to which L lives in shared memory
-constexpr int TRI_MAXR = 32;  // registers per lane in the substitution: M1 <= 1024
+constexpr int CHOL_MAX_M1 = 1024;  // the large substitution's shared vector
 
 // 1/sqrt(d) for a positive normal d: an FP32 estimate refined by two
 // Newton-Raphson steps for f(r) = 1/r^2 - d, r <- r (3 - d r^2) / 2 (each
@@ -257,75 +352,131 @@ __device__ __forceinline__ void chol_pivot(double *L, const double *adiag, int M
 }
 
 // Blocked right-looking Cholesky for M1 > SMEM_SOLVE_MAX, in panels of CHB
-// columns, so that the O(M1^3) part runs on the whole GPU: chol_panel_kernel
-// (one CTA) factorises a panel's columns one after the other over every row
-// below them, with chol_pivot's drop rule, and chol_update_kernel (one CTA per
-// 32 x 32 tile) subtracts the panel's L21 L21^T from the trailing lower
-// triangle.  The layout is that of the shared-memory kernel below: the
+// columns: chol_diag_kernel factorises the panel's diagonal block with
+// chol_pivot's drop rule (in registers), chol_rows_kernel
+// takes every row below through the same columns (one row a thread, so the rows
+// spread over the SMs), and chol_update_kernel (one CTA per 32 x 32 tile) subtracts
+// the panel's L21 L21^T from the trailing lower triangle.  Per element the
+// operations and their order are those of a factorisation column by column.  One
+// CTA doing a panel's columns over all rows in global memory, four barriers a
+// column, took 0.26 ms a panel at M1 = 513; diagonal block and rows take 0.055.
+// The layout is that of the shared-memory kernel below: the
 // scaled L (L_ij = a_ij / sqrt(d_j)) in the lower
 // triangle of work, the reciprocal diagonal after it (0 for a dropped pivot),
 // flag[0] for a non-finite pivot and flag[1] counting the drops.
 constexpr int CHB = 32;
-constexpr int CHB_THREADS = 256;
 
-__global__ void __launch_bounds__(CHB_THREADS) chol_panel_kernel(const double *__restrict__ A,
-                                                                 int M1, int p0, int w,
-                                                                 double *__restrict__ work,
-                                                                 int *flag)
+// Four warps, because a sub-partition issues one FP64 instruction in 64 clocks: lane
+// = row, warp w holds the columns 4 q + w.  The owner of column j + 1 updates it
+// first and finishes it while the others still take column j off theirs.
+constexpr int CHD_WARPS = 4;
+
+__global__ void __launch_bounds__(32 * CHD_WARPS) chol_diag_kernel(const double *__restrict__ A, int M1, int p0,
+                                                                   int w, double *__restrict__ work, int *flag)
 {
+    __shared__ double col[2][CHB];
+    constexpr int Q = CHB / CHD_WARPS;
     double *L = work;
     double *rinv = work + (size_t) M1 * M1;
-    __shared__ double r_sh;
-    __shared__ double colj[CHB];  // the scaled column j in the panel's later rows
-    __shared__ int bad, ndrop;
-    const int tid = threadIdx.x;
-    const int kend = p0 + w;
-    if (tid == 0) {
-        bad = 0;
-        ndrop = 0;
-    }
-    for (int j = p0; j < kend; j++) {
-        __syncthreads();
-        if (tid == 0) {
-            const size_t jj = (size_t) j * M1 + j;
-            const double d = L[jj], ajj = A[jj];
-            double r = 0.0;
-            if (!isfinite(d)) {
-                bad = 1;
-                L[jj] = 0.0;
-            } else if (!(d > CHOL_DROP * ajj)) {
-                ndrop++;
-                L[jj] = 0.0;  // marks a dropped unknown
-            } else {
-                r = rsqrt_nr(d);
-                L[jj] = d * r;
-            }
-            rinv[j] = r;
-            r_sh = r;
+    const int i = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    double a[Q];  // row p0 + i, columns CHD_WARPS q + wp
+    const double *row = L + (size_t) (p0 + min(i, w - 1)) * M1 + p0;
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+        a[q] = CHD_WARPS * q + wp < w ? row[CHD_WARPS * q + wp] : 0.0;
+    const double diag = A[(size_t) (p0 + min(i, w - 1)) * M1 + p0 + min(i, w - 1)];
+    int bad = 0, ndrop = 0;
+    // column j in registers q of its owner: pivot and scaling
+    auto finish = [&](double &x, int j) {
+        const double d = __shfl_sync(0xffffffffu, x, j), ajj = __shfl_sync(0xffffffffu, diag, j);
+        double r = 0.0, ljj = 0.0;  // 0 marks a dropped unknown
+        if (!isfinite(d)) {
+            bad = 1;
+        } else if (!(d > CHOL_DROP * ajj)) {
+            ndrop++;
+        } else {
+            r = rsqrt_nr(d);
+            ljj = d * r;
         }
-        __syncthreads();
-        const double r = r_sh;
-        for (int i = j + 1 + tid; i < M1; i += CHB_THREADS)
-            L[(size_t) i * M1 + j] *= r;
-        __syncthreads();
-        if (tid < kend - j - 1)
-            colj[tid] = L[(size_t) (j + 1 + tid) * M1 + j];
-        __syncthreads();
-        // the panel's later columns k (j < k < kend), rows i >= k
-        for (int i = j + 1 + tid; i < M1; i += CHB_THREADS) {
-            double *Li = L + (size_t) i * M1;
-            const double lij = Li[j];
-            const int kmax = min(i, kend - 1);
-            for (int k = j + 1; k <= kmax; k++)
-                Li[k] = fma(-lij, colj[k - j - 1], Li[k]);
-        }
-    }
+        x = i == j ? ljj : i > j ? x * r : x;
+        col[j & 1][i] = x;
+        if (i == j)
+            rinv[p0 + j] = r;
+    };
+    if (wp == 0)
+        finish(a[0], 0);
     __syncthreads();
-    if (tid == 0) {
+#pragma unroll
+    for (int j = 0; j < CHB; j++) {
+        if (j + 1 < w) {  // uniform
+            const double lij = col[j & 1][i];
+            // column j + 1 first, by its owner
+            const int qn = (j + 1) / CHD_WARPS;
+            if (wp == (j + 1) % CHD_WARPS) {
+                const double lkj = col[j & 1][j + 1];
+                if (i >= j + 1)
+                    a[qn < Q ? qn : 0] = fma(-lij, lkj, a[qn < Q ? qn : 0]);
+                finish(a[qn < Q ? qn : 0], j + 1);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                const int k = CHD_WARPS * q + wp;
+                if (CHD_WARPS * q + CHD_WARPS - 1 > j + 1 && k > j + 1) {
+                    const double lkj = col[j & 1][k];
+                    if (i >= k)
+                        a[q] = fma(-lij, lkj, a[q]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (i < w) {
+        double *dst = L + (size_t) (p0 + i) * M1 + p0;
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+            if (CHD_WARPS * q + wp <= i)
+                dst[CHD_WARPS * q + wp] = a[q];
+    }
+    if (i == 0) {
         if (bad)
             flag[0] = DGTM_ENONFINITE;
-        flag[1] += ndrop;
+        if (ndrop)
+            atomicAdd(&flag[1], ndrop);
     }
+}
+
+// rows below the diagonal block: column j scaled by r_j, then the later columns less
+// l_ij l_kj
+__global__ void __launch_bounds__(32) chol_rows_kernel(int M1, int p0, double *__restrict__ work)
+{
+    __shared__ double Ld[CHB][CHB + 1], r[CHB];
+    double *L = work;
+    const double *rinv = work + (size_t) M1 * M1;
+    const int i0 = p0 + CHB + blockIdx.x * 32, lane = threadIdx.x;
+    __shared__ double T[32][CHB + 1];  // the 32 rows, through shared memory for whole lines
+    for (int q = 0; q < 32; q++) {
+        Ld[q][lane] = L[(size_t) (p0 + q) * M1 + p0 + lane];
+        T[q][lane] = i0 + q < M1 ? L[(size_t) (i0 + q) * M1 + p0 + lane] : 0.0;
+    }
+    r[lane] = rinv[p0 + lane];
+    __syncwarp();
+    double a[CHB];
+#pragma unroll
+    for (int k = 0; k < CHB; k++)
+        a[k] = T[lane][k];
+#pragma unroll
+    for (int j = 0; j < CHB; j++) {
+        a[j] *= r[j];
+#pragma unroll
+        for (int k = j + 1; k < CHB; k++)
+            a[k] = fma(-a[j], Ld[k][j], a[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < CHB; k++)
+        T[lane][k] = a[k];
+    __syncwarp();
+    for (int q = 0; q < 32 && i0 + q < M1; q++)
+        L[(size_t) (i0 + q) * M1 + p0 + lane] = T[q][lane];
 }
 
 // L[i][k] -= sum_q L[i][p0 + q] L[k][p0 + q] over the panel's w columns, for
@@ -445,39 +596,36 @@ __global__ void __launch_bounds__(CHOL_THREADS) cholesky_small_kernel(const doub
     }
 }
 
-// Forward (L y = b) and back (L^T w = y) substitution, right-looking: one warp
-// per right-hand side (column of B), lane l holding entries l, l + 32, ...
-// in NR = ceil(M1 / 32) registers; step i broadcasts the finished entry i and
-// every lane updates the registers that can still hold later (forward) or
-// earlier (back) entries with one FMA each.  Many blocks, so the D columns
-// run on many SMs.
-constexpr int TRI_WARPS = 4;
+// Forward (L y = b) and back (L^T w = y) substitution, right-looking, one
+// right-hand side (column of B) a CTA.  For an entry p the finished entries i are
+// taken off in the order i = 0, 1, .. (forward) and from the end (back), one FMA
+// each, in both kernels.
+//
+// L in shared memory (M1 <= SMEM_SOLVE_MAX): one warp, lane l holding entries l,
+// l + 32, ... in NR = ceil(M1 / 32) registers; step i broadcasts the finished entry
+// and every lane updates the registers that can still change.  The CTA's other
+// warps only load L.
+constexpr int TRI_THREADS = 128;
 
 template <int NR>
-__global__ void __launch_bounds__(TRI_WARPS * 32) tri_solve_kernel(const double *__restrict__ Lg,
-                                                                  const double *__restrict__ B,
-                                                                  int M1, int D, int l_in_smem,
-                                                                  const int *__restrict__ flag,
-                                                                  double *__restrict__ W)
+__global__ void __launch_bounds__(TRI_THREADS) tri_solve_kernel(const double *__restrict__ Lg,
+                                                                const double *__restrict__ B,
+                                                                int M1, int D,
+                                                                const int *__restrict__ flag,
+                                                                double *__restrict__ W)
 {
     extern __shared__ double sh[];
     if (flag[0] != 0)
         return;  // non-finite factorisation: reported by the host
-    const double *L = Lg;
-    const double *inv = Lg + (size_t) M1 * M1;
-    if (l_in_smem) {
-        const size_t n = (size_t) M1 * M1 + M1;
+    const int n = M1 * M1 + M1;
 #pragma unroll 8
-        for (size_t i = threadIdx.x; i < n; i += blockDim.x)
-            sh[i] = Lg[i];
-        __syncthreads();
-        L = sh;
-        inv = sh + (size_t) M1 * M1;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int c = blockIdx.x * TRI_WARPS + warp;
-    if (c >= D)
+    for (int i = threadIdx.x; i < n; i += TRI_THREADS)
+        sh[i] = Lg[i];
+    __syncthreads();
+    if (threadIdx.x >= 32)
         return;
+    const double *L = sh, *inv = sh + (size_t) M1 * M1;
+    const int lane = threadIdx.x, c = blockIdx.x;
     double x[NR];
 #pragma unroll
     for (int r = 0; r < NR; r++) {
@@ -527,26 +675,117 @@ __global__ void __launch_bounds__(TRI_WARPS * 32) tri_solve_kernel(const double 
     }
 }
 
-using TriKernel = void (*)(const double *, const double *, int, int, int, const int *, double *);
+// L beyond shared memory: blocks of 32 entries.  Warp 0 solves a block against L's
+// 32 x 32 diagonal block; then all four warps (a sub-partition issues one FP64
+// instruction in 64 clocks) take its 32 entries off the others, a thread an entry at
+// a time, with L read by whole lines: a forward step needs columns, from the
+// transposed copy LT.  M1 = 513, D = 166: 0.54 ms; 3.0 ms with one warp reading
+// columns across rows, four right-hand sides a CTA.
+__global__ void __launch_bounds__(TRI_THREADS) tri_solve_large_kernel(const double *__restrict__ L,
+                                                                      const double *__restrict__ LT,
+                                                                      const double *__restrict__ inv,
+                                                                      const double *__restrict__ B, int M1, int D,
+                                                                      const int *__restrict__ flag,
+                                                                      double *__restrict__ W)
+{
+    __shared__ double x[1024 + 32], y[32], dg[32][33];
+    if (flag[0] != 0)
+        return;
+    const int tid = threadIdx.x, lane = tid & 31, c = blockIdx.x;
+    for (int p = tid; p < M1; p += TRI_THREADS)
+        x[p] = B[(size_t) p * D + c];
+    const int nb = (M1 + 31) / 32;
+    for (int pass = 0; pass < 2; pass++) {
+        for (int q = 0; q < nb; q++) {
+            const int b = pass ? nb - 1 - q : q, i0 = 32 * b, w = min(32, M1 - i0);
+            // dg[s][l]: what step s takes off entry l of the block (L_{l s} forward, L_{s l} back)
+            for (int s = tid >> 5; s < 32; s += TRI_THREADS / 32)
+                dg[s][lane] = (s < w && lane < w) ? (pass ? L : LT)[(size_t) (i0 + s) * M1 + i0 + lane] : 0.0;
+            __syncthreads();
+            if (tid < 32) {
+                double v = lane < w ? x[i0 + lane] : 0.0;
+                const double iv = lane < w ? inv[i0 + lane] : 0.0;
+                for (int t = 0; t < w; t++) {
+                    const int s = pass ? w - 1 - t : t;
+                    const double f = __shfl_sync(0xffffffffu, v, s) * __shfl_sync(0xffffffffu, iv, s);
+                    if (lane == s)
+                        v = f;
+                    else if (pass ? lane < s : (lane > s && lane < w))
+                        v = fma(-dg[s][lane], f, v);
+                }
+                y[lane] = v;
+                if (lane < w)
+                    x[i0 + lane] = v;
+            }
+            __syncthreads();
+            // the entries after (before) the block, up to four of a thread side by side
+            // (their chains are independent, and so are their loads)
+            const int pa = pass ? 0 : i0 + 32, pe = pass ? i0 : M1;
+            const double *M = (pass ? L : LT) + (size_t) i0 * M1;
+            for (int pb = pa; pb < pe; pb += 4 * TRI_THREADS) {
+                double v[4];
+                int p[4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    p[r] = min(pb + tid + TRI_THREADS * r, pe - 1);
+                    v[r] = x[p[r]];
+                }
+                const int nr = min(4, (pe - pb + TRI_THREADS - 1) / TRI_THREADS);
+                auto steps = [&](auto NR) {
+                    constexpr int R = decltype(NR)::value;
+#pragma unroll 4
+                    for (int t = 0; t < w; t++) {
+                        const int s = pass ? w - 1 - t : t;
+                        double l[R];
+#pragma unroll
+                        for (int r = 0; r < R; r++)
+                            l[r] = M[(size_t) s * M1 + p[r]];
+#pragma unroll
+                        for (int r = 0; r < R; r++)
+                            v[r] = fma(-l[r], y[s], v[r]);
+                    }
+                };
+                if (nr == 1)
+                    steps(std::integral_constant<int, 1>());
+                else if (nr == 2)
+                    steps(std::integral_constant<int, 2>());
+                else if (nr == 3)
+                    steps(std::integral_constant<int, 3>());
+                else
+                    steps(std::integral_constant<int, 4>());
+#pragma unroll
+                for (int r = 0; r < 4; r++)
+                    if (pb + tid + TRI_THREADS * r < pe)
+                        x[p[r]] = v[r];
+            }
+            __syncthreads();
+        }
+    }
+    for (int p = tid; p < M1; p += TRI_THREADS)
+        W[(size_t) p * D + c] = x[p];
+}
 
-// exact register counts up to 8, then buckets (the registers past M1 hold 0
-// and take no steps)
+// LT[i][p] = L[p][i], p >= i
+__global__ void __launch_bounds__(256) transpose_kernel(const double *__restrict__ L, int M1,
+                                                        double *__restrict__ LT)
+{
+    __shared__ double t[32][33];
+    const int p0 = blockIdx.x * 32, i0 = blockIdx.y * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int r = w; r < 32; r += 8)
+        t[r][lane] = (p0 + r < M1 && i0 + lane < M1) ? L[(size_t) (p0 + r) * M1 + i0 + lane] : 0.0;
+    __syncthreads();
+    for (int r = w; r < 32; r += 8)
+        if (i0 + r < M1 && p0 + lane < M1)
+            LT[(size_t) (i0 + r) * M1 + p0 + lane] = t[lane][r];
+}
+
+using TriKernel = void (*)(const double *, const double *, int, int, const int *, double *);
+
+// ceil(M1 / 32) for M1 <= SMEM_SOLVE_MAX
 TriKernel tri_solve_for(int nr)
 {
-    switch (nr) {
-    case 1: return tri_solve_kernel<1>;
-    case 2: return tri_solve_kernel<2>;
-    case 3: return tri_solve_kernel<3>;
-    case 4: return tri_solve_kernel<4>;
-    case 5: return tri_solve_kernel<5>;
-    case 6: return tri_solve_kernel<6>;
-    case 7: return tri_solve_kernel<7>;
-    case 8: return tri_solve_kernel<8>;
-    default:
-        return nr <= 12 ? tri_solve_kernel<12>
-                        : nr <= 16 ? tri_solve_kernel<16>
-                                   : nr <= 24 ? tri_solve_kernel<24> : tri_solve_kernel<32>;
-    }
+    return nr == 1 ? tri_solve_kernel<1> : nr == 2 ? tri_solve_kernel<2>
+           : nr == 3 ? tri_solve_kernel<3> : tri_solve_kernel<4>;
 }
 
 // Parallel cyclic Jacobi (round-robin pairing) on the symmetric A; the
@@ -735,16 +974,17 @@ int solve_launches(int M1, int solver)
         return 2;
     if (M1 <= SMEM_SOLVE_MAX)
         return 2;
-    // np panels, np - 1 trailing updates (none after the last), the substitution
+    // np diagonal blocks, np - 1 of the rows below and trailing updates (none after
+    // the last), L's transpose, the substitution
     const int np = ceil_div(M1, CHB);
-    return np + (np - 1) + 1;
+    return np + 2 * (np - 1) + 2;
 }
 
 int launch_solve(const double *A, const double *B, int M1, int D, int solver, double *W,
                  double *work, int *flag, cudaStream_t s)
 {
-    if (solver != DGTM_SOLVE_SVD && M1 > 32 * TRI_MAXR) {
-        set_error(DGTM_ENOTSUP, "the Cholesky solver supports M1 <= %d", 32 * TRI_MAXR);
+    if (solver != DGTM_SOLVE_SVD && M1 > CHOL_MAX_M1) {
+        set_error(DGTM_ENOTSUP, "the Cholesky solver supports M1 <= %d", CHOL_MAX_M1);
         return DGTM_ENOTSUP;
     }
     if (solver == DGTM_SOLVE_SVD && M1 > 2 * SVD_THREADS - 2) {
@@ -780,20 +1020,29 @@ int launch_solve(const double *A, const double *B, int M1, int D, int solver, do
                                           cudaMemcpyDeviceToDevice, s));
             for (int p0 = 0; p0 < M1; p0 += CHB) {
                 const int w = M1 - p0 < CHB ? M1 - p0 : CHB;
-                chol_panel_kernel<<<1, CHB_THREADS, 0, s>>>(A, M1, p0, w, work, flag);
+                chol_diag_kernel<<<1, 32 * CHD_WARPS, 0, s>>>(A, M1, p0, w, work, flag);
                 const int nt = ceil_div(M1 - p0 - w, 32);
-                if (nt > 0)
+                if (nt > 0) {
+                    chol_rows_kernel<<<nt, 32, 0, s>>>(M1, p0, work);
                     chol_update_kernel<<<nt * (nt + 1) / 2, 256, 0, s>>>(M1, p0, w, work);
+                }
             }
         }
         DGTM_CUDA_TRY(cudaGetLastError());
-        const size_t lbytes = sizeof(double) * ((size_t) M1 * M1 + M1);
-        const int l_in_smem = lbytes <= 96 * 1024;
-        const size_t tsmem = l_in_smem ? lbytes : 16;
-        const TriKernel tri = tri_solve_for(ceil_div(M1, 32));
-        DGTM_CUDA_TRY(cudaFuncSetAttribute(tri, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int) tsmem));
-        tri<<<ceil_div(D, TRI_WARPS), TRI_WARPS * 32, tsmem, s>>>(work, B, M1, D, l_in_smem, flag, W);
+        if (M1 <= SMEM_SOLVE_MAX) {
+            const size_t tsmem = sizeof(double) * ((size_t) M1 * M1 + M1);
+            const TriKernel tri = tri_solve_for(ceil_div(M1, 32));
+            DGTM_CUDA_TRY(cudaFuncSetAttribute(tri, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int) tsmem));
+            tri<<<D, TRI_THREADS, tsmem, s>>>(work, B, M1, D, flag, W);
+        } else {
+            const double *inv = work + (size_t) M1 * M1;
+            double *LT = work + (size_t) M1 * M1 + M1;  // within the solver's 2 M1^2 + M1 D
+            const int nt = ceil_div(M1, 32);
+            transpose_kernel<<<dim3(nt, nt), 256, 0, s>>>(work, M1, LT);
+            DGTM_CUDA_TRY(cudaGetLastError());
+            tri_solve_large_kernel<<<D, TRI_THREADS, 0, s>>>(work, LT, inv, B, M1, D, flag, W);
+        }
     }
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;

@@ -35,3 +35,13 @@ def test_svd_sizes(pkg, M1, D):
                                     (33000, 30, 64), (700, 250, 20)])
 def test_normal_equations_by_slices(pkg, K, M1, D):
     solve_case(pkg, M1, D, K, "cholesky")
+
+
+# the blocked Cholesky and the two substitutions: the last order in shared memory, the
+# first beyond it, whole and partial panels, every register bucket; the multiply-add
+# normal equations of the FP32 form at tiles of 64 that are only partly filled
+@pytest.mark.parametrize("M1,D,precision", [(32, 3, "fp64"), (33, 65, "fp32"), (110, 7, "fp32"), (111, 7, "fp32"),
+                                            (128, 64, "fp32"), (129, 2, "fp32"), (257, 5, "fp32"),
+                                            (400, 6, "fp64"), (513, 9, "fp32"), (700, 3, "fp64")])
+def test_cholesky_sizes(pkg, M1, D, precision):
+    solve_case(pkg, M1, D, 2 * M1 + 20, "cholesky", precision)
