@@ -26,29 +26,39 @@ def _stream(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+def _check_pair(Y, T):
+    """N, K, D of a pair of float32 CUDA matrices."""
+    if Y.dtype != torch.float32 or T.dtype != torch.float32 or not Y.is_cuda or not T.is_cuda:
+        raise TypeError("Y and T must be float32 CUDA tensors")
+    K, D = Y.shape
+    N, D2 = T.shape
+    if D != D2:
+        raise ValueError("Y and T must have the same number of columns")
+    return N, K, D
+
+
+def _workspace(lib, N, K, D, device):
+    """A workspace tensor, its 256-byte aligned address and usable bytes."""
+    nbytes = ctypes.c_size_t()
+    _pkg._check(lib.dgtm_fe_workspace_size(N, K, D, ctypes.byref(nbytes)))
+    ws = torch.empty(nbytes.value + 256, dtype=torch.uint8, device=device)
+    return ws, ws.data_ptr() + (-ws.data_ptr()) % 256, nbytes.value
+
+
 class FreeEnergy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, Y, T, beta, temp):
-        if Y.dtype != torch.float32 or T.dtype != torch.float32 or not Y.is_cuda or not T.is_cuda:
-            raise TypeError("Y and T must be float32 CUDA tensors")
+        N, K, D = _check_pair(Y, T)
         Y = Y.contiguous()
         T = T.contiguous()
-        K, D = Y.shape
-        N, D2 = T.shape
-        if D != D2:
-            raise ValueError("Y and T must have the same number of columns")
         b = float(beta)
         lib = _pkg.load_library()
-        nbytes = ctypes.c_size_t()
-        _pkg._check(lib.dgtm_fe_workspace_size(N, K, D, ctypes.byref(nbytes)))
-        ws = torch.empty(nbytes.value + 256, dtype=torch.uint8, device=Y.device)
-        off = (-ws.data_ptr()) % 256
-        ws_ptr = ws.data_ptr() + off
+        ws, ws_ptr, nbytes = _workspace(lib, N, K, D, Y.device)
         F = torch.empty((), dtype=torch.float64, device=Y.device)
         _pkg._check(lib.dgtm_fe_forward(Y.data_ptr(), T.data_ptr(), N, K, D, b, float(temp),
-                                        ws_ptr, nbytes.value, _stream(Y.device), F.data_ptr()))
+                                        ws_ptr, nbytes, _stream(Y.device), F.data_ptr()))
         ctx.save_for_backward(Y, T, ws)
-        ctx.meta = (N, K, D, b, float(temp), ws_ptr, nbytes.value)
+        ctx.meta = (N, K, D, b, float(temp), ws_ptr, nbytes)
         ctx.beta_is_tensor = torch.is_tensor(beta)
         return F
 
@@ -81,12 +91,26 @@ def project(T_new, Y, beta, temp=1.0, steps=50, lr=None):
     step size ``lr`` (default 1/beta, which makes one step the exact
     fixed-point update t <- sum_k R_kn y_k at temp = 1).
     """
-    T = T_new.detach().clone().contiguous().requires_grad_(True)
+    T = T_new.detach().clone().contiguous()
     Yd = Y.detach().contiguous()
     step = (1.0 / float(beta)) if lr is None else lr
+    if steps < 1:
+        return T
+    if not torch.is_grad_enabled():
+        raise RuntimeError("project needs gradients: it cannot run where they are disabled")
+    N, K, D = _check_pair(Yd, T)
+    lib = _pkg.load_library()
+    stream = _stream(T.device)
+    ws, ws_ptr, nbytes = _workspace(lib, N, K, D, T.device)
+    F = torch.empty((), dtype=torch.float64, device=T.device)
+    g = torch.empty_like(T)
+    one = torch.ones((), dtype=torch.float64, device=T.device)
+    b = float(beta)
+    # the forward and the gradient in T of each step, without a graph
     for _ in range(steps):
-        F = free_energy(Yd, T, float(beta), temp)
-        (g,) = torch.autograd.grad(F, T)
-        with torch.no_grad():
-            T += step * g  # F increases towards the centres: ascend
-    return T.detach()
+        _pkg._check(lib.dgtm_fe_forward(Yd.data_ptr(), T.data_ptr(), N, K, D, b, float(temp), ws_ptr,
+                                        nbytes, stream, F.data_ptr()))
+        _pkg._check(lib.dgtm_fe_backward(Yd.data_ptr(), T.data_ptr(), N, K, D, b, float(temp), ws_ptr,
+                                         nbytes, stream, one.data_ptr(), None, g.data_ptr(), None))
+        T.add_(g, alpha=step)  # F increases towards the centres: ascend
+    return T

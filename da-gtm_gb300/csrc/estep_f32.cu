@@ -55,20 +55,6 @@ __host__ __device__ __forceinline__ Pair split(double v)
     return r;
 }
 
-// an FP32 value as FP64, by its bits (non-finite values by conversion); a subnormal
-// is first scaled by 2^24, exactly: responsibilities reach them
-__device__ __forceinline__ double widen(float f)
-{
-    const bool small = fabsf(f) < 1.17549435e-38f;
-    const uint32_t b = __float_as_uint(small ? __fmul_rn(f, 16777216.f) : f), m = b & 0x7FFFFFFFu;
-    if (m >= 0x7F800000u) {
-        asm volatile("");  // keeps the conversion behind the branch
-        return (double) f;
-    }
-    const uint32_t hi = (m >> 3) + (small ? 0x38000000u - (24u << 20) : 0x38000000u);
-    return __hiloint2double((int) ((b & 0x80000000u) | (m ? hi : 0u)), (int) (b << 29));
-}
-
 // s + e = a + b exactly
 __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
 {

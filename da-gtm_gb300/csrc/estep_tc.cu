@@ -1020,7 +1020,10 @@ constexpr int P3_SEG = 32;       // chunks per segment of the output accumulator
 struct P3Params {
     int N, D, Npad, Kpad, nchunk, nstage, nout;  // nout = D rounded up to 64
     const float4 *colq;  // Npad: (m, scale, log2 s) of each point at the temperature
-    float *C;            // N x D
+    float *C;            // N x D: the output accumulator, then dT = -g beta (t - C)
+    const float *T;      // N x D
+    const double *gF;    // g (null: 1)
+    double beta;
     int *status;
 };
 
@@ -1099,9 +1102,10 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
             for (int pn = 0; pn < NP; pn++)
                 tma_load_2d(dstage + (tp * NP + pn) * DPANEL, &tmT, t_full, PANEL_ELEMS * pn,
                             tp * p.Npad + n0);
+        int q = 0;
+        uint32_t ph = 0;
         for (int it = 0; it < 2 * p.nchunk; it++) {
-            const int q = it % nslot;
-            if (it >= nslot && !mbar_wait(&y_empty[q], ((it / nslot) & 1) ^ 1u, p.status, 41)) {
+            if (it >= nslot && !mbar_wait(&y_empty[q], ph ^ 1u, p.status, 41)) {
                 failed = 1;
                 break;
             }
@@ -1115,6 +1119,10 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
             for (int pn = 0; pn < NP; pn++)
                 tma_load_2d(Yslot + q * SLOT + pn * YPANEL, &tmY, &y_full[q], PANEL_ELEMS * pn,
                             piece * p.Kpad + c * P3_BK);
+            if (++q == nslot) {
+                q = 0;
+                ph ^= 1u;
+            }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (whole warp; one elected lane issues) ----------------
@@ -1138,6 +1146,10 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
             ok = mbar_wait_w(t_done, 0, p.status, 43);
             tc_fence_after();
         }
+        // ring positions by counters: the chunk's divisions by nslot stood on the issuer's
+        // serial path
+        int q1 = 0, q2 = 0;  // the next slot to multiply by, and to multiply R by
+        uint32_t ph1 = 0;
         for (int c = 0; ok && c <= p.nchunk; c++) {
             if (c < p.nchunk) {
                 const int b = c & 1;
@@ -1148,13 +1160,16 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
                 const uint32_t d = tmem + (uint32_t) (S_COL + b * P3_BK);
 #pragma unroll
                 for (int piece = 0; piece < 2; piece++) {
-                    const int it = 2 * c + piece, q = it % nslot;
-                    if (!mbar_wait_w(&y_full[q], (it / nslot) & 1, p.status, 45)) {
+                    if (!mbar_wait_w(&y_full[q1], ph1, p.status, 45)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t bd = yk + (uint64_t) (q * (SLOT >> 4));
+                    const uint64_t bd = yk + (uint64_t) (q1 * (SLOT >> 4));
+                    if (++q1 == nslot) {
+                        q1 = 0;
+                        ph1 ^= 1u;
+                    }
 #pragma unroll
                     for (int tp = 0; tp < (piece == 0 ? NT : 1); tp++)
 #pragma unroll
@@ -1181,7 +1196,10 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
                 }
                 tc_fence_after();
                 const uint32_t a0 = tmem + (uint32_t) (S_COL + b * P3_BK);
-                const int qh = (2 * j) % nslot, ql = (2 * j + 1) % nslot;
+                const int qh = q2;
+                q2 = q2 + 1 == nslot ? 0 : q2 + 1;
+                const int ql = q2;
+                q2 = q2 + 1 == nslot ? 0 : q2 + 1;
 #pragma unroll
                 for (int pr = 0; pr < 3; pr++) {
                     // (R hi, Y hi), (R hi, Y lo), (R lo, Y hi)
@@ -1214,8 +1232,11 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
         const uint32_t lane_base = tmem + ((uint32_t) (q * 32) << 16);
         const float4 cq = p.colq[n];  // n < Npad: padding points carry R = 0
         bool ok = true;
-        // OUT (this thread's row) to C: 32-column batches, batch i to half i % 2
-        auto drain_out = [&](bool add) {
+        // OUT (this thread's row) to C: 32-column batches, batch i to half i % 2;
+        // the last one leaves dT (NaN once a bounded wait of the call has given up)
+        auto drain_out = [&](bool add, bool last) {
+            const double g = p.gF ? p.gF[0] : 1.0;
+            const float gb = (float) (-(*(volatile int *) p.status ? NAN : g) * p.beta);
 #pragma unroll 1
             for (int c0 = 32 * h; c0 < p.nout; c0 += 64) {
                 uint32_t v[32];
@@ -1223,10 +1244,13 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
                 tmem_ld_wait();
                 if (n < p.N) {
                     float *dst = p.C + (size_t) n * p.D + c0;
+                    const float *t = p.T + (size_t) n * p.D + c0;
 #pragma unroll
                     for (int e = 0; e < 32; e++) {
-                        if (c0 + e < p.D)
-                            dst[e] = add ? dst[e] + __uint_as_float(v[e]) : __uint_as_float(v[e]);
+                        if (c0 + e < p.D) {
+                            const float o = add ? dst[e] + __uint_as_float(v[e]) : __uint_as_float(v[e]);
+                            dst[e] = last ? gb * (t[e] - o) : o;
+                        }
                     }
                 }
             }
@@ -1263,13 +1287,17 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
                     break;
                 }
                 tc_fence_after();
-                drain_out(seg > 0);
+                drain_out(seg > 0, c == p.nchunk - 1);
                 if (seg + 1 < nseg) {
                     tc_fence_before();
                     mbar_arrive(o_empty);
                 }
             }
         }
+        if (!ok && n < p.N)  // this tile's rows are not complete
+            for (int d = 32 * h; d < p.D; d += 64)
+                for (int e = d; e < min(d + 32, p.D); e++)
+                    p.C[(size_t) n * p.D + e] = NAN;
         if (!ok)
             failed = 1;
     }
@@ -1324,28 +1352,41 @@ __global__ void t_class_kernel(const double *__restrict__ T64, size_t n, int *fl
 // T pieces (nT x Npad x Dp): value pieces, three columns of ones, zero
 // padding.  F: the data as the caller holds it (FP64 for a context, FP32 for
 // the free energy); the second piece is the remainder t - hi, rounded to BF16.
+// A thread writes eight columns (16 bytes of each piece); Dp is a multiple of 64.
 template <typename F>
-__global__ void t_split_kernel(const F *__restrict__ T, int N, int D, int Dp, int Npad, int nT,
-                               __nv_bfloat16 *__restrict__ Tb)
+__global__ void __launch_bounds__(256) t_split_kernel(const F *__restrict__ T, int N, int D, int Dp, int Npad,
+                                                      int nT, __nv_bfloat16 *__restrict__ Tb)
 {
-    const size_t total = (size_t) Npad * Dp;
-    for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < total;
-         i += (size_t) gridDim.x * blockDim.x) {
-        const int n = (int) (i / Dp), d = (int) (i % Dp);
-        float hi = 0.f, lo = 0.f;
-        if (n < N) {
-            if (d < D) {
-                const F t = T[(size_t) n * D + d];
-                const __nv_bfloat16 h = __float2bfloat16_rn((float) t);
-                hi = __bfloat162float(h);
-                lo = (float) (t - (F) hi);
-            } else if (d < D + 3) {
-                hi = 1.f;
-            }
+    const int per = Dp / 8;
+    const size_t total = (size_t) Npad * per, plane = (size_t) Npad * Dp;
+    for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < total; i += (size_t) gridDim.x * 256) {
+        const int n = (int) (i / per), d0 = (int) (i - (size_t) n * per) * 8;
+        F t[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+            t[e] = (n < N && d0 + e < D) ? T[(size_t) n * D + d0 + e] : F(0);
+        float hi[8], lo[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            const int d = d0 + e;
+            hi[e] = __bfloat162float(__float2bfloat16_rn((float) t[e]));
+            lo[e] = (float) (t[e] - (F) hi[e]);
+            if (n < N && d >= D && d < D + 3)
+                hi[e] = 1.f;
         }
-        Tb[i] = __float2bfloat16_rn(hi);
-        if (nT == 2)
-            Tb[total + i] = __float2bfloat16_rn(lo);
+        uint4 h, l;
+        h.x = pack_bf16(hi[0], hi[1]);
+        h.y = pack_bf16(hi[2], hi[3]);
+        h.z = pack_bf16(hi[4], hi[5]);
+        h.w = pack_bf16(hi[6], hi[7]);
+        *(uint4 *) (Tb + 8 * i) = h;
+        if (nT == 2) {
+            l.x = pack_bf16(lo[0], lo[1]);
+            l.y = pack_bf16(lo[2], lo[3]);
+            l.z = pack_bf16(lo[4], lo[5]);
+            l.w = pack_bf16(lo[6], lo[7]);
+            *(uint4 *) (Tb + plane + 8 * i) = l;
+        }
     }
 }
 
@@ -1470,6 +1511,10 @@ P1Kernel pass1_for(int np, int kl, int nt)
 // fastest of 256 / 384 / 512 / 640 (5.56 ms against 5.72 / 5.65 / 5.63).
 static int p2_unit_tiles(int ntiles, int ktiles, int grid_max)
 {
+    // a free-energy call plans from its sizes alone, several times a step
+    static thread_local int known[4] = {-1, -1, -1, 0};
+    if (known[0] == ntiles && known[1] == ktiles && known[2] == grid_max)
+        return known[3];
     int best = 256;
     double best_cost = 0.0;
     std::vector<long> work;
@@ -1488,6 +1533,10 @@ static int p2_unit_tiles(int ntiles, int ktiles, int grid_max)
             best = ut;
         }
     }
+    known[0] = ntiles;
+    known[1] = ktiles;
+    known[2] = grid_max;
+    known[3] = best;
     return best;
 }
 
@@ -1689,7 +1738,7 @@ int tc_create(TcState **out, int N, int D, int K, int sms, const double *T64, co
         set_error(DGTM_ENOMEM, "tc_create: %s", cudaGetErrorString(e));
         return fail(DGTM_ENOMEM);
     }
-    t_split_kernel<double><<<grid_for(tpl), 256, 0, s>>>(T64, N, D, st->Dp, st->Npad, st->nT,
+    t_split_kernel<double><<<grid_for(tpl / 8), 256, 0, s>>>(T64, N, D, st->Dp, st->Npad, st->nT,
                                                          st->Tb);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1890,16 +1939,14 @@ int tc_fe_estep(const TcFeLayout &L, void *ws, const float *Y, const float *T, i
         return rc;
     st.Y32 = const_cast<float *>(Y);
     st.T32 = T;
-    DGTM_CUDA_TRY(cudaMemsetAsync(st.status, 0, sizeof(int), s));
     const size_t tpl = (size_t) st.Npad * st.Dp;
-    t_split_kernel<float><<<grid_for(tpl), 256, 0, s>>>(T, N, D, st.Dp, st.Npad, 2, st.Tb);
+    t_split_kernel<float><<<grid_for(tpl / 8), 256, 0, s>>>(T, N, D, st.Dp, st.Npad, 2, st.Tb);
     DGTM_CUDA_TRY(cudaGetLastError());
     y_split_kernel<float><<<grid_for((size_t) st.Kpad * 32, 256, 4096), 256, 0, s>>>(
         Y, K, D, st.Dp, st.Kpad, st.Yb, nullptr);
     DGTM_CUDA_TRY(cudaGetLastError());
     int nl = 0;
-    // tc_estep clears the status word again; a failure of this call shows
-    // there.  The free energy needs the statistics at `temp` only.
+    // tc_estep clears the status word.  The free energy needs the statistics at `temp` only.
     return tc_estep(&st, nullptr, c1, c2, 1, colstat, part, s, &nl, false);
 }
 
@@ -1917,8 +1964,8 @@ int tc_fe_stats(const TcFeLayout &L, void *ws, int N, int K, int D, int sms, dou
     return tc_mstep_reduce(&st, G, RT, s, &nl);
 }
 
-int tc_fe_rty(const TcFeLayout &L, void *ws, int N, int K, int D, int sms, float *C,
-              cudaStream_t s)
+int tc_fe_rty(const TcFeLayout &L, void *ws, const float *T, int N, int K, int D, int sms, double beta,
+              const double *gF, float *dT, cudaStream_t s)
 {
     TcState st{};
     TcFeLayout L2;
@@ -1934,7 +1981,10 @@ int tc_fe_rty(const TcFeLayout &L, void *ws, int N, int K, int D, int sms, float
     p.nstage = st.nstage3;
     p.nout = round_up(D, PANEL_ELEMS);  // whole 128-byte swizzle atoms of the MN-major Y
     p.colq = st.colq;
-    p.C = C;
+    p.C = dT;
+    p.T = T;
+    p.gF = gF;
+    p.beta = beta;
     p.status = st.status;
     st.pass3<<<st.Npad / P3_TILE, P3_THREADS, st.smem3, s>>>(st.tmY3, st.tmT1, p);
     DGTM_CUDA_TRY(cudaGetLastError());

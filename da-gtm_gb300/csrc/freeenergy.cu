@@ -26,8 +26,10 @@ namespace dgtm {
 
 namespace {
 
+constexpr int SQ_BLOCKS = 304;  // partial sums of |t|^2
+
 struct FeLayout {
-    size_t tt, yy, colstat, part, Gpart, RTpart, G, RT, Cpart, C, bterm, scal, tc, total;
+    size_t tt, yy, sq, colstat, part, Gpart, RTpart, G, RT, Cpart, C, bterm, tc, total;
     int nblk1, nsplit_k, n_per_split_k, nsplit_n, k_per_split_n;
     bool use_tc;
     TcFeLayout tcl;
@@ -49,14 +51,12 @@ FeLayout fe_layout(int N, int K, int D, int sms)
             return at;
         };
         L.nblk1 = L.tcl.pass1_blocks;
-        L.tt = take(sizeof(double) * N);
-        L.yy = take(sizeof(double) * K);
         L.colstat = take(sizeof(double2) * N);
         L.part = take(sizeof(double) * 2 * L.nblk1);
+        L.sq = take(sizeof(double) * SQ_BLOCKS);
         L.G = take(sizeof(double) * K);
         L.RT = take(sizeof(double) * (size_t) K * D);
         L.bterm = take(sizeof(double) * K);
-        L.scal = take(sizeof(double) * 8);
         L.tc = take(L.tcl.total);
         L.total = o;
         return L;
@@ -91,7 +91,7 @@ FeLayout fe_layout(int N, int K, int D, int sms)
     L.Cpart = take(sizeof(double) * (size_t) L.nsplit_n * ((size_t) N * D + N));
     L.C = take(sizeof(double) * ((size_t) N * D + N));
     L.bterm = take(sizeof(double) * K);
-    L.scal = take(sizeof(double) * 8);
+    L.sq = take(sizeof(double) * SQ_BLOCKS);
     L.total = o;
     return L;
 }
@@ -118,39 +118,50 @@ __global__ void norms_f32_kernel(const float *__restrict__ X, int rows, int D,
 // outputs of the call are then NaN.
 __device__ __forceinline__ bool fe_failed(const int *status) { return status && *status != 0; }
 
-// F = base + temp * S2 (S2 = sum of the per-point tempered log-sum-exp terms)
-__global__ void fe_value_kernel(const double *__restrict__ S, double base, double temp,
-                                const int *__restrict__ status, double *__restrict__ F)
+// F = base + temp * S2, S2 = the sum of the per-point tempered log-sum-exp terms of
+// pass 1's blocks (in a fixed order)
+__global__ void __launch_bounds__(1024) fe_value_kernel(const double *__restrict__ part, int nb, double base,
+                                                        double temp, const int *__restrict__ status,
+                                                        double *__restrict__ F)
 {
-    F[0] = fe_failed(status) ? NAN : base + temp * S[1];
+    __shared__ double red[32];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < nb; i += blockDim.x)  // coalesced, fixed order
+        s += part[2 * i + 1];
+    s = block_sum_fixed(s, red);
+    if (threadIdx.x == 0)
+        F[0] = fe_failed(status) ? NAN : base + temp * s;
 }
 
-// bterm_k = G_k |y_k|^2 - 2 y_k . RT_k ; dY = -g beta (G_k y_k - RT_k)
+// bterm_k = G_k |y_k|^2 - 2 y_k . RT_k (bterm may be null); dY = -g beta (G_k y_k - RT_k)
 __global__ void fe_dy_kernel(const float *__restrict__ Y, const double *__restrict__ G,
-                             const double *__restrict__ RT, const double *__restrict__ yy, int K,
-                             int D, double beta, const double *__restrict__ gF,
+                             const double *__restrict__ RT, int K, int D, double beta, const double *__restrict__ gF,
                              const int *__restrict__ status, float *__restrict__ dY,
                              double *__restrict__ bterm)
 {
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     const double g = fe_failed(status) ? NAN : (gF ? gF[0] : 1.0);
     for (int k = blockIdx.x * wpb + (threadIdx.x >> 5); k < K; k += gridDim.x * wpb) {
-        double yrt = 0.0;
+        const double gk = G[k];
+        double b = 0.0;
         for (int d = lane; d < D; d += 32) {
             const double y = (double) Y[(size_t) k * D + d], rt = RT[(size_t) k * D + d];
-            yrt += y * rt;
+            if (bterm)
+                b = fma(y, fma(gk, y, -2.0 * rt), b);
             if (dY)
-                dY[(size_t) k * D + d] = (float) (-g * beta * (G[k] * y - rt));
+                dY[(size_t) k * D + d] = (float) (-g * beta * (gk * y - rt));
         }
+        if (!bterm)
+            continue;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
-            yrt += __shfl_xor_sync(0xffffffffu, yrt, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
         if (lane == 0)
-            bterm[k] = G[k] * yy[k] - 2.0 * yrt;
+            bterm[k] = b;
     }
 }
 
-// dT = -g beta (t_n - sum_k R_kn y_k); C FP64 (CUDA-core path) ...
+// dT = -g beta (t_n - sum_k R_kn y_k) (CUDA-core path)
 __global__ void fe_dt_kernel(const float *__restrict__ T, const double *__restrict__ C, int N,
                              int D, double beta, const double *__restrict__ gF,
                              float *__restrict__ dT)
@@ -162,25 +173,56 @@ __global__ void fe_dt_kernel(const float *__restrict__ T, const double *__restri
         dT[i] = (float) (-g * beta * ((double) T[i] - C[i]));
 }
 
-// ... or FP32 in dT itself (tensor-core path), overwritten in place
-__global__ void fe_dt_inplace_kernel(const float *__restrict__ T, int N, int D, double beta,
-                                     const double *__restrict__ gF, const int *__restrict__ status,
-                                     float *__restrict__ dT)
+// part[b] = the sum of squares of block b's share of x: sum_n |t_n|^2 needs no norm
+// per point, and no reduction across a warp per point (FP64: 46 us of a call's 10^6
+// gradient at N = 65536, D = 64; this 8 us)
+__global__ void __launch_bounds__(256) fe_sumsq_kernel(const float *__restrict__ x, size_t n,
+                                                       double *__restrict__ part)
 {
-    const float gb = (float) (-(fe_failed(status) ? NAN : (gF ? gF[0] : 1.0)) * beta);
-    const size_t total = (size_t) N * D;
-    for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < total;
-         i += (size_t) gridDim.x * blockDim.x)
-        dT[i] = gb * (T[i] - dT[i]);
+    __shared__ double red[32];
+    double s = 0.0;
+    const size_t step = (size_t) gridDim.x * 256;
+    size_t i = blockIdx.x * (size_t) 256 + threadIdx.x;
+    for (; i + 7 * step < n; i += 8 * step) {
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            v[q] = x[i + q * step];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const double d = widen(v[q]);
+            s = fma(d, d, s);
+        }
+    }
+    for (; i < n; i += step) {
+        const double d = widen(x[i]);
+        s = fma(d, d, s);
+    }
+    s = block_sum_fixed(s, red);
+    if (threadIdx.x == 0)
+        part[blockIdx.x] = s;
 }
 
-// dbeta = g (N D / (2 beta) - sum R o D / 2), sum R o D = S[0]
-__global__ void fe_dbeta_kernel(const double *__restrict__ S, double ND, double beta,
-                                const double *__restrict__ gF, const int *__restrict__ status,
-                                double *__restrict__ dbeta)
+// dbeta = g (N D / (2 beta) - sum R o D / 2), and
+// sum R o D = sum_k (G_k |y_k|^2 - 2 y_k.RT_k) + sum_n |t_n|^2
+__global__ void __launch_bounds__(1024) fe_dbeta_kernel(const double *__restrict__ bterm, int K,
+                                                        const double *__restrict__ sq, int nsq, double ND,
+                                                        double beta, const double *__restrict__ gF,
+                                                        const int *__restrict__ status,
+                                                        double *__restrict__ dbeta)
 {
-    const double g = fe_failed(status) ? NAN : (gF ? gF[0] : 1.0);
-    dbeta[0] = g * (ND / (2.0 * beta) - 0.5 * S[0]);
+    __shared__ double red[32];
+    double s = 0.0, t = 0.0;
+    for (int i = threadIdx.x; i < K; i += blockDim.x)  // coalesced, fixed order
+        s += bterm[i];
+    for (int i = threadIdx.x; i < nsq; i += blockDim.x)
+        t += sq[i];
+    s = block_sum_fixed(s, red);
+    t = block_sum_fixed(t, red);
+    if (threadIdx.x == 0) {
+        const double g = fe_failed(status) ? NAN : (gF ? gF[0] : 1.0);
+        dbeta[0] = g * (ND / (2.0 * beta) - 0.5 * (s + t));
+    }
 }
 
 int grid_rows(int rows)
@@ -265,10 +307,6 @@ int dgtm_fe_forward(const float *Y, const float *T, int N, int K, int D, double 
         return DGTM_EINVAL;
     }
     cudaStream_t s = (cudaStream_t) stream;
-    double *tt = WS(double *, tt), *yy = WS(double *, yy);
-    if ((r = launch_norms_f32(T, N, D, tt, s)) != DGTM_OK ||
-        (r = launch_norms_f32(Y, K, D, yy, s)) != DGTM_OK)
-        return r;
     const int *status = nullptr;
     if (L.use_tc) {
         void *tcws = static_cast<char *>(ws) + L.tc;
@@ -277,16 +315,17 @@ int dgtm_fe_forward(const float *Y, const float *T, int N, int K, int D, double 
             return r;
         status = tc_fe_status(L.tcl, tcws);
     } else {
+        double *tt = WS(double *, tt), *yy = WS(double *, yy);
+        if ((r = launch_norms_f32(T, N, D, tt, s)) != DGTM_OK ||
+            (r = launch_norms_f32(Y, K, D, yy, s)) != DGTM_OK)
+            return r;
         Pass1Args<float> a{T, Y, tt, yy, N, D, K, beta / 2.0, beta / (2.0 * temp), 1,
                            WS(double2 *, colstat), WS(double *, part)};
         if ((r = launch_pass1_simt<float>(a, s)) != DGTM_OK)
             return r;
     }
-    double *S = WS(double *, scal);
-    if ((r = launch_sum_pairs(WS(double *, part), L.nblk1, S, s)) != DGTM_OK)
-        return r;
     const double base = N * ((D / 2.0) * log(beta / (2.0 * M_PI)) - log((double) K));
-    fe_value_kernel<<<1, 1, 0, s>>>(S, base, temp, status, F);
+    fe_value_kernel<<<1, 1024, 0, s>>>(WS(double *, part), L.nblk1, base, temp, status, F);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
@@ -303,7 +342,7 @@ int dgtm_fe_backward(const float *Y, const float *T, int N, int K, int D, double
     cudaStream_t s = (cudaStream_t) stream;
     const double c = beta / (2.0 * temp);
     double *tt = WS(double *, tt), *yy = WS(double *, yy), *G = WS(double *, G),
-           *RT = WS(double *, RT), *S = WS(double *, scal);
+           *RT = WS(double *, RT);
     const double2 *cs = WS(double2 *, colstat);
     void *tcws = L.use_tc ? static_cast<char *>(ws) + L.tc : nullptr;
     const int *status = L.use_tc ? tc_fe_status(L.tcl, tcws) : nullptr;
@@ -321,17 +360,14 @@ int dgtm_fe_backward(const float *Y, const float *T, int N, int K, int D, double
                                           D, G, RT, s)) != DGTM_OK)
                 return r;
         }
-        fe_dy_kernel<<<grid_rows(K), 256, 0, s>>>(Y, G, RT, yy, K, D, beta, gF, status, dY,
-                                                   WS(double *, bterm));
+        double *bterm = dbeta ? WS(double *, bterm) : nullptr;
+        fe_dy_kernel<<<grid_rows(K), 256, 0, s>>>(Y, G, RT, K, D, beta, gF, status, dY, bterm);
         DGTM_CUDA_TRY(cudaGetLastError());
         if (dbeta) {
-            // sum_kn R_kn d_kn = sum_k (G_k |y_k|^2 - 2 y_k.RT_k) + sum_n |t_n|^2
-            double *tsum = S + 4;
-            if ((r = launch_sum_ratio(tt, N, 0.0, 1.0, tsum, s)) != DGTM_OK)
-                return r;
-            if ((r = launch_sum_ratio_dev(WS(double *, bterm), K, tsum, S, s)) != DGTM_OK)
-                return r;
-            fe_dbeta_kernel<<<1, 1, 0, s>>>(S, (double) N * D, beta, gF, status, dbeta);
+            double *sq = WS(double *, sq);
+            fe_sumsq_kernel<<<SQ_BLOCKS, 256, 0, s>>>(T, (size_t) N * D, sq);
+            DGTM_CUDA_TRY(cudaGetLastError());
+            fe_dbeta_kernel<<<1, 1024, 0, s>>>(bterm, K, sq, SQ_BLOCKS, (double) N * D, beta, gF, status, dbeta);
             DGTM_CUDA_TRY(cudaGetLastError());
         }
     }
@@ -341,12 +377,7 @@ int dgtm_fe_backward(const float *Y, const float *T, int N, int K, int D, double
         if (blocks > 8192)
             blocks = 8192;
         if (L.use_tc) {
-            // sum_k R_kn y_k into dT itself, then dT = -g beta (t_n - that)
-            if ((r = tc_fe_rty(L.tcl, tcws, N, K, D, sms, dT, s)) != DGTM_OK)
-                return r;
-            fe_dt_inplace_kernel<<<(unsigned) blocks, 256, 0, s>>>(T, N, D, beta, gF, status, dT);
-            DGTM_CUDA_TRY(cudaGetLastError());
-            return DGTM_OK;
+            return tc_fe_rty(L.tcl, tcws, T, N, K, D, sms, beta, gF, dT, s);
         }
         // sum_k R_kn y_k: points own the rows (with their statistics), centres streamed
         Pass2Args<float> a{Y, T, yy, tt, cs, K, D, N, c, L.k_per_split_n,

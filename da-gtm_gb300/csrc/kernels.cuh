@@ -131,9 +131,6 @@ int launch_norms_f32(const float *X, int rows, int D, double *out, cudaStream_t 
 // out[0] = sum_i v[i] (fixed order) + add; out[1] = num / out[0].
 int launch_sum_ratio(const double *v, int n, double add, double num, double *out,
                      cudaStream_t s);
-// out[0] = sum_i v[i] (fixed order) + add_dev[0].
-int launch_sum_ratio_dev(const double *v, int n, const double *add_dev, double *out,
-                         cudaStream_t s);
 // Sum of the pass-1 block partials: out[0] = sum part[2b], out[1] = sum part[2b+1].
 int launch_sum_pairs(const double *part, int nblocks, double *out, cudaStream_t s);
 // Element-wise conversion to FP32.

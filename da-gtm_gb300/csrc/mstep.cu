@@ -1382,26 +1382,6 @@ int launch_sum_ratio(const double *v, int n, double add, double num, double *out
     return DGTM_OK;
 }
 
-__global__ void __launch_bounds__(1024) sum_dev_kernel(const double *__restrict__ v, int n,
-                                                      const double *__restrict__ add, double *out)
-{
-    __shared__ double red[32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x)  // coalesced, fixed order
-        s += v[i];
-    s = block_sum_fixed(s, red);
-    if (threadIdx.x == 0)
-        out[0] = s + add[0];
-}
-
-int launch_sum_ratio_dev(const double *v, int n, const double *add_dev, double *out,
-                         cudaStream_t s)
-{
-    sum_dev_kernel<<<1, 1024, 0, s>>>(v, n, add_dev, out);
-    DGTM_CUDA_TRY(cudaGetLastError());
-    return DGTM_OK;
-}
-
 __global__ void __launch_bounds__(1024) sum_pairs_kernel(const double *__restrict__ part,
                                                         int nb, double *out)
 {

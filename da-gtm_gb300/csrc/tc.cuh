@@ -50,9 +50,10 @@ int tc_fe_estep(const TcFeLayout &L, void *ws, const float *Y, const float *T, i
 // Pass 2 and the slot sum: G = rowsum R and RT = R T (FP64) of the tempered R.
 int tc_fe_stats(const TcFeLayout &L, void *ws, int N, int K, int D, int sms, double *G,
                 double *RT, cudaStream_t s);
-// Pass 3: C = R^T Y (N x D, FP32), C_n = sum_k R_kn y_k.
-int tc_fe_rty(const TcFeLayout &L, void *ws, int N, int K, int D, int sms, float *C,
-              cudaStream_t s);
+// Pass 3: dT = -g beta (t_n - sum_k R_kn y_k) (N x D, FP32); gF: g on the device, or
+// null for 1.
+int tc_fe_rty(const TcFeLayout &L, void *ws, const float *T, int N, int K, int D, int sms, double beta,
+              const double *gF, float *dT, cudaStream_t s);
 // The device status word (non-zero: a bounded wait gave up).
 int *tc_fe_status(const TcFeLayout &L, void *ws);
 
