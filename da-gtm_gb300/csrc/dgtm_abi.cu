@@ -651,8 +651,8 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
         DGTM_TRY(launch_form_ab(ctx->FI, ctx->G, ctx->RT, K, M1, D, ctx->A, ctx->B, ctx->abpart,
                                 ctx->flag, ctx->stream));
     }
-    DGTM_TRY(launch_solve(ctx->A, ctx->B, M1, D, ctx->solver, ctx->W, ctx->work, ctx->flag,
-                          ctx->stream));
+    DGTM_TRY(launch_solve(ctx->A, ctx->B, M1, D, ctx->solver, ctx->precision == DGTM_FP64, ctx->W,
+                          ctx->work, ctx->flag, ctx->stream));
     // the E-step's copies of the new centres come out of the same kernel
     YCopies cp;
     if (ctx->precision == DGTM_FP32)

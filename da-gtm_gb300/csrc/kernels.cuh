@@ -78,7 +78,9 @@ int launch_form_ab(const double *FI, const double *G, const double *RT, int K, i
 // (flag[0..1] zero before).
 // kernel launches of one launch_solve
 int solve_launches(int M1, int solver);
-int launch_solve(const double *A, const double *B, int M1, int D, int solver, double *W,
+// fp64: the FP64 form (its pseudo-inverse may round differently from one version to
+// the next; the other forms' may not).
+int launch_solve(const double *A, const double *B, int M1, int D, int solver, bool fp64, double *W,
                  double *work, int *flag, cudaStream_t s);
 // Copies of the centres that the E-step of a form reads, written by
 // launch_update_y with Y (each may be null): the FP32 copy (K x D) and the

@@ -792,21 +792,35 @@ TriKernel tri_solve_for(int nr)
 // eigenvectors go to work[M1 M1 ..) and the inverted eigenvalues (0 where an
 // eigenvalue is exactly 0) to work[2 M1 M1 ..); then W = V diag(inv) V^T B.
 //
-// One CTA, because the M1 - 1 rounds of a sweep depend on each other; what
-// bounds it is the FP64 pipe (2 operations a clock) and, for small M1, the
-// chain of a round: angles, barrier, updates, barrier.  So S and V stay in
-// shared memory (in global memory beyond the 227 KB a block can hold:
-// M1 > SVD_SMEM_MAX); a round's rotations act on S as independent 2 x 2 blocks,
-// one per pair of pivot pairs (t <= u, mirrored), J_t^T S_tu J_u in one step
-// instead of a row pass, a barrier and a column pass; and the angle is taken
-// in FP32, with c = 1 / sqrt(1 + t^2) from it in FP64: c^2 + s^2 = 1 holds to
-// FP64, a pivot element is left at ~1e-7 of itself instead of at rounding, and
-// the next sweep removes it.  M1 = 26: 0.69 ms a solve, 5.73 ms with S and V in
-// global memory, FP64 angles and separate row and column passes.
+// One CTA, because the M1 - 1 rounds of a sweep depend on each other.  A round's
+// rotations act on S as independent 2 x 2 blocks, one per pair of pivot pairs
+// (t <= u, mirrored): J_t^T S_tu J_u in one step.  What bounds it is FP64: an SM
+// sub-partition issues one FP64 instruction in 64 clocks, so a chain of them in one
+// warp costs 64 clocks each.  Therefore:
+//   * S and V stay in shared memory (in global memory beyond M1 = SVD_SMEM_MAX);
+//   * the angle is taken in FP32 (on the pivot elements' leading bits, scaled by
+//     their larger exponent) as tan(theta / 2), and c = 2 r - 1, s = 2 tan r with
+//     r = 1 / (1 + tan^2) in FP64, so c^2 + s^2 = 1 to FP64: ten FP64 instructions.
+//     A pivot element is left at ~1e-7 of itself instead of at rounding, and the
+//     next sweep removes it;
+//   * the eigenvectors of a round are rotated by the other warps while the first
+//     ones take the next round's angles.
+// M1 = 26: 5.73 ms a solve with S and V in global memory and FP64 angles, 0.74 ms
+// with the angles' FP64 division and square root and V after S; 0.41 ms this way.
 constexpr int SVD_THREADS = 512;
 constexpr int SVD_SMEM_MAX = 112;  // 2 M1^2 doubles within 200 KB
 
 __device__ __forceinline__ int jacobi_slot(int x, int n) { return x >= n - 1 ? x - (n - 1) : x; }
+
+// x 2^-(e - 1023) to FP32's leading bits (truncated), for an exponent field of x at most e
+__device__ __forceinline__ float leading_bits(double x, int e)
+{
+    const uint32_t hi = (uint32_t) __double2hiint(x), lo = (uint32_t) __double2loint(x);
+    const int fe = (int) ((hi >> 20) & 0x7FF) - e + 127;
+    if (fe <= 0)
+        return 0.f;
+    return __uint_as_float((hi & 0x80000000u) | ((uint32_t) fe << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29));
+}
 
 template <bool SM>
 __global__ void __launch_bounds__(SVD_THREADS) jacobi_kernel(const double *__restrict__ A, int M1,
@@ -816,17 +830,33 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_kernel(const double *__res
     double *S = SM ? sh : work;                       // M1 x M1 (becomes diagonal)
     double *V = SM ? sh + (size_t) M1 * M1            // M1 x M1 eigenvectors (columns)
                    : work + (size_t) M1 * M1;
-    __shared__ double cs[SVD_THREADS], sn[SVD_THREADS];
-    __shared__ short2 pq[SVD_THREADS];
+    __shared__ double cs[2][SVD_THREADS], sn[2][SVD_THREADS];  // two rounds' rotations
+    __shared__ short2 pq[2][SVD_THREADS];
     __shared__ double red[32];
     const int tid = threadIdx.x;
     const int n = M1 + (M1 & 1);  // even number of slots; slot M1 (if any) is a dummy
-    const int h = n / 2;
+    const int h = n / 2, noff = h * (h - 1) / 2, noff32 = (noff + 31) & ~31;
+    const int na = (h + 31) & ~31;              // threads that take angles
+    const bool overlap = na <= SVD_THREADS / 2;  // the others rotate V meanwhile
     for (int i = tid; i < M1 * M1; i += SVD_THREADS) {
         S[i] = A[i];
         V[i] = ((i / M1) == (i % M1)) ? 1.0 : 0.0;
     }
+    // V <- V J of the rotations in buffer b, by threads t0 .. SVD_THREADS
+    auto rotate_v = [&](int b, int t0) {
+        for (int idx = tid - t0; idx < h * M1; idx += SVD_THREADS - t0) {
+            const int t = idx / M1, k = idx - t * M1;
+            const int p = pq[b][t].x, q = pq[b][t].y;
+            const double c = cs[b][t], s = sn[b][t];
+            if (s == 0.0)
+                continue;
+            const double vp = V[k * M1 + p], vq = V[k * M1 + q];
+            V[k * M1 + p] = c * vp - s * vq;
+            V[k * M1 + q] = s * vp + c * vq;
+        }
+    };
     __syncthreads();
+    int round = 0;  // rounds so far; their rotations alternate between the buffers
     for (int sweep = 0; sweep < 60; sweep++) {
         double off = 0.0, tot = 0.0;
         for (int i = tid; i < M1 * M1; i += SVD_THREADS) {
@@ -839,37 +869,58 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_kernel(const double *__res
         tot = block_sum_fixed(tot, red);
         if (off <= 1e-32 * tot)  // the same value in every thread
             break;
-        for (int r = 0; r < n - 1; r++) {
+        for (int r = 0; r < n - 1; r++, round++) {
+            const int b = round & 1;
             // round-robin: slot 0 fixed, the others rotate
             if (tid < h) {
-                const int a = (tid == 0) ? 0 : 1 + jacobi_slot(tid - 1 + r, n);
-                const int b = 1 + jacobi_slot(n - 2 - tid + r, n);
-                const int p = min(a, b), q = max(a, b);
+                const int x = (tid == 0) ? 0 : 1 + jacobi_slot(tid - 1 + r, n);
+                const int y = 1 + jacobi_slot(n - 2 - tid + r, n);
+                const int p = min(x, y), q = max(x, y);
                 double c = 1.0, s = 0.0;
                 if (q < M1) {
-                    const double apq = S[p * M1 + q];
+                    const double apq = S[p * M1 + q], d = S[q * M1 + q] - S[p * M1 + p];
                     if (apq != 0.0) {
-                        const float th = (float) ((S[q * M1 + q] - S[p * M1 + p]) / (2.0 * apq));
-                        const float t = copysignf(1.0f / (fabsf(th) + sqrtf(fmaf(th, th, 1.0f))), th);
-                        const double d = fma((double) t, (double) t, 1.0);
-                        c = rsqrt_nr(d);
-                        c = fma(0.5 * c, fma(-d * c, c, 1.0), c);  // to half an ulp
-                        s = (double) t * c;
+                        const int e = max((__double2hiint(apq) >> 20) & 0x7FF, (__double2hiint(d) >> 20) & 0x7FF);
+                        // fast FP32 forms: the angle only has to be near
+                        const float th = fminf(fmaxf(__fdividef(0.5f * leading_bits(d, e), leading_bits(apq, e)),
+                                                     -1e18f), 1e18f);
+                        const float a2 = fmaf(th, th, 1.0f);
+                        const float t = copysignf(__fdividef(1.0f, fabsf(th) + a2 * rsqrtf(a2)), th);
+                        const float b2 = fmaf(t, t, 1.0f);
+                        const float hf = __fdividef(t, 1.0f + b2 * rsqrtf(b2));  // tan(theta / 2)
+                        const double hd = widen(hf), den = fma(hd, hd, 1.0);
+                        double ri = widen(__fdividef(1.0f, fmaf(hf, hf, 1.0f)));
+                        ri = fma(ri, fma(-den, ri, 1.0), ri);
+                        ri = fma(ri, fma(-den, ri, 1.0), ri);
+                        c = fma(2.0, ri, -1.0);
+                        s = 2.0 * hd * ri;
                     }
                 }
-                pq[tid] = make_short2((short) p, (short) q);
-                cs[tid] = c;
-                sn[tid] = s;
+                pq[b][tid] = make_short2((short) p, (short) q);
+                cs[b][tid] = c;
+                sn[b][tid] = s;
+            } else if (overlap && tid >= na && round > 0) {
+                rotate_v(b ^ 1, na);
             }
             __syncthreads();
-            // S <- J^T S J: block (t, u) of the pairs t <= u; then V <- V J
-            const int nb = h * h;
-            for (int idx = tid; idx < nb; idx += SVD_THREADS) {
-                const int t = idx / h, u = idx - t * h;
-                if (t > u)
-                    continue;
-                const int p = pq[t].x, q = pq[t].y;
-                const double c1 = cs[t], s1 = sn[t];
+            // S <- J^T S J: block (t, u) of the pairs t < u, then (in warps of their own)
+            // the pivot blocks t = u
+            for (int idx = tid; idx < noff32 + h; idx += SVD_THREADS) {
+                int t, u;
+                if (idx < noff32) {
+                    if (idx >= noff)
+                        continue;
+                    u = (int) ((sqrtf(8.0f * (float) idx + 1.0f) + 1.0f) * 0.5f);
+                    while (u * (u + 1) / 2 <= idx)
+                        u++;
+                    while (u * (u - 1) / 2 > idx)
+                        u--;
+                    t = idx - u * (u - 1) / 2;
+                } else {
+                    t = u = idx - noff32;
+                }
+                const int p = pq[b][t].x, q = pq[b][t].y;
+                const double c1 = cs[b][t], s1 = sn[b][t];
                 if (t == u) {
                     if (q >= M1 || s1 == 0.0)
                         continue;
@@ -881,8 +932,8 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_kernel(const double *__res
                     S[p * M1 + q] = S[q * M1 + p] = s1 * cx + c1 * cy;
                     continue;
                 }
-                const int v = pq[u].x, w = pq[u].y;
-                const double c2 = cs[u], s2 = sn[u];
+                const int v = pq[b][u].x, w = pq[b][u].y;
+                const double c2 = cs[b][u], s2 = sn[b][u];
                 if (s1 == 0.0 && s2 == 0.0)
                     continue;
                 const bool hq = q < M1, hw = w < M1;  // p and v are real slots
@@ -898,19 +949,14 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_kernel(const double *__res
                 if (hq && hw)
                     S[q * M1 + w] = S[w * M1 + q] = s2 * rqv + c2 * rqw;
             }
-            for (int idx = tid; idx < h * M1; idx += SVD_THREADS) {
-                const int k = idx / h, t = idx - k * h;
-                const int p = pq[t].x, q = pq[t].y;
-                const double c = cs[t], s = sn[t];
-                if (s == 0.0)
-                    continue;
-                const double vp = V[k * M1 + p], vq = V[k * M1 + q];
-                V[k * M1 + p] = c * vp - s * vq;
-                V[k * M1 + q] = s * vp + c * vq;
-            }
+            if (!overlap)
+                rotate_v(b, 0);
             __syncthreads();
         }
     }
+    if (overlap && round > 0)
+        rotate_v((round - 1) & 1, 0);  // the last round's
+    __syncthreads();
     // the inverted eigenvalues after V, which the global variant has in place
     for (int i = tid; i < M1; i += SVD_THREADS) {
         const double lam = S[i * M1 + i];
@@ -920,6 +966,105 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_kernel(const double *__res
         for (int i = tid; i < M1 * M1; i += SVD_THREADS)
             work[M1 * M1 + i] = V[i];
     if (tid == 0)
+        flag[0] = 0;
+}
+
+// The same decomposition for the FP32 and split forms, whose rounded centres would
+// follow a last bit of W that changes (see launch_form_ab's callers): FP64 angles, and
+// a row pass and a column pass over the whole of S, element by element as these forms
+// have always had them.  S and V in shared memory where they fit.
+template <bool SM>
+__global__ void __launch_bounds__(SVD_THREADS) jacobi_passes_kernel(const double *__restrict__ A, int M1,
+                                                                   double *__restrict__ work, int *flag)
+{
+    extern __shared__ double sh[];
+    double *S = SM ? sh : work;                                  // M1 x M1 (becomes diagonal)
+    double *V = (SM ? sh : work) + (size_t) M1 * M1;             // M1 x M1 eigenvectors (columns)
+    __shared__ double cs[SVD_THREADS], sn[SVD_THREADS];
+    __shared__ int pp[SVD_THREADS], qq[SVD_THREADS];
+    __shared__ double red[32];
+    __shared__ int done;
+    const int n = M1 + (M1 & 1);  // even number of slots; slot M1 (if any) is a dummy
+    for (int i = threadIdx.x; i < M1 * M1; i += blockDim.x) {
+        S[i] = A[i];
+        V[i] = ((i / M1) == (i % M1)) ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    for (int sweep = 0; sweep < 60; sweep++) {
+        double off = 0.0, tot = 0.0;
+        for (int i = threadIdx.x; i < M1 * M1; i += blockDim.x) {
+            const double v = S[i] * S[i];
+            tot += v;
+            if ((i / M1) != (i % M1))
+                off += v;
+        }
+        off = block_sum_fixed(off, red);
+        tot = block_sum_fixed(tot, red);
+        if (threadIdx.x == 0)
+            done = (off <= 1e-32 * tot);
+        __syncthreads();
+        if (done)
+            break;
+        for (int r = 0; r < n - 1; r++) {
+            // round-robin: slot 0 fixed, the others rotate
+            for (int t = threadIdx.x; t < n / 2; t += blockDim.x) {
+                int a = (t == 0) ? 0 : 1 + ((t - 1 + r) % (n - 1));
+                int b = 1 + ((n - 2 - t + r) % (n - 1));
+                int p = min(a, b), q = max(a, b);
+                double c = 1.0, s = 0.0;
+                if (q < M1) {
+                    const double apq = S[(size_t) p * M1 + q];
+                    if (apq != 0.0) {
+                        const double app = S[(size_t) p * M1 + p], aqq = S[(size_t) q * M1 + q];
+                        const double th = (aqq - app) / (2.0 * apq);
+                        const double tt = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
+                        c = 1.0 / sqrt(tt * tt + 1.0);
+                        s = tt * c;
+                    }
+                }
+                pp[t] = p;
+                qq[t] = q;
+                cs[t] = c;
+                sn[t] = s;
+            }
+            __syncthreads();
+            // rows: S <- J^T S
+            for (int idx = threadIdx.x; idx < (n / 2) * M1; idx += blockDim.x) {
+                const int t = idx / M1, k = idx % M1;
+                const int p = pp[t], q = qq[t];
+                if (q >= M1 || sn[t] == 0.0)
+                    continue;
+                const double c = cs[t], s = sn[t];
+                const double sp = S[(size_t) p * M1 + k], sq = S[(size_t) q * M1 + k];
+                S[(size_t) p * M1 + k] = c * sp - s * sq;
+                S[(size_t) q * M1 + k] = s * sp + c * sq;
+            }
+            __syncthreads();
+            // columns: S <- S J, V <- V J
+            for (int idx = threadIdx.x; idx < (n / 2) * M1; idx += blockDim.x) {
+                const int t = idx / M1, k = idx % M1;
+                const int p = pp[t], q = qq[t];
+                if (q >= M1 || sn[t] == 0.0)
+                    continue;
+                const double c = cs[t], s = sn[t];
+                const double sp = S[(size_t) k * M1 + p], sq = S[(size_t) k * M1 + q];
+                S[(size_t) k * M1 + p] = c * sp - s * sq;
+                S[(size_t) k * M1 + q] = s * sp + c * sq;
+                const double vp = V[(size_t) k * M1 + p], vq = V[(size_t) k * M1 + q];
+                V[(size_t) k * M1 + p] = c * vp - s * vq;
+                V[(size_t) k * M1 + q] = s * vp + c * vq;
+            }
+            __syncthreads();
+        }
+    }
+    for (int i = threadIdx.x; i < M1; i += blockDim.x) {
+        const double lam = S[(size_t) i * M1 + i];
+        work[2 * (size_t) M1 * M1 + i] = lam != 0.0 ? 1.0 / lam : 0.0;
+    }
+    if (SM)
+        for (int i = threadIdx.x; i < M1 * M1; i += blockDim.x)
+            work[(size_t) M1 * M1 + i] = V[i];
+    if (threadIdx.x == 0)
         flag[0] = 0;
 }
 
@@ -980,7 +1125,7 @@ int solve_launches(int M1, int solver)
     return np + 2 * (np - 1) + 2;
 }
 
-int launch_solve(const double *A, const double *B, int M1, int D, int solver, double *W,
+int launch_solve(const double *A, const double *B, int M1, int D, int solver, bool fp64, double *W,
                  double *work, int *flag, cudaStream_t s)
 {
     if (solver != DGTM_SOLVE_SVD && M1 > CHOL_MAX_M1) {
@@ -992,15 +1137,12 @@ int launch_solve(const double *A, const double *B, int M1, int D, int solver, do
         return DGTM_ENOTSUP;
     }
     if (solver == DGTM_SOLVE_SVD) {
-        if (M1 <= SVD_SMEM_MAX) {
-            const size_t smem = sizeof(double) * 2 * (size_t) M1 * M1;
-            DGTM_CUDA_TRY(cudaFuncSetAttribute(jacobi_kernel<true>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int) smem));
-            jacobi_kernel<true><<<1, SVD_THREADS, smem, s>>>(A, M1, work, flag);
-        } else {
-            jacobi_kernel<false><<<1, SVD_THREADS, 0, s>>>(A, M1, work, flag);
-        }
+        const bool sm = M1 <= SVD_SMEM_MAX;
+        const size_t smem = sm ? sizeof(double) * 2 * (size_t) M1 * M1 : 0;
+        const auto jacobi = fp64 ? (sm ? jacobi_kernel<true> : jacobi_kernel<false>)
+                                 : (sm ? jacobi_passes_kernel<true> : jacobi_passes_kernel<false>);
+        DGTM_CUDA_TRY(cudaFuncSetAttribute(jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        jacobi<<<1, SVD_THREADS, smem, s>>>(A, M1, work, flag);
         DGTM_CUDA_TRY(cudaGetLastError());
         const size_t asmem = sizeof(double) * 2 * SVD_COLS * (size_t) M1;
         DGTM_CUDA_TRY(cudaFuncSetAttribute(svd_apply_kernel,

@@ -24,9 +24,10 @@ def solve_case(pkg, M1, D, K, solver, precision="fp64"):
 
 
 # odd and even orders, one pair, the last size in shared memory and the first beyond it
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("M1,D", [(1, 3), (2, 5), (3, 1), (26, 9), (65, 33), (112, 6), (113, 6)])
-def test_svd_sizes(pkg, M1, D):
-    solve_case(pkg, M1, D, 3 * M1 + 20, "svd")
+def test_svd_sizes(pkg, M1, D, precision):
+    solve_case(pkg, M1, D, 3 * M1 + 20, "svd", precision)
 
 
 # the normal equations by digit slices: one tile and several, ragged K, M1 and D,
