@@ -1233,7 +1233,10 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
         const float4 cq = p.colq[n];  // n < Npad: padding points carry R = 0
         bool ok = true;
         // OUT (this thread's row) to C: 32-column batches, batch i to half i % 2;
-        // the last one leaves dT (NaN once a bounded wait of the call has given up)
+        // the last one leaves dT (NaN once a bounded wait of the call has given up).
+        // A batch's loads are all issued before its first store: C and T may be any
+        // buffers, so between stores each load would wait out its own latency.
+        const bool quads = (p.D & 3) == 0 && (((uintptr_t) p.C | (uintptr_t) p.T) & 15) == 0;
         auto drain_out = [&](bool add, bool last) {
             const double g = p.gF ? p.gF[0] : 1.0;
             const float gb = (float) (-(*(volatile int *) p.status ? NAN : g) * p.beta);
@@ -1241,17 +1244,40 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
             for (int c0 = 32 * h; c0 < p.nout; c0 += 64) {
                 uint32_t v[32];
                 tmem_ld32(lane_base + (uint32_t) (O_COL + c0), v);
-                tmem_ld_wait();
-                if (n < p.N) {
-                    float *dst = p.C + (size_t) n * p.D + c0;
-                    const float *t = p.T + (size_t) n * p.D + c0;
+                float *dst = p.C + (size_t) n * p.D + c0;
+                const float *t = p.T + (size_t) n * p.D + c0;
+                const int left = n < p.N ? p.D - c0 : 0;  // columns of this row and batch
+                __align__(16) float prev[32], tv[32];
+                if (quads) {
+#pragma unroll
+                    for (int e = 0; e < 32; e += 4) {
+                        const bool in = e < left;
+                        *(float4 *) (prev + e) = add && in ? *(const float4 *) (dst + e) : float4{0.f, 0.f, 0.f, 0.f};
+                        *(float4 *) (tv + e) = last && in ? *(const float4 *) (t + e) : float4{0.f, 0.f, 0.f, 0.f};
+                    }
+                } else {
 #pragma unroll
                     for (int e = 0; e < 32; e++) {
-                        if (c0 + e < p.D) {
-                            const float o = add ? dst[e] + __uint_as_float(v[e]) : __uint_as_float(v[e]);
-                            dst[e] = last ? gb * (t[e] - o) : o;
-                        }
+                        prev[e] = add && e < left ? dst[e] : 0.f;
+                        tv[e] = last && e < left ? t[e] : 0.f;
                     }
+                }
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 32; e++) {
+                    const float o = add ? prev[e] + __uint_as_float(v[e]) : __uint_as_float(v[e]);
+                    prev[e] = last ? gb * (tv[e] - o) : o;
+                }
+                if (quads) {
+#pragma unroll
+                    for (int e = 0; e < 32; e += 4)
+                        if (e < left)
+                            *(float4 *) (dst + e) = *(const float4 *) (prev + e);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 32; e++)
+                        if (e < left)
+                            dst[e] = prev[e];
                 }
             }
         };
