@@ -67,6 +67,50 @@ constexpr int SMEM_LIMIT = 227 * 1024;
 
 __host__ __device__ constexpr int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
+// four consecutive elements, for 16-byte loads
+template <typename F>
+struct __align__(16) Quad {
+    F x, y, z, w;
+};
+
+// sum_d (y[d] - t[d])^2 in one FP32 chain.  The rows of a warp's points lie D apart, so
+// each load is a round trip to L2 or memory by itself: with rows on 16-byte boundaries 32
+// dimensions are fetched (float4, double2) before the first is used, else eight.
+template <typename F>
+__device__ __forceinline__ float sum_sq_diff(const float *__restrict__ y, const F *__restrict__ t, int D)
+{
+    float sum = 0.f;
+    int d0 = 0;
+    if ((D & 3) == 0 && (((uintptr_t) y | (uintptr_t) t) & 15) == 0) {
+        using F4 = Quad<F>;
+#pragma unroll 1
+        for (; d0 + 32 <= D; d0 += 32) {
+            float4 yv[8];
+            F4 tv[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                yv[i] = *(const float4 *) (y + d0 + 4 * i);
+                tv[i] = *(const F4 *) (t + d0 + 4 * i);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float a = yv[i].x - (float) tv[i].x, b = yv[i].y - (float) tv[i].y;
+                const float c = yv[i].z - (float) tv[i].z, d = yv[i].w - (float) tv[i].w;
+                sum = fmaf(a, a, sum);
+                sum = fmaf(b, b, sum);
+                sum = fmaf(c, c, sum);
+                sum = fmaf(d, d, sum);
+            }
+        }
+    }
+#pragma unroll 8
+    for (int d = d0; d < D; d++) {
+        const float df = y[d] - (float) t[d];
+        sum = fmaf(df, df, sum);
+    }
+    return sum;
+}
+
 struct P1Params {
     int N, D, Dp, npanel, nT, Npad, Kpad, K, nchunk, nstage, ntile;
     int ksteps;           // 16-deep MMA steps covering the D + 3 used columns
@@ -496,20 +540,11 @@ __global__ void __launch_bounds__(P1_THREADS, 1)
                         }
                     }
                 }
-            } else if (active && p.T32) {
-                const float *tn = p.T32 + (size_t) n * p.D;
-#pragma unroll 8
-                for (int d = 0; d < p.D; d++) {
-                    const float df = yk[d] - tn[d];
-                    dsum = fmaf(df, df, dsum);
-                }
             } else if (active) {
-                const double *tn = p.T64 + (size_t) n * p.D;
-#pragma unroll 8
-                for (int d = 0; d < p.D; d++) {
-                    const float df = yk[d] - (float) tn[d];
-                    dsum = fmaf(df, df, dsum);
-                }
+                if (p.T32)
+                    dsum = sum_sq_diff(yk, p.T32 + (size_t) n * p.D, p.D);
+                else
+                    dsum = sum_sq_diff(yk, p.T64 + (size_t) n * p.D, p.D);
             }
             if (active) {
                 const double dstar = (double) dsum;
