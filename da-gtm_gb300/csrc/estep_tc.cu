@@ -1034,23 +1034,27 @@ P2Kernel pass2_for(int np, int kl, int nt)
 // The transpose of pass 2's problem: points own the rows and the centres are
 // streamed.  One CTA per 128-point tile; the tile's data pieces live in
 // tensor memory as the A operand of the distance product, like pass 1.  Per
-// 64-centre chunk of Y (hi and lo pieces through a TMA ring):
-//   MMA 1  S = T Y^T (M = 128 points, N = 64 centres, A from tensor memory);
-//   eight warps (four lane quarters x two 32-centre halves) turn S into
+// chunk of Y (hi and lo pieces through a TMA ring; 128 centres, or 64 where
+// three panels leave tensor memory no room for two 128-column S buffers):
+//   MMA 1  S = T Y^T (M = 128 points, N = a chunk, A from tensor memory);
+//   four warps (the lane quarters) for each 32 centres turn S into
 //          R = exp2(scale (S - m) - log2 s) with the forward's per-point
 //          statistics, split into BF16 hi / lo and written over S;
 //   MMA 2  OUT += R Y (M = 128 points, N = D rounded up to 64, K = 16
 //          centres, A = R from tensor memory, B = the same Y chunk read
 //          MN-major): R_hi Y_hi + R_hi Y_lo + R_lo Y_hi.
 // Two S buffers let MMA 1 of the next chunk run while the warps work.  OUT
-// is moved to C (FP32, global) every P3_SEG chunks (a segment) so that no
-// accumulator runs over more than 2048 centres: the tensor pipe's FP32
-// accumulation drifts low over long runs of MMAs, as measured for pass 2.
+// is moved to C (FP32, global) every P3_SEG centres (a segment) so that no
+// accumulator runs over more: the tensor pipe's FP32 accumulation drifts low
+// over long runs of MMAs, as measured for pass 2.
 // ---------------------------------------------------------------------------
-constexpr int P3_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 responsibilities
-constexpr int P3_TILE = 128;     // points per CTA (MMA M)
-constexpr int P3_BK = 64;        // centres per chunk
-constexpr int P3_SEG = 32;       // chunks per segment of the output accumulator
+constexpr int P3_TILE = 128;  // points per CTA (MMA M)
+constexpr int P3_SEG = 2048;  // centres per segment of the output accumulator
+// centres per chunk, and threads: warp 0 TMA, warp 1 MMA, the others responsibilities
+__host__ __device__ constexpr int p3_bk(int np) { return np <= 2 ? 128 : 64; }
+__host__ __device__ constexpr int p3_threads(int np) { return 64 + 4 * p3_bk(np); }
+// ring slots (a chunk each) that first hold the data pieces
+__host__ __device__ constexpr int p3_ndata(int np, int nt) { return (nt * 64 + p3_bk(np) - 1) / p3_bk(np); }
 
 struct P3Params {
     int N, D, Npad, Kpad, nchunk, nstage, nout;  // nout = D rounded up to 64
@@ -1063,20 +1067,22 @@ struct P3Params {
 };
 
 template <int NP, int KL, int NT>
-__global__ void __launch_bounds__(P3_THREADS, 1)
+__global__ void __launch_bounds__(p3_threads(NP), 1)
     tc_rty_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmT,
                   const P3Params p)
 {
     constexpr int ACOL = NP * 32;          // TMEM columns of one data piece
     constexpr int KS = 4 * (NP - 1) + KL;  // 16-deep steps of the distance product
-    constexpr int YPANEL = P3_BK * 128;    // 8 KB: 64 centres x 64 depths
-    constexpr int SLOT = NP * YPANEL;      // one piece (hi or lo) of a chunk
+    constexpr int BK = p3_bk(NP), SEG = P3_SEG / BK;
+    constexpr int YPANEL = BK * 128;       // a chunk's centres x 64 depths
+    constexpr int PIECE = NP * YPANEL;     // hi or lo of a chunk
+    constexpr int SLOT = 2 * PIECE;
     constexpr int DPANEL = P3_TILE * 128;  // 16 KB: 128 points x 64 depths
-    constexpr int NDATA = 2 * NT;          // ring slots that first hold the data pieces
-    constexpr int S_COL = NT * ACOL;       // two 64-column S / R buffers
-    constexpr int O_COL = S_COL + 2 * P3_BK;
+    constexpr int NDATA = p3_ndata(NP, NT);
+    constexpr int S_COL = NT * ACOL;       // two S / R buffers
+    constexpr int O_COL = S_COL + 2 * BK;
     static_assert(O_COL + NP * 64 <= 512, "pass 3 tensor memory plan");
-    static_assert(NDATA * SLOT == NT * NP * DPANEL, "data pieces fill whole ring slots");
+    static_assert(NDATA * SLOT >= NT * NP * DPANEL, "data pieces fit their ring slots");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int nslot = p.nstage;
@@ -1087,8 +1093,7 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
     uint64_t *t_full = bars + 2 * nslot;
     uint64_t *t_done = t_full + 1;
     uint64_t *s_full = t_done + 1;   // [2]
-    uint64_t *s_free = s_full + 2;   // [2]
-    uint64_t *p_full = s_free + 2;   // [2]
+    uint64_t *p_full = s_full + 2;   // [2]
     uint64_t *o_full = p_full + 2;
     uint64_t *o_empty = o_full + 1;
     uint64_t *drain = o_empty + 1;
@@ -1097,7 +1102,7 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * P3_TILE;
-    const int nseg = (p.nchunk + P3_SEG - 1) / P3_SEG;
+    const int nseg = (p.nchunk + SEG - 1) / SEG;
 
     if (threadIdx.x == 0) {
         failed = 0;
@@ -1109,11 +1114,10 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
         mbar_init(t_done, 1);
         for (int b = 0; b < 2; b++) {
             mbar_init(&s_full[b], 1);
-            mbar_init(&s_free[b], 1);
-            mbar_init(&p_full[b], 256);
+            mbar_init(&p_full[b], 4 * BK);
         }
         mbar_init(o_full, 1);
-        mbar_init(o_empty, 256);
+        mbar_init(o_empty, 4 * BK);
         mbar_init(drain, 1);
         fence_barrier_init();
     }
@@ -1139,21 +1143,22 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
                             tp * p.Npad + n0);
         int q = 0;
         uint32_t ph = 0;
-        for (int it = 0; it < 2 * p.nchunk; it++) {
-            if (it >= nslot && !mbar_wait(&y_empty[q], ph ^ 1u, p.status, 41)) {
+        for (int c = 0; c < p.nchunk; c++) {
+            if (c >= nslot && !mbar_wait(&y_empty[q], ph ^ 1u, p.status, 41)) {
                 failed = 1;
                 break;
             }
-            if (it < nslot && q >= nslot - NDATA && !mbar_wait(t_done, 0, p.status, 42)) {
+            if (c < nslot && q >= nslot - NDATA && !mbar_wait(t_done, 0, p.status, 42)) {
                 failed = 1;
                 break;
             }
-            const int c = it >> 1, piece = it & 1;
             mbar_expect_tx(&y_full[q], (uint32_t) SLOT);
 #pragma unroll
-            for (int pn = 0; pn < NP; pn++)
-                tma_load_2d(Yslot + q * SLOT + pn * YPANEL, &tmY, &y_full[q], PANEL_ELEMS * pn,
-                            piece * p.Kpad + c * P3_BK);
+            for (int piece = 0; piece < 2; piece++)
+#pragma unroll
+                for (int pn = 0; pn < NP; pn++)
+                    tma_load_2d(Yslot + q * SLOT + piece * PIECE + pn * YPANEL, &tmY, &y_full[q],
+                                PANEL_ELEMS * pn, piece * p.Kpad + c * BK);
             if (++q == nslot) {
                 q = 0;
                 ph ^= 1u;
@@ -1161,7 +1166,7 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (whole warp; one elected lane issues) ----------------
-        const uint32_t id1 = idesc_bf16(P3_TILE, P3_BK, 0, 0);
+        const uint32_t id1 = idesc_bf16(P3_TILE, BK, 0, 0);
         const uint32_t id2 = idesc_bf16(P3_TILE, p.nout, 0, 1);
         const uint64_t yk = sdesc_sw128(smem_u32(Yslot), 16, 1024);      // K-major (MMA 1)
         const uint64_t ymn = sdesc_sw128(smem_u32(Yslot), YPANEL, 1024);  // MN-major (MMA 2)
@@ -1181,40 +1186,45 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
             ok = mbar_wait_w(t_done, 0, p.status, 43);
             tc_fence_after();
         }
-        // ring positions by counters: the chunk's divisions by nslot stood on the issuer's
-        // serial path
-        int q1 = 0, q2 = 0;  // the next slot to multiply by, and to multiply R by
-        uint32_t ph1 = 0;
+        // ring positions by counters: divisions by nslot would stand on the issuer's serial path
+        int q1 = 0, q2 = 0, qf = 0;  // the next slot to multiply by, to multiply R by, and
+        uint32_t ph1 = 0, phf = 0;   // the one whose emptying frees the next S buffer
         for (int c = 0; ok && c <= p.nchunk; c++) {
             if (c < p.nchunk) {
                 const int b = c & 1;
-                if (c >= 2 && !mbar_wait_w(&s_free[b], ((c - 2) >> 1) & 1, p.status, 44)) {
-                    ok = false;
-                    break;
-                }
-                const uint32_t d = tmem + (uint32_t) (S_COL + b * P3_BK);
-#pragma unroll
-                for (int piece = 0; piece < 2; piece++) {
-                    if (!mbar_wait_w(&y_full[q1], ph1, p.status, 45)) {
+                if (c >= 2) {
+                    // MMA 2 of chunk c - 2, the last reader of S buffer b, emptied its slot
+                    if (!mbar_wait_w(&y_empty[qf], phf, p.status, 44)) {
                         ok = false;
                         break;
                     }
-                    tc_fence_after();
-                    const uint64_t bd = yk + (uint64_t) (q1 * (SLOT >> 4));
-                    if (++q1 == nslot) {
-                        q1 = 0;
-                        ph1 ^= 1u;
+                    if (++qf == nslot) {
+                        qf = 0;
+                        phf ^= 1u;
                     }
+                }
+                if (!mbar_wait_w(&y_full[q1], ph1, p.status, 45)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d = tmem + (uint32_t) (S_COL + b * BK);
+                const uint64_t bd = yk + (uint64_t) (q1 * (SLOT >> 4));
+#pragma unroll
+                for (int piece = 0; piece < 2; piece++) {
 #pragma unroll
                     for (int tp = 0; tp < (piece == 0 ? NT : 1); tp++)
 #pragma unroll
                         for (int ks = 0; ks < KS; ks++)
                             mma_ts_w(d, tmem + (uint32_t) (tp * ACOL + ks * 8),
-                                     bd + (uint64_t) ((ks >> 2) * (YPANEL >> 4) + 2 * (ks & 3)), id1,
-                                     (piece | tp | ks) ? 1u : 0u);
+                                     bd + (uint64_t) (piece * (PIECE >> 4) + (ks >> 2) * (YPANEL >> 4) +
+                                                      2 * (ks & 3)),
+                                     id1, (piece | tp | ks) ? 1u : 0u);
                 }
-                if (!ok)
-                    break;
+                if (++q1 == nslot) {
+                    q1 = 0;
+                    ph1 ^= 1u;
+                }
                 mma_commit_w(&s_full[b]);
             }
             if (c > 0) {
@@ -1223,36 +1233,35 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
                     ok = false;
                     break;
                 }
-                const int seg = j / P3_SEG;
-                const bool seg_first = (j % P3_SEG) == 0;
+                const int seg = j / SEG;
+                const bool seg_first = (j % SEG) == 0;
                 if (seg_first && seg > 0 && !mbar_wait_w(o_empty, (seg - 1) & 1, p.status, 47)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t a0 = tmem + (uint32_t) (S_COL + b * P3_BK);
-                const int qh = q2;
-                q2 = q2 + 1 == nslot ? 0 : q2 + 1;
-                const int ql = q2;
-                q2 = q2 + 1 == nslot ? 0 : q2 + 1;
+                const uint32_t a0 = tmem + (uint32_t) (S_COL + b * BK);
 #pragma unroll
-                for (int pr = 0; pr < 3; pr++) {
-                    // (R hi, Y hi), (R hi, Y lo), (R lo, Y hi)
-                    const int rp = pr == 2 ? 1 : 0;
-                    const uint64_t bd = ymn + (uint64_t) ((pr == 1 ? ql : qh) * (SLOT >> 4));
+                for (int blk = 0; blk < BK / 64; blk++) {
 #pragma unroll
-                    for (int kk = 0; kk < P3_BK / 16; kk++)
-                        // centres 16 kk .. 16 kk + 15 belong to half kk / 2, whose 32
-                        // columns hold R hi (16) then R lo (16)
-                        mma_ts_w(tmem + (uint32_t) O_COL,
-                                 a0 + (uint32_t) ((kk >> 1) * 32 + rp * 16 + (kk & 1) * 8),
-                                 bd + (uint64_t) (kk * (2048 >> 4)), id2,
-                                 (!seg_first || pr || kk) ? 1u : 0u);
+                    for (int pr = 0; pr < 3; pr++) {
+                        // (R hi, Y hi), (R hi, Y lo), (R lo, Y hi)
+                        const int rp = pr == 2 ? 1 : 0;
+                        const uint64_t bd = ymn + (uint64_t) (q2 * (SLOT >> 4) + (pr == 1 ? PIECE >> 4 : 0));
+#pragma unroll
+                        for (int kk = 4 * blk; kk < 4 * blk + 4; kk++)
+                            // centres 16 kk .. 16 kk + 15 belong to group kk / 2, whose 32
+                            // columns hold R hi (16) then R lo (16)
+                            mma_ts_w(tmem + (uint32_t) O_COL,
+                                     a0 + (uint32_t) ((kk >> 1) * 32 + rp * 16 + (kk & 1) * 8),
+                                     bd + (uint64_t) (kk * (2048 >> 4)), id2,
+                                     (!seg_first || blk || pr || (kk & 3)) ? 1u : 0u);
+                    }
                 }
-                mma_commit_w(&y_empty[qh]);
-                mma_commit_w(&y_empty[ql]);
-                mma_commit_w(&s_free[b]);
-                if ((j % P3_SEG) == P3_SEG - 1 || j == p.nchunk - 1)
+                mma_commit_w(&y_empty[q2]);
+                if (++q2 == nslot)
+                    q2 = 0;
+                if ((j % SEG) == SEG - 1 || j == p.nchunk - 1)
                     mma_commit_w(o_full);
             }
         }
@@ -1261,13 +1270,13 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
     } else if (warp >= 2) {
         // ---------------- responsibilities and the segment drains ----------------
         const int q = warp & 3;          // TMEM lane quarter: points 32 q .. 32 q + 31
-        const int h = (warp - 2) >> 2;   // centres 32 h .. 32 h + 31 of a chunk
+        const int h = (warp - 2) >> 2;   // centres 32 h .. 32 h + 31 of a chunk, BK / 32 groups
         const int row = q * 32 + lane;
         const int n = n0 + row;
         const uint32_t lane_base = tmem + ((uint32_t) (q * 32) << 16);
         const float4 cq = p.colq[n];  // n < Npad: padding points carry R = 0
         bool ok = true;
-        // OUT (this thread's row) to C: 32-column batches, batch i to half i % 2;
+        // OUT (this thread's row) to C: 16-column batches, batch i to group i % (BK / 32);
         // the last one leaves dT (NaN once a bounded wait of the call has given up).
         // A batch's loads are all issued before its first store: C and T may be any
         // buffers, so between stores each load would wait out its own latency.
@@ -1276,41 +1285,41 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
             const double g = p.gF ? p.gF[0] : 1.0;
             const float gb = (float) (-(*(volatile int *) p.status ? NAN : g) * p.beta);
 #pragma unroll 1
-            for (int c0 = 32 * h; c0 < p.nout; c0 += 64) {
-                uint32_t v[32];
-                tmem_ld32(lane_base + (uint32_t) (O_COL + c0), v);
+            for (int c0 = 16 * h; c0 < p.nout; c0 += BK / 2) {
+                uint32_t v[16];
+                tmem_ld16p(lane_base + (uint32_t) (O_COL + c0), v);
                 float *dst = p.C + (size_t) n * p.D + c0;
                 const float *t = p.T + (size_t) n * p.D + c0;
                 const int left = n < p.N ? p.D - c0 : 0;  // columns of this row and batch
-                __align__(16) float prev[32], tv[32];
+                __align__(16) float prev[16], tv[16];
                 if (quads) {
 #pragma unroll
-                    for (int e = 0; e < 32; e += 4) {
+                    for (int e = 0; e < 16; e += 4) {
                         const bool in = e < left;
                         *(float4 *) (prev + e) = add && in ? *(const float4 *) (dst + e) : float4{0.f, 0.f, 0.f, 0.f};
                         *(float4 *) (tv + e) = last && in ? *(const float4 *) (t + e) : float4{0.f, 0.f, 0.f, 0.f};
                     }
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 32; e++) {
+                    for (int e = 0; e < 16; e++) {
                         prev[e] = add && e < left ? dst[e] : 0.f;
                         tv[e] = last && e < left ? t[e] : 0.f;
                     }
                 }
                 tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 32; e++) {
+                for (int e = 0; e < 16; e++) {
                     const float o = add ? prev[e] + __uint_as_float(v[e]) : __uint_as_float(v[e]);
                     prev[e] = last ? gb * (tv[e] - o) : o;
                 }
                 if (quads) {
 #pragma unroll
-                    for (int e = 0; e < 32; e += 4)
+                    for (int e = 0; e < 16; e += 4)
                         if (e < left)
                             *(float4 *) (dst + e) = *(const float4 *) (prev + e);
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 32; e++)
+                    for (int e = 0; e < 16; e++)
                         if (e < left)
                             dst[e] = prev[e];
                 }
@@ -1323,7 +1332,7 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
                 break;
             }
             tc_fence_after();
-            const uint32_t col0 = (uint32_t) (S_COL + b * P3_BK + h * 32);
+            const uint32_t col0 = (uint32_t) (S_COL + b * BK + h * 32);
             uint32_t va[32];
             tmem_ld32(lane_base + col0, va);
             tmem_ld_wait();
@@ -1341,8 +1350,8 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&p_full[b]);
-            if ((c % P3_SEG) == P3_SEG - 1 || c == p.nchunk - 1) {
-                const int seg = c / P3_SEG;
+            if ((c % SEG) == SEG - 1 || c == p.nchunk - 1) {
+                const int seg = c / SEG;
                 if (!mbar_wait(o_full, seg & 1, p.status, 49)) {
                     ok = false;
                     break;
@@ -1356,8 +1365,8 @@ __global__ void __launch_bounds__(P3_THREADS, 1)
             }
         }
         if (!ok && n < p.N)  // this tile's rows are not complete
-            for (int d = 32 * h; d < p.D; d += 64)
-                for (int e = d; e < min(d + 32, p.D); e++)
+            for (int d = 16 * h; d < p.D; d += BK / 2)
+                for (int e = d; e < min(d + 16, p.D); e++)
                     p.C[(size_t) n * p.D + e] = NAN;
         if (!ok)
             failed = 1;
@@ -1678,9 +1687,9 @@ static int tc_plan(TcState *st, int N, int D, int K, int sms, int nT)
     if (ns2 > 8)
         ns2 = 8;
     st->pass2 = (st->npanel <= 3) ? pass2_for(st->npanel, klast, nT) : nullptr;
-    // pass 3: Y slots of one 64-centre chunk piece; the first 2 nT slots
-    // stage the data tile on its way to tensor memory
-    const size_t slot3 = (size_t) st->npanel * P3_BK * 128;
+    // pass 3: Y slots of one chunk, both pieces; the last ones stage the data
+    // tile on its way to tensor memory
+    const size_t slot3 = (size_t) st->npanel * p3_bk(st->npanel) * 128 * 2;
     int ns3 = (int) ((SMEM_LIMIT - 1024 - bar_bytes) / slot3);
     if (ns3 > 12)
         ns3 = 12;
@@ -1689,7 +1698,7 @@ static int tc_plan(TcState *st, int N, int D, int K, int sms, int nT)
         set_error(DGTM_ENOTSUP, "the split-BF16 form supports D <= 189 (D = %d)", D);
         return DGTM_ENOTSUP;
     }
-    if (ns1 < 2 || ns2 < 2 || ns3 < 4 || ns3 < 2 * nT || !st->pass1) {
+    if (ns1 < 2 || ns2 < 2 || ns3 < 2 || ns3 < p3_ndata(st->npanel, nT) || !st->pass1) {
         set_error(DGTM_ENOTSUP, "the split-BF16 form does not fit shared memory (D = %d)", D);
         return DGTM_ENOTSUP;
     }
@@ -1726,7 +1735,7 @@ static int tc_maps(TcState *st)
                              P2_TILE, PANEL_ELEMS)) != DGTM_OK ||
         (rc = make_tmap_bf16(&st->tmY1, st->Yb, 2 * (uint64_t) st->Kpad, st->Dp, st->Dp, P1_BK,
                              PANEL_ELEMS)) != DGTM_OK ||
-        (rc = make_tmap_bf16(&st->tmY3, st->Yb, 2 * (uint64_t) st->Kpad, st->Dp, st->Dp, P3_BK,
+        (rc = make_tmap_bf16(&st->tmY3, st->Yb, 2 * (uint64_t) st->Kpad, st->Dp, st->Dp, p3_bk(st->npanel),
                              PANEL_ELEMS)) != DGTM_OK)
         return rc;
     return DGTM_OK;
@@ -2038,7 +2047,7 @@ int tc_fe_rty(const TcFeLayout &L, void *ws, const float *T, int N, int K, int D
     p.D = D;
     p.Npad = st.Npad;
     p.Kpad = st.Kpad;
-    p.nchunk = st.Kpad / P3_BK;
+    p.nchunk = st.Kpad / p3_bk(st.npanel);
     p.nstage = st.nstage3;
     p.nout = round_up(D, PANEL_ELEMS);  // whole 128-byte swizzle atoms of the MN-major Y
     p.colq = st.colq;
@@ -2047,7 +2056,7 @@ int tc_fe_rty(const TcFeLayout &L, void *ws, const float *T, int N, int K, int D
     p.gF = gF;
     p.beta = beta;
     p.status = st.status;
-    st.pass3<<<st.Npad / P3_TILE, P3_THREADS, st.smem3, s>>>(st.tmY3, st.tmT1, p);
+    st.pass3<<<st.Npad / P3_TILE, p3_threads(st.npanel), st.smem3, s>>>(st.tmY3, st.tmT1, p);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
