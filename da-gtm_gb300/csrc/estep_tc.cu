@@ -56,7 +56,6 @@ using namespace sm100;
 namespace {
 
 constexpr int P1_THREADS = 320;       // warp 0 TMA, warp 1 MMA, warps 2-9 statistics
-constexpr int P2_THREADS = 320;       // warp 0 TMA, warp 1 MMA, warps 2-9 responsibilities
 constexpr int P1_TILE = 128;          // points per tile (MMA M); a CTA holds 1 or 2 tiles
 constexpr int P1_BK = 128;            // centres per chunk (MMA N)
 constexpr int PANEL_ELEMS = 64;       // BF16 elements per 128-byte swizzle row
@@ -620,22 +619,28 @@ struct P2Params {
     int *status;
 };
 
-constexpr int P2_TILE = 64;  // points per tile (MMA N of the distance product)
-// R T is accumulated in tensor memory over at most this many tiles (4096
-// points), a segment.  The tensor pipe's FP32 accumulation rounds each MMA's
+constexpr int P2_GRAIN = 64;  // points: units are counted in these
+// Points per tile (MMA N of the distance product), and threads: warp 0 TMA, warp 1 MMA,
+// the others responsibilities (four for each 32 points).  A tile's round through its
+// barriers takes about as long as its MMAs at one or two panels, so a tile is as many
+// points as tensor memory holds two buffers of beside the accumulator and the centres
+// (N = 65536, K = 4096, D = 64: 198 us a pass with 128, 220 with 64).
+__host__ __device__ constexpr int p2_tile(int np) { return np <= 2 ? 128 : 64; }
+__host__ __device__ constexpr int p2_threads(int np) { return 64 + 4 * p2_tile(np); }
+// R T is accumulated in tensor memory over at most this many points, a segment.  The tensor pipe's FP32 accumulation rounds each MMA's
 // sum down a little, which over a whole 16384-point unit came to ~6e-5 of G
 // and R T (4096 points: ~1e-5).  A power of two: the MMA warp finds segment
 // starts with a mask.
-constexpr int P2_SEG_TILES = 64;
-static_assert((P2_SEG_TILES & (P2_SEG_TILES - 1)) == 0, "segment length");
+constexpr int P2_SEG = 4096;
+static_assert((P2_SEG & (P2_SEG - 1)) == 0, "segment length");
 
 // Where the segments of a unit are summed.  With shared memory to spare
-// (128 x (Dp + 4) FP32 beside at least four ring stages) they are summed
+// (128 x (Dp + 4) FP32 beside at least three ring stages) they are summed
 // there in FP32 (round-to-nearest) and the unit's total is stored to its
-// slot.  Otherwise (two data pieces and three panels: the ring would drop to
-// two stages, which measured 1.5x slower) the first segment is stored to
-// the slot and the later ones are added at L2 with red.global.add.
-__host__ __device__ constexpr bool p2_segbuf(int np, int nt) { return nt * np <= 4; }
+// slot.  Otherwise (two data pieces and two or three panels: the ring would
+// drop to two stages, which measured 1.5x slower with three) the first segment
+// is stored to the slot and the later ones are added at L2 with red.global.add.
+__host__ __device__ constexpr bool p2_segbuf(int np, int nt) { return nt * np <= 3; }
 
 // The CTAs take units v = blockIdx.x, blockIdx.x + gridDim.x, ... in point-
 // major order, so at any time all CTAs stream the same few point tiles (which
@@ -651,37 +656,40 @@ __device__ __forceinline__ void unit_of(const P2Params &p, int v, int &u, int &k
 }
 
 // Pass 2, a template on the operand shape like pass 1.  Tensor memory holds
-// the unit's R T accumulator (columns 0 .. Dp-1), two 64-point buffers in
+// the unit's R T accumulator (columns 0 .. Dp-1), two buffers of a tile's points in
 // which the distance accumulator S is turned into R (BF16 hi/lo), and the
 // unit's 128 centres (Y hi, Y lo) as the A operand of the distance product,
-// so shared memory is left to a deep ring of point tiles.  Per 64-point tile:
-// MMA 1 (A = Y from tensor memory, B = T tile, N = 64) gives S; eight warps
-// (two 32-point groups x four lane quarters) form R and write it over S; MMA 2
+// so shared memory is left to a deep ring of point tiles.  Per tile:
+// MMA 1 (A = Y from tensor memory, B = T tile, N = its points) gives S; a
+// group of four warps (the lane quarters) for each 32 points forms R and writes it over S; MMA 2
 // (A = R from tensor memory, B = the same T tile read MN-major, N = Dp)
 // accumulates R T.  At a unit boundary the same warps drain R T to the
 // unit's slot and load the next unit's centres into tensor memory.
 template <int NP, int KL, int NT>
-__global__ void __launch_bounds__(P2_THREADS, 1)
+__global__ void __launch_bounds__(p2_threads(NP), 1)
     tc_pass2_kernel(const __grid_constant__ CUtensorMap tmT, const P2Params p)
 {
     constexpr int KS = 4 * (NP - 1) + KL;               // 16-deep steps of the distance product
     constexpr int DP = NP * PANEL_ELEMS;
+    constexpr int TP = p2_tile(NP);                     // points of a tile
+    constexpr int G = TP / 32;                          // groups of four warps
+    constexpr int SEG_TILES = P2_SEG / TP;
     constexpr int YCOLS = (KS * 8 + 15) / 16 * 16;      // TMEM columns of one Y piece
-    constexpr int SP_COL = DP;                          // S / P buffers: 2 x 64 columns
-    constexpr int Y_COL = DP + 2 * P2_TILE;             // Y hi, then Y lo
+    constexpr int SP_COL = DP;                          // S / P buffers: 2 x TP columns
+    constexpr int Y_COL = DP + 2 * TP;             // Y hi, then Y lo
     static_assert(Y_COL + 2 * YCOLS <= 512, "pass 2 tensor memory plan");
-    constexpr int TPANEL_BYTES = P2_TILE * 128;         // 8 KB
+    constexpr int TPANEL_BYTES = TP * 128;
     constexpr int TSTAGE_BYTES = NT * NP * TPANEL_BYTES;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int nstage = p.nstage;
     unsigned char *Tst = base;
-    float4 *cq = (float4 *) (Tst + nstage * TSTAGE_BYTES);  // nstage x 64
+    float4 *cq = (float4 *) (Tst + nstage * TSTAGE_BYTES);  // nstage x TP
     // the unit's segment sums: 128 rows of DP + 4 floats (the pad spreads a
     // quarter-warp's float4 accesses to one row each over all banks)
     constexpr bool SEGBUF = p2_segbuf(NP, NT);
     constexpr int RB = DP + 4;
-    float *rtbuf = (float *) (cq + nstage * P2_TILE);
+    float *rtbuf = (float *) (cq + nstage * TP);
     uint64_t *bars = (uint64_t *) (rtbuf + (SEGBUF ? P2_BK * RB : 0));
     uint64_t *t_full = bars;
     uint64_t *t_empty = bars + nstage;
@@ -703,10 +711,10 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&s_full[b], 1);
-            mbar_init(&p_full[b], 256);
+            mbar_init(&p_full[b], 4 * TP);
         }
         mbar_init(rt_full, 1);
-        mbar_init(y_ready, 256);
+        mbar_init(y_ready, 4 * TP);
         mbar_init(drain, 1);
         fence_barrier_init();
     }
@@ -733,14 +741,14 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
                     ok = false;
                     break;
                 }
-                mbar_expect_tx(&t_full[s], (uint32_t) (TSTAGE_BYTES + P2_TILE * 16));
+                mbar_expect_tx(&t_full[s], (uint32_t) (TSTAGE_BYTES + TP * 16));
 #pragma unroll
                 for (int tp = 0; tp < NT; tp++)
 #pragma unroll
                     for (int pn = 0; pn < NP; pn++)
                         tma_load_2d(Tst + s * TSTAGE_BYTES + (tp * NP + pn) * TPANEL_BYTES, &tmT,
-                                    &t_full[s], PANEL_ELEMS * pn, tp * p.Npad + t * P2_TILE);
-                bulk_load(cq + s * P2_TILE, p.colq + (size_t) t * P2_TILE, (uint32_t) (P2_TILE * 16),
+                                    &t_full[s], PANEL_ELEMS * pn, tp * p.Npad + t * TP);
+                bulk_load(cq + s * TP, p.colq + (size_t) t * TP, (uint32_t) (TP * 16),
                           &t_full[s]);
                 if (++s == nstage) {
                     s = 0;
@@ -752,7 +760,7 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
             failed = 1;
     } else if (warp == 1) {
         // ---------------- MMA issuer (whole warp; one elected lane issues) ----------------
-        const uint32_t id1 = idesc_bf16(P2_BK, P2_TILE, 0, 0);
+        const uint32_t id1 = idesc_bf16(P2_BK, TP, 0, 0);
         const uint32_t id2 = idesc_bf16(P2_BK, DP, 0, 1);
         const uint64_t tdesc_k = sdesc_sw128(smem_u32(Tst), 16, 1024);            // K-major (MMA 1)
         const uint64_t tdesc_mn = sdesc_sw128(smem_u32(Tst), TPANEL_BYTES, 1024); // MN-major (MMA 2)
@@ -773,14 +781,14 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
             tc_fence_after();
             for (int t = t0; t <= t1; t++) {
                 if (t < t1) {
-                    // S = Y T^T for tile jt: M = 128 centres, N = 64 points
+                    // S = Y T^T for tile jt: M = 128 centres, N = TP points
                     const int b = jt & 1;
                     if (!mbar_wait_w(&t_full[s], ph, p.status, 24)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t d = tmem + (uint32_t) (SP_COL + b * P2_TILE);
+                    const uint32_t d = tmem + (uint32_t) (SP_COL + b * TP);
                     const uint64_t bd = tdesc_k + (uint64_t) (s * (TSTAGE_BYTES >> 4));
 #pragma unroll
                     for (int piece = 0; piece < 2; piece++) {
@@ -805,20 +813,23 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
                     }
                     tc_fence_after();
                     const uint64_t bd = tdesc_mn + (uint64_t) (sp * (TSTAGE_BYTES >> 4));
-                    const uint32_t a0 = tmem + (uint32_t) (SP_COL + b * P2_TILE);
+                    const uint32_t a0 = tmem + (uint32_t) (SP_COL + b * TP);
 #pragma unroll
-                    for (int rp = 0; rp < 2; rp++) {
+                    for (int blk = 0; blk < TP / 64; blk++) {
 #pragma unroll
-                        for (int tp = 0; tp < (rp == 0 ? NT : 1); tp++) {
+                        for (int rp = 0; rp < 2; rp++) {
 #pragma unroll
-                            for (int kk = 0; kk < P2_TILE / 16; kk++)
-                                // points 16 kk .. 16 kk + 15 belong to group kk / 2, whose
-                                // 32 columns hold R hi (16) then R lo (16)
-                                mma_ts_w(rt_tmem,
-                                         a0 + (uint32_t) ((kk >> 1) * 32 + rp * 16 + (kk & 1) * 8),
-                                         bd + (uint64_t) (tp * NP * (TPANEL_BYTES >> 4) + kk * (2048 >> 4)),
-                                         id2, (((uint32_t) (t - 1 - t0) & (P2_SEG_TILES - 1)) != 0u ||
-                                               rp | tp | kk) ? 1u : 0u);
+                            for (int tp = 0; tp < (rp == 0 ? NT : 1); tp++) {
+#pragma unroll
+                                for (int kk = 4 * blk; kk < 4 * blk + 4; kk++)
+                                    // points 16 kk .. 16 kk + 15 belong to group kk / 2, whose
+                                    // 32 columns hold R hi (16) then R lo (16)
+                                    mma_ts_w(rt_tmem,
+                                             a0 + (uint32_t) ((kk >> 1) * 32 + rp * 16 + (kk & 1) * 8),
+                                             bd + (uint64_t) (tp * NP * (TPANEL_BYTES >> 4) + kk * (2048 >> 4)),
+                                             id2, (((uint32_t) (t - 1 - t0) & (SEG_TILES - 1)) != 0u ||
+                                                   blk | rp | tp | (kk & 3)) ? 1u : 0u);
+                            }
                         }
                     }
                     // also tells the responsibility warps that a segment's
@@ -847,26 +858,30 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
         const int g = (warp - 2) >> 2;          // point group: points 32 g .. 32 g + 31 of a tile
         const int row = q * 32 + lane;          // centre within the tile
         const uint32_t lane_base = tmem + ((uint32_t) (q * 32) << 16);
-        // This group's half of row `row` of the R T accumulator (FP32) out of
+        // This group's part (DP / G columns) of row `row` of the R T accumulator (FP32) out of
         // tensor memory, at the end of a segment (last: the unit's last one;
         // later: not the unit's first one).  With the shared-memory sums the
         // segment is stored or added there, and after the unit's last one the
-        // thread's half row (384 B at D_p = 192) goes to the unit's slot as one
+        // thread's part of the row (384 B at D_p = 192) goes to the unit's slot as one
         // bulk copy by the TMA engine.  Without them every segment goes to the
         // slot, stored or added at L2.  Each element has this one owner
         // thread, in program order.
         float *const buf = rtbuf + row * RB;
         auto move_rt = [&](bool last, bool later, int uslot) {
+            constexpr int CB = DP / G < 32 ? 16 : 32;  // columns per batch
             float *dst = p.RTpart + ((size_t) uslot * P2_BK + row) * DP;
             if constexpr (SEGBUF)
-                bulk_wait_read();  // the previous unit's copy has left the half row
+                bulk_wait_read();  // the previous unit's copy has left it
 #pragma unroll 1
-            for (int c0 = g * (DP / 2); c0 < (g + 1) * (DP / 2); c0 += 32) {
-                uint32_t vv[32];
-                tmem_ld32(lane_base + (uint32_t) c0, vv);
+            for (int c0 = g * (DP / G); c0 < (g + 1) * (DP / G); c0 += CB) {
+                uint32_t vv[CB];
+                if constexpr (CB == 32)
+                    tmem_ld32p(lane_base + (uint32_t) c0, vv);
+                else
+                    tmem_ld16p(lane_base + (uint32_t) c0, vv);
                 tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 32; j += 4) {
+                for (int j = 0; j < CB; j += 4) {
                     float4 x = make_float4(__uint_as_float(vv[j]), __uint_as_float(vv[j + 1]),
                                            __uint_as_float(vv[j + 2]), __uint_as_float(vv[j + 3]));
                     if constexpr (SEGBUF) {
@@ -888,32 +903,37 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
             if constexpr (SEGBUF) {
                 if (last) {
                     fence_proxy_async_smem();
-                    bulk_store(dst + g * (DP / 2), buf + g * (DP / 2), (uint32_t) (DP / 2 * 4));
+                    bulk_store(dst + g * (DP / G), buf + g * (DP / G), (uint32_t) (DP / G * 4));
                     bulk_commit();
                 }
             }
         };
-        // The centre row of centre tile ktc (group 0: Y hi, group 1: Y lo) into
+        // The centre row of centre tile ktc (even groups: Y hi, odd: Y lo; with four
+        // groups the first two and the last two take alternate 16 columns) into
         // tensor memory, column j holding depths 2 j and 2 j + 1, then y_ready.
         // Every load is issued before the first store: one L2 round trip.
         auto load_y = [&](int ktc) {
+            constexpr int STEP = 8 * G;                     // columns between a thread's batches
+            constexpr int NB = (YCOLS + STEP - 1) / STEP;   // its batches, at most
+            const int piece = g & 1, c1 = (g >> 1) * 16;
             const uint4 *src =
-                (const uint4 *) (p.Yb + ((size_t) g * p.Kpad + (size_t) ktc * P2_BK + row) * (DP / 2));
-            uint4 x[YCOLS / 4];
+                (const uint4 *) (p.Yb + ((size_t) piece * p.Kpad + (size_t) ktc * P2_BK + row) * (DP / 2) + c1);
+            uint4 x[4 * NB];
 #pragma unroll
-            for (int i = 0; i < YCOLS / 4; i++)
-                x[i] = src[i];
+            for (int i = 0; i < 4 * NB; i++)
+                x[i] = STEP * (i / 4) + c1 < YCOLS ? src[STEP / 4 * (i / 4) + i % 4] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-            for (int c0 = 0; c0 < YCOLS; c0 += 16) {
+            for (int i = 0; i < NB; i++) {
                 uint32_t w[16];
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    w[4 * i] = x[c0 / 4 + i].x;
-                    w[4 * i + 1] = x[c0 / 4 + i].y;
-                    w[4 * i + 2] = x[c0 / 4 + i].z;
-                    w[4 * i + 3] = x[c0 / 4 + i].w;
+                for (int k = 0; k < 4; k++) {
+                    w[4 * k] = x[4 * i + k].x;
+                    w[4 * k + 1] = x[4 * i + k].y;
+                    w[4 * k + 2] = x[4 * i + k].z;
+                    w[4 * k + 3] = x[4 * i + k].w;
                 }
-                tmem_st16(lane_base + (uint32_t) (Y_COL + g * YCOLS + c0), w);
+                if (STEP * i + c1 < YCOLS)
+                    tmem_st16(lane_base + (uint32_t) (Y_COL + piece * YCOLS + STEP * i + c1), w);
             }
             tmem_st_wait();
             tc_fence_before();
@@ -927,8 +947,8 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
             unit_of(p, v, u, kt, t0, t1);
             if (nunit == 0)
                 load_y(kt);
-            const bool multi = t1 - t0 > P2_SEG_TILES;
-            int seg_r = t0 + P2_SEG_TILES;  // the first tile of the next segment
+            const bool multi = t1 - t0 > SEG_TILES;
+            int seg_r = t0 + SEG_TILES;  // the first tile of the next segment
             for (int t = t0; t < t1; t++, jt++) {
                 const int b = jt & 1;
                 if (!mbar_wait(&t_full[s], ph, p.status, 27) ||
@@ -937,11 +957,11 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
                     break;
                 }
                 tc_fence_after();
-                const uint32_t col0 = (uint32_t) (SP_COL + b * P2_TILE + g * 32);
+                const uint32_t col0 = (uint32_t) (SP_COL + b * TP + g * 32);
                 uint32_t va[32];
                 tmem_ld32(lane_base + col0, va);
                 tmem_ld_wait();
-                const float4 *cqs = cq + s * P2_TILE + g * 32;
+                const float4 *cqs = cq + s * TP + g * 32;
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
@@ -967,8 +987,8 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
                         break;
                     }
                     tc_fence_after();
-                    move_rt(false, t > t0 + P2_SEG_TILES, u);
-                    seg_r += P2_SEG_TILES;
+                    move_rt(false, t > t0 + SEG_TILES, u);
+                    seg_r += SEG_TILES;
                 }
                 tc_fence_before();
                 mbar_arrive(&p_full[b]);
@@ -1588,7 +1608,7 @@ static int p2_unit_tiles(int ntiles, int ktiles, int grid_max)
     int best = 256;
     double best_cost = 0.0;
     std::vector<long> work;
-    for (int ut = 256; ut <= 640; ut += P2_SEG_TILES) {
+    for (int ut = 256; ut <= 640; ut += P2_SEG / P2_GRAIN) {
         const long upk = (ntiles + ut - 1) / ut;
         const long nunits = upk * ktiles;
         const int grid = nunits < grid_max ? (int) nunits : grid_max;
@@ -1662,7 +1682,7 @@ static int tc_plan(TcState *st, int N, int D, int K, int sms, int nT)
     // exact 0/1 data: two 128-point tiles per pass-1 CTA; split data (two T
     // pieces) one, to fit tensor memory.  Pass-2 tiles are 64 points.
     st->ntile1 = (nT == 1) ? 2 : 1;
-    st->bn2 = P2_TILE;
+    st->bn2 = P2_GRAIN;
     st->ntiles2 = st->Npad / st->bn2;
     const int ktiles2 = (K + P2_BK - 1) / P2_BK;
     st->unit_tiles = p2_unit_tiles(st->ntiles2, ktiles2, sms);
@@ -1680,7 +1700,7 @@ static int tc_plan(TcState *st, int N, int D, int K, int sms, int nT)
     st->pass1 = pass1_for(st->npanel, klast, nT);
     // pass 2: the point-tile ring (T pieces + column statistics); the centres
     // live in tensor memory
-    const size_t ts2 = (size_t) nT * st->npanel * P2_TILE * 128 + P2_TILE * 16;
+    const size_t ts2 = (size_t) p2_tile(st->npanel) * (nT * st->npanel * 128 + 16);
     const size_t rtbuf2 =
         p2_segbuf(st->npanel, nT) ? (size_t) P2_BK * (st->npanel * PANEL_ELEMS + 4) * 4 : 0;
     int ns2 = (int) ((SMEM_LIMIT - 1024 - bar_bytes - rtbuf2) / ts2);
@@ -1732,7 +1752,7 @@ static int tc_maps(TcState *st)
     if ((rc = make_tmap_bf16(&st->tmT1, st->Tb, (uint64_t) st->nT * st->Npad, st->Dp, st->Dp,
                              P1_TILE, PANEL_ELEMS)) != DGTM_OK ||
         (rc = make_tmap_bf16(&st->tmT2, st->Tb, (uint64_t) st->nT * st->Npad, st->Dp, st->Dp,
-                             P2_TILE, PANEL_ELEMS)) != DGTM_OK ||
+                             p2_tile(st->npanel), PANEL_ELEMS)) != DGTM_OK ||
         (rc = make_tmap_bf16(&st->tmY1, st->Yb, 2 * (uint64_t) st->Kpad, st->Dp, st->Dp, P1_BK,
                              PANEL_ELEMS)) != DGTM_OK ||
         (rc = make_tmap_bf16(&st->tmY3, st->Yb, 2 * (uint64_t) st->Kpad, st->Dp, st->Dp, p3_bk(st->npanel),
@@ -1901,8 +1921,9 @@ int tc_mstep_pass(TcState *st, const double2 *, double, cudaStream_t s, int *nla
     p.Dp = st->Dp;
     p.Npad = st->Npad;
     p.Kpad = st->Kpad;
-    p.ntiles = st->ntiles2;
-    p.unit_tiles = st->unit_tiles;
+    const int per = p2_tile(st->npanel) / P2_GRAIN;
+    p.ntiles = st->ntiles2 / per;  // Npad is a multiple of 256, a unit of P2_SEG
+    p.unit_tiles = st->unit_tiles / per;
     p.units_per_k = st->units_per_k;
     p.ktiles = (st->K + P2_BK - 1) / P2_BK;
     p.nunits = st->nunits;
@@ -1911,7 +1932,7 @@ int tc_mstep_pass(TcState *st, const double2 *, double, cudaStream_t s, int *nla
     p.colq = st->colq;
     p.RTpart = st->RTpart;
     p.status = st->status;
-    st->pass2<<<st->grid2, P2_THREADS, st->smem2, s>>>(st->tmT2, p);
+    st->pass2<<<st->grid2, p2_threads(st->npanel), st->smem2, s>>>(st->tmT2, p);
     DGTM_CUDA_TRY(cudaGetLastError());
     *nlaunch = 1;
     return DGTM_OK;
