@@ -18,9 +18,10 @@
 //   * FP32 values become FP64 by integer operations, and sums over lanes are
 //     reduced and scattered at once (the same tree, an eighth of the additions).
 //
-// N = 100,000, K = 8000, D = 166: pass 1 29.9 -> 16.8 ms, pass 2 85.7 -> 20.8 ms.
-// What bounds them now is issue and latency at two blocks an SM (2.1 instructions a
-// clock; FMA pipe 27 and 32 %, FP64 pipe 21 and 30 % busy).
+// N = 100,000, K = 8000, D = 166: pass 1 29.9 -> 13.6 ms (16.8 while a chunk of centres
+// was loaded between two barriers), pass 2 85.7 -> 20.7 ms.  What bounds pass 1 now is
+// issue and latency at two blocks an SM; pass 2 shared memory: 1010 wavefronts a warp
+// and tile of 64 points for 2100 FP32 multiply-adds' clocks over four schedulers.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "sm100.cuh"
@@ -64,13 +65,14 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
 }
 
 // h + l rounded to FP32; ok is cleared when it is not safely away from a rounding
-// boundary (or not finite)
+// boundary (or not finite).  The remainder e may be off by 2^-42 |r|, at most 2^-17 of
+// the distance to the nearest boundary from r, so r is safe if e grown by 2^-16 still
+// rounds to it.
 __device__ __forceinline__ float settle(float h, float l, bool &ok)
 {
     const float r = __fadd_rn(h, l);
     const float e = __fsub_rn(l, __fsub_rn(r, h));
-    const float d = __fmul_rn(fabsf(r), 0x1p-42f);
-    ok = ok && __fadd_rn(r, __fadd_rn(e, d)) == r && __fadd_rn(r, __fsub_rn(e, d)) == r;
+    ok = ok && __fadd_rn(r, __fmul_rn(e, 1.f + 0x1p-16f)) == r;
     return r;
 }
 
@@ -98,16 +100,32 @@ __device__ __forceinline__ void times(Pair c, float xh, float xl, float &h, floa
 
 // ---------------------------------------------------------------------------
 // Pass 1: column statistics.  Block: 64 points (resident in shared memory), all
-// centres in chunks of 64; thread: 4 points x 4 centres (tx + 16 j, as the generic
+// centres in chunks of 64, half their depths at a time through two buffers that
+// cp.async fills ahead of the products; thread: 4 points x 4 centres (tx + 16 j, as the generic
 // kernel's lanes, whose summation tree this keeps).  Two blocks an SM.
 // ---------------------------------------------------------------------------
+// a row of half the depths (an even number of quads: see row_stride)
+template <int J>
+__host__ __device__ constexpr int half_stride() { return 16 * J + 4; }
+
+__device__ __forceinline__ void copy_async(float *dst, const float *src, bool in, bool two)
+{
+    const uint32_t d = smem_u32(dst);
+    if (two)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(in ? 8 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+
 template <int J>
 __global__ void __launch_bounds__(FT, J <= 6 ? 2 : 1) pass1_f32_kernel(Pass1Args<float> a, Pair c1, Pair c2)
 {
     extern __shared__ __align__(16) float sm[];
     constexpr int ld = row_stride<J>();
     const int D = a.D, D4 = (D + 3) / 4 * 4;
-    float *Ts = sm, *Ys = sm + TILE * ld, *yys = Ys + TILE * ld;  // points, centres, |y|^2
+    constexpr int lh = half_stride<J>();
+    const int hd = (D4 + 7) / 8 * 4;  // depths of the first half
+    float *Ts = sm, *Ys = sm + TILE * ld, *yys = Ys + 2 * TILE * lh;  // points, centres, |y|^2
     __shared__ double red[32];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -127,40 +145,68 @@ __global__ void __launch_bounds__(FT, J <= 6 ? 2 : 1) pass1_f32_kernel(Pass1Args
     const double oc = ot ? a.c2 : a.c1;
     double s = 0.0;
 
+    // depths d0 .. d1 - 1 of the centres k .. k + 63 into half buffer b; zeros outside
+    auto fill = [&](int k, int b) {
+        const int d0 = b * hd, n = b ? D4 - hd : hd;
+        float *dst = Ys + b * TILE * lh;
+        const bool two = (D & 1) == 0;  // rows start on 8 bytes
+        const int step = two ? 2 : 1;
+        for (int r = warp; r < TILE; r += FT / 32) {
+            const float *src = a.Y + (size_t) min(k + r, a.K - 1) * D;
+            for (int d = step * lane; d < n; d += 32 * step) {
+                const bool in = k + r < a.K && d0 + d < D;
+                copy_async(dst + r * lh + d, in ? src + d0 + d : a.Y, in, two);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fill(0, 0);
+
     for (int k0 = 0; k0 < a.K; k0 += TILE) {
-        __syncthreads();
-        for (int r = warp; r < TILE; r += FT / 32)
-            for (int d = lane; d < D4; d += 32)
-                Ys[r * ld + d] = (k0 + r < a.K && d < D) ? a.Y[(size_t) (k0 + r) * D + d] : 0.f;
-        if (threadIdx.x < TILE)
-            yys[threadIdx.x] = (float) (k0 + (int) threadIdx.x < a.K ? a.yy[k0 + threadIdx.x] : 0.0);
-        __syncthreads();
         float acc[4][4];
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++)
                 acc[i][j] = 0.f;
-        // columns D .. D4 are zero in both operands: adding 0 x 0 keeps every bit
-        // (a sum that is -0 cannot arise from products added to +0)
+#pragma unroll 1
+        for (int b = 0; b < 2; b++) {
+            // this half has arrived for every thread, and the other buffer's readers are done
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (b == 0)
+                fill(k0, 1);
+            else if (k0 + TILE < a.K)
+                fill(k0 + TILE, 0);
+            float yy = 0.f;
+            if (b == 0 && threadIdx.x < TILE)
+                yy = (float) (k0 + (int) threadIdx.x < a.K ? a.yy[k0 + threadIdx.x] : 0.0);
+            const float *tp = Ts + b * hd, *yp = Ys + b * TILE * lh;
+            const int n = b ? D4 - hd : hd;
+            // columns D .. D4 are zero in both operands: adding 0 x 0 keeps every bit
+            // (a sum that is -0 cannot arise from products added to +0)
 #pragma unroll 2
-        for (int d = 0; d < D4; d += 4) {
-            float4 t[4], y[4];
+            for (int d = 0; d < n; d += 4) {
+                float4 t[4], y[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                t[i] = *(const float4 *) &Ts[(ty * 4 + i) * ld + d];
+                for (int i = 0; i < 4; i++)
+                    t[i] = *(const float4 *) &tp[(ty * 4 + i) * ld + d];
 #pragma unroll
-            for (int j = 0; j < 4; j++)
-                y[j] = *(const float4 *) &Ys[(tx + 16 * j) * ld + d];
+                for (int j = 0; j < 4; j++)
+                    y[j] = *(const float4 *) &yp[(tx + 16 * j) * lh + d];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+                for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    acc[i][j] = __fmaf_rn(t[i].x, y[j].x, acc[i][j]);
-                    acc[i][j] = __fmaf_rn(t[i].y, y[j].y, acc[i][j]);
-                    acc[i][j] = __fmaf_rn(t[i].z, y[j].z, acc[i][j]);
-                    acc[i][j] = __fmaf_rn(t[i].w, y[j].w, acc[i][j]);
-                }
+                    for (int j = 0; j < 4; j++) {
+                        acc[i][j] = __fmaf_rn(t[i].x, y[j].x, acc[i][j]);
+                        acc[i][j] = __fmaf_rn(t[i].y, y[j].y, acc[i][j]);
+                        acc[i][j] = __fmaf_rn(t[i].z, y[j].z, acc[i][j]);
+                        acc[i][j] = __fmaf_rn(t[i].w, y[j].w, acc[i][j]);
+                    }
+            }
+            // read after the second half's barrier; the last chunk's readers passed the first's
+            if (b == 0 && threadIdx.x < TILE)
+                yys[threadIdx.x] = yy;
         }
         float yf[4];
 #pragma unroll
@@ -504,7 +550,7 @@ template <int J>
 constexpr Kernels kernels_of()
 {
     constexpr int J2 = (J + 1) / 2;
-    return Kernels{pass1_f32_kernel<J>, pass2_f32_kernel<J2>, row_stride<J>(), row_stride<2 * J2>()};
+    return Kernels{pass1_f32_kernel<J>, pass2_f32_kernel<J2>, row_stride<J>() + 2 * half_stride<J>(), row_stride<2 * J2>()};
 }
 
 const Kernels KERNELS[8] = {kernels_of<1>(), kernels_of<2>(), kernels_of<3>(), kernels_of<4>(),
@@ -528,7 +574,7 @@ int launch_pass1_f32(const Pass1Args<float> &a, cudaStream_t s)
     const int rc = depth_class(a.D, &k);
     if (rc != DGTM_OK)
         return rc;
-    const size_t smem = sizeof(float) * (2 * (size_t) TILE * k->ld1 + TILE);
+    const size_t smem = sizeof(float) * ((size_t) TILE * k->ld1 + TILE);
     DGTM_CUDA_TRY(cudaFuncSetAttribute(k->p1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     k->p1<<<ceil_div(a.N, TILE), FT, smem, s>>>(a, split(a.c1), split(a.c2));
     DGTM_CUDA_TRY(cudaGetLastError());
