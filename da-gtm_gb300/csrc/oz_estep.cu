@@ -40,6 +40,7 @@ constexpr int PANEL = 64;
 constexpr long long CHUNK = 10000000;   // centre-point pairs a chunk
 constexpr int ST_PTS = 8;               // points of a statistics or map block
 constexpr int DG_K = 2;                 // centres of a digits block
+constexpr int NARROW = 8;               // depths whose products are formed as 64-bit integers
 constexpr int64_t ZERO_COLUMN = INT64_MIN;  // aref of a point whose R is 1/K
 constexpr size_t TAB_BYTES = sizeof(uint64_t) * oz::TAB;
 
@@ -93,12 +94,13 @@ __global__ void __launch_bounds__(256) oz_absmax_kernel(const double *__restrict
 }
 
 // planes[i][r][d] = digit i of X[r][d] on the common grid of bits[0]; zero past rows
-// and D.  With sc: the grid of the products with T (tbits: its max |t| and |t|^2;
+// and D.  fixed (instead of planes): [r][d] = X[r][d] as an integer below 2^61, ld of a row.  With sc: the grid of the products with T (tbits: its max |t| and |t|^2;
 // sa its planes) and h_k = |y_k|^2 / 2 on it.
 __global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__restrict__ X, int rows, int D,
                                                             int prows, int ld,
                                                             const unsigned long long *__restrict__ bits,
                                                             __nv_bfloat16 *__restrict__ planes,
+                                                            int64_t *__restrict__ fixed,
                                                             const unsigned long long *__restrict__ tbits,
                                                             int sa, const double *__restrict__ xx,
                                                             OzScale *sc, int64_t *__restrict__ h)
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__rest
     const size_t n2 = (size_t) prows * ld / 2;
     if (sc) {
         // |t.y| + |y|^2 / 2, and differences of two such, within 2^62 units
-        const int base = sa == 1 ? e - 55 : oz::exponent_of(tbits[0]) + e - 53;
+        const int base = sa == 1 ? e - 55 : oz::exponent_of(tbits[0]) + e - (fixed ? 58 : 53);
         const double tt = oz::bits_double(tbits[1]), yy = oz::bits_double(bits[1]);
         const double bound = 2.0 * (sqrt(tt) * sqrt(yy) + 0.5 * yy);
         const int need = oz::exponent_of(oz::double_bits(bound)) - 62;
@@ -120,6 +122,13 @@ __global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__rest
         }
         for (int k = blockIdx.x * 256 + threadIdx.x; k < rows; k += gridDim.x * 256)
             h[k] = bad ? 0 : oz::scaled_int(xx[k], -1 - u);
+    }
+    if (fixed) {
+        for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < (size_t) rows * ld; i += (size_t) gridDim.x * 256) {
+            const int r = (int) (i / ld), d = (int) (i % ld);
+            fixed[i] = d < D ? oz::scaled_int(X[(size_t) r * D + d], 61 - e) : 0;
+        }
+        return;
     }
     for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < n2; i += (size_t) gridDim.x * 256) {
         const int r = (int) (2 * i / ld), d = (int) (2 * i % ld);
@@ -137,16 +146,52 @@ __global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__rest
     }
 }
 
+// The products of up to 8 depths as 64-bit integers: out[k ldm + m] = y_k . t_m in
+// units of 2^u, each product's upper 64 bits (in 2^-58 of the operands' 2^e, eight of
+// them below 2^61) added exactly.  Eight digits of either operand leave 2^-54 of the largest product, which
+// at few depths is more than an FP64 sum loses: the error of R at D = 5 was 1.9e-15 of
+// its norm, 1.2e-15 by FP64 products, and is 4.9e-16 here (D >= 9: the digits are the
+// more exact, 2.2e-15 against 2.6e-15 at D = 9, 4.1e-15 against 1.4e-14 at D = 37).  A thread holds a point, DP >= D depths of it, and goes through 64
+// centres; bound by integer issue, about 10 instructions a product.
+template <int DP>
+__global__ void __launch_bounds__(256) oz_narrow_kernel(const int64_t *__restrict__ T, const int64_t *__restrict__ Y,
+                                                        int nn, int K, const OzScale *__restrict__ sc, size_t ldm,
+                                                        int64_t *__restrict__ out)
+{
+    const int m = blockIdx.x * 256 + threadIdx.x;
+    if (m >= nn)
+        return;
+    const int shift = sc->shift;
+    const int64_t half = shift ? 1ll << (shift - 1) : 0;
+    int64_t t[DP];
+#pragma unroll
+    for (int d = 0; d < DP; d++)
+        t[d] = T[(size_t) m * DP + d];
+    const int k1 = min(K, (int) (blockIdx.y + 1) * 64);
+#pragma unroll 4
+    for (int k = blockIdx.y * 64; k < k1; k++) {
+        int64_t sum = half;
+#pragma unroll
+        for (int d = 0; d < DP; d++)
+            sum += __mul64hi(t[d], Y[(size_t) k * DP + d]);
+        out[(size_t) k * ldm + m] = sum >> shift;
+    }
+}
+
 __device__ __forceinline__ void load_table(uint64_t *tab, const uint64_t *__restrict__ gtab)
 {
     for (int i = threadIdx.x; i < oz::TAB; i += blockDim.x)
         tab[i] = gtab[i];
 }
 
-// the base-2 exponent of a double's natural logarithm term, as a fixed-point value
+// the base-2 exponent of a double's natural logarithm term, as a fixed-point value; the
+// product's rounding error (log2 e as two doubles) and the bias are added as integers
 __device__ __forceinline__ uint64_t lam_of(double ln_s)
 {
-    return oz::to_wfix(ln_s * 1.4426950408889634 + (double) oz::WBIAS);
+    const double p = ln_s * 1.4426950408889634;
+    const double e = fma(ln_s, 2.0355273740931033e-17, fma(ln_s, 1.4426950408889634, -p));
+    return (uint64_t) (oz::scaled_int(p, oz::WFRAC) + oz::scaled_int(e, oz::WFRAC)) +
+           ((uint64_t) oz::WBIAS << oz::WFRAC);
 }
 
 struct OzStatsArgs {
@@ -670,6 +715,7 @@ int grid_of(size_t n, int cap)
 struct OzE {
     OzEArgs a;
     unsigned char *arena = nullptr;  // every buffer below, one allocation
+    int narrow = 0;  // depths of a row of 64-bit integers in Town and Yp, 0: digit planes
     int sa = 8, panels = 0, Dp = 0, Np = 0, Kp = 0, chunk = 0, nchunks = 0;
     const __nv_bfloat16 *Tp = nullptr;  // data planes (own or the caller's)
     __nv_bfloat16 *Town = nullptr, *Yp = nullptr;
@@ -732,6 +778,7 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     const int N = a.N, D = a.D, K = a.K;
     st->sa = a.Tb ? 1 : 8;
     st->Dp = a.Tb ? a.Tb_ld : rup(D, PANEL);
+    st->narrow = a.Tb || D > NARROW ? 0 : D <= 2 ? 2 : D <= 4 ? 4 : 8;
     st->panels = st->Dp / PANEL;
     st->Np = a.Tb ? a.Tb_rows : rup(N, 128);
     st->Kp = rup(K, 64);
@@ -793,7 +840,8 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         oz_absmax_kernel<<<grid_of((size_t) N * D, 1216), 256, 0, s>>>(a.T64, (size_t) N * D, a.tt, N, st->bits);
         if (!a.Tb)
             oz_slice_rows_kernel<<<grid_of((size_t) st->Np * st->Dp / 2, 16384), 256, 0, s>>>(
-                a.T64, N, D, st->Np, st->Dp, st->bits, st->Town, nullptr, 8, nullptr, nullptr, nullptr);
+                a.T64, N, D, st->Np, st->narrow ? st->narrow : st->Dp, st->bits, st->Town,
+                st->narrow ? (int64_t *) st->Town : nullptr, nullptr, 8, nullptr, nullptr, nullptr);
         e = cudaGetLastError();
         st->Tp = a.Tb ? a.Tb : st->Town;
     }
@@ -843,15 +891,32 @@ int slice_centres(OzE *st, const double *Y, const double *yy, cudaStream_t s)
     oz_absmax_kernel<<<grid_of((size_t) K * D, 608), 256, 0, s>>>(Y, (size_t) K * D, yy, K, st->bits + 2);
     DGTM_CUDA_TRY(cudaGetLastError());
     oz_slice_rows_kernel<<<grid_of((size_t) st->Kp * st->Dp / 2, 4864), 256, 0, s>>>(
-        Y, K, D, st->Kp, st->Dp, st->bits + 2, st->Yp, st->bits, st->sa, yy, st->sc, st->h);
+        Y, K, D, st->Kp, st->narrow ? st->narrow : st->Dp, st->bits + 2, st->Yp,
+        st->narrow ? (int64_t *) st->Yp : nullptr, st->bits, st->sa, yy, st->sc, st->h);
     DGTM_CUDA_TRY(cudaGetLastError());
     st->acc_whole = st->own_stats = 0;
+    return DGTM_OK;
+}
+
+// points m0 .. m0 + nn - 1 with centres k0 .. k0 + nk - 1 into out (narrow state)
+int narrow_products(OzE *st, int m0, int nn, int k0, int nk, size_t ldm, int64_t *out, cudaStream_t s)
+{
+    const int dp = st->narrow;
+    const auto kernel = dp == 2 ? oz_narrow_kernel<2> : dp == 4 ? oz_narrow_kernel<4> : oz_narrow_kernel<8>;
+    const dim3 grid(ceil_div(nn, 256), ceil_div(nk, 64));
+    kernel<<<grid, 256, 0, s>>>((const int64_t *) st->Tp + (size_t) m0 * dp, (const int64_t *) st->Yp + (size_t) k0 * dp,
+                                nn, nk, st->sc, ldm, out);
+    DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
 
 // the integer products of chunk c
 int chunk_products(OzE *st, int c, cudaStream_t s)
 {
+    if (st->narrow) {
+        const int n0 = c * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
+        return narrow_products(st, n0, nn, 0, st->a.K, st->ldm, st->acc, s);
+    }
     OzGemm g;
     g.A = st->Tp;
     g.B = st->Yp;
@@ -1058,7 +1123,10 @@ int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colst
         g.mtiles = ceil_div(m1 - m0, 128);
         g.mrows = (int) (m1 - m0);
         g.ldm = (size_t) g.mrows;
-        OZ_TRY(launch_oz_gemm(g, st->a.sms, st->a.status, s));
+        if (st->narrow)
+            OZ_TRY(narrow_products(st, (int) m0, m1 - (int) m0, k0, nk, g.ldm, st->acc, s));
+        else
+            OZ_TRY(launch_oz_gemm(g, st->a.sms, st->a.status, s));
         const int na = m0 < n0 ? n0 : (int) m0;
         OZ_TRY(launch(st->acc + (na - m0), g.ldm, na, m1 - na));
     }

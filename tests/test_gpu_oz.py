@@ -109,6 +109,33 @@ def test_map_matches_cuda_cores(pkg, monkeypatch, form, binary, D):
     assert rel(out[0], out[1]) <= 1e-12
 
 
+# few depths, whose products are 64-bit integers: both sides of every row length and of
+# the switch to digits, points and centres off the blocks of 256 and 64
+@pytest.mark.parametrize("N,D,K", [(520, 1, 65), (300, 2, 129), (257, 3, 130), (1030, 4, 64), (511, 5, 67),
+                                   (700, 8, 81), (513, 9, 66)])
+def test_few_depths(pkg, N, D, K):
+    """Responsibilities against extended precision.  Their relative error is c times
+    the errors of the distances to the centre and to the nearest one, two roundings
+    of |y|^2 / 2 and an integer unit each (under 2^-51 |y|^2 + 2^-53 |t||y| D), and a few
+    roundings of the exponent, its sum's logarithm and the result."""
+    T, Y, FI, X = problem(N, D, K, N + D)
+    beta, temp = 6.0, 1.5
+    with pkg.Context(T, FI, "fp64") as c:
+        assert c.path == "exact_slices"
+        c.set_Y(Y)
+        c.estep(beta, 1, temp)
+        R = c.R_block(0, K, 0, N)
+    q = np.longdouble
+    d = ((T[None].astype(q) - Y[:, None].astype(q)) ** 2).sum(2)
+    v = -d * (q(beta) / 2 / q(temp))
+    e = np.exp(v - v.max(0))
+    ref = e / e.sum(0)
+    y2, t2 = np.max(np.sum(Y * Y, 1)), np.max(np.sum(T * T, 1))
+    arg = float(-(v - v.max(0)).min()) + np.log(K)
+    tol = beta / (2 * temp) * 2 * (2.0**-51 * y2 + 2.0**-53 * D * np.sqrt(y2 * t2)) + 2.0**-52 * (arg + 4)
+    assert np.max(np.abs(R - ref) / ref) <= tol
+
+
 # the FP64 critical temperatures by digit slices against the CUDA-core scatter,
 # centre by centre: two dimensions, one and several tiles of features and of
 # centres, several batches of centres (a small budget), several chunks of points
