@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__rest
 // units of 2^u, each product's upper 64 bits (in 2^-58 of the operands' 2^e, eight of
 // them below 2^61) added exactly.  Eight digits of either operand leave 2^-54 of the largest product, which
 // at few depths is more than an FP64 sum loses: the error of R at D = 5 was 1.9e-15 of
-// its norm, 1.2e-15 by FP64 products, and is 4.9e-16 here (D >= 9: the digits are the
+// its norm, 1.2e-15 by FP64 products, and is 5.6e-16 here (D >= 9: the digits are the
 // more exact, 2.2e-15 against 2.6e-15 at D = 9, 4.1e-15 against 1.4e-14 at D = 37).  A thread holds a point, DP >= D depths of it, and goes through 64
 // centres; bound by integer issue, about 10 instructions a product.
 template <int DP>
@@ -184,14 +184,10 @@ __device__ __forceinline__ void load_table(uint64_t *tab, const uint64_t *__rest
         tab[i] = gtab[i];
 }
 
-// the base-2 exponent of a double's natural logarithm term, as a fixed-point value; the
-// product's rounding error (log2 e as two doubles) and the bias are added as integers
+// the base-2 exponent of a double's natural logarithm term, as a fixed-point value
 __device__ __forceinline__ uint64_t lam_of(double ln_s)
 {
-    const double p = ln_s * 1.4426950408889634;
-    const double e = fma(ln_s, 2.0355273740931033e-17, fma(ln_s, 1.4426950408889634, -p));
-    return (uint64_t) (oz::scaled_int(p, oz::WFRAC) + oz::scaled_int(e, oz::WFRAC)) +
-           ((uint64_t) oz::WBIAS << oz::WFRAC);
+    return oz::to_wfix(ln_s * 1.4426950408889634 + (double) oz::WBIAS);
 }
 
 struct OzStatsArgs {
