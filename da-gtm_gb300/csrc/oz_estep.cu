@@ -215,7 +215,7 @@ struct OzStatsArgs {
 __device__ __forceinline__ void add_power(uint64_t x, const oz::Mul &k, const uint64_t *tab, uint64_t &lo,
                                           uint32_t &hi)
 {
-    const uint64_t W = oz::mul_w(k, x <= k.lim ? x : k.lim);  // lim is 2000 bits down (or 0)
+    const uint64_t W = oz::mul_w(k, x <= k.lim ? x : k.lim);  // lim is 1024 bits down at least (or 0)
     const int n = (int) (W >> oz::WFRAC);
     if (n < 64 && x <= k.lim) {
         const uint64_t t = oz::exp2_neg(W, tab) >> n;
@@ -410,8 +410,10 @@ __device__ __forceinline__ uint64_t r_exponent(const OzPoint &o, int64_t v, cons
         return o.lam;
     const int64_t x = o.aref - v;
     const uint64_t ax = (uint64_t) (x < 0 ? -x : x);
-    if (ax > k.lim)
-        return x < 0 ? 0ull : ~0ull;
+    if (ax > k.lim) {
+        const uint64_t far = x < 0 ? ~0ull : oz::mul_far(k, ax);
+        return x < 0 ? 0ull : far == ~0ull ? far : o.lam + far;
+    }
     const uint64_t wv = oz::mul_w(k, ax);
     if (x >= 0)
         return o.lam + wv;

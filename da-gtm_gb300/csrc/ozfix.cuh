@@ -133,12 +133,15 @@ OZ_HD uint32_t digit_field(uint64_t biased, int i)
     return (uint32_t) (biased >> (7 * (DIGITS - 1 - i))) & (i == 0 ? 255u : 127u);
 }
 
-// w = x kappa in units of 2^-53, for 0 <= x <= lim: (mulhi(x << a, m)) >> b
+// w = x kappa in units of 2^-53, for 0 <= x <= lim: (mulhi(x << a, m)) >> b.  Beyond
+// lim, x << a has more than 64 bits (w is then 1024 at least) or w is 2000 or more.
 struct Mul {
     uint64_t m;
-    uint64_t lim;  // beyond it w leaves the exponents' range: the power is 0
+    uint64_t lim;
     int a, b;
 };
+
+constexpr uint64_t W_END = 2000ull << WFRAC;  // a power from here on is 0
 
 // kappa = k0 2^u with k0 known on the host and u (the unit of x) on the device
 struct MulBase {
@@ -164,16 +167,27 @@ OZ_HD Mul mul_at(const MulBase &k, int u)
     r.m = k.m;
     // x kappa 2^53 = x m 2^(ex + u + 53 - 64) = mulhi(x << a, m) >> b
     const int sh = k.ex + u + WFRAC;  // a - b
-    r.a = sh > 0 ? (sh < 63 ? sh : 63) : 0;
+    r.a = sh > 0 ? (sh < 65 ? sh : 65) : 0;         // above 63 only x = 0 is within lim
     r.b = sh < 0 ? (sh > -63 ? -sh : 63) : 0;
-    const uint64_t cap = (1ull << (63 - r.a)) - 1;  // x << a below 2^63
+    const uint64_t cap = sh > 63 ? 0ull : ~0ull >> r.a;  // x << a below 2^64
     const int ls = -(k.ex + u) - 20;                // lim = l0 2^ls, l0 < 2^32
     uint64_t l = ls >= 31 ? ~0ull >> 1 : ls >= 0 ? k.l0 << ls : ls > -64 ? k.l0 >> -ls : 0ull;
-    r.lim = sh > 63 ? 0ull : (l < cap ? l : cap);
+    r.lim = l < cap ? l : cap;
     return r;
 }
 
-OZ_HD uint64_t mul_w(const Mul &k, uint64_t x) { return mulhi(x << k.a, k.m) >> k.b; }
+OZ_HD uint64_t mul_w(const Mul &k, uint64_t x) { return mulhi(x << (k.a & 63), k.m) >> k.b; }
+
+// w of x > lim: ~0 from 2000 on.  What x << a has no room for below that has one bit
+// too many (m >= 2^63), so it is 2 mulhi(x << (a - 1), m): every power that FP64 can
+// hold, 2^-1074 the last, is kept whatever kappa's mantissa.
+OZ_HD uint64_t mul_far(const Mul &k, uint64_t x)
+{
+    if (k.a < 1 || k.a > 64 || x > ~0ull >> (k.a - 1))
+        return ~0ull;
+    const uint64_t h = mulhi(x << (k.a - 1), k.m);
+    return h < W_END / 2 ? 2 * h : ~0ull;
+}
 
 // 2^-(W 2^-53) = E 2^-63 2^-n with n = W >> 53: returns E in (2^62, 2^63].
 // 2^-f = T[f's top 12 bits] (1 - x), x = y - y^2/2 + y^3/6 - y^4/24 for

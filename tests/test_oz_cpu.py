@@ -20,3 +20,15 @@ def test_fixed_point_pieces(tmp_path):
     assert float(exp2) <= 2.0 ** -57
     assert float(dbl) <= 2.0 ** -53 + 2.0 ** -57
     assert float(prod) <= 1.0
+
+
+def test_exponents_over_the_whole_range(tmp_path):
+    """Every power that FP64 can hold (to 2^-1074) has an exponent, whatever the
+    mantissa of kappa and the unit (tests/oz_range_check.cc); within two units."""
+    exe = str(tmp_path / "oz_range_check")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-o", exe,
+                           os.path.join(ROOT, "tests", "oz_range_check.cc"), "-lm"])
+    dropped, beyond, worst = subprocess.run([exe], capture_output=True, text=True, timeout=300,
+                                            check=True).stdout.split()
+    assert int(dropped) == 0 and int(beyond) == 0
+    assert float(worst) <= 2.0
