@@ -145,11 +145,13 @@ __global__ void __launch_bounds__(FT, J <= 6 ? 2 : 1) pass1_f32_kernel(Pass1Args
     const double oc = ot ? a.c2 : a.c1;
     double s = 0.0;
 
+    // 8-byte copies where every row starts on 8 bytes: an even D, and a pointer that does
+    // (Y may be a caller's array, which is only known to start on 4)
+    const bool two = (D & 1) == 0 && ((uintptr_t) a.Y & 7) == 0;
     // depths d0 .. d1 - 1 of the centres k .. k + 63 into half buffer b; zeros outside
     auto fill = [&](int k, int b) {
         const int d0 = b * hd, n = b ? D4 - hd : hd;
         float *dst = Ys + b * TILE * lh;
-        const bool two = (D & 1) == 0;  // rows start on 8 bytes
         const int step = two ? 2 : 1;
         for (int r = warp; r < TILE; r += FT / 32) {
             const float *src = a.Y + (size_t) min(k + r, a.K - 1) * D;
@@ -367,6 +369,7 @@ __global__ void __launch_bounds__(FT, J <= 3 ? 2 : 1) pass2_f32_kernel(Pass2Args
     for (int i = 0; i < 4; i++)
         yf[i] = (float) (kw + i < a.K ? a.yy[kw + i] : 0.0);
     const float invK = (float) (1.0 / (double) a.K);
+    const bool two = (D & 1) == 0 && ((uintptr_t) a.T & 7) == 0;  // every row starts on 8 bytes
     // G of two centres (lanes 0-15: kw, kw + 1; 16-31: kw + 2, kw + 3) over the
     // points lane % 16 + 16 j, j = 0 .. 3, in this order
     double g[2] = {0.0, 0.0};
@@ -379,7 +382,7 @@ __global__ void __launch_bounds__(FT, J <= 3 ? 2 : 1) pass2_f32_kernel(Pass2Args
 
     for (int n0 = nb; n0 < ne; n0 += TILE) {
         __syncthreads();
-        if ((D & 1) == 0) {  // rows start on 8 bytes
+        if (two) {
 #pragma unroll 4
             for (int r = warp; r < TILE; r += FT / 32)
 #pragma unroll
