@@ -390,7 +390,7 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
     // bits flips some of those roundings, and a run would no longer repeat what
     // it gave before to better than the form's own 1e-5.
     if (precision == DGTM_FP64 && ozab_wanted(K, M1, D))
-        CK(unless_enomem(ozab_create(&c->ozab, K, M1, D, c->sms)));
+        CK(unless_enomem(ozab_create(&c->ozab, K, M1, D, c->sms, c->stream)));
     if (!c->ozab)
         CK(dev_alloc(&c->abpart, form_ab_scratch_doubles(M1, D)));
     // scalars, then the status words; on the host W follows where it is small

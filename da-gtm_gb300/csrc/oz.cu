@@ -34,6 +34,7 @@
 #include "sm100.cuh"
 
 #include <math.h>
+#include <new>
 #include <vector>
 
 namespace dgtm {
@@ -463,10 +464,14 @@ void ozab_destroy(OzAB *st)
     delete st;
 }
 
-int ozab_create(OzAB **out, int K, int M1, int D, int sms)
+int ozab_create(OzAB **out, int K, int M1, int D, int sms, cudaStream_t s)
 {
     *out = nullptr;
-    OzAB *st = new OzAB();
+    OzAB *st = new (std::nothrow) OzAB();
+    if (!st) {
+        set_error(DGTM_ENOMEM, "host allocation failed");
+        return DGTM_ENOMEM;
+    }
     st->K = K;
     st->M1 = M1;
     st->D = D;
@@ -497,8 +502,10 @@ int ozab_create(OzAB **out, int K, int M1, int D, int sms)
         e = cudaMalloc((void **) &st->part, sizeof(int64_t) * TM * TN * (size_t) st->ntile * st->splits);
     if (e == cudaSuccess)
         e = cudaMalloc((void **) &st->tiles, sizeof(int) * tiles.size());
+    // on the stream of their readers; from pageable memory the call returns once the
+    // list is staged
     if (e == cudaSuccess)
-        e = cudaMemcpy(st->tiles, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(st->tiles, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) {
         const int code = e == cudaErrorMemoryAllocation ? DGTM_ENOMEM : DGTM_ECUDA;
         cudaGetLastError();

@@ -46,7 +46,7 @@ int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s);
 
 // A = FI^T diag(G) FI and B = FI^T RT by digit slices; FI's planes are kept.
 struct OzAB;
-int ozab_create(OzAB **out, int K, int M1, int D, int sms);
+int ozab_create(OzAB **out, int K, int M1, int D, int sms, cudaStream_t s);
 int ozab_basis(OzAB *st, const double *FI, cudaStream_t s);
 void ozab_destroy(OzAB *st);
 // flag: [0..2] set to 0 (as launch_form_ab does), [3] the bounded waits' status word

@@ -829,7 +829,7 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     if (e == cudaSuccess)
         lay_out(st->arena);
     if (e == cudaSuccess)
-        e = cudaMemcpy(st->tab, host_table(), TAB_BYTES, cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(st->tab, host_table(), TAB_BYTES, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(st->bits, 0, sizeof(unsigned long long) * (4 + D + 1), s);
     if (e == cudaSuccess)
