@@ -389,7 +389,7 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
     // rounds the centres to FP32 / BF16 pieces, so a W that differs in its last
     // bits flips some of those roundings, and a run would no longer repeat what
     // it gave before to better than the form's own 1e-5.
-    if (precision == DGTM_FP64 && ozab_wanted(K, M1, D))
+    if (precision == DGTM_FP64 && slices_on() && ozab_wanted(K, M1, D))
         CK(unless_enomem(ozab_create(&c->ozab, K, M1, D, c->sms, c->stream)));
     if (!c->ozab)
         CK(dev_alloc(&c->abpart, form_ab_scratch_doubles(M1, D)));

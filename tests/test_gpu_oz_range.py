@@ -36,3 +36,28 @@ def test_far_centre_beyond_512_bits(pkg, orc, c):
     assert G[9] == pytest.approx(gk, rel=1e-11)
     assert np.max(np.abs(RT[9] - R[9] @ T)) <= 1e-11 * np.max(np.abs(R[9] @ T))
     assert np.isfinite(got_k[9]) and np.isfinite(got) and got == np.max(got_k)
+
+
+def test_switch_keeps_the_normal_equations_on_the_cuda_cores(pkg, monkeypatch):
+    """DGTM_X64=0 is the arm without digit slices: also for A = FI^T diag(G) FI, whose
+    slices take five launches instead of two."""
+    rng = np.random.default_rng(8)
+    K, M1, D = 8000, 65, 166
+    T = rng.random((260, D))
+    FI = np.concatenate([rng.random((K, M1 - 1)), np.ones((K, 1))], axis=1)
+    Y = rng.random((K, D))
+    launches, W = [], []
+    for on in ("1", "0"):
+        monkeypatch.setenv("DGTM_X64", on)
+        with pkg.Context(T, FI, "fp64") as c:
+            assert (c.path == "cuda_cores") == (on == "0")
+            c.set_timing(True)
+            c.set_Y(Y)
+            c.estep(2.0, 1, 1.5)
+            W.append(c.mstep()[1])
+            G, RT = c.get_stats()
+            launches.append(c.timing()["mstep_solve"]["launches"])
+    # the reduction of the CUDA-core responsibility pass is one launch more there
+    assert launches[0] == launches[1] - 1 + 3
+    tol = 16 * M1 * np.finfo(float).eps * np.linalg.cond(FI.T @ (G[:, None] * FI))
+    assert np.linalg.norm(W[0] - W[1]) <= tol * np.linalg.norm(W[1])
