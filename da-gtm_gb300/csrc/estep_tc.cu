@@ -1083,7 +1083,7 @@ struct P3Params {
     const float *T;      // N x D
     const double *gF;    // g (null: 1)
     double beta;
-    int *status;
+    int *status;         // the waits' status word, then the CTAs that are done (0 between launches)
 };
 
 template <int NP, int KL, int NT>
@@ -1297,13 +1297,13 @@ __global__ void __launch_bounds__(p3_threads(NP), 1)
         const float4 cq = p.colq[n];  // n < Npad: padding points carry R = 0
         bool ok = true;
         // OUT (this thread's row) to C: 16-column batches, batch i to group i % (BK / 32);
-        // the last one leaves dT (NaN once a bounded wait of the call has given up).
+        // the last one leaves dT.
         // A batch's loads are all issued before its first store: C and T may be any
         // buffers, so between stores each load would wait out its own latency.
         const bool quads = (p.D & 3) == 0 && (((uintptr_t) p.C | (uintptr_t) p.T) & 15) == 0;
         auto drain_out = [&](bool add, bool last) {
             const double g = p.gF ? p.gF[0] : 1.0;
-            const float gb = (float) (-(*(volatile int *) p.status ? NAN : g) * p.beta);
+            const float gb = (float) (-g * p.beta);
 #pragma unroll 1
             for (int c0 = 16 * h; c0 < p.nout; c0 += BK / 2) {
                 uint32_t v[16];
@@ -1384,10 +1384,6 @@ __global__ void __launch_bounds__(p3_threads(NP), 1)
                 }
             }
         }
-        if (!ok && n < p.N)  // this tile's rows are not complete
-            for (int d = 16 * h; d < p.D; d += BK / 2)
-                for (int e = d; e < min(d + 16, p.D); e++)
-                    p.C[(size_t) n * p.D + e] = NAN;
         if (!ok)
             failed = 1;
     }
@@ -1401,6 +1397,21 @@ __global__ void __launch_bounds__(p3_threads(NP), 1)
     tc_fence_after();
     if (warp == 0)
         tmem_dealloc(tmem, 512);
+    // The last CTA sees every CTA's waits: once one of this call has given up, all of
+    // dT is NaN, whichever tiles had finished before.
+    __shared__ int poison;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const bool last = atomicAdd(p.status + 1, 1) == (int) gridDim.x - 1;
+        if (last)
+            p.status[1] = 0;
+        __threadfence();
+        poison = last && *(volatile int *) p.status != 0;
+    }
+    __syncthreads();
+    if (poison)
+        for (size_t i = threadIdx.x; i < (size_t) p.N * p.D; i += p3_threads(NP))
+            p.C[i] = NAN;
 }
 
 using P3Kernel = void (*)(const CUtensorMap, const CUtensorMap, const P3Params);
@@ -1794,7 +1805,7 @@ int tc_create(TcState **out, int N, int D, int K, int sms, const double *T64, co
         tc_destroy(st);
         return code;
     };
-    cudaError_t e = cudaMalloc((void **) &st->status, sizeof(int));
+    cudaError_t e = cudaMalloc((void **) &st->status, 2 * sizeof(int));
     if (e == cudaSuccess)
         e = cudaMallocHost((void **) &st->hstatus, sizeof(int));
     if (e == cudaSuccess)
@@ -1907,7 +1918,7 @@ int tc_estep(TcState *st, const double *, double c1, double c2, int isDA, double
     p.colq = st->colq;
     p.part = part;
     p.status = st->status;
-    DGTM_CUDA_TRY(cudaMemsetAsync(st->status, 0, sizeof(int), s));
+    DGTM_CUDA_TRY(cudaMemsetAsync(st->status, 0, 2 * sizeof(int), s));  // and pass 3's count
     st->pass1<<<tc_pass1_blocks(st), P1_THREADS, st->smem1, s>>>(st->tmY1, st->tmT1, p);
     DGTM_CUDA_TRY(cudaGetLastError());
     *nlaunch = 1;
@@ -1970,7 +1981,8 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t) 255; }
 // A plan over the workspace: T always in two BF16 pieces (the data of a
 // gradient step are real-valued, and the piece count must be known without
 // inspecting them); Y pieces with the folded -|y|^2/2 columns; the column
-// statistics; the pass-2 slots; the status word of the bounded waits.
+// statistics; the pass-2 slots; the status word of the bounded waits and pass 3's count
+// of finished CTAs.
 static int fe_state(int N, int K, int D, int sms, TcState *st, TcFeLayout *L)
 {
     int rc = sm10x_or_fail();
@@ -1988,7 +2000,7 @@ static int fe_state(int N, int K, int D, int sms, TcState *st, TcFeLayout *L)
     L->Yb = take(sizeof(__nv_bfloat16) * 2 * (size_t) st->Kpad * st->Dp);
     L->colq = take(sizeof(float4) * (size_t) st->Npad);
     L->RTpart = take(sizeof(float) * (size_t) st->nunits * P2_BK * st->Dp);
-    L->status = take(sizeof(int));
+    L->status = take(2 * sizeof(int));
     L->total = o;
     L->pass1_blocks = tc_pass1_blocks(st);
     return DGTM_OK;
@@ -2037,7 +2049,7 @@ int tc_fe_estep(const TcFeLayout &L, void *ws, const float *Y, const float *T, i
         Y, K, D, st.Dp, st.Kpad, st.Yb, nullptr);
     DGTM_CUDA_TRY(cudaGetLastError());
     int nl = 0;
-    // tc_estep clears the status word.  The free energy needs the statistics at `temp` only.
+    // tc_estep clears the status words.  The free energy needs the statistics at `temp` only.
     return tc_estep(&st, nullptr, c1, c2, 1, colstat, part, s, &nl, false);
 }
 
