@@ -89,16 +89,19 @@ def project(T_new, Y, beta, temp=1.0, steps=50, lr=None):
 
     Each step moves the points along -dF/dT, i.e. towards sum_k R_kn y_k, with
     step size ``lr`` (default 1/beta, which makes one step the exact
-    fixed-point update t <- sum_k R_kn y_k at temp = 1).
+    fixed-point update t <- sum_k R_kn y_k at temp = 1; a number, or a tensor that
+    broadcasts against the points).
     """
-    T = T_new.detach().clone().contiguous()
+    # floating-point points only, whatever the number of steps
+    T = T_new.detach().clone().contiguous().requires_grad_(True).detach()
     Yd = Y.detach().contiguous()
     step = (1.0 / float(beta)) if lr is None else lr
-    if steps < 1:
+    rounds = range(steps)
+    if not rounds:
         return T
+    N, K, D = _check_pair(Yd, T)
     if not torch.is_grad_enabled():
         raise RuntimeError("project needs gradients: it cannot run where they are disabled")
-    N, K, D = _check_pair(Yd, T)
     lib = _pkg.load_library()
     stream = _stream(T.device)
     ws, ws_ptr, nbytes = _workspace(lib, N, K, D, T.device)
@@ -107,10 +110,16 @@ def project(T_new, Y, beta, temp=1.0, steps=50, lr=None):
     one = torch.ones((), dtype=torch.float64, device=T.device)
     b = float(beta)
     # the forward and the gradient in T of each step, without a graph
-    for _ in range(steps):
+    for _ in rounds:
         _pkg._check(lib.dgtm_fe_forward(Yd.data_ptr(), T.data_ptr(), N, K, D, b, float(temp), ws_ptr,
                                         nbytes, stream, F.data_ptr()))
         _pkg._check(lib.dgtm_fe_backward(Yd.data_ptr(), T.data_ptr(), N, K, D, b, float(temp), ws_ptr,
                                          nbytes, stream, one.data_ptr(), None, g.data_ptr(), None))
-        T.add_(g, alpha=step)  # F increases towards the centres: ascend
+        # F increases towards the centres: ascend; a rate may also be a tensor, one per
+        # point or coordinate
+        if isinstance(step, (int, float)):
+            T.add_(g, alpha=step)
+        else:
+            with torch.no_grad():
+                T += step * g
     return T
