@@ -584,6 +584,18 @@ int launch_pass1_f32(const Pass1Args<float> &a, cudaStream_t s)
     return DGTM_OK;
 }
 
+// Device code is loaded kernel by kernel on first use: this loads pass 1 of every D.
+int load_pass1_f32()
+{
+    for (const Kernels &k : KERNELS) {
+        cudaFuncAttributes attr;
+        DGTM_CUDA_TRY(cudaFuncGetAttributes(&attr, (const void *) k.p1));
+        const size_t smem = sizeof(float) * ((size_t) TILE * k.ld1 + TILE);
+        DGTM_CUDA_TRY(cudaFuncSetAttribute(k.p1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    }
+    return DGTM_OK;
+}
+
 int launch_pass2_f32(const Pass2Args<float> &a, int nsplit, cudaStream_t s)
 {
     const Kernels *k = nullptr;

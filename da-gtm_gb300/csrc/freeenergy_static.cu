@@ -73,6 +73,7 @@ bool current_context_id(unsigned long long *id)
 // array's device address (cudaGetSymbolAddress).  The first lookup in a
 // process may make the driver load this library's device code, which is
 // when the array is reserved on that device; later calls reuse the address.
+// The E-step kernel differs with D (eight classes): all are loaded here.
 int scratch_on_current_device(void **out)
 {
     int dev = 0;
@@ -99,6 +100,10 @@ int scratch_on_current_device(void **out)
             set_error(DGTM_ECUDA, "no current CUDA context for the no-alloc scratch");
             return DGTM_ECUDA;
         }
+        // a later call may be the first of its D: its kernel is loaded here as well
+        const int r = load_pass1_f32();
+        if (r != DGTM_OK)
+            return r;
         g_scratch[dev] = ScratchAddr{id, p};
     }
     *out = g_scratch[dev].addr;

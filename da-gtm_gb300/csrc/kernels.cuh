@@ -49,6 +49,7 @@ int launch_pass2_simt(const Pass2Args<F> &a, int nsplit, cudaStream_t s, bool ow
 // the FP32 form's passes (estep_f32.cu)
 int launch_pass1_f32(const Pass1Args<float> &a, cudaStream_t s);
 int launch_pass2_f32(const Pass2Args<float> &a, int nsplit, cudaStream_t s);
+int load_pass1_f32();
 int pass1_simt_blocks(int N);
 int pass2_simt_ktiles(int K);
 // M = R^T X (N x L, L <= 8) and explicit R blocks, FP64, from the column
