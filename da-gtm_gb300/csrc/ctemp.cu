@@ -48,7 +48,6 @@ constexpr int EIG_SMALL_D = 96;
 // largest dynamic shared memory a block may opt into on sm_10x (227 KB), less
 // room for the kernel's static arrays
 constexpr size_t EIG_SMEM_MAX = 232448 - 1024;
-constexpr double GG_MIN = 1e-250;  // comm/mpicomm.c:601-612
 constexpr size_t ALIGN = 256;
 
 size_t align_up(size_t b) { return (b + ALIGN - 1) / ALIGN * ALIGN; }
@@ -308,17 +307,11 @@ __global__ void __launch_bounds__(EIG_THREADS) eig_kernel(const double *__restri
             out[(size_t) kl * 2 + which] = 0.0;
         return;
     }
-    // gg < GG_MIN: the reference scales H by 1 / GG_MIN before gsl_eigen_symm
-    // and the eigenvalues back.  The FP32 arithmetic takes H / gg (1e250 is
-    // outside FP32) and multiplies the eigenvalues by gg; H was formed with
-    // weights scaled by r_scale, which the matrix scale takes back out.
-    double sc = 1.0, back = 1.0;
-    if (sizeof(F) == 8) {
-        if (gk < GG_MIN)
-            sc = 1.0 / GG_MIN, back = GG_MIN;
-    } else {
-        sc = 1.0 / (gk * r_scale(rmax, kl)), back = gk;
-    }
+    // The FP32 arithmetic takes H / gg (an H below gg = 1e-250, which the reference
+    // scales by 1e250, comm/mpicomm.c:601-612, is outside FP32) and multiplies the
+    // eigenvalues by gg; H was formed with weights scaled by r_scale, which the matrix
+    // scale takes back out.
+    const double sc = 1.0 / (gk * r_scale(rmax, kl)), back = gk;
     for (int e = threadIdx.x; e < D * D; e += EIG_THREADS) {
         const int i = e / D, j = e - i * D;
         const size_t at = i <= j ? (size_t) i * D + j : (size_t) j * D + i;
@@ -506,12 +499,22 @@ __global__ void __launch_bounds__(NT) eig64_kernel(const double *__restrict__ S,
             out[(size_t) kl * 2 + which] = 0.0;
         return;
     }
-    // gg < GG_MIN: the reference scales H by 1 / GG_MIN and the eigenvalues back
-    const double sc = gk < GG_MIN ? 1.0 / GG_MIN : 1.0, back = gk < GG_MIN ? GG_MIN : 1.0;
+    // S follows R, which is far below 1 at a far centre: from 2^-500 on its squares leave
+    // FP64's range, and every column would count as reduced.  Past 2^+-300 the matrix is
+    // brought near 1 by a power of two and the eigenvalues back (below gg = 1e-250 the
+    // reference scales H by 1e250, comm/mpicomm.c:601-612, inside a scaled reduction).
+    double top = 0.0;  // of S1's diagonal, which bounds every entry
+    for (int i = lane; i < D; i += 32)
+        top = fmax(top, S1[(size_t) i * D + i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    const int e0 = top > 0.0 && isfinite(top) ? ilogb(top) : 0, back = abs(e0) > 300 ? e0 : 0;
+    const double sc1 = ldexp(1.0, -(back / 2)), sc2 = ldexp(1.0, -(back - back / 2));
     for (int e = tid; e < D * D; e += NT) {
         const int i = e / D, j = e - i * D;
         const size_t at = i <= j ? (size_t) i * D + j : (size_t) j * D + i;
-        M[i * LD + j] = (which == 0 ? 2.0 * S1[at] : 2.0 * (S1[at] - S2[at])) * sc;
+        M[i * LD + j] = (which == 0 ? 2.0 * S1[at] : 2.0 * (S1[at] - S2[at])) * sc1 * sc2;
     }
     const int rw = (D + 31) & ~31;       // row threads
     const int ng = NT / rw;              // column groups
@@ -610,7 +613,7 @@ __global__ void __launch_bounds__(NT) eig64_kernel(const double *__restrict__ S,
         hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
     const double norm = fmax(fabs(lo), fabs(hi));
-    const double limit = lim_scale * gk / back;
+    const double limit = lim_scale * (gk * sc1 * sc2);
     double mx = 0.0;
     if (norm > 0.0 && isfinite(norm)) {
         const int ex = ilogb(norm);
@@ -646,7 +649,7 @@ __global__ void __launch_bounds__(NT) eig64_kernel(const double *__restrict__ S,
                 lo = nlo;
                 hi = nhi;
             }
-            const double lam = ldexp(0.5 * (lo + hi), ex) * back;
+            const double lam = ldexp(0.5 * (lo + hi), ex + back);
             mx = (c < D) ? fmax(lam, 0.0) : lam;
         }
     }  // else the zero matrix, or non-finite entries: 0

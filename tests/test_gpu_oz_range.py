@@ -61,3 +61,29 @@ def test_switch_keeps_the_normal_equations_on_the_cuda_cores(pkg, monkeypatch):
     assert launches[0] == launches[1] - 1 + 3
     tol = 16 * M1 * np.finfo(float).eps * np.linalg.cond(FI.T @ (G[:, None] * FI))
     assert np.linalg.norm(W[0] - W[1]) <= tol * np.linalg.norm(W[1])
+
+
+@pytest.mark.parametrize("pairs", ["1", "0"])
+@pytest.mark.parametrize("c", [3.0, 1.04])
+def test_critical_temperature_of_a_far_centre(pkg, orc, monkeypatch, pairs, c):
+    """The squares of a scatter matrix that follows R = 2^-850 are outside FP64: the
+    eigenvalue step still finds its eigenvalues, from both scatters."""
+    monkeypatch.setenv("DGTM_CTEMP_PAIRS", pairs)
+    rng = np.random.default_rng(4)
+    N, D, K, temp, eps = 3000, 40, 30, 1.1, 1e-6
+    s = 0.2 / np.sqrt(c)
+    T = s * rng.normal(size=(N, D))
+    Y = s * rng.normal(size=(K, D))
+    beta = 2.0 * temp * c
+    Y[9] = 0.0
+    Y[9, 0] = np.sqrt(2.0 * 640.0 / beta) + 0.5
+    R, _, _ = orc.resp(orc.dist(Y, T), beta, 1, temp)
+    with pkg.Context(T, np.ones((K, 1)), "fp64") as ctx:
+        ctx.set_Y(Y)
+        ctx.estep(beta, 1, temp)
+        got_k = ctx.next_ctemp(temp, beta, eps, per_centre=True)[1]
+    X = T - Y[9]
+    lam = np.linalg.eigvalsh((X * (R[9] / R[9].sum())[:, None]).T @ X * 2.0)  # R^2 is below FP64's range
+    lam[lam >= (temp - eps) * 2.0 / beta] = 0.0
+    # 2^-53 of the largest eigenvalue, which is 1600 times this one
+    assert got_k[9] == pytest.approx(beta / 2.0 * lam.max(), rel=1e-10)
