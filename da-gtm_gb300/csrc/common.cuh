@@ -47,19 +47,4 @@ __device__ __forceinline__ double block_sum_fixed(double v, double *scratch)
     return r;
 }
 
-// An FP32 value as FP64 by integer operations (a conversion takes the FP64 pipe's 16
-// clocks of the SM per warp); a subnormal is first scaled by 2^24, exactly, and
-// non-finite values are converted.
-__device__ __forceinline__ double widen(float f)
-{
-    const bool small = fabsf(f) < 1.17549435e-38f;
-    const uint32_t b = __float_as_uint(small ? __fmul_rn(f, 16777216.f) : f), m = b & 0x7FFFFFFFu;
-    if (m >= 0x7F800000u) {
-        asm volatile("");  // keeps the conversion behind the branch
-        return (double) f;
-    }
-    const uint32_t hi = (m >> 3) + (small ? 0x38000000u - (24u << 20) : 0x38000000u);
-    return __hiloint2double((int) ((b & 0x80000000u) | (m ? hi : 0u)), (int) (b << 29));
-}
-
 }  // namespace dgtm

@@ -23,6 +23,7 @@
 // issue and latency at two blocks an SM; pass 2 shared memory: 1010 wavefronts a warp
 // and tile of 64 points for 2100 FP32 multiply-adds' clocks over four schedulers.
 #include "common.cuh"
+#include "f32pair.cuh"
 #include "kernels.cuh"
 #include "sm100.cuh"
 
@@ -42,59 +43,6 @@ constexpr int P2C = 32;   // centres of a pass-2 block: four per warp
 // room for 32 lanes x J, so that every address is a base and a constant.
 template <int J>
 __host__ __device__ constexpr int row_stride() { return 32 * J + 4; }
-
-// a double as an unevaluated sum of two FP32 (48 bits)
-struct Pair {
-    float h, l;
-};
-
-__host__ __device__ __forceinline__ Pair split(double v)
-{
-    Pair r;
-    r.h = (float) v;
-    r.l = (float) (v - (double) r.h);
-    return r;
-}
-
-// s + e = a + b exactly
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
-{
-    s = __fadd_rn(a, b);
-    const float t = __fsub_rn(s, a);
-    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
-}
-
-// h + l rounded to FP32; ok is cleared when it is not safely away from a rounding
-// boundary (or not finite).  The remainder e may be off by 2^-42 |r|, at most 2^-17 of
-// the distance to the nearest boundary from r, so r is safe if e grown by 2^-16 still
-// rounds to it.
-__device__ __forceinline__ float settle(float h, float l, bool &ok)
-{
-    const float r = __fadd_rn(h, l);
-    const float e = __fsub_rn(l, __fsub_rn(r, h));
-    ok = ok && __fadd_rn(r, __fmul_rn(e, 1.f + 0x1p-16f)) == r;
-    return r;
-}
-
-// Whether c x is exactly h + l with h = c.h xh: then its rounding is that of the
-// FP64 product too, even half way between two FP32 numbers (a beta / 2 of a few
-// bits, such as 3, puts a quarter of the products there)
-__device__ __forceinline__ bool exact_product(Pair c, float xh, float xl)
-{
-    const float h = __fmul_rn(c.h, xh), l = __fmaf_rn(c.h, xh, -h), p = __fmul_rn(c.h, xl);
-    float s, e;
-    two_sum(l, p, s, e);
-    return c.l == 0.f && __fmaf_rn(c.h, xl, -p) == 0.f && e == 0.f;
-}
-
-// c x as a pair, x = xh + xl
-__device__ __forceinline__ void times(Pair c, float xh, float xl, float &h, float &l)
-{
-    h = __fmul_rn(c.h, xh);
-    l = __fmaf_rn(c.h, xh, -h);
-    l = __fmaf_rn(c.h, xl, l);
-    l = __fmaf_rn(c.l, xh, l);
-}
 
 }  // namespace
 
@@ -234,16 +182,14 @@ __global__ void __launch_bounds__(FT, J <= 6 ? 2 : 1) pass1_f32_kernel(Pass1Args
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const bool in = k0 + tx + 16 * j < a.K;
-                float xh, xl, h, l;
+                float xh, xl;
                 two_sum(in ? dd[j] : nm, -nm, xh, xl);
-                times(c1, xh, xl, h, l);
                 bool ok = true;
-                p1[j] = -settle(h, l, ok);
+                p1[j] = pass1_argument(c1, xh, xl, ok);
                 bad |= ok ? 0u : 1u << j;
                 if (a.isDA) {
-                    times(c2, xh, xl, h, l);
                     ok = true;
-                    p2[j] = -settle(h, l, ok);
+                    p2[j] = pass1_argument(c2, xh, xl, ok);
                     bad |= ok ? 0u : 16u << j;
                 }
             }
@@ -438,12 +384,7 @@ __global__ void __launch_bounds__(FT, J <= 3 ? 2 : 1) pass2_f32_kernel(Pass2Args
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 dd[i][e] = __fadd_rn(__fmaf_rn(-2.f, acc[i][e], yf[i]), p.w);
-                float xh, xl, h, l, t, u;
-                two_sum(dd[i][e], -p.x, xh, xl);
-                times(c, xh, xl, h, l);
-                two_sum(h, p.y, t, u);
-                u = __fadd_rn(u, __fadd_rn(l, p.z));
-                r[i][e] = -settle(t, u, ok);
+                r[i][e] = pass2_argument(c, dd[i][e], p.x, p.y, p.z, ok);
             }
         }
         if (!ok) {

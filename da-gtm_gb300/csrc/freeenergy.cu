@@ -17,6 +17,7 @@
 // R T for dF/dY and dF/dbeta; pass 3 gives sum_k R_kn y_k for dF/dT.  Other
 // shapes use the FP32 CUDA-core kernels of the FP32 form.
 #include "common.cuh"
+#include "f32pair.cuh"
 #include "kernels.cuh"
 #include "tc.cuh"
 

@@ -18,6 +18,7 @@
 //
 // Every reduction runs in a fixed order, so repeated runs are bit-identical.
 #include "common.cuh"
+#include "f32pair.cuh"
 #include "kernels.cuh"
 
 #include <cuda_bf16.h>
