@@ -848,7 +848,7 @@ int map_impl(dgtm_ctx *ctx, const double *X, int L, double *M, int ldM, bool rd)
                                     ctx->stream);
     if (e == cudaSuccess) {
         if (oz) {
-            r = oze_map(oz, ctx->Y64, ctx->yy, ctx->colstat, c, dX, L, dM, ctx->stream);
+            r = oze_map(oz, ctx->Y64, ctx->yy, ctx->colstat, ctx->beta / 2.0, c, dX, L, dM, ctx->stream);
             if (r == DGTM_OK)
                 r = fetch_ctl(ctx);
         } else if (rd)
@@ -899,7 +899,7 @@ int r_block_impl(dgtm_ctx *ctx, int k0, int nk, int n0, int nn, double *R, int l
     // from the E-step's own distances where those are digit slices; the other forms
     // have the slices after a large map, and use them for blocks worth their launches
     OzE *oz = rd ? nullptr : ctx->oze ? ctx->oze : (size_t) nk * nn >= 65536 ? ctx->ozmap : nullptr;
-    int r = oz ? oze_r_block(oz, ctx->Y64, ctx->yy, ctx->colstat, c, dcut, k0, nk, n0, nn, dR, ctx->stream)
+    int r = oz ? oze_r_block(oz, ctx->Y64, ctx->yy, ctx->colstat, ctx->beta / 2.0, c, dcut, k0, nk, n0, nn, dR, ctx->stream)
             : rd ? launch_r_block(ctx->T64, ctx->Yprev, ctx->tt, ctx->yyprev, ctx->colstat, ctx->D,
                                 ctx->K, c, k0, nk, n0, nn, dR, ctx->stream, ctx->Y64, ctx->yy, dcut)
                : launch_r_block(ctx->T64, ctx->Y64, ctx->tt, ctx->yy, ctx->colstat, ctx->D, ctx->K,
@@ -1006,7 +1006,7 @@ int dgtm_next_ctemp_k(dgtm_ctx *ctx, double temp, double beta, double eps, const
         std::vector<double> spread(K);
         rc = dev_alloc(&dspread, (size_t) K);
         if (rc == DGTM_OK)
-            rc = oz_ctemp(slices, ctx->T64, ctx->Y64, ctx->yy, ctx->colstat, N, D, K, ctx->sms, c, dcut,
+            rc = oz_ctemp(slices, ctx->T64, ctx->Y64, ctx->yy, ctx->colstat, N, D, K, ctx->sms, ctx->beta / 2.0, c, dcut,
                           gg ? dgg : nullptr, lim_scale, bounded ? budget : gbudget, dgsum, dout, dspread,
                           ctx->flag + 3, ctx->stream);
         if (rc == DGTM_OK)

@@ -66,7 +66,8 @@ struct OzParams {
     int64_t *out;
     size_t ldm;
     int mrows, ncols;
-    const int *shift;
+    const OzUnit *units;
+    const oz::Centre *cen;
     int *status;
 };
 
@@ -249,8 +250,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
         const int q = warp & 3, h = (warp - 2) >> 2;  // lane quarter, 16 of the columns
         const uint32_t lane_base = tmem + ((uint32_t) (q * 32) << 16) + (uint32_t) (16 * h);
         const int row = q * 32 + lane;
-        const int shift = SUM ? 8 + p.ext : (p.shift ? *p.shift : 0);
-        const int64_t half = SUM ? (1ll << (shift - 1)) : 0;
+        const int shift = 8 + p.ext;  // sums
+        const int64_t half = 1ll << (shift - 1);
         int nseg = 0;
         bool ok = true;
         for (int it = blockIdx.x; ok && it < p.nitems; it += gridDim.x) {
@@ -262,6 +263,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
                 for (int c = 0; c < 16; c++)
                     acc[c] = 0;
             }
+            OzUnit un{0, 0};
+            if constexpr (!SUM)
+                un = p.units[min(mt * TM + row, p.mrows - 1)];
             for (int pn = p0; pn < p1; pn += SEG, nseg++) {
                 if (!mbar_wait(acc_full, (uint32_t) (nseg & 1), p.status, 76)) {
                     ok = false;
@@ -275,6 +279,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
 #pragma unroll
                     for (int l = 0; l < SB; l++)
                         tmem_ld4p(lane_base + (uint32_t) (l * TN + 4 * cb), v + 4 * l);
+                    oz::Centre cen[SUM ? 1 : 4];
+                    if constexpr (!SUM) {
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            cen[c] = p.cen[min(nt * TN + 16 * h + 4 * cb + c, p.ncols - 1)];
+                    }
                     tmem_ld_wait();
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
@@ -285,11 +295,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
                             acc[4 * cb + c] += hi * (1 << (28 - shift)) + ((lo + half) >> shift);
                         } else {
                             // units 2^-61 (sa = 8): 8 bits down; sa = 1: exact in 2^-55
-                            int64_t I = SA == 1 ? hi * 268435456 + lo : hi * 1048576 + ((lo + 128) >> 8);
-                            I >>= shift;
+                            const int64_t I = SA == 1 ? hi * 268435456 + lo : hi * 1048576 + ((lo + 128) >> 8);
                             const int n = nt * TN + 16 * h + 4 * cb + c, m = mt * TM + row;
                             if (m < p.mrows && n < p.ncols)
-                                p.out[(size_t) n * p.ldm + m] = I;
+                                p.out[(size_t) n * p.ldm + m] = oz::level(I, cen[c], un.p, un.u);
                         }
                     }
                 }
@@ -382,7 +391,8 @@ int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
     p.ldm = g.ldm;
     p.mrows = g.mrows;
     p.ncols = g.ncols;
-    p.shift = g.shift;
+    p.units = g.units;
+    p.cen = g.cen;
     p.status = status;
     using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const OzParams);
     // |S_l| <= (l + 1) 64 panels 4096: at most 2^22 for two panels, and for 0/1 data

@@ -10,6 +10,11 @@
 
 namespace dgtm {
 
+// a point's unit 2^u and p (oz::level)
+struct OzUnit {
+    int p, u;
+};
+
 // One product C[m][n] = sum_k A[m][k] B[n][k] over digit planes: A has sa planes
 // (8, or 1 for values that are small integers themselves) of a_rows x 64
 // a_panels BF16, B has 8 planes of b_rows x 64 b_panels; a_rows a multiple of
@@ -32,12 +37,14 @@ struct OzGemm {
     // integers of all splits can be added
     int64_t *out64 = nullptr;
     int item_panels = 0;
-    // distances (out64 == null, panels <= 4): out[n ldm + m] = sum >> shift in units of
-    // 2^-53 (sa = 8) or 2^-55 (sa = 1) of the operands' 2^e, for m < mrows, n < ncols
+    // distances (out64 == null, panels <= 4): out[n ldm + m] = oz::level of the sum, which
+    // is in units of 2^-53 (sa = 8) or 2^-55 (sa = 1) of the operands' 2^e, for m < mrows,
+    // n < ncols; units of A's rows from a_tile0, centres of B's rows from b_row0
     int64_t *out = nullptr;
     size_t ldm = 0;
     int mrows = 0, ncols = 0;
-    const int *shift = nullptr;  // device: further right shift (see oz.cu)
+    const OzUnit *units = nullptr;
+    const oz::Centre *cen = nullptr;
 };
 
 int oz_sum_ext(int panels);
@@ -78,21 +85,23 @@ int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, 
               double2 *colstat, double *part, double dcut, double *sums, int *nlaunch, cudaStream_t s);
 int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaStream_t s);
 // The parts other products with R are made of.  oze_refer: the centres' planes and
-// the points' references (kept when they are those of the last oze_estep);
+// the points' references (kept when they are those of the last oze_estep; c1 = beta / 2,
+// c the exponents' factor);
 // oze_chunks: how many chunks, and their points; oze_r_digits: R (or R^2) of the
 // centres k0 .. k0 + kb over a chunk as eight planes of prows x (points rounded
 // up to 64), and the integer exponents of their grids: an integer sum of the
 // product with B counts 2^(5 - nmin[k]) of B's grid (oz_sum_ext).  products: form
 // the chunk's distances first (they stay until the next chunk's).
-int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat, double dcut, cudaStream_t s);
+int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c1, double c, double dcut,
+              cudaStream_t s);
 int oze_chunks(const OzE *st, int *points);
 int oze_r_digits(OzE *st, int ch, int k0, int kb, double c, bool squares, bool products, int prows,
                  __nv_bfloat16 *planes, int *nmin, cudaStream_t s);
 // R of the centres k0 .. k0 + nk and the points n0 .. n0 + nn (nk x nn)
-int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c, double dcut,
+int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c1, double c, double dcut,
                 int k0, int nk, int n0, int nn, double *R, cudaStream_t s);
 // M = R^T X from a context's column statistics
-int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c,
+int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c1, double c,
             const double *X, int L, double *M, cudaStream_t s);
 
 // The AUTO schedule's scatter in FP64 accuracy as digit-slice products of R and
@@ -100,7 +109,7 @@ int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, 
 // spread[k] = tr(sum R x x^T) / tr(S1) about the data's mean: what the expansion
 // cancels.  DGTM_ENOMEM (nothing done) if not even 128 centres fit the budget.
 int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, const double2 *colstat, int N,
-             int D, int K, int sms, double c, double dcut, const double *gg_dev, double lim_scale,
+             int D, int K, int sms, double c1, double c, double dcut, const double *gg_dev, double lim_scale,
              size_t budget, double *gsum_dev, double *out_dev, double *spread_dev, int *status,
              cudaStream_t s);
 

@@ -253,7 +253,7 @@ size_t align_up(size_t b) { return (b + 255) / 256 * 256; }
     } while (0)
 
 int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, const double2 *colstat, int N,
-             int D, int K, int sms, double c, double dcut, const double *gg_dev, double lim_scale,
+             int D, int K, int sms, double c1, double c, double dcut, const double *gg_dev, double lim_scale,
              size_t budget, double *gsum_dev, double *out_dev, double *spread_dev, int *status,
              cudaStream_t s)
 {
@@ -314,7 +314,7 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
         zmax_kernel<<<dim3(blocks, ceil_div(D, 32)), 256, 0, s>>>(T64, N, D, mean, zbits);
         feature_table_kernel<<<ceil_div(Fp, 256), 256, 0, s>>>(F, Fp, D, zbits, ftab);
         DGTM_CUDA_TRY(cudaGetLastError());
-        OZ_TRY(oze_refer(st, Y, yy, colstat, dcut, s));
+        OZ_TRY(oze_refer(st, Y, yy, colstat, c1, c, dcut, s));
         for (int k0 = 0; k0 < K; k0 += kpad) {
             const int kb = K - k0 < kpad ? K - k0 : kpad;
             // rows without a centre count as zero

@@ -7,10 +7,12 @@
 // Here the contraction runs on the tensor cores and what is left per pair on the
 // integer pipe:
 //
-//   distances.  acc_kn = y_k.t_n - |y_k|^2 / 2 = (|t_n|^2 - d_kn) / 2 as a 64-bit
-//     integer on one power-of-two grid (unit 2^u, at most 2^-53 of the largest
-//     product), so the best centre is an integer comparison and
-//     d_kn - d_min = 2 (acc_max - acc_kn) 2^u an exact integer difference.
+//   distances.  v_kn = y_k.t_n - |y_k|^2 / 2 = (|t_n|^2 - d_kn) / 2 as a 64-bit integer in
+//     units 2^u of the point's own (ozfix.cuh), so the best centre is an integer
+//     comparison and d_kn - d_min = 2 (v_max - v_kn) 2^u an exact integer difference.
+//     Every point and every centre is cut into digits on the power-of-two grid of its
+//     own largest coordinate: the error of d_kn follows |t_n| and |y_k|, as that of an
+//     FP64 sum does, whatever other points and centres hold.
 //   exponentials.  2^-W for the fixed-point W = c log2(e) (d_kn - d_min) (+ log2 of
 //     the column sum), units of 2^-53 (ozfix.cuh): no FP64 operation.
 //   column sums.  2^-63 integers with a carry word: exact, order-free.
@@ -31,6 +33,7 @@
 #include <math.h>
 #include <new>
 #include <type_traits>
+#include <vector>
 
 namespace dgtm {
 
@@ -46,123 +49,120 @@ constexpr size_t TAB_BYTES = sizeof(uint64_t) * oz::TAB;
 
 __host__ __device__ constexpr int rup(int a, int b) { return (a + b - 1) / b * b; }
 
-// the centres' grid, set by oz_slice_rows_kernel
+// what the centres' kernel leaves for the units; two of them take turns, the idle one
+// reset by oz_units_kernel
 struct OzScale {
-    int shift;  // right shift of the product's integers (oz.cuh)
-    int u;      // one unit of acc is 2^u
-    int bad;    // a centre is not finite
+    int ymin;  // least exponent of a centre's |y|^2
+    int bad;   // a centre is not finite
 };
+constexpr int YMIN_START = 1 << 20;
 
 // a point's reference and the exponent its responsibilities start from
 struct OzPoint {
-    int64_t aref;   // (t^2 - d_ref) / 2 in units, or ZERO_COLUMN
+    int64_t aref;   // v of its d_ref, or ZERO_COLUMN
     uint64_t lam;   // log2 s + WBIAS (2^-53)
 };
 
-// max |y| and max |y|^2 of the centres, as bits
-__global__ void __launch_bounds__(256) oz_absmax_kernel(const double *__restrict__ X, size_t n,
-                                                        const double *__restrict__ xx, int rows,
-                                                        unsigned long long *__restrict__ bits)
-{
-    unsigned long long m = 0ull, q = 0ull;
-    for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < n; i += (size_t) gridDim.x * 256) {
-        const unsigned long long b = oz::double_bits(X[i]) & oz::ABS_MASK;
-        m = b > m ? b : m;
-        if (i < (size_t) rows) {
-            const unsigned long long c = oz::double_bits(xx[i]) & oz::ABS_MASK;
-            q = c > q ? c : q;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long a = __shfl_xor_sync(0xffffffffu, m, o), b = __shfl_xor_sync(0xffffffffu, q, o);
-        m = a > m ? a : m;
-        q = b > q ? b : q;
-    }
-    __shared__ unsigned long long red[2][8];
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = m;
-        red[1][threadIdx.x >> 5] = q;
-    }
-    __syncthreads();
-    if (threadIdx.x < 2) {
-        m = 0ull;
-        for (int i = 0; i < 8; i++)
-            m = red[threadIdx.x][i] > m ? red[threadIdx.x][i] : m;
-        atomicMax(&bits[threadIdx.x], m);
-    }
-}
-
-// planes[i][r][d] = digit i of X[r][d] on the common grid of bits[0]; zero past rows
-// and D.  fixed (instead of planes): [r][d] = X[r][d] as an integer below 2^61, ld of a row.  With sc: the grid of the products with T (tbits: its max |t| and |t|^2;
-// sa its planes) and h_k = |y_k|^2 / 2 on it.
+// planes[i][r][d] = digit i of X[r][d] on the grid of row r's largest value; zero past rows
+// and D.  fixed (instead of planes): [r][d] = X[r][d] as an integer below 2^61, ld of a row.
+// ex: the rows' exponents (may be null).  cen: the rows as centres, with xx = |x|^2, and
+// their sc (both may be null).  A warp a row, ld <= 256.
 __global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__restrict__ X, int rows, int D,
                                                             int prows, int ld,
-                                                            const unsigned long long *__restrict__ bits,
                                                             __nv_bfloat16 *__restrict__ planes,
-                                                            int64_t *__restrict__ fixed,
-                                                            const unsigned long long *__restrict__ tbits,
-                                                            int sa, const double *__restrict__ xx,
-                                                            OzScale *sc, int64_t *__restrict__ h)
+                                                            int64_t *__restrict__ fixed, int *__restrict__ ex,
+                                                            const double *__restrict__ xx,
+                                                            oz::Centre *__restrict__ cen, OzScale *sc)
 {
-    const int e = oz::exponent_of(bits[0]);
+    const int lane = threadIdx.x & 31;
     const size_t n2 = (size_t) prows * ld / 2;
-    if (sc) {
-        // |t.y| + |y|^2 / 2, and differences of two such, within 2^62 units
-        const int base = sa == 1 ? e - 55 : oz::exponent_of(tbits[0]) + e - (fixed ? 58 : 53);
-        const double tt = oz::bits_double(tbits[1]), yy = oz::bits_double(bits[1]);
-        const double bound = 2.0 * (sqrt(tt) * sqrt(yy) + 0.5 * yy);
-        const int need = oz::exponent_of(oz::double_bits(bound)) - 62;
-        const int u = need > base ? need : base;
-        const int bad = bits[0] >= oz::INF_BITS || bits[1] >= oz::INF_BITS;
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            sc->shift = u - base < 60 ? u - base : 60;
-            sc->u = u;
-            sc->bad = bad;
-        }
-        for (int k = blockIdx.x * 256 + threadIdx.x; k < rows; k += gridDim.x * 256)
-            h[k] = bad ? 0 : oz::scaled_int(xx[k], -1 - u);
-    }
-    if (fixed) {
-        for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < (size_t) rows * ld; i += (size_t) gridDim.x * 256) {
-            const int r = (int) (i / ld), d = (int) (i % ld);
-            fixed[i] = d < D ? oz::scaled_int(X[(size_t) r * D + d], 61 - e) : 0;
-        }
-        return;
-    }
-    for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < n2; i += (size_t) gridDim.x * 256) {
-        const int r = (int) (2 * i / ld), d = (int) (2 * i % ld);
-        int64_t a = 0, b = 0;
-        if (r < rows) {
-            const double *x = X + (size_t) r * D;
-            a = d < D ? oz::to_fixed(x[d], e) : 0;
-            b = d + 1 < D ? oz::to_fixed(x[d + 1], e) : 0;
-        }
-        uint32_t *dst = (uint32_t *) planes + i, w[oz::DIGITS];
-        digit_pairs(a, b, w);
+    int ymin = YMIN_START, bad = 0;
+    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < prows; r += gridDim.x * 8) {
+        double x[8];  // depths 2 lane + 64 i, + 1
+        unsigned long long m = 0ull;
 #pragma unroll
-        for (int p = 0; p < oz::DIGITS; p++)
-            dst[(size_t) p * n2] = w[p];
+        for (int i = 0; i < 8; i++) {
+            const int d = 2 * lane + 64 * (i >> 1) + (i & 1);
+            x[i] = r < rows && d < D ? X[(size_t) r * D + d] : 0.0;
+            const unsigned long long b = oz::double_bits(x[i]) & oz::ABS_MASK;
+            m = b > m ? b : m;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long b = __shfl_xor_sync(0xffffffffu, m, o);
+            m = b > m ? b : m;
+        }
+        const int e = oz::exponent_of(m);
+        if (r < rows && lane == 0) {
+            if (ex)
+                ex[r] = e;
+            if (cen) {
+                cen[r] = oz::make_centre(m, xx[r]);
+                ymin = min(ymin, oz::exponent_of(oz::double_bits(xx[r]) & oz::ABS_MASK));
+                bad |= m >= oz::INF_BITS;
+            }
+        }
+        if (fixed) {
+            if (r < rows)
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    if (2 * lane + i < ld)
+                        fixed[(size_t) r * ld + 2 * lane + i] = oz::scaled_int(x[i], 61 - e);
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            const int d = 2 * lane + 32 * i;
+            if (d >= ld)
+                break;
+            uint32_t w[oz::DIGITS];
+            digit_pairs(oz::to_fixed(x[i], e), oz::to_fixed(x[i + 1], e), w);
+            uint32_t *dst = (uint32_t *) planes + ((size_t) r * ld + d) / 2;
+#pragma unroll
+            for (int p = 0; p < oz::DIGITS; p++)
+                dst[(size_t) p * n2] = w[p];
+        }
+    }
+    if (sc && lane == 0) {
+        atomicMin(&sc->ymin, ymin);
+        if (bad)
+            atomicOr(&sc->bad, 1);
     }
 }
 
-// The products of up to 8 depths as 64-bit integers: out[k ldm + m] = y_k . t_m in
-// units of 2^u, each product's upper 64 bits (in 2^-58 of the operands' 2^e, eight of
-// them below 2^61) added exactly.  Eight digits of either operand leave 2^-54 of the largest product, which
-// at few depths is more than an FP64 sum loses: the error of R at D = 5 was 1.9e-15 of
-// its norm, 1.2e-15 by FP64 products, and is 5.6e-16 here (D >= 9: the digits are the
-// more exact, 2.2e-15 against 2.6e-15 at D = 9, 4.1e-15 against 1.4e-14 at D = 37).  A thread holds a point, DP >= D depths of it, and goes through 64
-// centres; bound by integer issue, about 10 instructions a product.
+// The points' units for the centres that left sc; idle: the next call's sc.  The product is
+// in units of 2^(e + f - bits), or 2^(f - bits) where the data are exact (0/1).
+__global__ void __launch_bounds__(256) oz_units_kernel(const int *__restrict__ ex, const double *__restrict__ tt, int N,
+                                                       const OzScale *__restrict__ sc, OzScale *__restrict__ idle,
+                                                       int bits, bool exact, int ucap, OzUnit *__restrict__ units)
+{
+    const int ymin = sc->ymin;
+    for (int n = blockIdx.x * 256 + threadIdx.x; n < N; n += gridDim.x * 256) {
+        units[n] = OzUnit{exact ? -bits : ex[n] - bits,
+                          oz::point_unit(oz::exponent_of(oz::double_bits(tt[n])), ymin, ucap)};
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *idle = OzScale{YMIN_START, 0};
+}
+
+// The products of up to 8 depths as 64-bit integers: each product's upper 64 bits (in
+// 2^-58 of the operands' 2^e, eight of them below 2^61) added exactly, then oz::level.  Eight
+// digits of either operand leave 2^-54 of the largest product, which at few depths is more
+// than an FP64 sum loses: on one grid for all points the error of R at D = 5 was 1.9e-15 of
+// its norm, 1.2e-15 by FP64 products, and is 5.6e-16 this way (D >= 9: the digits were the more
+// exact, 2.2e-15 against 2.6e-15 at D = 9, 4.1e-15 against 1.4e-14 at D = 37).  A thread
+// holds a point, DP >= D depths of it, and goes through 64 centres; bound by integer issue,
+// about 10 instructions a product.
 template <int DP>
 __global__ void __launch_bounds__(256) oz_narrow_kernel(const int64_t *__restrict__ T, const int64_t *__restrict__ Y,
-                                                        int nn, int K, const OzScale *__restrict__ sc, size_t ldm,
+                                                        int nn, int K, const OzUnit *__restrict__ units,
+                                                        const oz::Centre *__restrict__ cen, size_t ldm,
                                                         int64_t *__restrict__ out)
 {
     const int m = blockIdx.x * 256 + threadIdx.x;
     if (m >= nn)
         return;
-    const int shift = sc->shift;
-    const int64_t half = shift ? 1ll << (shift - 1) : 0;
+    const OzUnit un = units[m];
     int64_t t[DP];
 #pragma unroll
     for (int d = 0; d < DP; d++)
@@ -170,11 +170,11 @@ __global__ void __launch_bounds__(256) oz_narrow_kernel(const int64_t *__restric
     const int k1 = min(K, (int) (blockIdx.y + 1) * 64);
 #pragma unroll 4
     for (int k = blockIdx.y * 64; k < k1; k++) {
-        int64_t sum = half;
+        int64_t sum = 0;
 #pragma unroll
         for (int d = 0; d < DP; d++)
             sum += __mul64hi(t[d], Y[(size_t) k * DP + d]);
-        out[(size_t) k * ldm + m] = sum >> shift;
+        out[(size_t) k * ldm + m] = oz::level(sum, cen[k], un.p, un.u);
     }
 }
 
@@ -193,8 +193,8 @@ __device__ __forceinline__ uint64_t lam_of(double ln_s)
 struct OzStatsArgs {
     const int64_t *acc;    // K x ldm
     size_t ldm;
-    const int64_t *h;      // K
     const OzScale *sc;
+    const OzUnit *units;   // this chunk's points
     const uint64_t *tab;
     const double *tt;      // this chunk's points
     int nn, K, isDA;
@@ -203,7 +203,6 @@ struct OzStatsArgs {
     double2 *colstat;
     OzPoint *pt;
     int64_t *thr;
-    unsigned long long *ybits;  // the centres' maxima, zeroed for the next call
     double *part;          // 2 per block of the call
     double *block_part;    // of this launch
     double *sums;          // totals, from the last block of the call
@@ -242,8 +241,7 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
     const int p = blockIdx.x * ST_PTS + pl;
     const bool live = p < a.nn;
     const int64_t *acc = a.acc + (live ? p : 0);
-    if (blockIdx.x == 0 && threadIdx.x < 2)
-        a.ybits[threadIdx.x] = 0ull;
+    const int u = a.units[live ? p : 0].u;
     load_table(tab, a.tab);
     int64_t m = INT64_MIN;
     for (int k0 = kg; k0 < a.K; k0 += 8 * ST_KG) {
@@ -251,7 +249,7 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const int k = min(k0 + j * ST_KG, a.K - 1);  // a repeated centre changes no maximum
-            v[j] = acc[(size_t) k * a.ldm] - a.h[k];
+            v[j] = acc[(size_t) k * a.ldm];
         }
 #pragma unroll
         for (int j = 0; j < 8; j++)
@@ -269,7 +267,6 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
 #pragma unroll
     for (int i = 1; i < ST_WARPS; i++)
         m = smax[i][pl] > m ? smax[i][pl] : m;
-    const int u = a.sc->u;
     const oz::Mul k1 = oz::mul_at(a.k1, u), k2 = oz::mul_at(a.k2, u);
     uint64_t lo1 = 0, lo2 = 0;
     uint32_t hi1 = 0, hi2 = 0;
@@ -278,7 +275,7 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int k = min(k0 + j * ST_KG, a.K - 1);
-            x[j] = (uint64_t) (m - (acc[(size_t) k * a.ldm] - a.h[k]));
+            x[j] = (uint64_t) (m - acc[(size_t) k * a.ldm]);
             if (k0 + j * ST_KG >= a.K)
                 x[j] = ~0ull;
         }
@@ -382,28 +379,26 @@ __global__ void __launch_bounds__(NT) oz_stats_kernel(const OzStatsArgs a)
 
 // references and exponents from a context's column statistics (d_ref, ln s)
 __global__ void oz_points_kernel(const double2 *__restrict__ colstat, const double *__restrict__ tt, int N,
-                                 int K, const OzScale *__restrict__ sc, double dcut,
-                                 OzPoint *__restrict__ pt, int64_t *__restrict__ thr,
-                                 unsigned long long *__restrict__ ybits)
+                                 int K, const OzScale *__restrict__ sc, const OzUnit *__restrict__ units,
+                                 double dcut, OzPoint *__restrict__ pt, int64_t *__restrict__ thr)
 {
-    if (blockIdx.x == 0 && threadIdx.x < 2)
-        ybits[threadIdx.x] = 0ull;
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
         const double2 cs = colstat[n];
+        const int u = units[n].u;
         OzPoint o;
         if (isnan(cs.y) || sc->bad) {
             o.aref = ZERO_COLUMN;
             o.lam = lam_of(log((double) K));
         } else {
-            o.aref = oz::scaled_int(tt[n] - cs.x, -1 - sc->u);
+            o.aref = oz::scaled_int(tt[n] - cs.x, -1 - u);
             o.lam = lam_of(cs.y);
         }
         pt[n] = o;
-        thr[n] = o.aref == ZERO_COLUMN ? INT64_MIN : oz::scaled_int(tt[n] - dcut, -1 - sc->u);
+        thr[n] = o.aref == ZERO_COLUMN ? INT64_MIN : oz::scaled_int(tt[n] - dcut, -1 - u);
     }
 }
 
-// W of R = 2^(WBIAS - W): w(aref - acc) + lam; ~0 where R is 0
+// W of R = 2^(WBIAS - W): w(aref - v) + lam; ~0 where R is 0
 __device__ __forceinline__ uint64_t r_exponent(const OzPoint &o, int64_t v, const oz::Mul &k)
 {
     if (o.aref == ZERO_COLUMN)
@@ -441,24 +436,25 @@ __device__ __forceinline__ int grid_of_w(float w)
 // The least exponents W of R_kn of DG_K centres over the points na .. nb (each
 // warp's own share), in FP32: enough for the grid of a centre's responsibilities
 // (grid_of_w takes a margin), and one conversion and one FMA a pair.
-__device__ __forceinline__ void least_exponents(const int64_t *const (&row)[DG_K], const int64_t (&hk)[DG_K],
-                                                int na, int nb, int u, const oz::MulBase &kb,
+__device__ __forceinline__ void least_exponents(const int64_t *const (&row)[DG_K], int na, int nb,
+                                                const oz::MulBase &kb, const OzUnit *__restrict__ units,
                                                 const OzPoint *__restrict__ pt, const int64_t *__restrict__ thr,
                                                 float (&w)[DG_K])
 {
-    // exponents from x >> xs, xs such that one of its units is at most 2^-8
-    const int xs = min(max(-8 - kb.ex - u, 0), 40);
-    const float kf = scalbnf((float) (kb.m >> 40), kb.ex - 24 + u + xs);
+    const float kf0 = (float) (kb.m >> 40) * 0x1p-24f;
 #pragma unroll
     for (int i = 0; i < DG_K; i++)
         w[i] = 4096.f;
     for (int n = na + threadIdx.x; n < nb; n += 256) {
         const OzPoint o = pt[n];
         const int64_t t = thr[n];
+        // exponents from x >> xs, xs such that one of its units is at most 2^-8
+        const int q = kb.ex + units[n].u, xs = min(max(-8 - q, 0), 40);
+        const float kf = kf0 * __int_as_float((min(q + xs, 64) + 127) << 23);
         const float lf = (float) (uint32_t) (o.lam >> 32) * 0x1p-21f;  // 53 - 32 bits of fraction
 #pragma unroll
         for (int i = 0; i < DG_K; i++) {
-            const int64_t v = row[i][n] - hk[i];
+            const int64_t v = row[i][n];
             const int64_t x = (o.aref - v) >> xs;
             const int xi = x > 0x7FFFFFFF ? 0x7FFFFFFF : (int) x;  // x >= -(a few): d_ref is the least
             const float f = o.aref == ZERO_COLUMN ? lf : fmaf((float) xi, kf, lf);
@@ -477,23 +473,18 @@ __device__ __forceinline__ void least_exponents(const int64_t *const (&row)[DG_K
 // wmin[k] = that of the whole chunk as FP32 bits (4096 where all R are 0).  Block:
 // DG_K centres (a point's constants are read once for all of them), a range of points.
 __global__ void __launch_bounds__(256) oz_rmax_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn, int K,
-                                                      const int64_t *__restrict__ h,
-                                                      const OzScale *__restrict__ sc,
+                                                      const OzUnit *__restrict__ units,
                                                       const OzPoint *__restrict__ pt,
                                                       const int64_t *__restrict__ thr, oz::MulBase kb, int range,
                                                       unsigned *__restrict__ wmin)
 {
     const int k0 = blockIdx.x * DG_K, na = blockIdx.y * range, nb = min(nn, na + range);
-    int64_t hk[DG_K];
     const int64_t *row[DG_K];
     float w[DG_K];
 #pragma unroll
-    for (int i = 0; i < DG_K; i++) {
-        const int k = min(k0 + i, K - 1);
-        hk[i] = h[k];
-        row[i] = acc + (size_t) k * ldm;
-    }
-    least_exponents(row, hk, na, nb, sc->u, kb, pt, thr, w);
+    for (int i = 0; i < DG_K; i++)
+        row[i] = acc + (size_t) min(k0 + i, K - 1) * ldm;
+    least_exponents(row, na, nb, kb, units, pt, thr, w);
 #pragma unroll
     for (int i = 0; i < DG_K; i++)
         if ((threadIdx.x & 31) == 0 && k0 + i < K)
@@ -509,8 +500,7 @@ __global__ void __launch_bounds__(256) oz_rmax_kernel(const int64_t *__restrict_
 // instructions a pair, half of them the exponential.
 template <bool SQ, bool FIND>
 __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn, int K,
-                                                        const int64_t *__restrict__ h,
-                                                        const OzScale *__restrict__ sc,
+                                                        const OzUnit *__restrict__ units,
                                                         const uint64_t *__restrict__ gtab,
                                                         const OzPoint *__restrict__ pt,
                                                         const int64_t *__restrict__ thr, oz::MulBase kb, int range,
@@ -520,21 +510,16 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
 {
     extern __shared__ uint64_t tab[];
     const int k0 = blockIdx.x * DG_K, ja = blockIdx.y * (range / 2), jb = min(ldn / 2, ja + range / 2);
-    const oz::Mul km = oz::mul_at(kb, sc->u);
-    int64_t hk[DG_K];
     const int64_t *row[DG_K];
     int nmin[DG_K];
     load_table(tab, gtab);
 #pragma unroll
-    for (int i = 0; i < DG_K; i++) {
-        const int k = min(k0 + i, K - 1);
-        hk[i] = h[k];
-        row[i] = acc + (size_t) k * ldm;
-    }
+    for (int i = 0; i < DG_K; i++)
+        row[i] = acc + (size_t) min(k0 + i, K - 1) * ldm;
     if constexpr (FIND) {
         __shared__ float red[8][DG_K];
         float w[DG_K];
-        least_exponents(row, hk, 0, nn, sc->u, kb, pt, thr, w);
+        least_exponents(row, 0, nn, kb, units, pt, thr, w);
         if ((threadIdx.x & 31) == 0) {
 #pragma unroll
             for (int i = 0; i < DG_K; i++)
@@ -559,10 +544,12 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
     for (int j = ja + threadIdx.x; j < jb; j += 256) {
         OzPoint o[2];
         int64_t t[2];
+        oz::Mul km[2];
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int n = min(2 * j + e, nn - 1);
             o[e] = pt[n];
+            km[e] = oz::mul_at(kb, units[n].u);
             t[e] = 2 * j + e < nn ? thr[n] : INT64_MAX;  // padding: R = 0
         }
 #pragma unroll
@@ -572,8 +559,8 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
             int64_t q[2];
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                const int64_t v = row[i][min(2 * j + e, nn - 1)] - hk[i];
-                uint64_t W = v < t[e] ? ~0ull : r_exponent(o[e], v, km);
+                const int64_t v = row[i][min(2 * j + e, nn - 1)];
+                uint64_t W = v < t[e] ? ~0ull : r_exponent(o[e], v, km[e]);
                 if (SQ)
                     W = r_square(W);
                 const int ex = (int) (W >> oz::WFRAC);
@@ -618,8 +605,7 @@ __global__ void __launch_bounds__(256) oz_rt_kernel(const int64_t *__restrict__ 
 // M = R^T X of a chunk, blocks as in oz_stats_kernel.
 template <int NT, int LMAX>
 __global__ void __launch_bounds__(NT) oz_map_kernel(const int64_t *__restrict__ acc, size_t ldm, int nn,
-                                                            const int64_t *__restrict__ h,
-                                                            const OzScale *__restrict__ sc,
+                                                            const OzUnit *__restrict__ units,
                                                             const uint64_t *__restrict__ gtab,
                                                             const OzPoint *__restrict__ pt, oz::MulBase kb,
                                                             int K, const double *__restrict__ X, int L,
@@ -634,7 +620,7 @@ __global__ void __launch_bounds__(NT) oz_map_kernel(const int64_t *__restrict__ 
     const bool live = p < nn;
     const int64_t *a = acc + (live ? p : 0);
     const OzPoint o = pt[live ? p : 0];
-    const oz::Mul km = oz::mul_at(kb, sc->u);
+    const oz::Mul km = oz::mul_at(kb, units[live ? p : 0].u);
     load_table(tab, gtab);
     __syncthreads();
     double m[LMAX] = {};
@@ -643,12 +629,13 @@ __global__ void __launch_bounds__(NT) oz_map_kernel(const int64_t *__restrict__ 
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int k = min(k0 + j * ST_KG, K - 1);
-            v[j] = a[(size_t) k * ldm] - h[k];
+            v[j] = a[(size_t) k * ldm];
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int k = k0 + j * ST_KG;
-            const uint64_t W = k < K ? r_exponent(o, v[j], km) : ~0ull;
+            // (no R is cut here but FAR, which stands for any distance beyond the unit's range)
+            const uint64_t W = k < K && (v[j] > oz::FAR || o.aref == ZERO_COLUMN) ? r_exponent(o, v[j], km) : ~0ull;
             const int n = (int) (W >> oz::WFRAC) - oz::WBIAS;
             if (n > 1080)  // R is 0 in FP64
                 continue;
@@ -681,8 +668,7 @@ __global__ void __launch_bounds__(NT) oz_map_kernel(const int64_t *__restrict__ 
 
 // R of a block of centres and points from its distances (acc: nk rows of ldm)
 __global__ void __launch_bounds__(256) oz_rblock_kernel(const int64_t *__restrict__ acc, size_t ldm, int nk, int nn,
-                                                        const int64_t *__restrict__ h,
-                                                        const OzScale *__restrict__ sc,
+                                                        const OzUnit *__restrict__ units,
                                                         const uint64_t *__restrict__ gtab,
                                                         const OzPoint *__restrict__ pt,
                                                         const int64_t *__restrict__ thr, oz::MulBase kb, size_t ldR,
@@ -691,12 +677,11 @@ __global__ void __launch_bounds__(256) oz_rblock_kernel(const int64_t *__restric
     extern __shared__ uint64_t tab[];
     load_table(tab, gtab);
     __syncthreads();
-    const oz::Mul km = oz::mul_at(kb, sc->u);
     const size_t total = (size_t) nk * nn;
     for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < total; i += (size_t) gridDim.x * 256) {
         const int k = (int) (i / nn), n = (int) (i - (size_t) k * nn);
-        const int64_t v = acc[(size_t) k * ldm + n] - h[k];
-        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, km);
+        const int64_t v = acc[(size_t) k * ldm + n];
+        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, oz::mul_at(kb, units[n].u));
         R[(size_t) k * ldR + n] =
             W == ~0ull ? 0.0 : oz::to_double(oz::exp2_neg(W, tab), (int) (W >> oz::WFRAC) - oz::WBIAS);
     }
@@ -717,15 +702,19 @@ struct OzE {
     int sa = 8, panels = 0, Dp = 0, Np = 0, Kp = 0, chunk = 0, nchunks = 0;
     const __nv_bfloat16 *Tp = nullptr;  // data planes (own or the caller's)
     __nv_bfloat16 *Town = nullptr, *Yp = nullptr;
-    unsigned long long *bits = nullptr;  // 0, 1: T; 2, 3: Y; 4 ..: columns of T, then ones
-    OzScale *sc = nullptr;
+    unsigned long long *bits = nullptr;  // maxima of the columns of T, then ones
+    OzScale *sc = nullptr;   // [2], sc_now the one of the centres in Yp
+    int sc_now = 0;
+    int *ex = nullptr;       // the points' exponents
+    OzUnit *units = nullptr; // and units for the centres in Yp
+    oz::Centre *cen = nullptr;
     uint64_t *tab = nullptr;
-    int64_t *h = nullptr, *acc = nullptr;
+    int64_t *acc = nullptr;
     size_t ldm = 0;
     OzPoint *pt = nullptr;
     int64_t *thr = nullptr;  // acc below it: the reference's R is 0
     int acc_whole = 0;  // acc holds all points of the centres in Yp
-    int own_stats = 0;  // Yp, h and pt are those of the last oze_estep
+    int own_stats = 0;  // Yp, cen, units and pt are those of the last oze_estep
     // responsibility pass
     int Wp = 0, Kp128 = 0, Npk = 0, rt_tiles = 0, rt_per = 0;
     __nv_bfloat16 *Tt = nullptr, *Rp = nullptr;
@@ -808,10 +797,12 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         if (!a.Tb)
             lay(&st->Town, planes * st->Np * st->Dp, base);
         lay(&st->Yp, planes * st->Kp * st->Dp, base);
-        lay(&st->bits, sizeof(unsigned long long) * (4 + D + 1), base);
-        lay(&st->sc, sizeof(OzScale), base);
+        lay(&st->bits, sizeof(unsigned long long) * (D + 1), base);
+        lay(&st->sc, 2 * sizeof(OzScale), base);
+        lay(&st->ex, sizeof(int) * N, base);
+        lay(&st->units, sizeof(OzUnit) * N, base);
+        lay(&st->cen, sizeof(oz::Centre) * K, base);
         lay(&st->tab, TAB_BYTES, base);
-        lay(&st->h, sizeof(int64_t) * K, base);
         lay(&st->acc, sizeof(int64_t) * st->ldm * K, base);
         lay(&st->pt, sizeof(OzPoint) * N, base);
         lay(&st->thr, sizeof(int64_t) * N, base);
@@ -831,31 +822,36 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(st->tab, host_table(), TAB_BYTES, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = cudaMemsetAsync(st->bits, 0, sizeof(unsigned long long) * (4 + D + 1), s);
+        e = cudaMemsetAsync(st->bits, 0, sizeof(unsigned long long) * (D + 1), s);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(st->done, 0, sizeof(unsigned), s);
+    const OzScale start[2] = {{YMIN_START, 0}, {YMIN_START, 0}};
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(st->sc, start, sizeof(start), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        oz_absmax_kernel<<<grid_of((size_t) N * D, 1216), 256, 0, s>>>(a.T64, (size_t) N * D, a.tt, N, st->bits);
-        if (!a.Tb)
-            oz_slice_rows_kernel<<<grid_of((size_t) st->Np * st->Dp / 2, 16384), 256, 0, s>>>(
-                a.T64, N, D, st->Np, st->narrow ? st->narrow : st->Dp, st->bits, st->Town,
-                st->narrow ? (int64_t *) st->Town : nullptr, nullptr, 8, nullptr, nullptr, nullptr);
+        // of 0/1 data, which are in Tb, only the exponents are wanted: rows of no columns
+        oz_slice_rows_kernel<<<grid_of((size_t) st->Np * 32, 16384), 256, 0, s>>>(
+            a.T64, N, D, a.Tb ? N : st->Np, a.Tb ? 0 : st->narrow ? st->narrow : st->Dp, st->Town,
+            st->narrow ? (int64_t *) st->Town : nullptr, st->ex, nullptr, nullptr, nullptr);
         e = cudaGetLastError();
         st->Tp = a.Tb ? a.Tb : st->Town;
     }
+    const OzSource src{nullptr, a.T64, nullptr, D, D, 0};
+    if (e == cudaSuccess) {
+        oz_colmax_kernel<<<dim3(ceil_div(N, 512), ceil_div(D + 1, 32)), 256, 0, s>>>(src, N, D + 1, 512, st->bits);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess && a.mstep) {
-        const OzSource src{nullptr, a.T64, nullptr, D, D, 0};
         e = cudaMemsetAsync(st->Tt, 0, planes * st->Wp * st->Npk, s);
-        oz_colmax_kernel<<<dim3(ceil_div(N, 512), ceil_div(D + 1, 32)), 256, 0, s>>>(src, N, D + 1, 512,
-                                                                                    st->bits + 4);
         oz_slice_t_kernel<<<dim3(st->Npk / PANEL, ceil_div(D + 1, 32)), 256, 0, s>>>(
-            src, N, D + 1, st->Wp, st->Npk, st->bits + 4, st->Tt);
+            src, N, D + 1, st->Wp, st->Npk, st->bits, st->Tt);
         if (e == cudaSuccess)
             e = cudaGetLastError();
     }
-    unsigned long long tb[2] = {0, 0};
+    // a column's largest value (the squares of all are finite below 2^500)
+    std::vector<unsigned long long> top(D + 1);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(tb, st->bits, sizeof(tb), cudaMemcpyDeviceToHost, s);
+        e = cudaMemcpyAsync(top.data(), st->bits, sizeof(unsigned long long) * (D + 1), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
@@ -865,10 +861,12 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         oze_destroy(st);
         return code;
     }
-    if (tb[0] >= oz::INF_BITS || tb[1] >= oz::INF_BITS) {
-        oze_destroy(st);  // non-finite data: the CUDA-core kernels carry them
-        return DGTM_OK;
-    }
+    // data, or squares of it, that are not finite: the CUDA-core kernels carry them
+    for (int d = 0; d < D; d++)
+        if (top[d] >= oz::double_bits(0x1p500)) {
+            oze_destroy(st);
+            return DGTM_OK;
+        }
     *out = st;
     return DGTM_OK;
 }
@@ -881,16 +879,18 @@ int oze_estep_blocks(const OzE *st)
 
 namespace {
 
-// the centres' planes, grid and h (what follows zeroes bits[2..3] for the next call)
-int slice_centres(OzE *st, const double *Y, const double *yy, cudaStream_t s)
+// the centres' planes, and the points' units for exponents c1 d and c2 d
+int slice_centres(OzE *st, const double *Y, const double *yy, double c1, double c2, cudaStream_t s)
 {
-    const int K = st->a.K, D = st->a.D;
-    // bits[2..3] are 0: set so at the start and by the kernel that reads them last
-    oz_absmax_kernel<<<grid_of((size_t) K * D, 608), 256, 0, s>>>(Y, (size_t) K * D, yy, K, st->bits + 2);
+    const int N = st->a.N, K = st->a.K, D = st->a.D;
+    st->sc_now ^= 1;
+    oz_slice_rows_kernel<<<grid_of((size_t) st->Kp * 32, 4864), 256, 0, s>>>(
+        Y, K, D, st->Kp, st->narrow ? st->narrow : st->Dp, st->Yp, st->narrow ? (int64_t *) st->Yp : nullptr,
+        nullptr, yy, st->cen, st->sc + st->sc_now);
     DGTM_CUDA_TRY(cudaGetLastError());
-    oz_slice_rows_kernel<<<grid_of((size_t) st->Kp * st->Dp / 2, 4864), 256, 0, s>>>(
-        Y, K, D, st->Kp, st->narrow ? st->narrow : st->Dp, st->bits + 2, st->Yp,
-        st->narrow ? (int64_t *) st->Yp : nullptr, st->bits, st->sa, yy, st->sc, st->h);
+    oz_units_kernel<<<grid_of((size_t) N, 1216), 256, 0, s>>>(
+        st->ex, st->a.tt, N, st->sc + st->sc_now, st->sc + (st->sc_now ^ 1), st->narrow ? 58 : st->sa == 1 ? 55 : 53,
+        st->sa == 1, oz::unit_cap(c1, c2), st->units);
     DGTM_CUDA_TRY(cudaGetLastError());
     st->acc_whole = st->own_stats = 0;
     return DGTM_OK;
@@ -903,7 +903,7 @@ int narrow_products(OzE *st, int m0, int nn, int k0, int nk, size_t ldm, int64_t
     const auto kernel = dp == 2 ? oz_narrow_kernel<2> : dp == 4 ? oz_narrow_kernel<4> : oz_narrow_kernel<8>;
     const dim3 grid(ceil_div(nn, 256), ceil_div(nk, 64));
     kernel<<<grid, 256, 0, s>>>((const int64_t *) st->Tp + (size_t) m0 * dp, (const int64_t *) st->Yp + (size_t) k0 * dp,
-                                nn, nk, st->sc, ldm, out);
+                                nn, nk, st->units + m0, st->cen + k0, ldm, out);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
@@ -930,7 +930,8 @@ int chunk_products(OzE *st, int c, cudaStream_t s)
     g.ldm = st->ldm;
     g.mrows = nn;
     g.ncols = st->a.K;
-    g.shift = &st->sc->shift;
+    g.units = st->units + n0;
+    g.cen = st->cen;
     return launch_oz_gemm(g, st->a.sms, st->a.status, s);
 }
 
@@ -959,7 +960,7 @@ constexpr double LOG2E_2 = 2.0 * 1.4426950408889634;
 int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, int isDA, double2 *colstat,
               double *part, double dcut, double *sums, int *nlaunch, cudaStream_t s)
 {
-    OZ_TRY(slice_centres(st, Y, yy, s));
+    OZ_TRY(slice_centres(st, Y, yy, c1, isDA ? c2 : c1, s));
     const bool two = isDA && c1 != c2;
     const int nt = wide_blocks(st->a.K) ? 1024 : 512;
     const auto kernel = nt == 512 ? (two ? oz_stats_kernel<512, true> : oz_stats_kernel<512, false>)
@@ -971,8 +972,8 @@ int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, 
         OzStatsArgs a{};
         a.acc = st->acc;
         a.ldm = st->ldm;
-        a.h = st->h;
-        a.sc = st->sc;
+        a.sc = st->sc + st->sc_now;
+        a.units = st->units + n0;
         a.tab = st->tab;
         a.tt = st->a.tt + n0;
         a.nn = nn;
@@ -986,7 +987,6 @@ int oze_estep(OzE *st, const double *Y, const double *yy, double c1, double c2, 
         a.pt = st->pt + n0;
         a.thr = st->thr + n0;
         a.dcut = dcut;
-        a.ybits = st->bits + 2;
         a.part = part;
         a.block_part = part + 2 * (size_t) (n0 / ST_PTS);
         a.sums = sums;
@@ -1028,7 +1028,7 @@ int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaS
         g.item_panels = st->rt_per;
         OZ_TRY(launch_oz_gemm(g, st->a.sms, st->a.status, s));
         oz_rt_kernel<<<dim3(st->rt_tiles, 32), 256, 0, s>>>(st->part, g.ntiles, ceil_div(g.panels, st->rt_per),
-                                                            oz_sum_ext(g.panels), st->nmin, st->bits + 4, K, D,
+                                                            oz_sum_ext(g.panels), st->nmin, st->bits, K, D,
                                                             ch == 0 ? 1 : 0, G, RT);
         DGTM_CUDA_TRY(cudaGetLastError());
         nl += 4;
@@ -1039,13 +1039,15 @@ int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaS
 }
 
 // the centres' planes and the points' references for a context's column statistics
-int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat, double dcut, cudaStream_t s)
+int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c1, double c, double dcut,
+              cudaStream_t s)
 {
     if (st->own_stats)
         return DGTM_OK;
-    OZ_TRY(slice_centres(st, Y, yy, s));
+    OZ_TRY(slice_centres(st, Y, yy, c1, c, s));
     oz_points_kernel<<<grid_of((size_t) st->a.N, 1216), 256, 0, s>>>(colstat, st->a.tt, st->a.N, st->a.K,
-                                                                    st->sc, dcut, st->pt, st->thr, st->bits + 2);
+                                                                    st->sc + st->sc_now, st->units, dcut, st->pt,
+                                                                    st->thr);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
@@ -1075,26 +1077,26 @@ int oze_r_digits(OzE *st, int ch, int k0, int kb, double c, bool squares, bool p
     OZ_TRY(table_smem(kernel));
     if (!squares && parts > 1) {
         DGTM_CUDA_TRY(cudaMemsetAsync(st->wmin, 0x7F, sizeof(unsigned) * kb, s));
-        oz_rmax_kernel<<<dim3(kblocks, parts), 256, 0, s>>>(acc, st->ldm, nn, kb, st->h + k0, st->sc, st->pt + n0,
+        oz_rmax_kernel<<<dim3(kblocks, parts), 256, 0, s>>>(acc, st->ldm, nn, kb, st->units + n0, st->pt + n0,
                                                             st->thr + n0, base, range, st->wmin);
         DGTM_CUDA_TRY(cudaGetLastError());
     }
-    kernel<<<dim3(kblocks, parts), 256, TAB_BYTES, s>>>(acc, st->ldm, nn, kb, st->h + k0, st->sc, st->tab,
+    kernel<<<dim3(kblocks, parts), 256, TAB_BYTES, s>>>(acc, st->ldm, nn, kb, st->units + n0, st->tab,
                                                         st->pt + n0, st->thr + n0, base, range, st->wmin, prows,
                                                         ldn, planes, nmin);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
 
-int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c, double dcut,
+int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c1, double c, double dcut,
                 int k0, int nk, int n0, int nn, double *R, cudaStream_t s)
 {
-    OZ_TRY(oze_refer(st, Y, yy, colstat, dcut, s));
+    OZ_TRY(oze_refer(st, Y, yy, colstat, c1, c, dcut, s));
     OZ_TRY(table_smem(oz_rblock_kernel));
     const oz::MulBase base = oz::make_mul(c * LOG2E_2);
     auto launch = [&](const int64_t *acc, size_t ldm, int n, int np) -> int {
         oz_rblock_kernel<<<grid_of((size_t) nk * np, 1216), 256, TAB_BYTES, s>>>(
-            acc, ldm, nk, np, st->h + k0, st->sc, st->tab, st->pt + n, st->thr + n, base, (size_t) nn, R + (n - n0));
+            acc, ldm, nk, np, st->units + n, st->tab, st->pt + n, st->thr + n, base, (size_t) nn, R + (n - n0));
         DGTM_CUDA_TRY(cudaGetLastError());
         return DGTM_OK;
     };
@@ -1112,12 +1114,13 @@ int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colst
     g.ntiles = ceil_div(nk, 64);
     g.out = st->acc;
     g.ncols = nk;
-    g.shift = &st->sc->shift;
+    g.cen = st->cen + k0;
     const int first = n0 / 128 * 128;
     const long long room = (long long) st->ldm * st->a.K / nk / 128 * 128;
     for (long long m0 = first; m0 < n0 + nn; m0 += room) {
         const int m1 = (int) (m0 + room < n0 + nn ? m0 + room : n0 + nn);
         g.a_tile0 = (int) (m0 / 128);
+        g.units = st->units + m0;
         g.mtiles = ceil_div(m1 - m0, 128);
         g.mrows = (int) (m1 - m0);
         g.ldm = (size_t) g.mrows;
@@ -1131,11 +1134,11 @@ int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colst
     return DGTM_OK;
 }
 
-int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c, const double *X,
+int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c1, double c, const double *X,
             int L, double *M, cudaStream_t s)
 {
     const int N = st->a.N, K = st->a.K;
-    OZ_TRY(oze_refer(st, Y, yy, colstat, 1e300, s));
+    OZ_TRY(oze_refer(st, Y, yy, colstat, c1, c, 1e300, s));
     const int nt = wide_blocks(K) ? 1024 : 512;
     const auto kernel = nt == 512 ? (L <= 2 ? oz_map_kernel<512, 2> : L == 3 ? oz_map_kernel<512, 3> : oz_map_kernel<512, 8>)
                                   : (L <= 2 ? oz_map_kernel<1024, 2> : L == 3 ? oz_map_kernel<1024, 3> : oz_map_kernel<1024, 8>);
@@ -1144,7 +1147,7 @@ int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, 
         if (!st->acc_whole)
             OZ_TRY(chunk_products(st, ch, s));
         const int n0 = ch * st->chunk, nn = N - n0 < st->chunk ? N - n0 : st->chunk;
-        kernel<<<ceil_div(nn, ST_PTS), nt, TAB_BYTES, s>>>(st->acc, st->ldm, nn, st->h, st->sc, st->tab,
+        kernel<<<ceil_div(nn, ST_PTS), nt, TAB_BYTES, s>>>(st->acc, st->ldm, nn, st->units + n0, st->tab,
                                                                    st->pt + n0, oz::make_mul(c * LOG2E_2), K,
                                                                    X, L, M + (size_t) n0 * L);
         DGTM_CUDA_TRY(cudaGetLastError());

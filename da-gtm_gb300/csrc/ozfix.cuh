@@ -220,6 +220,72 @@ OZ_HD double to_double(uint64_t E, int n)
     return bits_double(((uint64_t) (e + 1023) << 52) + m);
 }
 
+// Units of the distances.  v = t.y - |y|^2 / 2 = (|t|^2 - d) / 2 of a point and a centre
+// is a 64-bit integer in units 2^u of the point's own, because only one point's distances
+// are compared with each other; a value elsewhere in the data or on a far centre changes
+// nothing for it.  With |t|^2 < 2^x, and 2^ymin next above the least |y|^2 of the centres,
+//     u = max(max(x, ymin) - 59, ucap):
+// |t|^2 and the smallest centre's |y|^2 are at most 2^59 units, so v of the best
+// centre is above -2^60.  A centre with |y|^2 / 2 >= 2^62 has |y| >= 2^31.5 against
+// |t| <= 2^29.5, so v <= -|y|^2 / 4 <= -2^61: it gets FAR instead.  Any other has
+// |t.y| <= 2^61: nothing overflows.  ucap (unit_cap) bounds the unit from below by what
+// the exponentials can tell apart, so that FAR is beyond every distance with an R.
+constexpr int64_t FAR = -(1ll << 61);
+
+OZ_HD int point_unit(int x, int ymin, int ucap)
+{
+    const int u = (x > ymin ? x : ymin) - 59;
+    return u > ucap ? u : ucap;
+}
+
+// ucap for exponents c1 d and c2 d: 2^60 units are past the reference's cut c1 d = 746 and
+// past c2 (d - d_min) = 64, whose R adds nothing to a sum in FP64.  c1 u is then at most
+// 2^-50.3, or c2 u at most 2^-54.
+static inline int unit_cap(double c1, double c2)
+{
+    int ex = 0;
+    frexp(c1 / 400.0 < c2 / 32.0 ? 400.0 / c1 : 32.0 / c2, &ex);  // < 2^ex
+    return ex - 60;
+}
+
+// x 2^s, towards minus infinity, for a result within 63 bits
+OZ_HD int64_t shifted(int64_t x, int s)
+{
+    const int l = s > 0 ? (s < 63 ? s : 63) : 0, r = s < 0 ? (s > -63 ? -s : 63) : 0;
+    return (int64_t) ((uint64_t) x << l) >> r;
+}
+
+// a centre of a product: |y|^2 = yy 2^yx, yy in [2^52, 2^53) or 0; |y_d| < 2^f
+struct alignas(16) Centre {
+    int64_t yy;
+    int f, yx;
+};
+
+OZ_HD Centre make_centre(uint64_t ymax_bits, double yy)
+{
+    const uint64_t b = double_bits(yy) & ABS_MASK;
+    uint64_t m = b & 0xFFFFFFFFFFFFFull;
+    int E = (int) (b >> 52);
+    Centre c;
+    c.f = exponent_of(ymax_bits);
+    if (E) {
+        m |= 1ull << 52;  // an infinity (the square of a finite y) becomes 2^1024
+    } else if (m) {
+        for (E = 1; !(m >> 52); E--)
+            m <<= 1;
+    }
+    c.yy = (int64_t) m;
+    c.yx = m ? E - 1075 : -8192;
+    return c;
+}
+
+// v from the product I, in units of 2^(p + f) (2^p the point's: its |t_d| < 2^e, and the digits')
+OZ_HD int64_t level(int64_t I, const Centre &c, int p, int u)
+{
+    const int s = c.yx - 1 - u;
+    return s >= 10 ? FAR : shifted(I, p + c.f - u) - shifted(c.yy, s);
+}
+
 // an unsigned fixed-point value in units of 2^-53 from a double (v >= 0)
 OZ_HD uint64_t to_wfix(double v) { return (uint64_t) scaled_int(v, WFRAC); }
 

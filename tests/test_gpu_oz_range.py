@@ -89,3 +89,48 @@ def test_critical_temperature_of_a_far_centre(pkg, orc, monkeypatch, pairs, c):
     lam[lam >= (temp - eps) * 2.0 / beta] = 0.0
     # 2^-53 of the largest eigenvalue, which is 1600 times this one
     assert got_k[9] == pytest.approx(beta / 2.0 * lam.max(), rel=1e-10)
+
+
+def outlier_case(value, D, own, seed=5, N=1000, K=400):
+    """Unit-sized data with one coordinate of one point replaced; own: centre 7 sits on
+    that point."""
+    rng = np.random.default_rng(seed)
+    means = rng.random((16, D))
+    T = means[rng.integers(0, 16, N)] + 0.2 * rng.normal(size=(N, D))
+    Y = T[rng.integers(0, N, K)] + 0.1 * rng.normal(size=(K, D))
+    T[5, D // 2] = value
+    if own:
+        Y[7] = T[5]
+    return T, Y, rng.normal(size=(K, 2))
+
+
+OUTLIERS = [(v, D, own) for v in (1e3, 1e6, 1e30) for D in (2, 5, 12, 70) for own in (False, True)]
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32"])
+@pytest.mark.parametrize("value,D,own", OUTLIERS)
+def test_one_large_value_leaves_the_other_points_alone(pkg, orc, value, D, own, form):
+    """R and the map of every other point, at the bounds that hold without the value:
+    1e-13 on R, 1e-12 on the map (FP64 form; the FP32 form's statistics are FP32, and
+    one large centre or point does not make them worse)."""
+    N, K = (1000, 400) if form == "fp64" else (8000, 300)  # the FP32 form's map by slices
+    T, Y, X = outlier_case(value, D, own, N=N, K=K)
+    beta, temp = 60.0 * 12 / max(D, 12), 1.5
+    with np.errstate(over="ignore", invalid="ignore"):
+        R, _, _ = orc.resp(orc.dist(Y, T), beta, 1, temp)
+    others = np.arange(N) != 5
+    with pkg.Context(T, np.ones((K, 1)), form) as c:
+        c.set_Y(Y)
+        c.estep(beta, 1, temp)
+        M = c.map(X)
+        Rb = c.R_block(0, K, 0, N)
+    if form == "fp64":
+        assert np.max(np.abs(Rb - R)[:, others]) <= 1e-13
+        assert np.max(np.abs((M - R.T @ X)[others])) <= 1e-12 * np.max(np.abs(X))
+    else:
+        assert np.max(np.abs(Rb - R)[:, others]) <= 1e-3
+        assert np.max(np.abs((M - R.T @ X)[others])) <= 1e-3 * np.max(np.abs(X))
+    # the point itself: its own centre's, or (every exp(-beta d / 2) is 0) any centre's.
+    # (Its FP32 distance of 1e6 - 1e6 says nothing; |t|^2 = 1e60 is too much for FP64 too.)
+    if (form == "fp64" and value < 1e30) or not own:
+        assert np.max(np.abs(Rb[:, 5] - (np.eye(K)[7] if own else 1.0 / K))) <= 1e-13

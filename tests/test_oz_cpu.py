@@ -32,3 +32,16 @@ def test_exponents_over_the_whole_range(tmp_path):
                                             check=True).stdout.split()
     assert int(dropped) == 0 and int(beyond) == 0
     assert float(worst) <= 2.0
+
+
+def test_units_of_the_distances(tmp_path):
+    """v = t.y - |y|^2 / 2 on each point's own unit, for sizes over 400 powers of two
+    (tests/oz_unit_check.cc): within what an FP64 sum may lose, nothing within the
+    reference's cut taken for far away, and no overflow."""
+    exe = str(tmp_path / "oz_unit_check")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-o", exe,
+                           os.path.join(ROOT, "tests", "oz_unit_check.cc"), "-lm"])
+    worst, far, over = subprocess.run([exe], capture_output=True, text=True, timeout=300,
+                                      check=True).stdout.split()
+    assert float(worst) <= 1.0
+    assert int(far) == 0 and int(over) == 0
