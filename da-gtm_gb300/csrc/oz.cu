@@ -56,7 +56,8 @@ constexpr int B_PLANE = TN * 128;          // 8 KB
 constexpr int B_BUF = SB * B_PLANE;        // 64 KB
 constexpr int A_SLOTS = 5;
 constexpr int SEG = 8;                     // panels per exact segment (512 elements)
-constexpr size_t OZ_SMEM = 1024 + 2 * (size_t) B_BUF + A_SLOTS * (size_t) A_SLOT + 256;
+constexpr int COLS = TN / (DRAIN_WARPS / 4);  // columns of a drain warp
+constexpr size_t OZ_SMEM = 1024 + 2 * (size_t) B_BUF + A_SLOTS * (size_t) A_SLOT + 256 + DRAIN_WARPS * COLS * 16;
 
 struct OzParams {
     int panels, b_panel0, a_rows, b_rows, a_tile0, b_row0, mtiles, ntiles, nitems, splits, item_panels;
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
     uint64_t *b_full = bars + 2 * A_SLOTS, *b_empty = b_full + 2;
     uint64_t *acc_full = b_full + 4, *acc_empty = acc_full + 1, *drain = acc_full + 2;
     uint32_t *tmem_sh = (uint32_t *) (drain + 1);
+    int4 *cols_sh = (int4 *) ((unsigned char *) bars + 256);  // COLS centres of each drain warp
     __shared__ int failed;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -263,9 +265,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
                 for (int c = 0; c < 16; c++)
                     acc[c] = 0;
             }
+            // Distances: this warp's centres by way of shared memory, |y|^2 / 2 on one
+            // exponent (half_square).  Where that serves all 32 points (near_group: hardly
+            // ever not) an element costs two shifts by constants of its row and one by its
+            // centre's, else oz::level.  With the centres from global memory and level()
+            // for all, a chunk of 1e7 products took 59 us instead of 42.
             OzUnit un{0, 0};
-            if constexpr (!SUM)
+            bool near = true;
+            int rh = 0;
+            int4 *cols = cols_sh + (warp - 2) * COLS;
+            if constexpr (!SUM) {
                 un = p.units[min(mt * TM + row, p.mrows - 1)];
+                const oz::Centre c = p.cen[min(nt * TN + 16 * h + (lane & 15), p.ncols - 1)];
+                int top = c.yx;
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1)
+                    top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+                const int64_t hs = oz::half_square(c, top);
+                __syncwarp();
+                if (lane < COLS)
+                    cols[lane] = make_int4((int) hs, (int) (hs >> 32), c.f, 0);
+                __syncwarp();
+                near = __all_sync(0xffffffffu, oz::near_group(top, un.u));
+                rh = un.u - top + 10;
+            }
             for (int pn = p0; pn < p1; pn += SEG, nseg++) {
                 if (!mbar_wait(acc_full, (uint32_t) (nseg & 1), p.status, 76)) {
                     ok = false;
@@ -273,37 +296,67 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
                 }
                 __syncwarp();
                 tc_fence_after();
-#pragma unroll
-                for (int cb = 0; cb < 4; cb++) {
-                    uint32_t v[4 * SB];
+                // four columns a batch; the accumulators are free once the last one is read
+                auto fetch = [&](int cb, uint32_t *v) {
 #pragma unroll
                     for (int l = 0; l < SB; l++)
                         tmem_ld4p(lane_base + (uint32_t) (l * TN + 4 * cb), v + 4 * l);
-                    oz::Centre cen[SUM ? 1 : 4];
-                    if constexpr (!SUM) {
-#pragma unroll
-                        for (int c = 0; c < 4; c++)
-                            cen[c] = p.cen[min(nt * TN + 16 * h + 4 * cb + c, p.ncols - 1)];
-                    }
                     tmem_ld_wait();
+                    if (cb == 3) {
+                        tc_fence_before();
+                        mbar_arrive(acc_empty);
+                    }
+                };
+                // units 2^-61 (sa = 8): 8 bits down; sa = 1: exact in 2^-55
+                auto product = [&](const uint32_t *v) {
+                    int64_t hi, lo;
+                    level_pairs<NARROW>(v, hi, lo);
+                    return SA == 1 ? hi * 268435456 + lo : hi * 1048576 + ((lo + 128) >> 8);
+                };
+                const int m = mt * TM + row, n0 = nt * TN + 16 * h;
+                int64_t *out = SUM ? nullptr : p.out + (size_t) n0 * p.ldm + m;
+                if constexpr (SUM) {
 #pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        int64_t hi, lo;
-                        level_pairs<NARROW>(v + c, hi, lo);
-                        if constexpr (SUM) {
+                    for (int cb = 0; cb < 4; cb++) {
+                        uint32_t v[4 * SB];
+                        fetch(cb, v);
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            int64_t hi, lo;
+                            level_pairs<NARROW>(v + c, hi, lo);
                             // hi 2^28 + lo may need 72 bits: both are shifted down by >= 8
                             acc[4 * cb + c] += hi * (1 << (28 - shift)) + ((lo + half) >> shift);
-                        } else {
-                            // units 2^-61 (sa = 8): 8 bits down; sa = 1: exact in 2^-55
-                            const int64_t I = SA == 1 ? hi * 268435456 + lo : hi * 1048576 + ((lo + 128) >> 8);
-                            const int n = nt * TN + 16 * h + 4 * cb + c, m = mt * TM + row;
-                            if (m < p.mrows && n < p.ncols)
-                                p.out[(size_t) n * p.ldm + m] = oz::level(I, cen[c], un.p, un.u);
+                        }
+                    }
+                } else if (near) {
+#pragma unroll
+                    for (int cb = 0; cb < 4; cb++) {
+                        uint32_t v[4 * SB];
+                        fetch(cb, v);
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            const int j = 4 * cb + c;
+                            const int4 y = cols[j];
+                            const int64_t hs = (int64_t) (uint32_t) y.x | ((int64_t) y.y << 32);
+                            const int64_t x = oz::shifted(product(v + c), un.p + y.z - un.u) - oz::sar(hs, rh);
+                            if (m < p.mrows && n0 + j < p.ncols)
+                                out[(size_t) j * p.ldm] = x;
+                        }
+                    }
+                } else {
+#pragma unroll 1
+                    for (int cb = 0; cb < 4; cb++) {
+                        uint32_t v[4 * SB];
+                        fetch(cb, v);
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            const int j = 4 * cb + c;
+                            const int64_t x = oz::level(product(v + c), p.cen[min(n0 + j, p.ncols - 1)], un.p, un.u);
+                            if (m < p.mrows && n0 + j < p.ncols)
+                                out[(size_t) j * p.ldm] = x;
                         }
                     }
                 }
-                tc_fence_before();
-                mbar_arrive(acc_empty);
             }
             if constexpr (SUM) {
                 if (ok) {

@@ -159,22 +159,41 @@ __global__ void __launch_bounds__(256) oz_narrow_kernel(const int64_t *__restric
                                                         const oz::Centre *__restrict__ cen, size_t ldm,
                                                         int64_t *__restrict__ out)
 {
+    __shared__ longlong2 cols[64];  // |y|^2 / 2 on one exponent (as in oz_gemm_kernel) and f
+    __shared__ int tops[2];
+    const int kb = blockIdx.y * 64;
+    oz::Centre c;
+    if (threadIdx.x < 64) {
+        c = cen[min(kb + (int) threadIdx.x, K - 1)];
+        const int top = __reduce_max_sync(0xffffffffu, c.yx);
+        if ((threadIdx.x & 31) == 0)
+            tops[threadIdx.x >> 5] = top;
+    }
+    __syncthreads();
+    const int top = max(tops[0], tops[1]);
+    if (threadIdx.x < 64)
+        cols[threadIdx.x] = make_longlong2(oz::half_square(c, top), c.f);
+    __syncthreads();
     const int m = blockIdx.x * 256 + threadIdx.x;
     if (m >= nn)
         return;
     const OzUnit un = units[m];
+    const bool near = oz::near_group(top, un.u);
+    const int rh = un.u - top + 10;
     int64_t t[DP];
 #pragma unroll
     for (int d = 0; d < DP; d++)
         t[d] = T[(size_t) m * DP + d];
-    const int k1 = min(K, (int) (blockIdx.y + 1) * 64);
+    const int k1 = min(K, kb + 64);
 #pragma unroll 4
-    for (int k = blockIdx.y * 64; k < k1; k++) {
+    for (int k = kb; k < k1; k++) {
         int64_t sum = 0;
 #pragma unroll
         for (int d = 0; d < DP; d++)
             sum += __mul64hi(t[d], Y[(size_t) k * DP + d]);
-        out[(size_t) k * ldm + m] = oz::level(sum, cen[k], un.p, un.u);
+        const longlong2 y = cols[k - kb];
+        out[(size_t) k * ldm + m] = near ? oz::shifted(sum, un.p + (int) y.y - un.u) - oz::sar(y.x, rh)
+                                         : oz::level(sum, cen[k], un.p, un.u);
     }
 }
 
@@ -549,7 +568,7 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
         for (int e = 0; e < 2; e++) {
             const int n = min(2 * j + e, nn - 1);
             o[e] = pt[n];
-            km[e] = oz::mul_at(kb, units[n].u);
+            km[e] = oz::mul_unit(kb, units[n].u);
             t[e] = 2 * j + e < nn ? thr[n] : INT64_MAX;  // padding: R = 0
         }
 #pragma unroll
@@ -681,7 +700,7 @@ __global__ void __launch_bounds__(256) oz_rblock_kernel(const int64_t *__restric
     for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < total; i += (size_t) gridDim.x * 256) {
         const int k = (int) (i / nn), n = (int) (i - (size_t) k * nn);
         const int64_t v = acc[(size_t) k * ldm + n];
-        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, oz::mul_at(kb, units[n].u));
+        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, oz::mul_unit(kb, units[n].u));
         R[(size_t) k * ldR + n] =
             W == ~0ull ? 0.0 : oz::to_double(oz::exp2_neg(W, tab), (int) (W >> oz::WFRAC) - oz::WBIAS);
     }

@@ -176,6 +176,54 @@ OZ_HD Mul mul_at(const MulBase &k, int u)
     return r;
 }
 
+// x 2^s for s of 0 and more, zeros from 64 on; and x 2^-s towards minus infinity
+OZ_HD uint64_t shl(uint64_t x, int s)
+{
+#if defined(__CUDA_ARCH__)
+    uint64_t r;
+    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+    return r;
+#else
+    return s < 64 ? x << s : 0ull;
+#endif
+}
+
+OZ_HD int64_t sar(int64_t x, int s)
+{
+#if defined(__CUDA_ARCH__)
+    int64_t r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+    return r;
+#else
+    return x >> (s < 63 ? s : 63);
+#endif
+}
+
+OZ_HD uint64_t shr(uint64_t x, int s)
+{
+#if defined(__CUDA_ARCH__)
+    uint64_t r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+    return r;
+#else
+    return s < 64 ? x >> s : 0ull;
+#endif
+}
+
+// The same where a thread has few x of a unit: lim leaves out the last 32nd of what fits,
+// so that w stays below 1984 without a look at l0.
+OZ_HD Mul mul_unit(const MulBase &k, int u)
+{
+    Mul r;
+    const int sh = k.ex + u + WFRAC;
+    r.m = k.m;
+    r.a = sh > 0 ? sh : 0;
+    r.b = sh < 0 ? -sh : 0;
+    const uint64_t cap = shr(~0ull, r.a);
+    r.lim = cap - (cap >> 5);
+    return r;
+}
+
 OZ_HD uint64_t mul_w(const Mul &k, uint64_t x) { return mulhi(x << (k.a & 63), k.m) >> k.b; }
 
 // w of x > lim: ~0 from 2000 on.  What x << a has no room for below that has one bit
@@ -251,8 +299,7 @@ static inline int unit_cap(double c1, double c2)
 // x 2^s, towards minus infinity, for a result within 63 bits
 OZ_HD int64_t shifted(int64_t x, int s)
 {
-    const int l = s > 0 ? (s < 63 ? s : 63) : 0, r = s < 0 ? (s > -63 ? -s : 63) : 0;
-    return (int64_t) ((uint64_t) x << l) >> r;
+    return sar((int64_t) shl((uint64_t) x, s > 0 ? s : 0), s < 0 ? -s : 0);
 }
 
 // a centre of a product: |y|^2 = yy 2^yx, yy in [2^52, 2^53) or 0; |y_d| < 2^f
@@ -278,6 +325,14 @@ OZ_HD Centre make_centre(uint64_t ymax_bits, double yy)
     c.yx = m ? E - 1075 : -8192;
     return c;
 }
+
+// |y|^2 / 2 of a group of centres, the largest yx of which is top, as integers of one
+// exponent: |y|^2 / 2 = half_square 2^(top - 10), below 2^62, towards minus infinity.  For
+// a point with u >= top - 10 none of them is FAR, and |y|^2 / 2 in its units is
+// half_square >> (u - top + 10): the same integer as by level().
+OZ_HD int64_t half_square(const Centre &c, int top) { return shifted(c.yy, c.yx - top + 9); }
+
+OZ_HD bool near_group(int top, int u) { return u >= top - 10; }
 
 // v from the product I, in units of 2^(p + f) (2^p the point's: its |t_d| < 2^e, and the digits')
 OZ_HD int64_t level(int64_t I, const Centre &c, int p, int u)

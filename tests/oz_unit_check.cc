@@ -4,7 +4,7 @@
 //   1. the largest error of v relative to what is allowed,
 //      2^-51 (|t| |y| + |t|^2 + |y|^2), plus the exponents' own 2^-50 / c1 + 2^-54 / c2;
 //   2. how many centres got FAR although exp(-c1 d) > 0 or c2 (d - d_min) < 64;
-//   3. how many others left 63 bits.
+//   3. how many others left 63 bits, or came out otherwise by way of half_square.
 #include "../da-gtm_gb300/csrc/ozfix.cuh"
 #include <random>
 #include <stdio.h>
@@ -16,7 +16,7 @@ int main()
     std::mt19937_64 g(3);
     std::normal_distribution<double> nrm;
     auto uni = [&](double a, double b) { return a + (b - a) * (double) (g() >> 11) * 0x1p-53; };
-    long far = 0, over = 0;
+    long far = 0, over = 0, nearby = 0;
     long double worst = 0;
     const int dims[] = {1, 2, 8, 9, 37, 64, 200, 256};
     for (int it = 0; it < 4000; it++) {
@@ -78,6 +78,14 @@ int main()
             if (fabsl(il) > 0x1p62L)
                 over++;
             const int64_t v = level((int64_t) il, c[k], p, u);
+            int top = c[k].yx;  // of the centre and its neighbours
+            for (int j = 0; j < K; j++)
+                if (j / 3 == k / 3 && c[j].yx > top)
+                    top = c[j].yx;
+            if (near_group(top, u) &&
+                v != shifted((int64_t) il, p + c[k].f - u) - sar(half_square(c[k], top), u - top + 10))
+                over++;
+            nearby += near_group(top, u);
             if (v == FAR) {
                 if (c1 * dist[k] < 745.0L || c2 * (dist[k] - dmin) < 64.0L)
                     far++;
@@ -92,6 +100,8 @@ int main()
             worst = fmaxl(worst, fabsl(ldexpl((long double) v, u) - ref) / allowed);
         }
     }
+    if (nearby < 10000)
+        over++;
     printf("%.3Lf %ld %ld\n", worst, far, over);
     return 0;
 }
