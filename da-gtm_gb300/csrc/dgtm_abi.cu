@@ -436,8 +436,13 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
                 CK(xr);
             if (c->x64)
                 c->nblk1 = x64_pass1_blocks(c->x64);
-            else if (slices_on() && oze_wanted(N, D, K))
-                CK(unless_enomem(oze_create(&c->oze, oze_args(c, true), c->stream)));
+            else if (slices_on() && oze_wanted(N, D, K)) {
+                const int rc = oze_create(&c->oze, oze_args(c, true), c->stream);
+                CK(unless_enomem(rc));
+                // data the slices do not fit: nor for the map, whose R is that of the
+                // CUDA-core E-step
+                c->ozmap_tried = rc == DGTM_OK && !c->oze;
+            }
             if (c->oze)
                 c->nblk1 = oze_estep_blocks(c->oze);
         }

@@ -591,7 +591,7 @@ int ozab_basis(OzAB *st, const double *FI, cudaStream_t s)
     oz_colmax_kernel<<<dim3(ceil_div(K, 128), ceil_div(M1, 32)), 256, 0, s>>>(src, K, M1, 128, st->fbits);
     DGTM_CUDA_TRY(cudaGetLastError());
     oz_slice_t_kernel<<<dim3(st->panels, ceil_div(M1, 32)), 256, 0, s>>>(src, K, M1, st->Mp, st->Kp,
-                                                                        st->fbits, st->Fp);
+                                                                        st->fbits, st->Fp, nullptr);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
@@ -607,10 +607,10 @@ int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, dou
     DGTM_CUDA_TRY(cudaGetLastError());
     const OzSource left{G, FI, nullptr, M1, M1, 0}, right{nullptr, RT, nullptr, D, D, 0};
     oz_slice_t_kernel<<<dim3(st->panels, ceil_div(M1, 32)), 256, 0, s>>>(left, K, M1, st->Wp, st->Kp,
-                                                                        st->wbits, st->Wpl);
+                                                                        st->wbits, st->Wpl, nullptr);
     DGTM_CUDA_TRY(cudaGetLastError());
     oz_slice_t_kernel<<<dim3(st->panels, ceil_div(D, 32)), 256, 0, s>>>(
-        right, K, D, st->Wp, st->Kp, st->wbits + M1, st->Wpl + (size_t) st->Ap * st->Kp);
+        right, K, D, st->Wp, st->Kp, st->wbits + M1, st->Wpl + (size_t) st->Ap * st->Kp, nullptr);
     DGTM_CUDA_TRY(cudaGetLastError());
     OzGemm g;
     g.A = st->Fp;

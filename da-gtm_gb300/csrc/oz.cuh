@@ -76,7 +76,8 @@ struct OzEArgs {
     int *status;             // device: the bounded waits' status word
 };
 bool oze_wanted(int N, int D, int K);
-// *out stays null (and the call succeeds) where the data have a non-finite value
+// *out stays null (and the call succeeds) where the data have a non-finite value or, for
+// the responsibility pass, a column that does not fit one grid
 int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s);
 void oze_destroy(OzE *st);
 int oze_estep_blocks(const OzE *st);

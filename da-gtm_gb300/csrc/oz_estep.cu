@@ -19,7 +19,11 @@
 //   G and R T.  R_kn on its centre's power-of-two grid (the chunk's largest
 //     R of the centre within [2^-56, 1] of it: small responsibilities keep their
 //     relative precision), in eight digit planes, times the digit planes of
-//     T^T and a row of ones: 64-bit integer sums per chunk, FP64 across chunks.
+//     T^T and a row of ones: 64-bit integer sums per chunk, FP64 across chunks.  The
+//     points are what is summed over, so T^T has a grid per column; data with a column
+//     whose largest value is far above its others (plain_columns) stay on the CUDA cores
+//     altogether: their pass with these distances' d_ref would put R of the large point
+//     off by its |t|^2.
 //
 // Points go in chunks whose K x nn integers stay in L2 (8 M of them, 64 MB).
 // Everything per chunk is a launch of its own: the distances cross L2 once more
@@ -741,6 +745,7 @@ struct OzE {
     int *nmin = nullptr;
     unsigned *wmin = nullptr;
     unsigned *done = nullptr;  // statistics blocks finished in a call
+    unsigned *low = nullptr;   // values of each column of T (and of the ones) short of bits
 };
 
 // The digit-slice path has fixed costs (planes of the centres, four launches a
@@ -770,6 +775,19 @@ static const uint64_t *host_table()
     };
     static const Table t;
     return t.v;
+}
+
+// Whether every column of T keeps its precision on one grid: at most a quarter of its
+// values are below 2^-6 of the grid's end and not exact there.  A value at that line
+// keeps 50 bits, the column's sums then 2^-51 of its bulk.  Gaussian and uniform
+// columns, and 0/1 and other coarse values, pass (a Gaussian column of 1e6 points: 20 %);
+// a column with one value 16 standard deviations out does not (38 %).
+static bool plain_columns(const std::vector<unsigned> &low, int N)
+{
+    for (unsigned n : low)
+        if (4.0 * n > (double) N)
+            return false;
+    return true;
 }
 
 int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
@@ -827,6 +845,7 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         lay(&st->thr, sizeof(int64_t) * N, base);
         lay(&st->wmin, sizeof(unsigned) * K, base);
         lay(&st->done, sizeof(unsigned), base);
+        lay(&st->low, sizeof(unsigned) * (D + 1), base);
         if (a.mstep) {
             lay(&st->Tt, planes * st->Wp * st->Npk, base);
             lay(&st->Rp, planes * st->Kp128 * st->chunk, base);
@@ -860,15 +879,20 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         oz_colmax_kernel<<<dim3(ceil_div(N, 512), ceil_div(D + 1, 32)), 256, 0, s>>>(src, N, D + 1, 512, st->bits);
         e = cudaGetLastError();
     }
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(st->low, 0, sizeof(unsigned) * (D + 1), s);
     if (e == cudaSuccess && a.mstep) {
         e = cudaMemsetAsync(st->Tt, 0, planes * st->Wp * st->Npk, s);
         oz_slice_t_kernel<<<dim3(st->Npk / PANEL, ceil_div(D + 1, 32)), 256, 0, s>>>(
-            src, N, D + 1, st->Wp, st->Npk, st->bits, st->Tt);
+            src, N, D + 1, st->Wp, st->Npk, st->bits, st->Tt, st->low);
         if (e == cudaSuccess)
             e = cudaGetLastError();
     }
     // a column's largest value (the squares of all are finite below 2^500)
     std::vector<unsigned long long> top(D + 1);
+    std::vector<unsigned> low(D + 1);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(low.data(), st->low, sizeof(unsigned) * (D + 1), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(top.data(), st->bits, sizeof(unsigned long long) * (D + 1), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
@@ -880,12 +904,15 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         oze_destroy(st);
         return code;
     }
-    // data, or squares of it, that are not finite: the CUDA-core kernels carry them
+    // the CUDA-core kernels carry data, or squares of it, that are not finite, and sums
+    // that the grids would cost bits
+    bool fit = plain_columns(low, N);
     for (int d = 0; d < D; d++)
-        if (top[d] >= oz::double_bits(0x1p500)) {
-            oze_destroy(st);
-            return DGTM_OK;
-        }
+        fit = fit && top[d] < oz::double_bits(0x1p500);
+    if (!fit) {
+        oze_destroy(st);
+        return DGTM_OK;
+    }
     *out = st;
     return DGTM_OK;
 }

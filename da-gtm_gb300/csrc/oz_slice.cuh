@@ -64,22 +64,35 @@ static __global__ void __launch_bounds__(256) oz_colmax_kernel(OzSource src, int
 
 // planes[i][c][k] = digit i of column c of the source on the column's grid:
 // the transposed operand (contraction over the source's rows), zero past rows
-// and cols.  Block: 64 rows x 32 columns.
+// and cols.  low (may be null): low[c] += how many values of column c are short of bits on
+// its grid.  Block: 64 rows x 32 columns.
 static __global__ void __launch_bounds__(256) oz_slice_t_kernel(OzSource src, int rows, int cols, int prows,
                                                          int ld, const unsigned long long *__restrict__ bits,
-                                                         __nv_bfloat16 *__restrict__ planes)
+                                                         __nv_bfloat16 *__restrict__ planes,
+                                                         unsigned *__restrict__ low)
 {
     __shared__ int64_t qs[32][65];
+    __shared__ unsigned few[8][32];
     const int k0 = blockIdx.x * 64, c0 = blockIdx.y * 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int c = c0 + lane;
     const int e = c < cols ? oz::exponent_of(bits[c]) : 0;
+    unsigned n = 0;
 #pragma unroll
     for (int r = w; r < 64; r += 8) {
         const int k = k0 + r;
-        qs[lane][r] = (k < rows && c < cols) ? oz::to_fixed(src.at(k, c), e) : 0;
+        const double v = (k < rows && c < cols) ? src.at(k, c) : 0.0;
+        qs[lane][r] = oz::to_fixed(v, e);
+        n += oz::short_of_bits(v, e);
     }
+    few[w][lane] = n;
     __syncthreads();
+    if (low && w == 0 && c < cols) {
+        for (int i = 1; i < 8; i++)
+            n += few[i][lane];
+        if (n)
+            atomicAdd(&low[c], n);
+    }
 #pragma unroll
     for (int cc = w; cc < 32; cc += 8) {
         uint32_t v[oz::DIGITS];

@@ -100,6 +100,18 @@ OZ_HD int64_t to_fixed(double v, int e)
     return (b >> 63) ? -(int64_t) q : (int64_t) q;
 }
 
+// Whether v is below 2^(e - BULK) and not a whole number of the grid 2^(e - FIX): then
+// to_fixed keeps fewer than 50 bits of it.
+constexpr int BULK = 6;
+
+OZ_HD bool short_of_bits(double v, int e)
+{
+    const uint64_t b = double_bits(v);
+    const int E = (int) ((b >> 52) & 0x7FF), drop = e + 1020 - (E ? E : 1);
+    const uint64_t m = (b & 0xFFFFFFFFFFFFFull) | (E ? (1ull << 52) : 0ull);
+    return drop >= BULK - 2 && (m & ((1ull << (drop < 63 ? drop : 63)) - 1)) != 0;
+}
+
 // q 2^k as an int64 from a double q, rounded to nearest, saturated
 OZ_HD int64_t scaled_int(double v, int k)
 {

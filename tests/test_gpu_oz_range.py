@@ -134,3 +134,47 @@ def test_one_large_value_leaves_the_other_points_alone(pkg, orc, value, D, own, 
     # (Its FP32 distance of 1e6 - 1e6 says nothing; |t|^2 = 1e60 is too much for FP64 too.)
     if (form == "fp64" and value < 1e30) or not own:
         assert np.max(np.abs(Rb[:, 5] - (np.eye(K)[7] if own else 1.0 / K))) <= 1e-13
+
+
+@pytest.mark.parametrize("value,D,where", [(v, D, w) for v in (1e3, 1e6, 1e30) for D in (5, 12, 70)
+                                           for w in ("point", "centre", "both") if not (w == "both" and v == 1e30)])
+def test_one_large_value_leaves_the_statistics_alone(pkg, orc, value, D, where):
+    """G and R T centre by centre and column by column, 1e-12 of the sum of magnitudes, with
+    a far point (the CUDA-core kernels), a far centre (the slices) and a centre on the far
+    point."""
+    N, K = 1000, 400
+    T, Y, _ = outlier_case(value if where != "centre" else 0.5, D, where == "both")
+    if where == "centre":
+        Y[7, D // 2] = value
+    beta, temp = 60.0 * 12 / max(D, 12), 1.5
+    with np.errstate(over="ignore", invalid="ignore"):
+        R, _, _ = orc.resp(orc.dist(Y, T), beta, 1, temp)
+    with pkg.Context(T, np.ones((K, 1)), "fp64") as c:
+        assert c.path == ("exact_slices" if where == "centre" else "cuda_cores")
+        c.set_Y(Y)
+        c.estep(beta, 1, temp)
+        c.mstep()
+        G, RT = c.get_stats()
+    assert np.max(np.abs(G - R.sum(1)) / np.maximum(R.sum(1), 1e-300)) <= 1e-12
+    assert np.max(np.abs(RT - R @ T) / np.maximum(R @ np.abs(T), 1e-300)) <= 1e-12
+
+
+@pytest.mark.parametrize("kind,slices", [("gauss", True), ("uniform", True), ("sparse", True), ("offset", True),
+                                         ("outlier", False), ("lognormal", False)])
+def test_which_columns_keep_the_digit_slices(pkg, kind, slices):
+    """The rule on the columns: ordinary and exactly held data keep the slices."""
+    rng = np.random.default_rng(6)
+    N, D, K = 4000, 20, 100
+    T = rng.normal(size=(N, D))
+    if kind == "uniform":
+        T = rng.random((N, D))
+    elif kind == "sparse":  # mostly zeros, and values of few bits
+        T = (rng.random((N, D)) < 0.02) * rng.integers(1, 1000, (N, D)).astype(float)
+    elif kind == "offset":
+        T += 1e6
+    elif kind == "outlier":
+        T[17, 3] = 200.0
+    elif kind == "lognormal":
+        T[:, 4] = np.exp(2.0 * T[:, 4])
+    with pkg.Context(T, np.ones((K, 1)), "fp64") as c:
+        assert (c.path == "exact_slices") == slices
