@@ -48,6 +48,7 @@ constexpr long long CHUNK = 10000000;   // centre-point pairs a chunk
 constexpr int ST_PTS = 8;               // points of a statistics or map block
 constexpr int DG_K = 2;                 // centres of a digits block
 constexpr int NARROW = 8;               // depths whose products are formed as 64-bit integers
+constexpr int NARROW_K = 16;            // centres of a block of them
 constexpr int64_t ZERO_COLUMN = INT64_MIN;  // aref of a point whose R is 1/K
 constexpr size_t TAB_BYTES = sizeof(uint64_t) * oz::TAB;
 
@@ -155,30 +156,29 @@ __global__ void __launch_bounds__(256) oz_units_kernel(const int *__restrict__ e
 // than an FP64 sum loses: on one grid for all points the error of R at D = 5 was 1.9e-15 of
 // its norm, 1.2e-15 by FP64 products, and is 5.6e-16 this way (D >= 9: the digits were the more
 // exact, 2.2e-15 against 2.6e-15 at D = 9, 4.1e-15 against 1.4e-14 at D = 37).  A thread
-// holds a point, DP >= D depths of it, and goes through 64 centres; bound by integer issue,
-// about 10 instructions a product.
+// holds a point, DP >= D depths of it, and goes through 16 centres; bound by integer issue,
+// about 10 instructions a product, on small problems by the latency of that loop (N = 992,
+// K = 289, D = 4: 29 us with 64 centres).
 template <int DP>
 __global__ void __launch_bounds__(256) oz_narrow_kernel(const int64_t *__restrict__ T, const int64_t *__restrict__ Y,
                                                         int nn, int K, const OzUnit *__restrict__ units,
                                                         const oz::Centre *__restrict__ cen, size_t ldm,
                                                         int64_t *__restrict__ out)
 {
-    __shared__ longlong2 cols[64];  // |y|^2 / 2 on one exponent (as in oz_gemm_kernel) and f
-    __shared__ int tops[2];
-    const int kb = blockIdx.y * 64;
-    oz::Centre c;
-    if (threadIdx.x < 64) {
-        c = cen[min(kb + (int) threadIdx.x, K - 1)];
+    __shared__ longlong2 cols[NARROW_K];  // |y|^2 / 2 on one exponent (as in oz_gemm_kernel) and f
+    __shared__ int s_top;
+    const int kb = blockIdx.x * NARROW_K;
+    if (threadIdx.x < 32) {
+        const oz::Centre c = cen[min(kb + (int) threadIdx.x % NARROW_K, K - 1)];
         const int top = __reduce_max_sync(0xffffffffu, c.yx);
-        if ((threadIdx.x & 31) == 0)
-            tops[threadIdx.x >> 5] = top;
+        if (threadIdx.x < NARROW_K)
+            cols[threadIdx.x] = make_longlong2(oz::half_square(c, top), c.f);
+        if (threadIdx.x == 0)
+            s_top = top;
     }
     __syncthreads();
-    const int top = max(tops[0], tops[1]);
-    if (threadIdx.x < 64)
-        cols[threadIdx.x] = make_longlong2(oz::half_square(c, top), c.f);
-    __syncthreads();
-    const int m = blockIdx.x * 256 + threadIdx.x;
+    const int top = s_top;
+    const int m = blockIdx.y * 256 + threadIdx.x;
     if (m >= nn)
         return;
     const OzUnit un = units[m];
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(256) oz_narrow_kernel(const int64_t *__restric
 #pragma unroll
     for (int d = 0; d < DP; d++)
         t[d] = T[(size_t) m * DP + d];
-    const int k1 = min(K, kb + 64);
+    const int k1 = min(K, kb + NARROW_K);
 #pragma unroll 4
     for (int k = kb; k < k1; k++) {
         int64_t sum = 0;
@@ -237,7 +237,7 @@ struct OzStatsArgs {
 __device__ __forceinline__ void add_power(uint64_t x, const oz::Mul &k, const uint64_t *tab, uint64_t &lo,
                                           uint32_t &hi)
 {
-    const uint64_t W = oz::mul_w(k, x <= k.lim ? x : k.lim);  // lim is 1024 bits down at least (or 0)
+    const uint64_t W = oz::mul_w(k, x <= k.lim ? x : k.lim);  // lim is 992 bits down at least (or 0)
     const int n = (int) (W >> oz::WFRAC);
     if (n < 64 && x <= k.lim) {
         const uint64_t t = oz::exp2_neg(W, tab) >> n;
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
         for (int e = 0; e < 2; e++) {
             const int n = min(2 * j + e, nn - 1);
             o[e] = pt[n];
-            km[e] = oz::mul_unit(kb, units[n].u);
+            km[e] = oz::mul_at(kb, units[n].u);
             t[e] = 2 * j + e < nn ? thr[n] : INT64_MAX;  // padding: R = 0
         }
 #pragma unroll
@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(256) oz_rblock_kernel(const int64_t *__restric
     for (size_t i = blockIdx.x * (size_t) 256 + threadIdx.x; i < total; i += (size_t) gridDim.x * 256) {
         const int k = (int) (i / nn), n = (int) (i - (size_t) k * nn);
         const int64_t v = acc[(size_t) k * ldm + n];
-        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, oz::mul_unit(kb, units[n].u));
+        const uint64_t W = v < thr[n] ? ~0ull : r_exponent(pt[n], v, oz::mul_at(kb, units[n].u));
         R[(size_t) k * ldR + n] =
             W == ~0ull ? 0.0 : oz::to_double(oz::exp2_neg(W, tab), (int) (W >> oz::WFRAC) - oz::WBIAS);
     }
@@ -947,7 +947,7 @@ int narrow_products(OzE *st, int m0, int nn, int k0, int nk, size_t ldm, int64_t
 {
     const int dp = st->narrow;
     const auto kernel = dp == 2 ? oz_narrow_kernel<2> : dp == 4 ? oz_narrow_kernel<4> : oz_narrow_kernel<8>;
-    const dim3 grid(ceil_div(nn, 256), ceil_div(nk, 64));
+    const dim3 grid(ceil_div(nk, NARROW_K), ceil_div(nn, 256));
     kernel<<<grid, 256, 0, s>>>((const int64_t *) st->Tp + (size_t) m0 * dp, (const int64_t *) st->Yp + (size_t) k0 * dp,
                                 nn, nk, st->units + m0, st->cen + k0, ldm, out);
     DGTM_CUDA_TRY(cudaGetLastError());

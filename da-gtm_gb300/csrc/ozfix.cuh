@@ -145,49 +145,6 @@ OZ_HD uint32_t digit_field(uint64_t biased, int i)
     return (uint32_t) (biased >> (7 * (DIGITS - 1 - i))) & (i == 0 ? 255u : 127u);
 }
 
-// w = x kappa in units of 2^-53, for 0 <= x <= lim: (mulhi(x << a, m)) >> b.  Beyond
-// lim, x << a has more than 64 bits (w is then 1024 at least) or w is 2000 or more.
-struct Mul {
-    uint64_t m;
-    uint64_t lim;
-    int a, b;
-};
-
-constexpr uint64_t W_END = 2000ull << WFRAC;  // a power from here on is 0
-
-// kappa = k0 2^u with k0 known on the host and u (the unit of x) on the device
-struct MulBase {
-    uint64_t m;   // k0 = m 2^(ex - 64), m's top bit set
-    uint64_t l0;  // 2000 / (m 2^-64) in units of 2^-20
-    int ex;
-};
-
-static inline MulBase make_mul(double k0)
-{
-    MulBase r;
-    int ex = 0;
-    const double f = frexp(k0, &ex);  // k0 = f 2^ex, f in [0.5, 1)
-    r.m = (uint64_t) ldexp(f, 64);
-    r.l0 = (uint64_t) (2000.0 / f * 1048576.0);
-    r.ex = ex;
-    return r;
-}
-
-OZ_HD Mul mul_at(const MulBase &k, int u)
-{
-    Mul r;
-    r.m = k.m;
-    // x kappa 2^53 = x m 2^(ex + u + 53 - 64) = mulhi(x << a, m) >> b
-    const int sh = k.ex + u + WFRAC;  // a - b
-    r.a = sh > 0 ? (sh < 65 ? sh : 65) : 0;         // above 63 only x = 0 is within lim
-    r.b = sh < 0 ? (sh > -63 ? -sh : 63) : 0;
-    const uint64_t cap = sh > 63 ? 0ull : ~0ull >> r.a;  // x << a below 2^64
-    const int ls = -(k.ex + u) - 20;                // lim = l0 2^ls, l0 < 2^32
-    uint64_t l = ls >= 31 ? ~0ull >> 1 : ls >= 0 ? k.l0 << ls : ls > -64 ? k.l0 >> -ls : 0ull;
-    r.lim = l < cap ? l : cap;
-    return r;
-}
-
 // x 2^s for s of 0 and more, zeros from 64 on; and x 2^-s towards minus infinity
 OZ_HD uint64_t shl(uint64_t x, int s)
 {
@@ -222,21 +179,47 @@ OZ_HD uint64_t shr(uint64_t x, int s)
 #endif
 }
 
-// The same where a thread has few x of a unit: lim leaves out the last 32nd of what fits,
-// so that w stays below 1984 without a look at l0.
-OZ_HD Mul mul_unit(const MulBase &k, int u)
+// w = x kappa in units of 2^-53, for 0 <= x <= lim: (mulhi(x << a, m)) >> b.  lim leaves
+// out the last 32nd of what x << a has room for, so that w is below 1984 there; beyond it
+// w is 992 or more.
+struct Mul {
+    uint64_t m;
+    uint64_t lim;
+    int a, b;
+};
+
+constexpr uint64_t W_END = 2000ull << WFRAC;  // a power from here on is 0
+
+// kappa = k0 2^u with k0 known on the host and u (the unit of x) on the device
+struct MulBase {
+    uint64_t m;  // k0 = m 2^(ex - 64), m's top bit set
+    int ex;
+};
+
+static inline MulBase make_mul(double k0)
+{
+    MulBase r;
+    int ex = 0;
+    const double f = frexp(k0, &ex);  // k0 = f 2^ex, f in [0.5, 1)
+    r.m = (uint64_t) ldexp(f, 64);
+    r.ex = ex;
+    return r;
+}
+
+OZ_HD Mul mul_at(const MulBase &k, int u)
 {
     Mul r;
-    const int sh = k.ex + u + WFRAC;
+    // x kappa 2^53 = x m 2^(ex + u + 53 - 64) = mulhi(x << a, m) >> b
+    const int sh = k.ex + u + WFRAC;  // a - b
     r.m = k.m;
-    r.a = sh > 0 ? sh : 0;
+    r.a = sh > 0 ? sh : 0;  // from 64 on only x = 0 is within lim
     r.b = sh < 0 ? -sh : 0;
     const uint64_t cap = shr(~0ull, r.a);
     r.lim = cap - (cap >> 5);
     return r;
 }
 
-OZ_HD uint64_t mul_w(const Mul &k, uint64_t x) { return mulhi(x << (k.a & 63), k.m) >> k.b; }
+OZ_HD uint64_t mul_w(const Mul &k, uint64_t x) { return shr(mulhi(shl(x, k.a), k.m), k.b); }
 
 // w of x > lim: ~0 from 2000 on.  What x << a has no room for below that has one bit
 // too many (m >= 2^63), so it is 2 mulhi(x << (a - 1), m): every power that FP64 can

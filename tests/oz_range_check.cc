@@ -30,10 +30,6 @@ int main()
                     dropped++;
                 if (ref >= 2010.0L && w != ~0ull)
                     beyond++;
-                const Mul q = mul_unit(make_mul(k0), u);
-                const uint64_t w2 = whole(q, x);
-                if (w2 != w && !(ref >= 1980.0L && (w2 == ~0ull || w == ~0ull)) && !(ref >= 960.0L && w2 - w + 2 <= 4))
-                    dropped++;
                 if (w != ~0ull)
                     worst = fmaxl(worst, fabsl((long double) w - ref * 0x1p53L));
             }
