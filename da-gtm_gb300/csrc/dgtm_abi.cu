@@ -1022,7 +1022,8 @@ int dgtm_next_ctemp_k(dgtm_ctx *ctx, double temp, double beta, double eps, const
         if (rc == DGTM_OK && e == cudaSuccess && (e = cudaStreamSynchronize(ctx->stream)) == cudaSuccess)
             rc = check_oz_status(ctx);
         cudaFree(dspread);
-        // centres whose expansion about the data's mean cancels more than 8 bits
+        // centres that lose more than 8 bits to the expansion about the data's mean or to
+        // the features' grids
         for (int k = 0; rc == DGTM_OK && e == cudaSuccess && k < K; k++)
             if (!(spread[k] <= 256.0))
                 redo.push_back(k);

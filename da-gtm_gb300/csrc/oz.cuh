@@ -107,8 +107,8 @@ int oze_map(OzE *st, const double *Y, const double *yy, const double2 *colstat, 
 
 // The AUTO schedule's scatter in FP64 accuracy as digit-slice products of R and
 // R^2 with pair features (oz_ctemp.cu): out and gsum as launch_ctemp_batch;
-// spread[k] = tr(sum R x x^T) / tr(S1) about the data's mean: what the expansion
-// cancels.  DGTM_ENOMEM (nothing done) if not even 128 centres fit the budget.
+// spread[k]: what the expansion about the data's mean and the features' grids cost, as a
+// factor of 2^-53 (see there).  DGTM_ENOMEM (nothing done) if not even 128 centres fit the budget.
 int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, const double2 *colstat, int N,
              int D, int K, int sms, double c1, double c, double dcut, const double *gg_dev, double lim_scale,
              size_t budget, double *gsum_dev, double *out_dev, double *spread_dev, int *status,

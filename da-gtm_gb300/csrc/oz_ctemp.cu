@@ -12,8 +12,11 @@
 // and so has each centre's R.
 //
 // The expansion cancels where a centre's points lie close together and far from
-// the mean: tr P / tr S1 says by how much (a few units on spread-out data).  The
-// caller redoes the centres for which it is large with the CUDA-core scatter.
+// the mean: tr P / tr S1 says by how much (a few units on spread-out data).  And a
+// feature's grid is that of its largest value over all points, 2^-56 of which every point
+// may be off: against tr S1 that is g sum_d max z_d^2 / tr S1 (a value far from the others
+// makes it large).  The caller redoes the centres for which either loses more than 8 bits
+// of 2^-53 with the CUDA-core scatter.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "oz.cuh"
@@ -203,8 +206,10 @@ __global__ void __launch_bounds__(256) sums_kernel(const int64_t *__restrict__ p
 __global__ void __launch_bounds__(256) assemble_kernel(const double *__restrict__ P, int rows, int kpad, int D,
                                                        const Feature *__restrict__ ftab,
                                                        const double *__restrict__ Y,
-                                                       const double *__restrict__ mean, double *__restrict__ S,
-                                                       double *__restrict__ gsum, double *__restrict__ spread)
+                                                       const double *__restrict__ mean,
+                                                       const unsigned long long *__restrict__ zbits,
+                                                       double *__restrict__ S, double *__restrict__ gsum,
+                                                       double *__restrict__ spread)
 {
     extern __shared__ double sh[];  // w, a1, a2
     __shared__ double red[32];
@@ -218,7 +223,7 @@ __global__ void __launch_bounds__(256) assemble_kernel(const double *__restrict_
     __syncthreads();
     const double g1 = P[(size_t) (np + D) * rows + k], g2 = P[(size_t) (np + D) * rows + kpad + k];
     double *S1 = S + (size_t) k * 2 * D * D, *S2 = S1 + (size_t) D * D;
-    double tp = 0.0, ts = 0.0;
+    double tp = 0.0, ts = 0.0, tz = 0.0;  // traces: P, S1, the squares of the coordinates' maxima
     for (int f = threadIdx.x; f < np; f += 256) {
         const int i = ftab[f].i, j = ftab[f].j;
         const double p1 = P[(size_t) f * rows + k], p2 = P[(size_t) f * rows + kpad + k];
@@ -229,15 +234,21 @@ __global__ void __launch_bounds__(256) assemble_kernel(const double *__restrict_
         S1[(size_t) i * D + j] = s1;
         S2[(size_t) i * D + j] = s2;
         if (i == j) {
+            const double z = oz::bits_double(zbits[i]);
             tp += p1;
             ts += s1;
+            tz = fma(z, z, tz);
         }
     }
     tp = block_sum_fixed(tp, red);
     ts = block_sum_fixed(ts, red);
+    tz = block_sum_fixed(tz, red);
     if (threadIdx.x == 0) {
         gsum[k] = g1;
-        spread[k] = tp > 0.0 ? (ts > 0.0 ? tp / ts : INFINITY) : 0.0;
+        // 2^-56 of a feature against 2^-53 of P: an eighth.  tz >= tp / g: all zero only if
+        // tz is, or g
+        const double lost = fmax(tp, 0.125 * g1 * tz);
+        spread[k] = lost > 0.0 ? (ts > 0.0 ? lost / ts : INFINITY) : lost;
     }
 }
 
@@ -341,7 +352,7 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
                                                                        oz_sum_ext(g.panels), nmin, rows, F, ftab, ch == 0 ? 1 : 0, P);
                 DGTM_CUDA_TRY(cudaGetLastError());
             }
-            assemble_kernel<<<kb, 256, asmem, s>>>(P, rows, kpad, D, ftab, Y + (size_t) k0 * D, mean, S, gsum_dev + k0,
+            assemble_kernel<<<kb, 256, asmem, s>>>(P, rows, kpad, D, ftab, Y + (size_t) k0 * D, mean, zbits, S, gsum_dev + k0,
                                                    spread_dev + k0);
             DGTM_CUDA_TRY(cudaGetLastError());
             OZ_TRY(launch_ctemp_eig(pl, kb, D, S, Mg, gg_dev ? gg_dev + k0 : gsum_dev + k0, lim_scale,

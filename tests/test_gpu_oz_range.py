@@ -178,3 +178,25 @@ def test_which_columns_keep_the_digit_slices(pkg, kind, slices):
         T[:, 4] = np.exp(2.0 * T[:, 4])
     with pkg.Context(T, np.ones((K, 1)), "fp64") as c:
         assert (c.path == "exact_slices") == slices
+
+
+def test_scatter_with_one_value_far_from_the_mean(pkg, monkeypatch):
+    """A column around 1000 with one value of 30,000 fits its grid as data, but the squares
+    about the mean do not: those centres go through the CUDA-core scatter.  (2^-57 of the
+    square's grid is 4e-9 a point; the distances' own 1e6 2^-53 is 1e-10.)"""
+    rng = np.random.default_rng(12)
+    N, D, K = 6000, 20, 60
+    T = rng.normal(size=(N, D))
+    T[:, 0] += 1000.0
+    Y = T[rng.integers(0, N, K)] + 0.5 * rng.normal(size=(K, D))
+    T[11, 0] = 30000.0
+    beta = 0.3
+    out = []
+    for pairs in ("1", "0"):
+        monkeypatch.setenv("DGTM_CTEMP_PAIRS", pairs)
+        with pkg.Context(T, np.ones((K, 1)), "fp64") as c:
+            assert c.path == "exact_slices"
+            c.set_Y(Y)
+            c.estep(beta, 1, 2.0)
+            out.append(c.next_ctemp(50.0, beta, 1e-6, per_centre=True)[1])
+    np.testing.assert_allclose(out[0], out[1], rtol=1e-13)
