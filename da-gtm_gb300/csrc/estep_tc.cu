@@ -1083,7 +1083,7 @@ struct P3Params {
     const float *T;      // N x D
     const double *gF;    // g (null: 1)
     double beta;
-    int *status;         // the waits' status word, then the CTAs that are done (0 between launches)
+    int *status;
 };
 
 template <int NP, int KL, int NT>
@@ -1397,21 +1397,22 @@ __global__ void __launch_bounds__(p3_threads(NP), 1)
     tc_fence_after();
     if (warp == 0)
         tmem_dealloc(tmem, 512);
-    // The last CTA sees every CTA's waits: once one of this call has given up, all of
-    // dT is NaN, whichever tiles had finished before.
-    __shared__ int poison;
+    // Once a wait of this call has given up, all of dT is NaN: the CTA whose wait it was
+    // fills the whole of it, and a CTA that ends later its own rows.  (One that did not see
+    // the status word set after its last row wrote that row before the word was set, so
+    // before the filling.)
+    __shared__ int gave_up;
     if (threadIdx.x == 0) {
         __threadfence();
-        const bool last = atomicAdd(p.status + 1, 1) == (int) gridDim.x - 1;
-        if (last)
-            p.status[1] = 0;
-        __threadfence();
-        poison = last && *(volatile int *) p.status != 0;
+        gave_up = *(volatile int *) p.status != 0;
     }
     __syncthreads();
-    if (poison)
-        for (size_t i = threadIdx.x; i < (size_t) p.N * p.D; i += p3_threads(NP))
+    if (gave_up) {
+        const size_t i0 = failed ? 0 : (size_t) n0 * p.D;
+        const size_t i1 = failed ? (size_t) p.N * p.D : (size_t) min(n0 + P3_TILE, p.N) * p.D;
+        for (size_t i = i0 + threadIdx.x; i < i1; i += p3_threads(NP))
             p.C[i] = NAN;
+    }
 }
 
 using P3Kernel = void (*)(const CUtensorMap, const CUtensorMap, const P3Params);
@@ -1805,7 +1806,7 @@ int tc_create(TcState **out, int N, int D, int K, int sms, const double *T64, co
         tc_destroy(st);
         return code;
     };
-    cudaError_t e = cudaMalloc((void **) &st->status, 2 * sizeof(int));
+    cudaError_t e = cudaMalloc((void **) &st->status, sizeof(int));
     if (e == cudaSuccess)
         e = cudaMallocHost((void **) &st->hstatus, sizeof(int));
     if (e == cudaSuccess)
@@ -1918,7 +1919,7 @@ int tc_estep(TcState *st, const double *, double c1, double c2, int isDA, double
     p.colq = st->colq;
     p.part = part;
     p.status = st->status;
-    DGTM_CUDA_TRY(cudaMemsetAsync(st->status, 0, 2 * sizeof(int), s));  // and pass 3's count
+    DGTM_CUDA_TRY(cudaMemsetAsync(st->status, 0, sizeof(int), s));
     st->pass1<<<tc_pass1_blocks(st), P1_THREADS, st->smem1, s>>>(st->tmY1, st->tmT1, p);
     DGTM_CUDA_TRY(cudaGetLastError());
     *nlaunch = 1;
@@ -1981,8 +1982,7 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t) 255; }
 // A plan over the workspace: T always in two BF16 pieces (the data of a
 // gradient step are real-valued, and the piece count must be known without
 // inspecting them); Y pieces with the folded -|y|^2/2 columns; the column
-// statistics; the pass-2 slots; the status word of the bounded waits and pass 3's count
-// of finished CTAs.
+// statistics; the pass-2 slots; the status word of the bounded waits.
 static int fe_state(int N, int K, int D, int sms, TcState *st, TcFeLayout *L)
 {
     int rc = sm10x_or_fail();
@@ -2000,7 +2000,7 @@ static int fe_state(int N, int K, int D, int sms, TcState *st, TcFeLayout *L)
     L->Yb = take(sizeof(__nv_bfloat16) * 2 * (size_t) st->Kpad * st->Dp);
     L->colq = take(sizeof(float4) * (size_t) st->Npad);
     L->RTpart = take(sizeof(float) * (size_t) st->nunits * P2_BK * st->Dp);
-    L->status = take(2 * sizeof(int));
+    L->status = take(sizeof(int));
     L->total = o;
     L->pass1_blocks = tc_pass1_blocks(st);
     return DGTM_OK;
@@ -2049,7 +2049,7 @@ int tc_fe_estep(const TcFeLayout &L, void *ws, const float *Y, const float *T, i
         Y, K, D, st.Dp, st.Kpad, st.Yb, nullptr);
     DGTM_CUDA_TRY(cudaGetLastError());
     int nl = 0;
-    // tc_estep clears the status words.  The free energy needs the statistics at `temp` only.
+    // tc_estep clears the status word.  The free energy needs the statistics at `temp` only.
     return tc_estep(&st, nullptr, c1, c2, 1, colstat, part, s, &nl, false);
 }
 
