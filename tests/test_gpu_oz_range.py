@@ -199,4 +199,9 @@ def test_scatter_with_one_value_far_from_the_mean(pkg, monkeypatch):
             c.set_Y(Y)
             c.estep(beta, 1, 2.0)
             out.append(c.next_ctemp(50.0, beta, 1e-6, per_centre=True)[1])
-    np.testing.assert_allclose(out[0], out[1], rtol=1e-13)
+            R = c.R_block(0, K, 0, N)
+    # 8 bits of 2^-53 of the trace may go (it is the far point's where a centre has a share
+    # of it, and its eigenvalue is then cut and the next one taken)
+    trace = np.array([(R[k][:, None] * (T - Y[k]) ** 2).sum() for k in range(K)]) / R.sum(1)
+    assert np.median(trace) < 100.0
+    assert np.all(np.abs(out[0] - out[1]) <= 1e-13 * out[1] + 2.0 ** -45 * beta * trace)
