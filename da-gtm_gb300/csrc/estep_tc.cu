@@ -1297,13 +1297,13 @@ __global__ void __launch_bounds__(p3_threads(NP), 1)
         const float4 cq = p.colq[n];  // n < Npad: padding points carry R = 0
         bool ok = true;
         // OUT (this thread's row) to C: 16-column batches, batch i to group i % (BK / 32);
-        // the last one leaves dT.
+        // the last one leaves dT (NaN once a wait of the call has given up: see the end).
         // A batch's loads are all issued before its first store: C and T may be any
         // buffers, so between stores each load would wait out its own latency.
         const bool quads = (p.D & 3) == 0 && (((uintptr_t) p.C | (uintptr_t) p.T) & 15) == 0;
         auto drain_out = [&](bool add, bool last) {
             const double g = p.gF ? p.gF[0] : 1.0;
-            const float gb = (float) (-g * p.beta);
+            const float gb = (float) (-(*(volatile int *) p.status ? NAN : g) * p.beta);
 #pragma unroll 1
             for (int c0 = 16 * h; c0 < p.nout; c0 += BK / 2) {
                 uint32_t v[16];
@@ -1398,19 +1398,12 @@ __global__ void __launch_bounds__(p3_threads(NP), 1)
     if (warp == 0)
         tmem_dealloc(tmem, 512);
     // Once a wait of this call has given up, all of dT is NaN: the CTA whose wait it was
-    // fills the whole of it, and a CTA that ends later its own rows.  (One that did not see
-    // the status word set after its last row wrote that row before the word was set, so
-    // before the filling.)
-    __shared__ int gave_up;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        gave_up = *(volatile int *) p.status != 0;
-    }
-    __syncthreads();
-    if (gave_up) {
-        const size_t i0 = failed ? 0 : (size_t) n0 * p.D;
-        const size_t i1 = failed ? (size_t) p.N * p.D : (size_t) min(n0 + P3_TILE, p.N) * p.D;
-        for (size_t i = i0 + threadIdx.x; i < i1; i += p3_threads(NP))
+    // fills it, and a row drained after that is NaN by its factor (drain_out).  A row whose
+    // factor was read just before the status word was set is stored within microseconds of
+    // that; the filling starts a millisecond later.
+    if (failed) {
+        __nanosleep(1000000);
+        for (size_t i = threadIdx.x; i < (size_t) p.N * p.D; i += p3_threads(NP))
             p.C[i] = NAN;
     }
 }
