@@ -385,14 +385,7 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
     CK(dev_alloc(&c->B, (size_t) M1 * D));
     CK(dev_alloc(&c->work, 2 * (size_t) M1 * M1 + (size_t) M1 * D));
     CK(dev_alloc(&c->bterm, K));
-    // The FP32 and split forms keep form_ab's multiply-add chain: their E-step
-    // rounds the centres to FP32 / BF16 pieces, so a W that differs in its last
-    // bits flips some of those roundings, and a run would no longer repeat what
-    // it gave before to better than the form's own 1e-5.
-    if (precision == DGTM_FP64 && slices_on() && ozab_wanted(K, M1, D))
-        CK(unless_enomem(ozab_create(&c->ozab, K, M1, D, c->sms, c->stream)));
-    if (!c->ozab)
-        CK(dev_alloc(&c->abpart, form_ab_scratch_doubles(M1, D)));
+    CK(dev_alloc(&c->abpart, form_ab_scratch_doubles(M1, D)));
     // scalars, then the status words; on the host W follows where it is small
     CK(dev_alloc(&c->scal, CTL_DOUBLES));
     c->flag = (int *) (c->scal + 8);
@@ -408,8 +401,6 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
                           sizeof(double) * D, N, cudaMemcpyHostToDevice, c->stream));
     CKC(copy_rows(c->FI, sizeof(double) * M1, FI, sizeof(double) * (size_t) ldFI,
                           sizeof(double) * M1, K, cudaMemcpyHostToDevice, c->stream));
-    if (c->ozab)
-        CK(ozab_basis(c->ozab, c->FI, c->stream));
     if (precision != DGTM_FP64) {
         CK(dev_alloc(&c->FIp, (size_t) K * M1));
         CK(launch_to_pairs(c->FI, (size_t) K * M1, c->FIp, c->stream));
@@ -445,6 +436,16 @@ int dgtm_ctx_create(int N, int D, int K, int M1, const double *T, int ldT, const
             }
             if (c->oze)
                 c->nblk1 = oze_estep_blocks(c->oze);
+        }
+        // The FP32 and split forms keep form_ab's multiply-add chain: their E-step
+        // rounds the centres to FP32 / BF16 pieces, so a W that differs in its last
+        // bits flips some of those roundings, and a run would no longer repeat what
+        // it gave before to better than the form's own 1e-5.  The slices hold R T on a
+        // grid per column, as data that fit one do (0/1 data, and oze's).
+        if ((c->x64 || c->oze) && slices_on() && ozab_wanted(K, M1, D)) {
+            CK(unless_enomem(ozab_create(&c->ozab, K, M1, D, c->sms, c->stream)));
+            if (c->ozab)
+                CK(ozab_basis(c->ozab, c->FI, c->stream));
         }
         CK(dev_alloc(&c->part, 2 * (size_t) c->nblk1));
         if (!c->oze) {
@@ -649,7 +650,7 @@ int dgtm_mstep(dgtm_ctx *ctx, double *W, int ldW, double *Y, int ldY, double *be
     }
     if (ctx->ozab) {
         int nab = 0;
-        DGTM_TRY(ozab_form(ctx->ozab, ctx->FI, ctx->G, ctx->RT, ctx->A, ctx->B, ctx->flag, &nab,
+        DGTM_TRY(ozab_form(ctx->ozab, ctx->FI, ctx->G, ctx->RT, ctx->A, ctx->B, ctx->abpart, ctx->flag, &nab,
                            ctx->stream));
         nsmall += nab - 2;
     } else {

@@ -70,10 +70,11 @@ int launch_reduce_slices(const double *Gpart, const double *RTpart, int nsplit, 
                          int D, double *G, double *RT, cudaStream_t s);
 // A = FI^T diag(G) FI (M1 x M1), B = FI^T RT (M1 x D); scratch holds
 // form_ab_scratch_doubles(M1, D) doubles of slice partials.  flag[0..2], the
-// solver's status words and update_y's ticket, are set to 0.
+// solver's status words and update_y's ticket, are set to 0.  only (may be null): nothing is
+// done where *only is 0.
 size_t form_ab_scratch_doubles(int M1, int D);
 int launch_form_ab(const double *FI, const double *G, const double *RT, int K, int M1,
-                   int D, double *A, double *B, double *scratch, int *flag, cudaStream_t s);
+                   int D, double *A, double *B, double *scratch, int *flag, cudaStream_t s, const int *only = nullptr);
 // W = A^{-1} B by Cholesky (solver 0) or symmetric-eigen pseudo-inverse (solver 1).
 // work: M1*M1 + M1 doubles (+ M1*M1 for solver 1).  flag[0] != 0 on failure
 // (flag[0..1] zero before).

@@ -86,8 +86,11 @@ constexpr int AB_LD = AB_TILE + 2;
 
 __global__ void __launch_bounds__(AB_THREADS) form_ab_rows_kernel(
     const double *__restrict__ FI, const double *__restrict__ G, const double *__restrict__ RT,
-    int K, int M1, int D, int M1p, int Wp, int kc, int slice_len, double *__restrict__ Cpart)
+    int K, int M1, int D, int M1p, int Wp, int kc, int slice_len, double *__restrict__ Cpart,
+    const int *__restrict__ only)
 {
+    if (only && !*only)
+        return;
     extern __shared__ double sh[];
     double *FIs = sh;                       // kc x M1p
     double *Rs = sh + (size_t) kc * M1p;    // kc x Wp
@@ -155,8 +158,10 @@ __global__ void __launch_bounds__(AB_THREADS) form_ab_rows_kernel(
 
 __global__ void __launch_bounds__(AB_THREADS) form_ab_partial_kernel(
     const double *__restrict__ FI, const double *__restrict__ G, const double *__restrict__ RT,
-    int K, int M1, int D, int nct, int slice_len, double *__restrict__ Cpart)
+    int K, int M1, int D, int nct, int slice_len, double *__restrict__ Cpart, const int *__restrict__ only)
 {
+    if (only && !*only)
+        return;
     __shared__ __align__(16) double FIs[AB_KC * AB_LD], Rs[AB_KC * AB_LD];
     const int W = D + M1;
     const int mt = (blockIdx.y / nct) * AB_TILE, ct = (blockIdx.y % nct) * AB_TILE;
@@ -238,8 +243,10 @@ __global__ void __launch_bounds__(AB_THREADS) form_ab_partial_kernel(
 // mirrored, so it is exactly symmetric
 __global__ void form_ab_reduce_kernel(const double *__restrict__ Cpart, int nslice, int M1, int D,
                                       double *__restrict__ A, double *__restrict__ B,
-                                      int *__restrict__ flag)
+                                      int *__restrict__ flag, const int *__restrict__ only)
 {
+    if (only && !*only)
+        return;
     if (blockIdx.x == 0 && threadIdx.x < 3)
         flag[threadIdx.x] = 0;
     const int W = D + M1;
@@ -277,7 +284,7 @@ __global__ void form_ab_reduce_kernel(const double *__restrict__ Cpart, int nsli
 size_t form_ab_scratch_doubles(int M1, int D) { return (size_t) AB_SLICES * M1 * (D + M1); }
 
 int launch_form_ab(const double *FI, const double *G, const double *RT, int K, int M1, int D,
-                   double *A, double *B, double *scratch, int *flag, cudaStream_t s)
+                   double *A, double *B, double *scratch, int *flag, cudaStream_t s, const int *only)
 {
     const int slice_len = ceil_div(K, AB_SLICES);
     const int nslice = ceil_div(K, slice_len);
@@ -287,17 +294,17 @@ int launch_form_ab(const double *FI, const double *G, const double *RT, int K, i
         kc = kc > 16 ? 16 : kc;  // at least 11: M1 + D <= 384
         form_ab_rows_kernel<<<dim3(nslice, ceil_div((M1p / 4) * (Wp / 4), AB_THREADS)), AB_THREADS,
                               sizeof(double) * (size_t) kc * (M1p + Wp), s>>>(FI, G, RT, K, M1, D, M1p, Wp, kc,
-                                                                              slice_len, scratch);
+                                                                              slice_len, scratch, only);
     } else {
         const int nct = ceil_div(D + M1, AB_TILE);
         form_ab_partial_kernel<<<dim3(nslice, ceil_div(M1, AB_TILE) * nct), AB_THREADS, 0, s>>>(
-            FI, G, RT, K, M1, D, nct, slice_len, scratch);
+            FI, G, RT, K, M1, D, nct, slice_len, scratch, only);
     }
     DGTM_CUDA_TRY(cudaGetLastError());
     const size_t total = (size_t) M1 * (D + M1);
     // small blocks: a small basis has few elements, and their loads spread over the SMs
     const int blocks = (int) ((total + 63) / 64);
-    form_ab_reduce_kernel<<<blocks, 64, 0, s>>>(scratch, nslice, M1, D, A, B, flag);
+    form_ab_reduce_kernel<<<blocks, 64, 0, s>>>(scratch, nslice, M1, D, A, B, flag, only);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }

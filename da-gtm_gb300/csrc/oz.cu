@@ -69,6 +69,7 @@ struct OzParams {
     int mrows, ncols;
     const OzUnit *units;
     const oz::Centre *cen;
+    const int *skip;
     int *status;
 };
 
@@ -115,6 +116,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
                                                                const __grid_constant__ CUtensorMap tmB,
                                                                const OzParams p)
 {
+    if (p.skip && *p.skip)
+        return;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *sm = (unsigned char *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
     unsigned char *Bst = sm, *Ast = sm + 2 * B_BUF;
@@ -446,6 +449,7 @@ int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
     p.ncols = g.ncols;
     p.units = g.units;
     p.cen = g.cen;
+    p.skip = g.skip;
     p.status = status;
     using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const OzParams);
     // |S_l| <= (l + 1) 64 panels 4096: at most 2^22 for two panels, and for 0/1 data
@@ -470,9 +474,31 @@ struct OzAB {
     unsigned long long *fbits = nullptr, *wbits = nullptr;
     int64_t *part = nullptr;
     int *tiles = nullptr;
+    int *wide = nullptr;  // G spans too much for the columns' grids: form_ab's chain does it
 };
 
 namespace {
+
+// A column of diag(G) FI is on the grid of its largest value, and what a basis function
+// loses is 2^-56 of that times its own largest value.  Where G is far smaller in the reach
+// of one basis function than elsewhere, the terms that determine its weights are as far
+// below the grid.  The line is a factor of 2^4 between max G times the function's maximum
+// and the maximum of their product.  Against long double, at K = 1600 to 8000, M1 = 65 and
+// 82, bases of condition 3e4 to 1e14, G falling over 0 to 12 decades: the centres' error is
+// 0.03 to 1.1 times the multiply-add chain's up to there (0.5 in the middle), 2 at 2^6,
+// 5 at 2^8, 30 at 2^13, 1000 at 2^20.
+__global__ void __launch_bounds__(256) ozab_wide_kernel(const unsigned long long *__restrict__ fbits,
+                                                        const unsigned long long *__restrict__ wbits, int M1,
+                                                        int gcol, int *__restrict__ wide)
+{
+    const double g = oz::bits_double(wbits[gcol]);
+    int w = 0;
+    for (int m = threadIdx.x; m < M1; m += 256)
+        w |= !(oz::bits_double(fbits[m]) * g <= 16.0 * oz::bits_double(wbits[m]));
+    w = __syncthreads_or(w);
+    if (threadIdx.x == 0)
+        *wide = w;
+}
 
 // A and B from the tiles' split sums (exact integers); a column with a
 // non-finite value gives NaN.
@@ -482,8 +508,10 @@ __global__ void __launch_bounds__(256) ozab_reduce_kernel(const int64_t *__restr
                                                           const unsigned long long *__restrict__ fbits,
                                                           const unsigned long long *__restrict__ wbits,
                                                           double *__restrict__ A, double *__restrict__ B,
-                                                          int *__restrict__ flag)
+                                                          int *__restrict__ flag, const int *__restrict__ wide)
 {
+    if (*wide)
+        return;
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 3)
         flag[threadIdx.x] = 0;
     const int t = blockIdx.x, v = tiles[t], mt = v >> 16, nt = v & 0xFFFF;
@@ -511,6 +539,9 @@ __global__ void __launch_bounds__(256) ozab_reduce_kernel(const int64_t *__restr
 
 }  // namespace
 
+// The slices' launches and gaps take about 70 us; the chain's multiply-adds run at
+// 0.63 TFMA/s: 32 us at the line and 250 at K = 8000, M1 = 65, D = 166 (8.2e7), where the
+// slices take 70.
 bool ozab_wanted(int K, int M1, int D)
 {
     return K <= (1 << 26) && (double) K * M1 * (0.5 * M1 + D) >= 2e7;
@@ -520,7 +551,7 @@ void ozab_destroy(OzAB *st)
 {
     if (!st)
         return;
-    void *ptrs[] = {st->Fp, st->Wpl, st->fbits, st->wbits, st->part, st->tiles};
+    void *ptrs[] = {st->Fp, st->Wpl, st->fbits, st->wbits, st->part, st->tiles, st->wide};
     for (void *p : ptrs)
         if (p)
             cudaFree(p);
@@ -560,9 +591,11 @@ int ozab_create(OzAB **out, int K, int M1, int D, int sms, cudaStream_t s)
     if (e == cudaSuccess)
         e = cudaMalloc((void **) &st->fbits, sizeof(unsigned long long) * M1);
     if (e == cudaSuccess)
-        e = cudaMalloc((void **) &st->wbits, sizeof(unsigned long long) * (M1 + D));
+        e = cudaMalloc((void **) &st->wbits, sizeof(unsigned long long) * (M1 + D + 1));
     if (e == cudaSuccess)
         e = cudaMalloc((void **) &st->part, sizeof(int64_t) * TM * TN * (size_t) st->ntile * st->splits);
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **) &st->wide, sizeof(int));
     if (e == cudaSuccess)
         e = cudaMalloc((void **) &st->tiles, sizeof(int) * tiles.size());
     // on the stream of their readers; from pageable memory the call returns once the
@@ -591,26 +624,31 @@ int ozab_basis(OzAB *st, const double *FI, cudaStream_t s)
     oz_colmax_kernel<<<dim3(ceil_div(K, 128), ceil_div(M1, 32)), 256, 0, s>>>(src, K, M1, 128, st->fbits);
     DGTM_CUDA_TRY(cudaGetLastError());
     oz_slice_t_kernel<<<dim3(st->panels, ceil_div(M1, 32)), 256, 0, s>>>(src, K, M1, st->Mp, st->Kp,
-                                                                        st->fbits, st->Fp, nullptr);
+                                                                        st->fbits, st->Fp, nullptr, nullptr);
     DGTM_CUDA_TRY(cudaGetLastError());
     return DGTM_OK;
 }
 
-int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, double *A, double *B,
+int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, double *A, double *B, double *scratch,
               int *flag, int *nlaunch, cudaStream_t s)
 {
-    const int K = st->K, M1 = st->M1, D = st->D, W = M1 + D;
+    const int K = st->K, M1 = st->M1, D = st->D, W = M1 + D + 1;
     DGTM_CUDA_TRY(cudaMemsetAsync(st->wbits, 0, sizeof(unsigned long long) * W, s));
-    // diag(G) FI at rows 0 .. M1 of the planes, RT at rows Ap ..
+    // diag(G) FI at rows 0 .. M1 of the planes, RT at rows Ap ..; and G's own maximum
     const OzSource both{G, FI, RT, M1, M1, D};
     oz_colmax_kernel<<<dim3(ceil_div(K, 128), ceil_div(W, 32)), 256, 0, s>>>(both, K, W, 128, st->wbits);
     DGTM_CUDA_TRY(cudaGetLastError());
+    // every launch below looks at wide: the slices do nothing where it is set, the chain
+    // where it is not
+    ozab_wide_kernel<<<1, 256, 0, s>>>(st->fbits, st->wbits, M1, W - 1, st->wide);
+    DGTM_CUDA_TRY(cudaGetLastError());
     const OzSource left{G, FI, nullptr, M1, M1, 0}, right{nullptr, RT, nullptr, D, D, 0};
     oz_slice_t_kernel<<<dim3(st->panels, ceil_div(M1, 32)), 256, 0, s>>>(left, K, M1, st->Wp, st->Kp,
-                                                                        st->wbits, st->Wpl, nullptr);
+                                                                        st->wbits, st->Wpl, nullptr, st->wide);
     DGTM_CUDA_TRY(cudaGetLastError());
     oz_slice_t_kernel<<<dim3(st->panels, ceil_div(D, 32)), 256, 0, s>>>(
-        right, K, D, st->Wp, st->Kp, st->wbits + M1, st->Wpl + (size_t) st->Ap * st->Kp, nullptr);
+        right, K, D, st->Wp, st->Kp, st->wbits + M1, st->Wpl + (size_t) st->Ap * st->Kp, nullptr,
+        st->wide);
     DGTM_CUDA_TRY(cudaGetLastError());
     OzGemm g;
     g.A = st->Fp;
@@ -624,14 +662,17 @@ int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, dou
     g.ntile = st->ntile;
     g.out64 = st->part;
     g.item_panels = st->item_panels;
-    const int rc = launch_oz_gemm(g, st->sms, flag + 3, s);
+    g.skip = st->wide;
+    int rc = launch_oz_gemm(g, st->sms, flag + 3, s);
     if (rc != DGTM_OK)
         return rc;
     ozab_reduce_kernel<<<dim3(st->ntile, 32), 256, 0, s>>>(st->part, st->tiles, st->splits, oz_sum_ext(st->panels), M1, D, st->Ap,
-                                                          st->fbits, st->wbits, A, B, flag);
+                                                          st->fbits, st->wbits, A, B, flag, st->wide);
     DGTM_CUDA_TRY(cudaGetLastError());
+    if ((rc = launch_form_ab(FI, G, RT, K, M1, D, A, B, scratch, flag, s, st->wide)) != DGTM_OK)
+        return rc;
     if (nlaunch)
-        *nlaunch = 5;
+        *nlaunch = 8;
     return DGTM_OK;
 }
 

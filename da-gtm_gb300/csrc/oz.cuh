@@ -45,6 +45,7 @@ struct OzGemm {
     int mrows = 0, ncols = 0;
     const OzUnit *units = nullptr;
     const oz::Centre *cen = nullptr;
+    const int *skip = nullptr;  // device, may be null: nothing is done where it is set
 };
 
 int oz_sum_ext(int panels);
@@ -56,8 +57,10 @@ struct OzAB;
 int ozab_create(OzAB **out, int K, int M1, int D, int sms, cudaStream_t s);
 int ozab_basis(OzAB *st, const double *FI, cudaStream_t s);
 void ozab_destroy(OzAB *st);
-// flag: [0..2] set to 0 (as launch_form_ab does), [3] the bounded waits' status word
-int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, double *A, double *B,
+// flag: [0..2] set to 0 (as launch_form_ab does), [3] the bounded waits' status word.
+// scratch: form_ab_scratch_doubles, for the multiply-add chain that takes over where G
+// spans too much for the columns' grids
+int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, double *A, double *B, double *scratch,
               int *flag, int *nlaunch, cudaStream_t s);
 // whether the digit-slice product is the faster one at this size
 bool ozab_wanted(int K, int M1, int D);

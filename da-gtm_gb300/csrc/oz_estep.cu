@@ -884,7 +884,7 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     if (e == cudaSuccess && a.mstep) {
         e = cudaMemsetAsync(st->Tt, 0, planes * st->Wp * st->Npk, s);
         oz_slice_t_kernel<<<dim3(st->Npk / PANEL, ceil_div(D + 1, 32)), 256, 0, s>>>(
-            src, N, D + 1, st->Wp, st->Npk, st->bits, st->Tt, st->low);
+            src, N, D + 1, st->Wp, st->Npk, st->bits, st->Tt, st->low, nullptr);
         if (e == cudaSuccess)
             e = cudaGetLastError();
     }

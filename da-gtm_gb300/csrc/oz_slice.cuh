@@ -24,8 +24,8 @@ __device__ __forceinline__ void digit_pairs(int64_t a, int64_t b, uint32_t (&w)[
     }
 }
 
-// Column c of the source: c < c1: G[k] X1[k][c] (G may be null), else X2[k][c - c1]
-// (X2 null: 1).
+// Column c of the source: c < c1: G[k] X1[k][c] (G may be null), else X2[k][c - c1], then
+// G[k] (X2 null: 1).
 struct OzSource {
     const double *G, *X1, *X2;
     int c1, ld1, ld2;
@@ -35,7 +35,7 @@ struct OzSource {
             const double v = X1[(size_t) k * ld1 + c];
             return G ? G[k] * v : v;
         }
-        return X2 ? X2[(size_t) k * ld2 + (c - c1)] : 1.0;
+        return !X2 ? 1.0 : c - c1 < ld2 ? X2[(size_t) k * ld2 + (c - c1)] : G[k];
     }
 };
 
@@ -65,12 +65,15 @@ static __global__ void __launch_bounds__(256) oz_colmax_kernel(OzSource src, int
 // planes[i][c][k] = digit i of column c of the source on the column's grid:
 // the transposed operand (contraction over the source's rows), zero past rows
 // and cols.  low (may be null): low[c] += how many values of column c are short of bits on
-// its grid.  Block: 64 rows x 32 columns.
+// its grid.  skip (may be null): nothing is done where *skip is set.  Block: 64 rows x 32
+// columns.
 static __global__ void __launch_bounds__(256) oz_slice_t_kernel(OzSource src, int rows, int cols, int prows,
                                                          int ld, const unsigned long long *__restrict__ bits,
                                                          __nv_bfloat16 *__restrict__ planes,
-                                                         unsigned *__restrict__ low)
+                                                         unsigned *__restrict__ low, const int *__restrict__ skip)
 {
+    if (skip && *skip)
+        return;
     __shared__ int64_t qs[32][65];
     __shared__ unsigned few[8][32];
     const int k0 = blockIdx.x * 64, c0 = blockIdx.y * 32;
