@@ -807,12 +807,10 @@ TriKernel tri_solve_for(int nr)
 // warp costs 64 clocks each.  Therefore:
 //   * S and V stay in shared memory (in global memory beyond M1 = SVD_SMEM_MAX);
 //   * the angle is taken in FP32 (on the pivot elements' leading bits, scaled by
-//     their larger exponent) as tan(theta / 2) = h, and s = 2 h / (1 + h^2), c = 1 - h s in
-//     FP64: ten FP64 instructions.  A relative error of s leaves c^2 + s^2 = 1 within a
-//     third of it, so V stays as orthonormal as with angles taken in FP64 (against them,
-//     over 250 rounds at M1 = 26: 2e-15 and 7e-15 from I, and W's error the same; with
-//     c = 2 / (1 + h^2) - 1 W's error was 1.4 times theirs).  A pivot element is left at
-//     ~1e-7 of itself instead of at rounding, and the next sweep removes it;
+//     their larger exponent) as tan(theta / 2), and c = 2 r - 1, s = 2 tan r with
+//     r = 1 / (1 + tan^2) in FP64, so c^2 + s^2 = 1 to FP64: ten FP64 instructions.
+//     A pivot element is left at ~1e-7 of itself instead of at rounding, and the
+//     next sweep removes it;
 //   * the eigenvectors of a round are rotated by the other warps while the first
 //     ones take the next round's angles.
 // M1 = 26: 5.73 ms a solve with S and V in global memory and FP64 angles, 0.74 ms
@@ -902,8 +900,8 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_kernel(const double *__res
                         double ri = widen(__fdividef(1.0f, fmaf(hf, hf, 1.0f)));
                         ri = fma(ri, fma(-den, ri, 1.0), ri);
                         ri = fma(ri, fma(-den, ri, 1.0), ri);
+                        c = fma(2.0, ri, -1.0);
                         s = 2.0 * hd * ri;
-                        c = fma(-hd, s, 1.0);
                     }
                 }
                 pq[b][tid] = make_short2((short) p, (short) q);
