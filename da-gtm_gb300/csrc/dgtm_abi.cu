@@ -986,7 +986,9 @@ int dgtm_next_ctemp_k(dgtm_ctx *ctx, double temp, double beta, double eps, const
     double *scratch = nullptr, *dgg = nullptr, *dgsum = nullptr, *dout = nullptr;
     std::vector<double> out((size_t) 2 * K), gsum(K);
     // FP64 form: the scatter as digit-slice products, where the problem is large
-    // enough for its fixed costs (an explicit DGTM_CTEMP_SCRATCH_MB bounds it too)
+    // enough for its fixed costs (an explicit DGTM_CTEMP_SCRATCH_MB bounds it too): at
+    // the line a call takes 0.4 to 0.8 ms, by the CUDA-core scatter 3.8 ms (N = 1200,
+    // K = 30, D = 53) to 53 ms (N = 20000, K = 25, D = 15)
     OzE *slices = nullptr;
     if (ctx->precision == DGTM_FP64 && env_int("DGTM_CTEMP_PAIRS", 1, 0, 1) &&
         (double) N * K * D * D >= 1e8 && D >= 2)

@@ -176,7 +176,7 @@ __global__ void fe_dt_kernel(const float *__restrict__ T, const double *__restri
 
 // part[b] = the sum of squares of block b's share of x: sum_n |t_n|^2 needs no norm
 // per point, and no reduction across a warp per point.  Bound by the FP64 pipe: 16 us at
-// N = 65536, D = 64, where the norms took 46
+// N = 65536, D = 64, where the norms took 52
 __global__ void __launch_bounds__(256) fe_sumsq_kernel(const float *__restrict__ x, size_t n,
                                                        double *__restrict__ part)
 {

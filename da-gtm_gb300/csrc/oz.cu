@@ -422,7 +422,7 @@ int oz_item_panels(int ntile, int panels, int sms)
 int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
 {
     CUtensorMap tmA, tmB;
-    const uint64_t lda = (uint64_t) g.a_panels * PANEL, ldb = (uint64_t) g.b_panels * PANEL;
+    const uint64_t lda = (uint64_t) g.a_ld, ldb = (uint64_t) g.b_ld;
     int rc = make_tmap_bf16(&tmA, g.A, (uint64_t) g.sa * g.a_rows, lda, lda, TM, PANEL);
     if (rc == DGTM_OK)
         rc = make_tmap_bf16(&tmB, g.B, (uint64_t) SB * g.b_rows, ldb, ldb, TN, PANEL);
@@ -539,9 +539,10 @@ __global__ void __launch_bounds__(256) ozab_reduce_kernel(const int64_t *__restr
 
 }  // namespace
 
-// The slices' launches and gaps take about 70 us; the chain's multiply-adds run at
-// 0.63 TFMA/s: 32 us at the line and 250 at K = 8000, M1 = 65, D = 166 (8.2e7), where the
-// slices take 70.
+// Measured, the whole solve phase by slices against by the chain: 198 us against 215 at
+// K = 4000, M1 = 50, D = 75 and 196 against 260 at K = 8000, M1 = 50, D = 25 (2.0e7, the
+// line: below it the slices' six launches have little left to win), 398 against 582 at
+// K = 8000, M1 = 65, D = 166 (1.0e8).
 bool ozab_wanted(int K, int M1, int D)
 {
     return K <= (1 << 26) && (double) K * M1 * (0.5 * M1 + D) >= 2e7;
@@ -655,7 +656,8 @@ int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, dou
     g.B = st->Wpl;
     g.a_rows = st->Mp;
     g.b_rows = st->Wp;
-    g.panels = g.a_panels = g.b_panels = st->panels;
+    g.panels = st->panels;
+    g.a_ld = g.b_ld = st->Kp;
     g.mtiles = st->Mp / TM;
     g.ntiles = st->Wp / TN;
     g.tiles = st->tiles;

@@ -16,16 +16,17 @@ struct OzUnit {
 };
 
 // One product C[m][n] = sum_k A[m][k] B[n][k] over digit planes: A has sa planes
-// (8, or 1 for values that are small integers themselves) of a_rows x 64
-// a_panels BF16, B has 8 planes of b_rows x 64 b_panels; a_rows a multiple of
-// 128, b_rows of 64.  The contraction runs over `panels` panels of 64, from
-// panel 0 of A and panel b_panel0 of B.
+// (8, or 1 for values that are small integers themselves) of a_rows x a_ld BF16, B has
+// 8 planes of b_rows x b_ld; row lengths a multiple of 8.  The contraction runs over
+// `panels` panels of 64, from panel 0 of A and panel b_panel0 of B; columns past a row's
+// end count as zero.  Rows of a last tile past a_rows or b_rows are the next plane's:
+// what they give is finite and not read.
 struct OzGemm {
     const __nv_bfloat16 *A = nullptr, *B = nullptr;
     int sa = 8;
     int a_rows = 0, b_rows = 0;
     int panels = 0;        // 64-deep panels of the contraction
-    int a_panels = 0, b_panels = 0, b_panel0 = 0;
+    int a_ld = 0, b_ld = 0, b_panel0 = 0;
     int a_tile0 = 0;       // first 128-row tile of A
     int b_row0 = 0;        // first row of B (tiles of 64 from there)
     int mtiles = 0, ntiles = 0;

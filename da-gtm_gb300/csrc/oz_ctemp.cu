@@ -342,7 +342,8 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
                 g.B = U;
                 g.a_rows = rows;
                 g.b_rows = Fp;
-                g.panels = g.a_panels = g.b_panels = ldn / PANEL;
+                g.panels = ldn / PANEL;
+                g.a_ld = g.b_ld = ldn;
                 g.mtiles = rows / 128;
                 g.ntiles = ntiles;
                 g.out64 = part;

@@ -25,7 +25,7 @@
 //     altogether: their pass with these distances' d_ref would put R of the large point
 //     off by its |t|^2.
 //
-// Points go in chunks whose K x nn integers stay in L2 (8 M of them, 64 MB).
+// Points go in chunks whose K x nn integers stay in L2 (1e7 of them, 80 MB of 129).
 // Everything per chunk is a launch of its own: the distances cross L2 once more
 // than in a fused kernel (16 bytes a pair, against ~150 integer operations), and
 // one layout serves the statistics, the responsibilities and the map.
@@ -37,7 +37,6 @@
 #include <math.h>
 #include <new>
 #include <type_traits>
-#include <vector>
 
 namespace dgtm {
 
@@ -71,14 +70,18 @@ struct OzPoint {
 // planes[i][r][d] = digit i of X[r][d] on the grid of row r's largest value; zero past rows
 // and D.  fixed (instead of planes): [r][d] = X[r][d] as an integer below 2^61, ld of a row.
 // ex: the rows' exponents (may be null).  cen: the rows as centres, with xx = |x|^2, and
-// their sc (both may be null).  A warp a row, ld <= 256.
+// their sc (both may be null).  start: the two sc before their first use (may be null).  A
+// warp a row, ld <= 256.
 __global__ void __launch_bounds__(256) oz_slice_rows_kernel(const double *__restrict__ X, int rows, int D,
                                                             int prows, int ld,
                                                             __nv_bfloat16 *__restrict__ planes,
                                                             int64_t *__restrict__ fixed, int *__restrict__ ex,
                                                             const double *__restrict__ xx,
-                                                            oz::Centre *__restrict__ cen, OzScale *sc)
+                                                            oz::Centre *__restrict__ cen, OzScale *sc,
+                                                            OzScale *start)
 {
+    if (start && blockIdx.x == 0 && threadIdx.x < 2)
+        start[threadIdx.x] = OzScale{YMIN_START, 0};
     const int lane = threadIdx.x & 31;
     const size_t n2 = (size_t) prows * ld / 2;
     int ymin = YMIN_START, bad = 0;
@@ -722,10 +725,11 @@ struct OzE {
     OzEArgs a;
     unsigned char *arena = nullptr;  // every buffer below, one allocation
     int narrow = 0;  // depths of a row of 64-bit integers in Town and Yp, 0: digit planes
-    int sa = 8, panels = 0, Dp = 0, Np = 0, Kp = 0, chunk = 0, nchunks = 0;
+    int sa = 8, panels = 0, ldT = 0, ldY = 0, Np = 0, Kp = 0, chunk = 0, nchunks = 0;  // lds: of a row of planes
     const __nv_bfloat16 *Tp = nullptr;  // data planes (own or the caller's)
     __nv_bfloat16 *Town = nullptr, *Yp = nullptr;
-    unsigned long long *bits = nullptr;  // maxima of the columns of T, then ones
+    unsigned long long *bits = nullptr;  // maxima of the columns of T, then of the ones; then, 32 bits
+                                         // each, how many of their values are short of bits
     OzScale *sc = nullptr;   // [2], sc_now the one of the centres in Yp
     int sc_now = 0;
     int *ex = nullptr;       // the points' exponents
@@ -745,7 +749,6 @@ struct OzE {
     int *nmin = nullptr;
     unsigned *wmin = nullptr;
     unsigned *done = nullptr;  // statistics blocks finished in a call
-    unsigned *low = nullptr;   // values of each column of T (and of the ones) short of bits
 };
 
 // The digit-slice path has fixed costs (planes of the centres, four launches a
@@ -777,15 +780,17 @@ static const uint64_t *host_table()
     return t.v;
 }
 
-// Whether every column of T keeps its precision on one grid: at most a quarter of its
-// values are below 2^-6 of the grid's end and not exact there.  A value at that line
+// Whether every column of T (maxima, then counts of values short of bits) has squares
+// within FP64 and keeps its precision on one grid: at most a quarter of its values are
+// below 2^-6 of the grid's end and not exact there.  A value at that line
 // keeps 50 bits, the column's sums then 2^-51 of its bulk.  Gaussian and uniform
 // columns, and 0/1 and other coarse values, pass (a Gaussian column of 1e6 points: 20 %);
 // a column with one value 16 standard deviations out does not (38 %).
-static bool plain_columns(const std::vector<unsigned> &low, int N)
+static bool plain_columns(const unsigned long long *top, int D, int N)
 {
-    for (unsigned n : low)
-        if (4.0 * n > (double) N)
+    const unsigned *low = (const unsigned *) (top + D + 1);
+    for (int d = 0; d < D; d++)
+        if (top[d] >= oz::double_bits(0x1p500) || 4.0 * low[d] > (double) N)
             return false;
     return true;
 }
@@ -801,13 +806,18 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     st->a = a;
     const int N = a.N, D = a.D, K = a.K;
     st->sa = a.Tb ? 1 : 8;
-    st->Dp = a.Tb ? a.Tb_ld : rup(D, PANEL);
     st->narrow = a.Tb || D > NARROW ? 0 : D <= 2 ? 2 : D <= 4 ? 4 : 8;
-    st->panels = st->Dp / PANEL;
+    // rows of planes in whole panels, at few depths in whole 32 bytes (the product's panel is
+    // filled up with zeros on the way: a quarter of the memory at D = 9); or of 64-bit
+    // integers.  Rows of 16-byte multiples at D = 37 made a chunk's product 25 us longer.
+    st->ldY = st->narrow ? st->narrow : D <= PANEL / 2 ? rup(D, 16) : rup(D, PANEL);
+    st->ldT = a.Tb ? a.Tb_ld : st->ldY;
+    st->panels = ceil_div(D, PANEL);
     st->Np = a.Tb ? a.Tb_rows : rup(N, 128);
     st->Kp = rup(K, 64);
-    // points a chunk: whole waves of statistics blocks (8 points on each SM) where
-    // that many fit, in whole tiles of 128
+    // points a chunk: no more than whole waves of statistics blocks (8 points on each SM)
+    // where one fits, in whole tiles of 128 (which leave the last wave of an odd number of
+    // waves a little short: 1152 points for 1216 on 152 SMs)
     const long long wave = (long long) ST_PTS * a.sms;
     long long c = CHUNK / K;
     c = c >= wave ? c / wave * wave : c;
@@ -820,6 +830,7 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     st->Kp128 = rup(K, 128);
     st->Npk = rup(N, PANEL);
     const size_t planes = sizeof(__nv_bfloat16) * oz::DIGITS;
+    const size_t value = st->narrow ? sizeof(int64_t) : planes;  // bytes of one of T or Y
     const int cp = rup(st->chunk, PANEL) / PANEL;
     st->rt_tiles = (st->Kp128 / 128) * (st->Wp / 64);
     st->rt_per = oz_item_panels(st->rt_tiles, cp, a.sms);
@@ -832,9 +843,9 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     auto lay_out = [&](unsigned char *base) {
         bytes = 0;
         if (!a.Tb)
-            lay(&st->Town, planes * st->Np * st->Dp, base);
-        lay(&st->Yp, planes * st->Kp * st->Dp, base);
-        lay(&st->bits, sizeof(unsigned long long) * (D + 1), base);
+            lay(&st->Town, value * st->Np * st->ldT, base);
+        lay(&st->Yp, value * st->Kp * st->ldY, base);
+        lay(&st->bits, (sizeof(unsigned long long) + sizeof(unsigned)) * (D + 1), base);
         lay(&st->sc, 2 * sizeof(OzScale), base);
         lay(&st->ex, sizeof(int) * N, base);
         lay(&st->units, sizeof(OzUnit) * N, base);
@@ -845,9 +856,8 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         lay(&st->thr, sizeof(int64_t) * N, base);
         lay(&st->wmin, sizeof(unsigned) * K, base);
         lay(&st->done, sizeof(unsigned), base);
-        lay(&st->low, sizeof(unsigned) * (D + 1), base);
         if (a.mstep) {
-            lay(&st->Tt, planes * st->Wp * st->Npk, base);
+            lay(&st->Tt, planes * (D + 1) * st->Npk, base);
             lay(&st->Rp, planes * st->Kp128 * st->chunk, base);
             lay(&st->part, sizeof(int64_t) * 8192 * (size_t) st->rt_tiles * ceil_div(cp, st->rt_per), base);
             lay(&st->nmin, sizeof(int) * K, base);
@@ -859,18 +869,17 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         lay_out(st->arena);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(st->tab, host_table(), TAB_BYTES, cudaMemcpyHostToDevice, s);
+    const size_t nbits = (sizeof(unsigned long long) + sizeof(unsigned)) * (D + 1);
+    unsigned *low = (unsigned *) (st->bits + D + 1);
     if (e == cudaSuccess)
-        e = cudaMemsetAsync(st->bits, 0, sizeof(unsigned long long) * (D + 1), s);
+        e = cudaMemsetAsync(st->bits, 0, nbits, s);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(st->done, 0, sizeof(unsigned), s);
-    const OzScale start[2] = {{YMIN_START, 0}, {YMIN_START, 0}};
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(st->sc, start, sizeof(start), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         // of 0/1 data, which are in Tb, only the exponents are wanted: rows of no columns
         oz_slice_rows_kernel<<<grid_of((size_t) st->Np * 32, 16384), 256, 0, s>>>(
-            a.T64, N, D, a.Tb ? N : st->Np, a.Tb ? 0 : st->narrow ? st->narrow : st->Dp, st->Town,
-            st->narrow ? (int64_t *) st->Town : nullptr, st->ex, nullptr, nullptr, nullptr);
+            a.T64, N, D, a.Tb ? N : st->Np, a.Tb ? 0 : st->ldT, st->Town,
+            st->narrow ? (int64_t *) st->Town : nullptr, st->ex, nullptr, nullptr, nullptr, st->sc);
         e = cudaGetLastError();
         st->Tp = a.Tb ? a.Tb : st->Town;
     }
@@ -879,22 +888,15 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         oz_colmax_kernel<<<dim3(ceil_div(N, 512), ceil_div(D + 1, 32)), 256, 0, s>>>(src, N, D + 1, 512, st->bits);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(st->low, 0, sizeof(unsigned) * (D + 1), s);
     if (e == cudaSuccess && a.mstep) {
-        e = cudaMemsetAsync(st->Tt, 0, planes * st->Wp * st->Npk, s);
         oz_slice_t_kernel<<<dim3(st->Npk / PANEL, ceil_div(D + 1, 32)), 256, 0, s>>>(
-            src, N, D + 1, st->Wp, st->Npk, st->bits, st->Tt, st->low, nullptr);
+            src, N, D + 1, D + 1, st->Npk, st->bits, st->Tt, low, nullptr);
         if (e == cudaSuccess)
             e = cudaGetLastError();
     }
-    // a column's largest value (the squares of all are finite below 2^500)
-    std::vector<unsigned long long> top(D + 1);
-    std::vector<unsigned> low(D + 1);
+    unsigned long long cols[(4 * PANEL + 1) * 3 / 2 + 1];  // nbits, D <= 256 (oze_wanted)
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(low.data(), st->low, sizeof(unsigned) * (D + 1), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(top.data(), st->bits, sizeof(unsigned long long) * (D + 1), cudaMemcpyDeviceToHost, s);
+        e = cudaMemcpyAsync(cols, st->bits, nbits, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
@@ -906,10 +908,7 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
     }
     // the CUDA-core kernels carry data, or squares of it, that are not finite, and sums
     // that the grids would cost bits
-    bool fit = plain_columns(low, N);
-    for (int d = 0; d < D; d++)
-        fit = fit && top[d] < oz::double_bits(0x1p500);
-    if (!fit) {
+    if (!plain_columns(cols, D, N)) {
         oze_destroy(st);
         return DGTM_OK;
     }
@@ -931,8 +930,8 @@ int slice_centres(OzE *st, const double *Y, const double *yy, double c1, double 
     const int N = st->a.N, K = st->a.K, D = st->a.D;
     st->sc_now ^= 1;
     oz_slice_rows_kernel<<<grid_of((size_t) st->Kp * 32, 4864), 256, 0, s>>>(
-        Y, K, D, st->Kp, st->narrow ? st->narrow : st->Dp, st->Yp, st->narrow ? (int64_t *) st->Yp : nullptr,
-        nullptr, yy, st->cen, st->sc + st->sc_now);
+        Y, K, D, st->Kp, st->ldY, st->Yp, st->narrow ? (int64_t *) st->Yp : nullptr,
+        nullptr, yy, st->cen, st->sc + st->sc_now, nullptr);
     DGTM_CUDA_TRY(cudaGetLastError());
     oz_units_kernel<<<grid_of((size_t) N, 1216), 256, 0, s>>>(
         st->ex, st->a.tt, N, st->sc + st->sc_now, st->sc + (st->sc_now ^ 1), st->narrow ? 58 : st->sa == 1 ? 55 : 53,
@@ -967,7 +966,9 @@ int chunk_products(OzE *st, int c, cudaStream_t s)
     g.sa = st->sa;
     g.a_rows = st->Np;
     g.b_rows = st->Kp;
-    g.panels = g.a_panels = g.b_panels = st->panels;
+    g.panels = st->panels;
+    g.a_ld = st->ldT;
+    g.b_ld = st->ldY;
     const int n0 = c * st->chunk, nn = st->a.N - n0 < st->chunk ? st->a.N - n0 : st->chunk;
     g.a_tile0 = n0 / 128;
     g.mtiles = ceil_div(nn, 128);
@@ -1064,9 +1065,10 @@ int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaS
         g.A = st->Rp;
         g.B = st->Tt;
         g.a_rows = st->Kp128;
-        g.b_rows = st->Wp;
-        g.panels = g.a_panels = ldn / PANEL;
-        g.b_panels = st->Npk / PANEL;
+        g.b_rows = D + 1;
+        g.panels = ldn / PANEL;
+        g.a_ld = ldn;
+        g.b_ld = st->Npk;
         g.b_panel0 = n0 / PANEL;
         g.mtiles = st->Kp128 / 128;
         g.ntiles = st->Wp / 64;
@@ -1156,7 +1158,9 @@ int oze_r_block(OzE *st, const double *Y, const double *yy, const double2 *colst
     g.a_rows = st->Np;
     g.b_rows = st->Kp;
     g.b_row0 = k0;
-    g.panels = g.a_panels = g.b_panels = st->panels;
+    g.panels = st->panels;
+    g.a_ld = st->ldT;
+    g.b_ld = st->ldY;
     g.ntiles = ceil_div(nk, 64);
     g.out = st->acc;
     g.ncols = nk;

@@ -98,6 +98,8 @@ static __global__ void __launch_bounds__(256) oz_slice_t_kernel(OzSource src, in
     }
 #pragma unroll
     for (int cc = w; cc < 32; cc += 8) {
+        if (c0 + cc >= prows)
+            break;
         uint32_t v[oz::DIGITS];
         digit_pairs(qs[cc][2 * lane], qs[cc][2 * lane + 1], v);
         uint32_t *dst = (uint32_t *) (planes + (size_t) (c0 + cc) * ld + k0) + lane;

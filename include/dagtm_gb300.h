@@ -166,9 +166,10 @@ int dgtm_get_RD_block(dgtm_ctx *ctx, int k0, int nk, int n0, int nn, double *R, 
  * R and R^2 (split BF16) against the pair features (t_i t_j, t_i, 1), which
  * are exact in BF16, with DGTM_CTEMP_GEMM_MB (default 8192) of scratch;
  * DGTM_CTEMP_PAIRS=0 selects the CUDA-core scatter for those contexts too.
- * The FP64 form does the same at large sizes (N K D^2 at least 1e8) with FP64-accurate digit-slice products, in DGTM_CTEMP_GEMM_MB of
- * scratch, or in DGTM_CTEMP_SCRATCH_MB where that is set (the CUDA-core
- * scatter where not even 128 centres fit).
+ * The FP64 form does the same at large sizes (N K D^2 at least 1e8) with
+ * FP64-accurate digit-slice products, in DGTM_CTEMP_GEMM_MB of scratch, or in
+ * DGTM_CTEMP_SCRATCH_MB where that is set (the CUDA-core scatter where not
+ * even 128 centres fit, and for centres that would lose more than 8 bits).
  * Replaces dagtm_mpi_next_ctemp and its helper (comm/mpicomm.c:562-674) with
  * dagtm_vector_max (comm/comm.c:2149-2161), called at dagtm/dagtm.cxx:1919-1934.
  */
@@ -210,8 +211,11 @@ int dgtm_get_stream(dgtm_ctx *ctx, void **stream);
  * products from fixed-point digit slices of the centres on the tensor cores
  * (exact integers), exponentials and sums in double-float and 2^-48 fixed
  * point.  On other data they use digit slices of both operands and fixed-point
- * exponentials when N K is at least 32768 (D <= 256).  Setting
- * DGTM_X64=0 before dgtm_ctx_create keeps them on the CUDA-core FP64 kernels. */
+ * exponentials when N K is at least 32768 (D <= 256), unless a column of the
+ * data has values far above its others (more than a quarter of it below 2^-6
+ * of the power of two above its largest value, and not whole multiples of
+ * 2^-55 of that): those stay on the CUDA cores.  Setting DGTM_X64=0 before
+ * dgtm_ctx_create keeps all of them on the CUDA-core FP64 kernels. */
 #define DGTM_PATH_CUDA_CORES 0
 #define DGTM_PATH_SPLIT_BF16 1
 #define DGTM_PATH_EXACT_SLICES 2

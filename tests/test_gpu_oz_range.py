@@ -255,3 +255,20 @@ def test_normal_equations_where_the_weights_span_decades(pkg, monkeypatch, decad
             assert 0.5 * decades < np.log10(G.max() / G.min()) < 1.6 * decades
         err.append(float(np.max(np.abs(Yn - long_double_solve(FI, G, RT)))))
     assert err[0] <= 4.0 * err[1]
+
+
+@pytest.mark.parametrize("D,limit", [(5, 400), (9, 800), (37, 2200)])
+def test_memory_of_a_context_per_point(pkg, D, limit):
+    """Digit planes take what D needs (16 bytes of a value rounded up to 8, twice), not
+    whole panels of 64: bytes a point, from contexts of two sizes."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(1)
+    T = rng.random((2_000_000, D))
+    used = []
+    for N in (1_000_000, 2_000_000):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        with pkg.Context(T[:N], np.ones((64, 1)), "fp64") as c:
+            assert c.path == "exact_slices"
+            used.append(before - torch.cuda.mem_get_info()[0])
+    assert (used[1] - used[0]) / 1e6 <= limit
