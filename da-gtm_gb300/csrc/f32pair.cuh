@@ -19,6 +19,7 @@ namespace dgtm {
 
 #if defined(__CUDA_ARCH__)
 F32_HD float rn_add(float a, float b) { return __fadd_rn(a, b); }
+F32_HD float rn_sub(float a, float b) { return __fsub_rn(a, b); }
 F32_HD float rn_mul(float a, float b) { return __fmul_rn(a, b); }
 F32_HD float rn_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 F32_HD uint32_t float_bits(float f) { return __float_as_uint(f); }
@@ -26,6 +27,7 @@ F32_HD double double_of(uint32_t hi, uint32_t lo) { return __hiloint2double((int
 #else
 // compiled without contraction
 F32_HD float rn_add(float a, float b) { return a + b; }
+F32_HD float rn_sub(float a, float b) { return a - b; }
 F32_HD float rn_mul(float a, float b) { return a * b; }
 F32_HD float rn_fma(float a, float b, float c) { return fmaf(a, b, c); }
 F32_HD uint32_t float_bits(float f)
@@ -60,8 +62,8 @@ F32_HD Pair split(double v)
 F32_HD void two_sum(float a, float b, float &s, float &e)
 {
     s = rn_add(a, b);
-    const float t = rn_add(s, -a);
-    e = rn_add(rn_add(a, -rn_add(s, -t)), rn_add(b, -t));
+    const float t = rn_sub(s, a);
+    e = rn_add(rn_sub(a, rn_sub(s, t)), rn_sub(b, t));
 }
 
 // h + l rounded to FP32; ok is cleared when it is not safely away from a rounding
@@ -71,7 +73,7 @@ F32_HD void two_sum(float a, float b, float &s, float &e)
 F32_HD float settle(float h, float l, bool &ok)
 {
     const float r = rn_add(h, l);
-    const float e = rn_add(l, -rn_add(r, -h));
+    const float e = rn_sub(l, rn_sub(r, h));
     ok = ok && rn_add(r, rn_mul(e, 1.f + 0x1p-16f)) == r;
     return r;
 }
