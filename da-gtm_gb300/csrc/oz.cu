@@ -15,8 +15,8 @@
 // integer whatever the order.  Levels 0 .. 7 are kept (36 of the 64 digit
 // products); what is dropped is below 2^-58 of the operands' largest products
 // per term, under the rounding of an FP64 multiply-add chain.  The levels are
-// combined in 64-bit integers every 512 elements; FP64 comes back only once per
-// result.
+// combined in 96-bit integers every 512 elements; FP64 comes back only once per
+// item of a sum.
 //
 // oz_gemm_kernel: persistent, one CTA per SM (TMEM: 8 levels x 64 columns = all
 // 512).  Tile 128 (A rows, TMEM lanes) x 64 (B rows).  Per 64-deep panel the
@@ -62,8 +62,7 @@ constexpr size_t OZ_SMEM = 1024 + 2 * (size_t) B_BUF + A_SLOTS * (size_t) A_SLOT
 struct OzParams {
     int panels, b_panel0, a_rows, b_rows, a_tile0, b_row0, mtiles, ntiles, nitems, splits, item_panels;
     const int *tiles;
-    int64_t *out64;
-    int ext;
+    double *sums;
     int64_t *out;
     size_t ldm;
     int mrows, ncols;
@@ -255,18 +254,20 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
         const int q = warp & 3, h = (warp - 2) >> 2;  // lane quarter, 16 of the columns
         const uint32_t lane_base = tmem + ((uint32_t) (q * 32) << 16) + (uint32_t) (16 * h);
         const int row = q * 32 + lane;
-        const int shift = 8 + p.ext;  // sums
-        const int64_t half = 1ll << (shift - 1);
         int nseg = 0;
         bool ok = true;
         for (int it = blockIdx.x; ok && it < p.nitems; it += gridDim.x) {
             int mt, nt, p0, p1;
             oz_item(p, it, mt, nt, p0, p1);
-            int64_t acc[SUM ? 16 : 1];
+            // sums over all segments of an item: exact, in 96 bits (rounded once at its end;
+            // a unit that a whole contraction of full terms fits is too coarse for a centre
+            // whose R lies on few points: 2^-49 of the grids at 5000 points put critical
+            // temperatures 1e-12 off)
+            oz::Sum96 acc[SUM ? 16 : 1];
             if constexpr (SUM) {
 #pragma unroll
                 for (int c = 0; c < 16; c++)
-                    acc[c] = 0;
+                    acc[c] = oz::Sum96{0, 0, 0};
             }
             // Distances: this warp's centres by way of shared memory, |y|^2 / 2 on one
             // exponent (half_square).  Where that serves all 32 points (near_group: hardly
@@ -327,8 +328,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
                         for (int c = 0; c < 4; c++) {
                             int64_t hi, lo;
                             level_pairs<NARROW>(v + c, hi, lo);
-                            // hi 2^28 + lo may need 72 bits: both are shifted down by >= 8
-                            acc[4 * cb + c] += hi * (1 << (28 - shift)) + ((lo + half) >> shift);
+                            oz::add96(acc[4 * cb + c], hi, lo);
                         }
                     }
                 } else if (near) {
@@ -363,10 +363,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
             }
             if constexpr (SUM) {
                 if (ok) {
-                    int64_t *dst = p.out64 + (size_t) it * (TM * TN) + (size_t) (16 * h) * TM + row;
+                    double *dst = p.sums + (size_t) it * (TM * TN) + (size_t) (16 * h) * TM + row;
 #pragma unroll
                     for (int c = 0; c < 16; c++)
-                        dst[(size_t) c * TM] = acc[c];
+                        dst[(size_t) c * TM] = oz::to_double96(acc[c]);
                 }
             }
         }
@@ -388,17 +388,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const __grid_con
 __host__ __device__ constexpr int rup(int a, int b) { return (a + b - 1) / b * b; }
 
 }  // namespace
-
-// One term is below 2^53 units of 2^-53: 512 terms fit 62 bits, longer
-// contractions drop one bit per doubling (of the sum's magnitude, which grows
-// alike: the unit stays below the FP64 rounding of a sum of that many terms).
-int oz_sum_ext(int panels)
-{
-    int ext = 0;
-    while ((512ll << ext) < (long long) panels * PANEL)
-        ext++;
-    return ext;
-}
 
 // Splits of the contraction: whole panels an item, the count that gives the
 // shortest schedule of equal items on `sms` CTAs (36 x 128 clocks of MMA a panel,
@@ -437,12 +426,11 @@ int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
     p.b_row0 = g.b_row0;
     p.mtiles = g.mtiles;
     p.ntiles = g.ntiles;
-    p.item_panels = g.out64 ? g.item_panels : g.panels;
+    p.item_panels = g.sums ? g.item_panels : g.panels;
     p.splits = ceil_div(g.panels, p.item_panels);
     p.nitems = (g.tiles ? g.ntile : g.mtiles * g.ntiles) * p.splits;
     p.tiles = g.tiles;
-    p.out64 = g.out64;
-    p.ext = oz_sum_ext(g.panels);
+    p.sums = g.sums;
     p.out = g.out;
     p.ldm = g.ldm;
     p.mrows = g.mrows;
@@ -453,7 +441,7 @@ int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s)
     p.status = status;
     using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const OzParams);
     // |S_l| <= (l + 1) 64 panels 4096: at most 2^22 for two panels, and for 0/1 data
-    const Kernel k = g.out64      ? (Kernel) oz_gemm_kernel<8, true, false>
+    const Kernel k = g.sums       ? (Kernel) oz_gemm_kernel<8, true, false>
                      : g.sa == 1  ? (Kernel) oz_gemm_kernel<1, false, true>
                      : g.panels <= 2 ? (Kernel) oz_gemm_kernel<8, false, true>
                                      : (Kernel) oz_gemm_kernel<8, false, false>;
@@ -472,7 +460,7 @@ struct OzAB {
     int ntile = 0, splits = 0, item_panels = 0;
     __nv_bfloat16 *Fp = nullptr, *Wpl = nullptr;
     unsigned long long *fbits = nullptr, *wbits = nullptr;
-    int64_t *part = nullptr;
+    double *part = nullptr;
     int *tiles = nullptr;
     int *wide = nullptr;  // G spans too much for the columns' grids: form_ab's chain does it
 };
@@ -500,11 +488,10 @@ __global__ void __launch_bounds__(256) ozab_wide_kernel(const unsigned long long
         *wide = w;
 }
 
-// A and B from the tiles' split sums (exact integers); a column with a
-// non-finite value gives NaN.
-__global__ void __launch_bounds__(256) ozab_reduce_kernel(const int64_t *__restrict__ part,
+// A and B from the tiles' split sums; a column with a non-finite value gives NaN.
+__global__ void __launch_bounds__(256) ozab_reduce_kernel(const double *__restrict__ part,
                                                           const int *__restrict__ tiles, int splits,
-                                                          int ext, int M1, int D, int Ap,
+                                                          int M1, int D, int Ap,
                                                           const unsigned long long *__restrict__ fbits,
                                                           const unsigned long long *__restrict__ wbits,
                                                           double *__restrict__ A, double *__restrict__ B,
@@ -521,11 +508,11 @@ __global__ void __launch_bounds__(256) ozab_reduce_kernel(const int64_t *__restr
         const int j = isA ? c : c - Ap;
         if (m >= M1 || (isA ? (j >= M1 || j < m) : j >= D))
             continue;
-        int64_t sum = 0;
+        double sum = 0.0;
         for (int sp = 0; sp < splits; sp++)
             sum += part[((size_t) t * splits + sp) * (TM * TN) + e];
         const unsigned long long fb = fbits[m], wb = wbits[isA ? j : M1 + j];
-        double r = scalbn((double) sum, oz::exponent_of(fb) + oz::exponent_of(wb) - 53 + ext);
+        double r = scalbn(sum, oz::exponent_of(fb) + oz::exponent_of(wb) - OZ_SUM_BITS);
         if (fb >= oz::INF_BITS || wb >= oz::INF_BITS)
             r = NAN;
         if (isA) {
@@ -594,7 +581,7 @@ int ozab_create(OzAB **out, int K, int M1, int D, int sms, cudaStream_t s)
     if (e == cudaSuccess)
         e = cudaMalloc((void **) &st->wbits, sizeof(unsigned long long) * (M1 + D + 1));
     if (e == cudaSuccess)
-        e = cudaMalloc((void **) &st->part, sizeof(int64_t) * TM * TN * (size_t) st->ntile * st->splits);
+        e = cudaMalloc((void **) &st->part, sizeof(double) * TM * TN * (size_t) st->ntile * st->splits);
     if (e == cudaSuccess)
         e = cudaMalloc((void **) &st->wide, sizeof(int));
     if (e == cudaSuccess)
@@ -662,13 +649,13 @@ int ozab_form(OzAB *st, const double *FI, const double *G, const double *RT, dou
     g.ntiles = st->Wp / TN;
     g.tiles = st->tiles;
     g.ntile = st->ntile;
-    g.out64 = st->part;
+    g.sums = st->part;
     g.item_panels = st->item_panels;
     g.skip = st->wide;
     int rc = launch_oz_gemm(g, st->sms, flag + 3, s);
     if (rc != DGTM_OK)
         return rc;
-    ozab_reduce_kernel<<<dim3(st->ntile, 32), 256, 0, s>>>(st->part, st->tiles, st->splits, oz_sum_ext(st->panels), M1, D, st->Ap,
+    ozab_reduce_kernel<<<dim3(st->ntile, 32), 256, 0, s>>>(st->part, st->tiles, st->splits, M1, D, st->Ap,
                                                           st->fbits, st->wbits, A, B, flag, st->wide);
     DGTM_CUDA_TRY(cudaGetLastError());
     if ((rc = launch_form_ab(FI, G, RT, K, M1, D, A, B, scratch, flag, s, st->wide)) != DGTM_OK)

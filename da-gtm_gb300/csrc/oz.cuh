@@ -32,13 +32,12 @@ struct OzGemm {
     int mtiles = 0, ntiles = 0;
     const int *tiles = nullptr;  // (mt << 16 | nt) of each tile, or null: all mtiles x ntiles
     int ntile = 0;               // entries of tiles
-    // sums (out64 != null): an item is one tile over `item_panels` panels; it leaves
-    // 64 x 128 integers (column, row) in units of 2^(-53 + oz_sum_ext(panels)) of
-    // the operands' 2^e at out64 + item 8192, item = tile * splits + split; the
-    // integers of all splits can be added
-    int64_t *out64 = nullptr;
+    // sums (not null): an item is one tile over `item_panels` panels; it leaves 64 x 128
+    // doubles (column, row), each an exact sum rounded once, in units of 2^-OZ_SUM_BITS of
+    // the operands' 2^e, at sums + item 8192, item = tile * splits + split
+    double *sums = nullptr;
     int item_panels = 0;
-    // distances (out64 == null, panels <= 4): out[n ldm + m] = oz::level of the sum, which
+    // distances (sums == null, panels <= 4): out[n ldm + m] = oz::level of the sum, which
     // is in units of 2^-53 (sa = 8) or 2^-55 (sa = 1) of the operands' 2^e, for m < mrows,
     // n < ncols; units of A's rows from a_tile0, centres of B's rows from b_row0
     int64_t *out = nullptr;
@@ -49,7 +48,7 @@ struct OzGemm {
     const int *skip = nullptr;  // device, may be null: nothing is done where it is set
 };
 
-int oz_sum_ext(int panels);
+constexpr int OZ_SUM_BITS = 61;
 int oz_item_panels(int ntile, int panels, int sms);
 int launch_oz_gemm(const OzGemm &g, int sms, int *status, cudaStream_t s);
 
@@ -94,8 +93,8 @@ int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaS
 // c the exponents' factor);
 // oze_chunks: how many chunks, and their points; oze_r_digits: R (or R^2) of the
 // centres k0 .. k0 + kb over a chunk as eight planes of prows x (points rounded
-// up to 64), and the integer exponents of their grids: an integer sum of the
-// product with B counts 2^(5 - nmin[k]) of B's grid (oz_sum_ext).  products: form
+// up to 64), and the integer exponents of their grids: a sum of the
+// product with B counts 2^(5 - nmin[k]) of B's grid.  products: form
 // the chunk's distances first (they stay until the next chunk's).
 int oze_refer(OzE *st, const double *Y, const double *yy, const double2 *colstat, double c1, double c, double dcut,
               cudaStream_t s);

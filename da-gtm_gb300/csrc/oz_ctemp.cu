@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256) features_kernel(const double *__restrict_
 }
 
 // P[f][row] (+)= the product's sums, rows = R then R^2
-__global__ void __launch_bounds__(256) sums_kernel(const int64_t *__restrict__ part, int ntiles, int splits, int ext,
+__global__ void __launch_bounds__(256) sums_kernel(const double *__restrict__ part, int ntiles, int splits,
                                                    const int *__restrict__ nmin, int rows, int F,
                                                    const Feature *__restrict__ ftab, int first,
                                                    double *__restrict__ P)
@@ -192,11 +192,11 @@ __global__ void __launch_bounds__(256) sums_kernel(const int64_t *__restrict__ p
         const int r = mt * 128 + (e & 127), f = nt * 64 + (e >> 7);
         if (f >= F)
             continue;
-        int64_t sum = 0;
+        double sum = 0.0;
         for (int sp = 0; sp < splits; sp++)
             sum += part[((size_t) t * splits + sp) * (128 * 64) + e];
         const int nm = nmin[r];
-        const double v = nm >= 0 && nm < 2047 ? scalbn((double) sum, 5 - nm + ftab[f].e - 53 + ext) : 0.0;
+        const double v = nm >= 0 && nm < 2047 ? scalbn(sum, 5 - nm + ftab[f].e - OZ_SUM_BITS) : 0.0;
         double *dst = P + (size_t) f * rows + r;
         *dst = first ? v : *dst + v;
     }
@@ -284,7 +284,7 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
         per = oz_item_panels(2 * (kpad / 128) * ntiles, cpanels, sms);
         splits = ceil_div(cpanels, per);
         need = fixed + align_up(sizeof(__nv_bfloat16) * oz::DIGITS * 2 * (size_t) kpad * cpanels * PANEL) +
-               align_up(sizeof(int64_t) * 2 * (size_t) kpad * Fp * splits) +
+               align_up(sizeof(double) * 2 * (size_t) kpad * Fp * splits) +
                align_up(sizeof(double) * 2 * (size_t) kpad * F) +
                (pl.eig_in_smem ? 1 : 2) * align_up(sizeof(double) * (size_t) kpad * 2 * D * D) +
                align_up(sizeof(int) * 2 * kpad);
@@ -310,7 +310,7 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
     Feature *ftab = (Feature *) take(sizeof(Feature) * Fp);
     const int rows = 2 * kpad;
     __nv_bfloat16 *R = (__nv_bfloat16 *) take(sizeof(__nv_bfloat16) * oz::DIGITS * (size_t) rows * cpanels * PANEL);
-    int64_t *part = (int64_t *) take(sizeof(int64_t) * (size_t) rows * Fp * splits);
+    double *part = (double *) take(sizeof(double) * (size_t) rows * Fp * splits);
     double *P = (double *) take(sizeof(double) * (size_t) rows * F);
     double *S = (double *) take(sizeof(double) * (size_t) kpad * 2 * D * D);
     double *Mg = pl.eig_in_smem ? nullptr : (double *) take(sizeof(double) * (size_t) kpad * 2 * D * D);
@@ -346,11 +346,11 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
                 g.a_ld = g.b_ld = ldn;
                 g.mtiles = rows / 128;
                 g.ntiles = ntiles;
-                g.out64 = part;
+                g.sums = part;
                 g.item_panels = per;
                 OZ_TRY(launch_oz_gemm(g, sms, status, s));
                 sums_kernel<<<dim3(g.mtiles * ntiles, 8), 256, 0, s>>>(part, ntiles, ceil_div(g.panels, per),
-                                                                       oz_sum_ext(g.panels), nmin, rows, F, ftab, ch == 0 ? 1 : 0, P);
+                                                                       nmin, rows, F, ftab, ch == 0 ? 1 : 0, P);
                 DGTM_CUDA_TRY(cudaGetLastError());
             }
             assemble_kernel<<<kb, 256, asmem, s>>>(P, rows, kpad, D, ftab, Y + (size_t) k0 * D, mean, zbits, S, gsum_dev + k0,

@@ -19,7 +19,7 @@
 //   G and R T.  R_kn on its centre's power-of-two grid (the chunk's largest
 //     R of the centre within [2^-56, 1] of it: small responsibilities keep their
 //     relative precision), in eight digit planes, times the digit planes of
-//     T^T and a row of ones: 64-bit integer sums per chunk, FP64 across chunks.  The
+//     T^T and a row of ones: exact sums over the splits of a chunk, FP64 across them.  The
 //     points are what is summed over, so T^T has a grid per column; data with a column
 //     whose largest value is far above its others (plain_columns) stay on the CUDA cores
 //     altogether: their pass with these distances' d_ref would put R of the large point
@@ -608,8 +608,8 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const int64_t *__restric
 
 // G and R T of a chunk from the products' split sums; the first chunk sets, the
 // others add.  Column D of the product is the row of ones: G.
-__global__ void __launch_bounds__(256) oz_rt_kernel(const int64_t *__restrict__ part, int ntiles, int splits,
-                                                    int ext, const int *__restrict__ nmin,
+__global__ void __launch_bounds__(256) oz_rt_kernel(const double *__restrict__ part, int ntiles, int splits,
+                                                    const int *__restrict__ nmin,
                                                     const unsigned long long *__restrict__ cbits, int K, int D,
                                                     int first, double *__restrict__ G, double *__restrict__ RT)
 {
@@ -618,11 +618,11 @@ __global__ void __launch_bounds__(256) oz_rt_kernel(const int64_t *__restrict__ 
         const int k = mt * 128 + (e & 127), d = nt * 64 + (e >> 7);
         if (k >= K || d > D)
             continue;
-        int64_t sum = 0;
+        double sum = 0.0;
         for (int sp = 0; sp < splits; sp++)
             sum += part[((size_t) t * splits + sp) * (128 * 64) + e];
         const int nm = nmin[k];
-        const double v = nm < 2047 ? scalbn((double) sum, 5 - nm + oz::exponent_of(cbits[d]) - 53 + ext) : 0.0;
+        const double v = nm < 2047 ? scalbn(sum, 5 - nm + oz::exponent_of(cbits[d]) - OZ_SUM_BITS) : 0.0;
         double *dst = d < D ? RT + (size_t) k * D + d : G + k;
         *dst = first ? v : *dst + v;
     }
@@ -745,7 +745,7 @@ struct OzE {
     // responsibility pass
     int Wp = 0, Kp128 = 0, Npk = 0, rt_tiles = 0, rt_per = 0;
     __nv_bfloat16 *Tt = nullptr, *Rp = nullptr;
-    int64_t *part = nullptr;
+    double *part = nullptr;
     int *nmin = nullptr;
     unsigned *wmin = nullptr;
     unsigned *done = nullptr;  // statistics blocks finished in a call
@@ -859,7 +859,7 @@ int oze_create(OzE **out, const OzEArgs &a, cudaStream_t s)
         if (a.mstep) {
             lay(&st->Tt, planes * (D + 1) * st->Npk, base);
             lay(&st->Rp, planes * st->Kp128 * st->chunk, base);
-            lay(&st->part, sizeof(int64_t) * 8192 * (size_t) st->rt_tiles * ceil_div(cp, st->rt_per), base);
+            lay(&st->part, sizeof(double) * 8192 * (size_t) st->rt_tiles * ceil_div(cp, st->rt_per), base);
             lay(&st->nmin, sizeof(int) * K, base);
         }
     };
@@ -1072,11 +1072,11 @@ int oze_mstep_pass(OzE *st, double c, double *G, double *RT, int *nlaunch, cudaS
         g.b_panel0 = n0 / PANEL;
         g.mtiles = st->Kp128 / 128;
         g.ntiles = st->Wp / 64;
-        g.out64 = st->part;
+        g.sums = st->part;
         g.item_panels = st->rt_per;
         OZ_TRY(launch_oz_gemm(g, st->a.sms, st->a.status, s));
         oz_rt_kernel<<<dim3(st->rt_tiles, 32), 256, 0, s>>>(st->part, g.ntiles, ceil_div(g.panels, st->rt_per),
-                                                            oz_sum_ext(g.panels), st->nmin, st->bits, K, D,
+                                                            st->nmin, st->bits, K, D,
                                                             ch == 0 ? 1 : 0, G, RT);
         DGTM_CUDA_TRY(cudaGetLastError());
         nl += 4;

@@ -336,6 +336,59 @@ OZ_HD int64_t level(int64_t I, const Centre &c, int p, int u)
     return s >= 10 ? FAR : shifted(I, p + c.f - u) - shifted(c.yy, s);
 }
 
+// A signed 96-bit sum, as three words.
+struct Sum96 {
+    uint32_t w0, w1, w2;
+};
+
+// s += hi 2^28 + lo
+OZ_HD void add96(Sum96 &s, int64_t hi, int64_t lo)
+{
+    const uint32_t a0 = (uint32_t) ((uint64_t) hi << 28), a1 = (uint32_t) (hi >> 4), a2 = (uint32_t) (hi >> 36);
+    const uint32_t b0 = (uint32_t) lo, b1 = (uint32_t) ((uint64_t) lo >> 32), b2 = (uint32_t) (lo >> 63);
+#if defined(__CUDA_ARCH__)
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+        : "+r"(s.w0), "+r"(s.w1), "+r"(s.w2) : "r"(a0), "r"(a1), "r"(a2));
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+        : "+r"(s.w0), "+r"(s.w1), "+r"(s.w2) : "r"(b0), "r"(b1), "r"(b2));
+#else
+    uint64_t c = (uint64_t) s.w0 + a0 + b0;
+    s.w0 = (uint32_t) c;
+    c = (uint64_t) s.w1 + a1 + b1 + (c >> 32);
+    s.w1 = (uint32_t) c;
+    s.w2 += a2 + b2 + (uint32_t) (c >> 32);
+#endif
+}
+
+OZ_HD int clz64(uint64_t x)
+{
+#if defined(__CUDA_ARCH__)
+    return __clzll((long long) x);
+#else
+    return x ? __builtin_clzll(x) : 64;
+#endif
+}
+
+// the sum as a double, rounded once; integer operations only
+OZ_HD double to_double96(const Sum96 &s)
+{
+    const bool neg = (s.w2 >> 31) != 0;
+    uint64_t lo = ((uint64_t) s.w1 << 32) | s.w0, top = s.w2;  // |s| = top 2^64 + lo
+    if (neg) {
+        lo = ~lo + 1;
+        top = (uint32_t) ~s.w2 + (lo == 0 ? 1u : 0u);
+    }
+    const uint64_t up = (top << 32) | (lo >> 32);              // the upper 64 of 96 bits
+    // T 2^e, T's top bit set; what T does not hold is below 2^-63 of it
+    const int n = up >> 31 ? clz64(up) : 64;
+    const uint64_t T = n < 64 ? (n < 32 ? (up << n) | (n ? (uint32_t) lo >> (32 - n) : 0u) : lo << (n - 32)) : shl(lo, clz64(lo));
+    if (T == 0)
+        return 0.0;
+    const int e = n < 64 ? 95 - n : 63 - clz64(lo);
+    const uint64_t m = ((T << 1) >> 12) + ((T >> 10) & 1);      // 52 fraction bits (may carry)
+    return bits_double(((uint64_t) neg << 63) | ((((uint64_t) (e + 1023)) << 52) + m));
+}
+
 // an unsigned fixed-point value in units of 2^-53 from a double (v >= 0)
 OZ_HD uint64_t to_wfix(double v) { return (uint64_t) scaled_int(v, WFRAC); }
 

@@ -272,3 +272,25 @@ def test_memory_of_a_context_per_point(pkg, D, limit):
             assert c.path == "exact_slices"
             used.append(before - torch.cuda.mem_get_info()[0])
     assert (used[1] - used[0]) / 1e6 <= limit
+
+
+def test_sums_that_few_points_carry(pkg):
+    """Centres of 5000 points whose G lies on a few points each: a unit that 5000 full
+    terms would need is 2^-49 of the grids (1e-14 of G here); the sums' own rounding is
+    2^-53."""
+    rng = np.random.default_rng(15)
+    N, D, K = 5000, 9, 1000
+    T = rng.random((N, D)) + 0.5
+    Y = np.full((K, D), 40.0)  # far from all, but
+    Y[:N // 50] = T[:N // 50]  # on the first points
+    with pkg.Context(T, np.ones((K, 1)), "fp64") as c:
+        assert c.path == "exact_slices"
+        c.set_Y(Y)
+        c.estep(4000.0, 1, 1.0)
+        R = c.R_block(0, N // 50, 0, N)
+        c.mstep()
+        G, _ = c.get_stats()
+    g = R.sum(1, dtype=np.longdouble)
+    # 2^-53 each from the block's R and from G's rounding, and half a unit of R's digits
+    # (2^-55 of a grid that ends below 4.2 Rmax) from each of a few points
+    assert np.max(np.abs(G[:N // 50] / g - 1.0)) <= 2.0 ** -51

@@ -45,3 +45,14 @@ def test_units_of_the_distances(tmp_path):
                                       check=True).stdout.split()
     assert float(worst) <= 1.0
     assert int(far) == 0 and int(over) == 0
+
+
+def test_exact_sums(tmp_path):
+    """96-bit sums and their doubles (tests/oz_sum_check.cc) against 128-bit integers: the
+    sums equal, the doubles within half a unit in the last place."""
+    exe = str(tmp_path / "oz_sum_check")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-o", exe,
+                           os.path.join(ROOT, "tests", "oz_sum_check.cc"), "-lm"])
+    wrong, worst = subprocess.run([exe], capture_output=True, text=True, timeout=300,
+                                  check=True).stdout.split()
+    assert int(wrong) == 0 and float(worst) <= 1.0
