@@ -12,11 +12,12 @@
 // and so has each centre's R.
 //
 // The expansion cancels where a centre's points lie close together and far from
-// the mean: tr P / tr S1 says by how much (a few units on spread-out data).  And a
-// feature's grid is that of its largest value over all points, 2^-56 of which every point
-// may be off: against tr S1 that is g sum_d max z_d^2 / tr S1 (a value far from the others
-// makes it large).  The caller redoes the centres for which either loses more than 8 bits
-// of 2^-53 with the CUDA-core scatter.
+// the mean: tr P / tr S1 says by how much (a few units on spread-out data).  And every
+// point leaves what the digit products below level 7 would add, about 2^-56 of the grids of
+// the centre's R and of the feature, whatever its own R and z: sqrt(N) of that in a sum
+// (on few points in grids far above theirs it is much: N = 5001, D = 5, centres on a few
+// dozen points: 2e-13 of a critical temperature).  The caller redoes the centres for which
+// either is more than 8 bits of 2^-53 of tr S1 with the CUDA-core scatter.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "oz.cuh"
@@ -181,11 +182,12 @@ __global__ void __launch_bounds__(256) features_kernel(const double *__restrict_
     }
 }
 
-// P[f][row] (+)= the product's sums, rows = R then R^2
+// P[f][row] (+)= the product's sums, rows = R then R^2; noise[row] (+)= sqrt(points) times
+// the grid of the row's R
 __global__ void __launch_bounds__(256) sums_kernel(const double *__restrict__ part, int ntiles, int splits,
                                                    const int *__restrict__ nmin, int rows, int F,
-                                                   const Feature *__restrict__ ftab, int first,
-                                                   double *__restrict__ P)
+                                                   const Feature *__restrict__ ftab, int first, double rootn,
+                                                   double *__restrict__ P, double *__restrict__ noise)
 {
     const int t = blockIdx.x, mt = t / ntiles, nt = t - mt * ntiles;
     for (int e = blockIdx.y * 256 + threadIdx.x; e < 128 * 64; e += 256 * gridDim.y) {
@@ -199,6 +201,10 @@ __global__ void __launch_bounds__(256) sums_kernel(const double *__restrict__ pa
         const double v = nm >= 0 && nm < 2047 ? scalbn(sum, 5 - nm + ftab[f].e - OZ_SUM_BITS) : 0.0;
         double *dst = P + (size_t) f * rows + r;
         *dst = first ? v : *dst + v;
+        if (f == 0) {
+            const double d = nm >= 0 && nm < 2047 ? rootn * scalbn(1.0, 5 - nm) : 0.0;
+            noise[r] = first ? d : noise[r] + d;
+        }
     }
 }
 
@@ -207,8 +213,7 @@ __global__ void __launch_bounds__(256) assemble_kernel(const double *__restrict_
                                                        const Feature *__restrict__ ftab,
                                                        const double *__restrict__ Y,
                                                        const double *__restrict__ mean,
-                                                       const unsigned long long *__restrict__ zbits,
-                                                       double *__restrict__ S, double *__restrict__ gsum,
+                                                       const double *__restrict__ noise, double *__restrict__ S, double *__restrict__ gsum,
                                                        double *__restrict__ spread)
 {
     extern __shared__ double sh[];  // w, a1, a2
@@ -223,7 +228,7 @@ __global__ void __launch_bounds__(256) assemble_kernel(const double *__restrict_
     __syncthreads();
     const double g1 = P[(size_t) (np + D) * rows + k], g2 = P[(size_t) (np + D) * rows + kpad + k];
     double *S1 = S + (size_t) k * 2 * D * D, *S2 = S1 + (size_t) D * D;
-    double tp = 0.0, ts = 0.0, tz = 0.0;  // traces: P, S1, the squares of the coordinates' maxima
+    double tp = 0.0, ts = 0.0, tz = 0.0;  // traces: P, S1, the grids of the squares
     for (int f = threadIdx.x; f < np; f += 256) {
         const int i = ftab[f].i, j = ftab[f].j;
         const double p1 = P[(size_t) f * rows + k], p2 = P[(size_t) f * rows + kpad + k];
@@ -234,10 +239,9 @@ __global__ void __launch_bounds__(256) assemble_kernel(const double *__restrict_
         S1[(size_t) i * D + j] = s1;
         S2[(size_t) i * D + j] = s2;
         if (i == j) {
-            const double z = oz::bits_double(zbits[i]);
             tp += p1;
             ts += s1;
-            tz = fma(z, z, tz);
+            tz += scalbn(1.0, ftab[f].e);
         }
     }
     tp = block_sum_fixed(tp, red);
@@ -245,9 +249,8 @@ __global__ void __launch_bounds__(256) assemble_kernel(const double *__restrict_
     tz = block_sum_fixed(tz, red);
     if (threadIdx.x == 0) {
         gsum[k] = g1;
-        // 2^-56 of a feature against 2^-53 of P: an eighth.  tz >= tp / g: all zero only if
-        // tz is, or g
-        const double lost = fmax(tp, 0.125 * g1 * tz);
+        // 2^-56 of the grids against 2^-53 of P: an eighth
+        const double lost = fmax(tp, 0.125 * noise[k] * tz);
         spread[k] = lost > 0.0 ? (ts > 0.0 ? lost / ts : INFINITY) : lost;
     }
 }
@@ -287,7 +290,7 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
                align_up(sizeof(double) * 2 * (size_t) kpad * Fp * splits) +
                align_up(sizeof(double) * 2 * (size_t) kpad * F) +
                (pl.eig_in_smem ? 1 : 2) * align_up(sizeof(double) * (size_t) kpad * 2 * D * D) +
-               align_up(sizeof(int) * 2 * kpad);
+               align_up(sizeof(int) * 2 * kpad) + align_up(sizeof(double) * 2 * kpad);
         if (need <= budget || kpad == 128)
             break;
     }
@@ -315,6 +318,7 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
     double *S = (double *) take(sizeof(double) * (size_t) kpad * 2 * D * D);
     double *Mg = pl.eig_in_smem ? nullptr : (double *) take(sizeof(double) * (size_t) kpad * 2 * D * D);
     int *nmin = (int *) take(sizeof(int) * rows);
+    double *noise = (double *) take(sizeof(double) * rows);
     const size_t zsmem = sizeof(double) * 66 * (size_t) D, asmem = sizeof(double) * 3 * (size_t) D;
 
     auto body = [&]() -> int {
@@ -350,10 +354,11 @@ int oz_ctemp(OzE *st, const double *T64, const double *Y, const double *yy, cons
                 g.item_panels = per;
                 OZ_TRY(launch_oz_gemm(g, sms, status, s));
                 sums_kernel<<<dim3(g.mtiles * ntiles, 8), 256, 0, s>>>(part, ntiles, ceil_div(g.panels, per),
-                                                                       nmin, rows, F, ftab, ch == 0 ? 1 : 0, P);
+                                                                       nmin, rows, F, ftab, ch == 0 ? 1 : 0, sqrt((double) nn),
+                                                                       P, noise);
                 DGTM_CUDA_TRY(cudaGetLastError());
             }
-            assemble_kernel<<<kb, 256, asmem, s>>>(P, rows, kpad, D, ftab, Y + (size_t) k0 * D, mean, zbits, S, gsum_dev + k0,
+            assemble_kernel<<<kb, 256, asmem, s>>>(P, rows, kpad, D, ftab, Y + (size_t) k0 * D, mean, noise, S, gsum_dev + k0,
                                                    spread_dev + k0);
             DGTM_CUDA_TRY(cudaGetLastError());
             OZ_TRY(launch_ctemp_eig(pl, kb, D, S, Mg, gg_dev ? gg_dev + k0 : gsum_dev + k0, lim_scale,

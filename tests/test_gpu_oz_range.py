@@ -294,3 +294,22 @@ def test_sums_that_few_points_carry(pkg):
     # 2^-53 each from the block's R and from G's rounding, and half a unit of R's digits
     # (2^-55 of a grid that ends below 4.2 Rmax) from each of a few points
     assert np.max(np.abs(G[:N // 50] / g - 1.0)) <= 2.0 ** -51
+
+
+def test_scatter_where_few_points_carry_a_centre(pkg, monkeypatch):
+    """5001 points and centres whose R lies on a few dozen: the products' sums are rounded
+    where they are, not on a unit that 5001 full terms would need (2^-49 of the grids:
+    1e-12 of a critical temperature).  8 bits of 2^-53 may go to the expansion, 2.8e-14 of
+    the largest eigenvalue."""
+    rng = np.random.default_rng(14)
+    N, D, K = 5001, 5, 1500
+    T = rng.normal(size=(N, D))
+    Y = T[rng.integers(0, N, K)] + 0.3 * rng.normal(size=(K, D))
+    out = []
+    for pairs in ("1", "0"):
+        monkeypatch.setenv("DGTM_CTEMP_PAIRS", pairs)
+        with pkg.Context(T, np.ones((K, 1)), "fp64") as c:
+            c.set_Y(Y)
+            c.estep(5.2, 1, 3.0)
+            out.append(c.next_ctemp(1e9, 5.2, 1e-6, per_centre=True)[1])
+    assert np.max(np.abs(out[0] / out[1] - 1.0)) <= 1e-13
