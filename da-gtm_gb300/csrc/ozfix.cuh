@@ -202,7 +202,7 @@ static inline MulBase make_mul(double k0)
     int ex = 0;
     const double f = frexp(k0, &ex);  // k0 = f 2^ex, f in [0.5, 1)
     r.m = (uint64_t) ldexp(f, 64);
-    r.ex = ex;
+    r.ex = r.m ? ex : -4096;  // beta / 2 = 0: every exponent 0
     return r;
 }
 
@@ -287,7 +287,8 @@ OZ_HD int point_unit(int x, int ymin, int ucap)
 static inline int unit_cap(double c1, double c2)
 {
     int ex = 0;
-    frexp(c1 / 400.0 < c2 / 32.0 ? 400.0 / c1 : 32.0 / c2, &ex);  // < 2^ex
+    const double range = c1 / 400.0 < c2 / 32.0 ? 400.0 / c1 : 32.0 / c2;
+    frexp(range < 0x1p1000 ? range : 0x1p1000, &ex);  // < 2^ex (a c below 1e-298 tells nothing apart)
     return ex - 60;
 }
 

@@ -313,3 +313,18 @@ def test_scatter_where_few_points_carry_a_centre(pkg, monkeypatch):
             c.estep(5.2, 1, 3.0)
             out.append(c.next_ctemp(1e9, 5.2, 1e-6, per_centre=True)[1])
     assert np.max(np.abs(out[0] / out[1] - 1.0)) <= 1e-13
+
+
+@pytest.mark.parametrize("beta", [5e-324, 1e-310, 1e-200])
+def test_vanishing_beta(pkg, beta):
+    """beta so small that every exponent is 0 (its half too, for the smallest): R = 1 / K."""
+    rng = np.random.default_rng(16)
+    N, D, K = 900, 12, 64
+    T, X = rng.normal(size=(N, D)), rng.normal(size=(K, 2))
+    with pkg.Context(T, np.ones((K, 1)), "fp64") as c:
+        assert c.path == "exact_slices"
+        c.set_Y(rng.normal(size=(K, D)))
+        c.estep(beta, 1, 1.5)
+        R, M = c.R_block(0, K, 0, N), c.map(X)
+    assert np.max(np.abs(R * K - 1.0)) <= 1e-15
+    assert np.max(np.abs(M - X.mean(0))) <= 1e-14
